@@ -233,7 +233,6 @@ extern "C" int nn_shutdown(nn_context* c) {
     if (c->argmax_slot) cudaFree(c->argmax_slot);
     if (c->norm_scratch) cudaFree(c->norm_scratch);
     if (c->stage_img) cudaFree(c->stage_img);
-    if (c->pair_scratch) cudaFree(c->pair_scratch);
     if (c->sk_scratch) cudaFree(c->sk_scratch);
     if (c->sk_flags) cudaFree(c->sk_flags);
     if (c->status_host) cudaFreeHost(c->status_host);
@@ -424,72 +423,19 @@ bool nnb::resolve_weight(const nn_context* c, const void* W, int K, ResolvedW* o
 // ---------------------------------------------------------------------------------
 // operator dispatch
 // ---------------------------------------------------------------------------------
-// M > 16 with one weight and a plain or residual epilogue: tensor-core GEMM (quantised weights
-// are expanded to fp16 inside the kernel, stage by stage).
+// M > 16: the tensor-core GEMM, with whatever follows the product in its epilogue (quantised weights are expanded to fp16
+// inside the kernel).  Shapes it does not take are walked in slices of 16 rows by the streaming kernel.
 static int run_gemm_tc(nn_context* c, int fmt, const LinArgs& a, int M, const char* who, bool* done) {
     *done = false;
-    if (a.nseg != 1 || !(a.epi == EPI_STORE || a.epi == EPI_RESIDUAL)) return NN_OK;
-    const LinSeg& sg = a.seg[0];
-    if (!gemm_tc_supported(fmt, M, sg.N, a.K, a.x, sg.W, sg.out)) return NN_OK;
-    cudaError_t e = launch_gemm_tc(fmt, sg.W, sg.scale, a.x, sg.out, M, sg.N, a.K, sg.ld_out, a.epi, a.status, a.peer_out, a.npeer, &a.sig, c->stream);
-    if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: tensor-core launch failed: %s (M=%d N=%d K=%d)", who, cudaGetErrorString(e), M, sg.N, a.K);
-    c->launches++;
-    *done = true;
-    return NN_OK;
-}
-
-// The fused forms (three-weight QKV, SwiGLU over two weights, the in-place SiLU gate) at prefill row counts: one
-// tensor-core GEMM per weight, each with an fp16 result, and for the two-weight forms the element-wise SiLU-multiply
-// over those results -- the reference's own M > 1 sequence (src/models/lfm2-5-350m/src/layers/mlp.cpp:101-129).  The
-// single-pass streaming kernel would walk such a batch in slices of 16 rows, re-reading the weights for every slice.
-static int run_fused_forms_tc(nn_context* c, int fmt, const LinArgs& a, int M, const char* who, bool* done) {
-    *done = false;
-    if (a.npeer > 0 || a.sig.world > 0 || a.argmax_slot || a.norm_w) return NN_OK;
-    const bool qkv = a.epi == EPI_STORE && a.nseg > 1, swiglu = a.epi == EPI_SWIGLU && a.nseg == 1, gate = a.epi == EPI_SILU_GATE && a.nseg == 1;
-    if (!qkv && !swiglu && !gate) return NN_OK;
-    for (int i = 0; i < a.nseg; ++i)
-        if (!gemm_tc_supported(fmt, M, a.seg[i].N, a.K, a.x, a.seg[i].W, a.seg[i].out)) return NN_OK;
-    if (swiglu && !gemm_tc_supported(fmt, M, a.seg[0].N, a.K, a.x, a.W2, a.seg[0].out)) return NN_OK;
-    auto gemm = [&](const uint8_t* W, const uint16_t* scale, uint16_t* out, int N, int ld) -> int {
-        cudaError_t e = launch_gemm_tc(fmt, W, scale, a.x, out, M, N, a.K, ld, EPI_STORE, a.status, nullptr, 0, nullptr, c->stream);
-        if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: tensor-core launch failed: %s (M=%d N=%d K=%d)", who, cudaGetErrorString(e), M, N, a.K);
-        c->launches++;
-        return NN_OK;
-    };
-    if (qkv) {
-        for (int i = 0; i < a.nseg; ++i) {
-            const int rc = gemm(a.seg[i].W, a.seg[i].scale, a.seg[i].out, a.seg[i].N, a.seg[i].ld_out);
-            if (rc) return rc;
-        }
-        *done = true;
-        return NN_OK;
-    }
-    const int N = a.seg[0].N;
-    const size_t one = (size_t)M * N * 2, need = swiglu ? 2 * one : one;
-    if (need > c->pair_scratch_bytes) {
-        if (c->capturing) return NN_OK;   // cannot grow inside a recording: the sliced route still works
-        cudaSetDevice(c->device);
-        CUDA_TRY(cudaStreamSynchronize(c->stream));
-        if (c->pair_scratch) CUDA_TRY(cudaFree(c->pair_scratch));
-        c->pair_scratch = nullptr;
-        c->pair_scratch_bytes = 0;
-        CUDA_TRY(cudaMalloc(&c->pair_scratch, need));
-        c->pair_scratch_bytes = need;
-    }
-    uint16_t* s0 = (uint16_t*)c->pair_scratch;
-    uint16_t* s1 = (uint16_t*)((char*)c->pair_scratch + one);
-    if (swiglu) {
-        int rc = gemm(a.seg[0].W, a.seg[0].scale, s0, N, N);
-        if (!rc) rc = gemm(a.W2, a.scale2, s1, N, N);
-        if (rc) return rc;
-        CUDA_TRY(launch_silu_mul(s0, s1, a.seg[0].out, (size_t)M * N, c->stream));
-    } else {   // gate_inout = silu(gate_inout) * (x . W3^T)
-        const int rc = gemm(a.seg[0].W, a.seg[0].scale, s0, N, N);
-        if (rc) return rc;
-        if (a.seg[0].ld_out != N) return NN_FAIL(NN_ERR_UNSUPPORTED, "%s: the in-place gate form needs a dense [M, N] buffer", who);
-        CUDA_TRY(launch_silu_mul(a.seg[0].out, s0, a.seg[0].out, (size_t)M * N, c->stream));
-    }
-    c->launches++;
+    if (!gemm_tc_supported(fmt, a, M)) return NN_OK;
+    bool wait_first = false;
+    const size_t rb = fmt_rowbytes(fmt, a.K);
+    for (int i = 0; i < a.nseg; ++i) wait_first = wait_first || c->recently_written(a.seg[i].W, rb * (size_t)a.seg[i].N);
+    if (a.epi == EPI_SWIGLU) wait_first = wait_first || c->recently_written(a.W2, rb * (size_t)a.seg[0].N);
+    int n = 0;
+    cudaError_t e = launch_gemm_tc(fmt, a, M, wait_first, c->use_pdl, c->stream, &n);
+    c->launches += n;
+    if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: tensor-core launch failed: %s (M=%d N=%d K=%d)", who, cudaGetErrorString(e), M, a.seg[0].N, a.K);
     *done = true;
     return NN_OK;
 }
@@ -519,6 +465,7 @@ static void note_recorded(nn_context* c, int fmt, const LinArgs& a, const Stream
 }
 
 static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char* who) {
+    for (int i = 0; i < a.nseg; ++i) c->note_output(a.seg[i].out, (size_t)M_total * a.seg[i].ld_out * 2);
     a.sk_scratch = c->sk_scratch;
     a.sk_flags = c->sk_flags;
     if (a.norm_w) {
@@ -551,9 +498,7 @@ static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char
     }
     if (M_total > 16) {
         bool done = false;
-        int rc = run_gemm_tc(c, fmt, a, M_total, who, &done);
-        if (rc != NN_OK || done) return rc;
-        rc = run_fused_forms_tc(c, fmt, a, M_total, who, &done);
+        const int rc = run_gemm_tc(c, fmt, a, M_total, who, &done);
         if (rc != NN_OK || done) return rc;
     }
     // M > 16 is walked in slices of 16 activation rows (each slice re-streams the weights).
@@ -742,11 +687,18 @@ static int linear_qkv(nn_context* c, int M, int K, nn_buf x, nn_buf Wq, int Nq, 
     a.norm_w = (const uint16_t*)gamma;
     a.norm_eps = eps;
     if (bq) {
-        // The bias rides in the projection's epilogue when the call takes the streaming kernel (up to 16 rows); otherwise
-        // the projection runs as it would without one and the reference's bias kernel follows it.
+        // The bias rides in the projection's epilogue when the call takes the streaming kernel (up to 16 rows) or the
+        // tensor-core GEMM; otherwise the projection runs as it would without one and the reference's bias kernel follows it.
         const void* bs[3] = {bq, bk, bv};
-        bool fused = M <= 16;
-        if (fused) {
+        bool fused = true;
+        if (M > 16) {
+            LinArgs probe = a;
+            if (gamma) {   // normalised into the context's scratch first
+                probe.norm_w = nullptr;
+                probe.x = (const uint16_t*)c->norm_scratch;
+            }
+            fused = gemm_tc_supported(fmt, probe, M);
+        } else {
             LinArgs probe = a;
             probe.M = M;
             if (M >= 2) probe.norm_w = nullptr;
@@ -797,6 +749,7 @@ extern "C" int nn_bias_add(nn_context* c, int rows, int cols, nn_buf out, nn_buf
     a.nseg = 1;
     ProfScope prof(c, "bias_add_rows" + std::to_string(rows) + "_cols" + std::to_string(cols));
     CUDA_TRY(launch_bias_add(a, c->stream));
+    c->note_output(out, (size_t)rows * cols * 2);
     c->launches++;
     return NN_OK;
 }
@@ -813,6 +766,7 @@ extern "C" int nn_rmsnorm(nn_context* c, int rows, int cols, nn_buf x, nn_buf we
     if (rows == 0) return NN_OK;
     ProfScope prof(c, "rmsnorm_rows" + std::to_string(rows) + "_cols" + std::to_string(cols));
     CUDA_TRY(launch_rmsnorm((const uint16_t*)x, (const uint16_t*)weight, (uint16_t*)out, rows, cols, eps, c->stream));
+    c->note_output(out, (size_t)rows * cols * 2);
     c->launches++;
     return NN_OK;
 }

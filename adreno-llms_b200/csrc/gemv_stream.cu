@@ -779,39 +779,47 @@ EncodeTiledFn g_encode_tiled = nullptr;
 // Encoding a tensor map costs the host about a microsecond, and a decode loop asks for the same
 // few hundred (weight, tile) views token after token: keep them in a small direct-mapped,
 // per-thread cache.  A map only describes (address, extents, box), so a hit is always valid.
-struct MapSlot {
+struct MapKey {
     const void* base;
-    int rows, rowbytes, box_bytes, box_rows, swizzled;
-    bool valid;
+    uint64_t dim0, dim1, stride1;
+    uint32_t box0, box1, kind;  // kind: fp16 elements | 128-byte swizzle << 1 | 256-byte L2 promotion << 2 | 8
+    bool operator==(const MapKey& o) const {
+        return base == o.base && dim0 == o.dim0 && dim1 == o.dim1 && stride1 == o.stride1 && box0 == o.box0 && box1 == o.box1 && kind == o.kind;
+    }
+};
+struct MapSlot {
+    MapKey key;       // kind == 0: empty
     CUtensorMap map;
 };
 constexpr int MAP_SLOTS = 2048;
 thread_local MapSlot* t_map_cache = nullptr;
 
-bool cached_byte_map(CUtensorMap* m, const void* base, int rows, int rowbytes, int box_bytes, int box_rows, bool swizzled) {
+bool cached_map(CUtensorMap* m, const MapKey& k) {
     if (!g_encode_tiled) return false;
     if (!t_map_cache) t_map_cache = new MapSlot[MAP_SLOTS]();
-    uint64_t h = reinterpret_cast<uintptr_t>(base) >> 4;
-    h ^= (uint64_t)rows * 0x9E3779B97F4A7C15ull + (uint64_t)rowbytes * 0xC2B2AE3D27D4EB4Full + (uint64_t)(box_rows * 4 + box_bytes * 2 + (swizzled ? 1 : 0));
+    uint64_t h = reinterpret_cast<uintptr_t>(k.base) >> 4;
+    h ^= k.dim1 * 0x9E3779B97F4A7C15ull + k.dim0 * 0xC2B2AE3D27D4EB4Full + (uint64_t)(k.box1 * 16 + k.box0 * 32 + k.kind);
     MapSlot& s = t_map_cache[(h ^ (h >> 17) ^ (h >> 31)) % MAP_SLOTS];
-    if (s.valid && s.base == base && s.rows == rows && s.rowbytes == rowbytes && s.box_bytes == box_bytes && s.box_rows == box_rows &&
-        s.swizzled == (swizzled ? 1 : 0)) {
+    if (s.key == k) {
         *m = s.map;
         return true;
     }
-    const cuuint64_t dims[2] = {(cuuint64_t)rowbytes, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)rowbytes};
-    const cuuint32_t box[2] = {(cuuint32_t)box_bytes, (cuuint32_t)box_rows};
+    const cuuint64_t dims[2] = {k.dim0, k.dim1};
+    const cuuint64_t strides[1] = {k.stride1};
+    const cuuint32_t box[2] = {k.box0, k.box1};
     const cuuint32_t estr[2] = {1u, 1u};
-    if (g_encode_tiled(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                       swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                       swizzled ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+    if (g_encode_tiled(m, (k.kind & 1u) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(k.base), dims, strides,
+                       box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, (k.kind & 2u) ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                       (k.kind & 4u) ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return false;
-    s.base = base; s.rows = rows; s.rowbytes = rowbytes; s.box_bytes = box_bytes; s.box_rows = box_rows; s.swizzled = swizzled ? 1 : 0;
+    s.key = k;
     s.map = *m;
-    s.valid = true;
     return true;
+}
+bool cached_byte_map(CUtensorMap* m, const void* base, int rows, int rowbytes, int box_bytes, int box_rows, bool swizzled) {
+    return cached_map(m, MapKey{base, (uint64_t)rowbytes, (uint64_t)rows, (uint64_t)rowbytes, (uint32_t)box_bytes, (uint32_t)box_rows,
+                                8u | (swizzled ? 6u : 0u)});
 }
 
 template <int FMT, int NT, bool DUAL>
@@ -873,15 +881,7 @@ bool make_scale_map(CUtensorMap* m, const void* S, int rows, int rowbytes, int b
 
 bool encode_tiled_2d(void* map, bool half_elems, const void* base, uint64_t dim0, uint64_t dim1, uint64_t stride1_bytes,
                      uint32_t box0, uint32_t box1, bool swizzle128) {
-    if (!g_encode_tiled) return false;
-    const cuuint64_t dims[2] = {dim0, dim1};
-    const cuuint64_t strides[1] = {stride1_bytes};
-    const cuuint32_t box[2] = {box0, box1};
-    const cuuint32_t estr[2] = {1u, 1u};
-    return g_encode_tiled(static_cast<CUtensorMap*>(map), half_elems ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
-                          const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return cached_map(static_cast<CUtensorMap*>(map), MapKey{base, dim0, dim1, stride1_bytes, box0, box1, 8u | 4u | (half_elems ? 1u : 0u) | (swizzle128 ? 2u : 0u)});
 }
 
 cudaError_t stream_configure() {

@@ -47,8 +47,6 @@ struct nn_context {
     unsigned long long* argmax_slot = nullptr;
     void* stage_img = nullptr;      // staged activations of a batched call, written once per launch (stage_image.cu)
     size_t stage_img_bytes = 0;
-    void* pair_scratch = nullptr;   // fp16 results of the two projections of a two-weight form at prefill row counts
-    size_t pair_scratch_bytes = 0;
     void* norm_scratch = nullptr;   // normalised activations when the fused prologue does not apply
     size_t norm_scratch_bytes = 0;
     float* sk_scratch = nullptr;   // partial sums of blocks that share a tile (balanced K-streaming)
@@ -56,6 +54,20 @@ struct nn_context {
     void* flush_buf = nullptr;
     size_t flush_bytes = 0;
     bool use_pdl = true;
+    // outputs of the last calls (address ranges, oldest overwritten): launches overlap, so a "weight" that is one of these
+    // may still be in the making
+    uintptr_t recent_lo[16] = {}, recent_hi[16] = {};
+    unsigned recent_n = 0;
+    void note_output(const void* p, size_t bytes) {
+        recent_lo[recent_n % 16] = (uintptr_t)p;
+        recent_hi[recent_n % 16] = (uintptr_t)p + bytes;
+        ++recent_n;
+    }
+    bool recently_written(const void* p, size_t bytes) const {
+        for (int i = 0; i < 16; ++i)
+            if ((uintptr_t)p < recent_hi[i] && recent_lo[i] < (uintptr_t)p + bytes) return true;
+        return false;
+    }
     bool capturing = false;
     std::vector<nnb::RecordedOp> rec;  // streamed single-token operators of the recording in progress
     bool profiling = false;

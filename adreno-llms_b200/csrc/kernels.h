@@ -116,10 +116,10 @@ bool encode_tiled_2d(void* map, bool half_elems, const void* base, uint64_t dim0
 
 // gemm_tc.cu: tcgen05 / tensor-memory GEMM for M > 16
 cudaError_t gemm_tc_configure();
-bool gemm_tc_supported(int fmt, int M, int N, int K, const void* x, const void* W, const void* out);
-// W in its registered format; scale = int8 row scales / Q4 block scales / null
-cudaError_t launch_gemm_tc(int fmt, const void* W, const uint16_t* scale, const uint16_t* x, uint16_t* out, int M, int N, int K,
-                           int ld_out, int epi, int* status, uint16_t* const* peer_out, int npeer, const GatherSignal* sig, cudaStream_t st);
+bool gemm_tc_supported(int fmt, const LinArgs& a, int M);
+// out = x . W^T for M rows with every epilogue of LinArgs.  `wait_first`: a weight may be the output of a launch still in
+// flight, so none of it is fetched ahead of that launch's end.  Adds the number of launches to *launches.
+cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool wait_first, bool pdl, cudaStream_t st, int* launches);
 
 // gemv_generic.cu: any K, any alignment (the reference's gemv_rT_fp32acc role)
 cudaError_t launch_generic(int fmt, const LinArgs& a, cudaStream_t st);
@@ -175,7 +175,6 @@ inline bool q4_scale_views(const LinArgs& a, const uint16_t* base[4], int* pitch
     return true;
 }
 cudaError_t launch_l2_flush(void* buf, size_t bytes, cudaStream_t st);
-cudaError_t launch_silu_mul(const uint16_t* g, const uint16_t* u, uint16_t* out, size_t n, cudaStream_t st);
 // the staged activations of a batched call (layout of the streaming kernel's shared memory), with the optional RMSNorm
 size_t stage_image_bytes(int fmt, int M, int K);
 cudaError_t launch_stage_image(int fmt, const uint16_t* x, int M, int K, const uint16_t* norm_w, float eps, uint8_t* img, cudaStream_t st,
