@@ -490,7 +490,7 @@ static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char
                 CUDA_TRY(cudaMalloc(&c->norm_scratch, need));
                 c->norm_scratch_bytes = need;
             }
-            CUDA_TRY(launch_rmsnorm(a.x, a.norm_w, (uint16_t*)c->norm_scratch, M_total, a.K, a.norm_eps, c->stream));
+            CUDA_TRY(launch_rmsnorm(a.x, a.norm_w, (uint16_t*)c->norm_scratch, M_total, a.K, a.norm_eps, c->stream, c->use_pdl));
             c->launches++;
             a.x = (const uint16_t*)c->norm_scratch;
             a.norm_w = nullptr;
@@ -765,7 +765,7 @@ extern "C" int nn_rmsnorm(nn_context* c, int rows, int cols, nn_buf x, nn_buf we
     if (rows < 0 || cols <= 0) return NN_FAIL(NN_ERR_ARG, "nn_rmsnorm: bad shape rows=%d cols=%d", rows, cols);
     if (rows == 0) return NN_OK;
     ProfScope prof(c, "rmsnorm_rows" + std::to_string(rows) + "_cols" + std::to_string(cols));
-    CUDA_TRY(launch_rmsnorm((const uint16_t*)x, (const uint16_t*)weight, (uint16_t*)out, rows, cols, eps, c->stream));
+    CUDA_TRY(launch_rmsnorm((const uint16_t*)x, (const uint16_t*)weight, (uint16_t*)out, rows, cols, eps, c->stream, c->use_pdl));
     c->note_output(out, (size_t)rows * cols * 2);
     c->launches++;
     return NN_OK;

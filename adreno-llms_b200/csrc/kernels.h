@@ -189,6 +189,6 @@ struct BiasArgs {  // up to three [rows, cols] fp16 outputs with a bias row each
     int rows, nseg;
 };
 cudaError_t launch_bias_add(const BiasArgs& a, cudaStream_t st);
-cudaError_t launch_rmsnorm(const uint16_t* x, const uint16_t* w, uint16_t* out, int rows, int cols, float eps, cudaStream_t st);
+cudaError_t launch_rmsnorm(const uint16_t* x, const uint16_t* w, uint16_t* out, int rows, int cols, float eps, cudaStream_t st, bool pdl);
 
 }  // namespace nnb
