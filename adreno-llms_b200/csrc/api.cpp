@@ -62,10 +62,11 @@ std::string op_label(int M, int N, int K, int fmt, const char* form) {
 struct ProfScope {  // event pair around whatever the scope enqueues
     nn_context* c;
     size_t slot = (size_t)-1;
-    ProfScope(nn_context* ctx, const std::string& label) : c(ctx) {
+    template <class Label>   // called only when the profile is on: building a label costs more than a launch's other host work
+    ProfScope(nn_context* ctx, Label&& label) : c(ctx) {
         if (!c || !c->profiling || c->capturing) return;
         ProfPending p;
-        p.label = label;
+        p.label = label();
         if (cudaEventCreate(&p.start) != cudaSuccess) return;
         if (cudaEventCreate(&p.stop) != cudaSuccess) { cudaEventDestroy(p.start); return; }
         cudaEventRecord(p.start, c->stream);
@@ -594,7 +595,7 @@ static int one_weight(nn_context* c, int M, int N, int K, nn_buf x, nn_buf W, nn
     a.status = c->status_dev;
     a.norm_w = (const uint16_t*)gamma;
     a.norm_eps = eps;
-    ProfScope prof(c, op_label(M, N, K, r.fmt, epi == EPI_RESIDUAL ? "_add" : epi == EPI_SILU_GATE ? "_silu_gate" : gamma ? "_rmsnorm" : ""));
+    ProfScope prof(c, [&] { return std::string(op_label(M, N, K, r.fmt, epi == EPI_RESIDUAL ? "_add" : epi == EPI_SILU_GATE ? "_silu_gate" : gamma ? "_rmsnorm" : "")); });
     if (npeer < 0 || npeer > 7) return NN_FAIL(NN_ERR_ARG, "%s: %d peers", who, npeer);
     a.npeer = npeer;
     for (int p = 0; p < npeer; ++p) a.peer_out[p] = peers[p];
@@ -646,7 +647,7 @@ static int gate_up_silu(nn_context* c, int M, int N, int K, nn_buf x, nn_buf Wg,
     a.status = c->status_dev;
     a.norm_w = (const uint16_t*)gamma;
     a.norm_eps = eps;
-    ProfScope prof(c, op_label(M, N, K, rg.fmt, gamma ? "_rmsnorm_swiglu" : "_swiglu"));
+    ProfScope prof(c, [&] { return std::string(op_label(M, N, K, rg.fmt, gamma ? "_rmsnorm_swiglu" : "_swiglu")); });
     return run_linear(c, rg.fmt, a, M, who);
 }
 
@@ -706,12 +707,12 @@ static int linear_qkv(nn_context* c, int M, int K, nn_buf x, nn_buf Wq, int Nq, 
         }
         if (fused) {
             for (int i = 0; i < 3; ++i) a.seg[i].bias = (const uint16_t*)bs[i];
-            ProfScope prof(c, op_label(M, Nq + Nk + Nv, K, fmt, gamma ? "_rmsnorm_qkv_bias" : "_qkv_bias"));
+            ProfScope prof(c, [&] { return std::string(op_label(M, Nq + Nk + Nv, K, fmt, gamma ? "_rmsnorm_qkv_bias" : "_qkv_bias")); });
             return run_linear(c, fmt, a, M, who);
         }
         int rc;
         {
-            ProfScope prof(c, op_label(M, Nq + Nk + Nv, K, fmt, gamma ? "_rmsnorm_qkv" : "_qkv"));
+            ProfScope prof(c, [&] { return std::string(op_label(M, Nq + Nk + Nv, K, fmt, gamma ? "_rmsnorm_qkv" : "_qkv")); });
             rc = run_linear(c, fmt, a, M, who);
         }
         if (rc) return rc;
@@ -723,12 +724,12 @@ static int linear_qkv(nn_context* c, int M, int K, nn_buf x, nn_buf Wq, int Nq, 
         }
         ba.rows = M;
         ba.nseg = 3;
-        ProfScope prof(c, "bias_add_qkv_rows" + std::to_string(M));
+        ProfScope prof(c, [&] { return std::string("bias_add_qkv_rows" + std::to_string(M)); });
         CUDA_TRY(launch_bias_add(ba, c->stream));
         c->launches++;
         return NN_OK;
     }
-    ProfScope prof(c, op_label(M, Nq + Nk + Nv, K, fmt, gamma ? "_rmsnorm_qkv" : "_qkv"));
+    ProfScope prof(c, [&] { return std::string(op_label(M, Nq + Nk + Nv, K, fmt, gamma ? "_rmsnorm_qkv" : "_qkv")); });
     return run_linear(c, fmt, a, M, who);
 }
 
@@ -747,7 +748,7 @@ extern "C" int nn_bias_add(nn_context* c, int rows, int cols, nn_buf out, nn_buf
     a.cols[0] = cols;
     a.rows = rows;
     a.nseg = 1;
-    ProfScope prof(c, "bias_add_rows" + std::to_string(rows) + "_cols" + std::to_string(cols));
+    ProfScope prof(c, [&] { return std::string("bias_add_rows" + std::to_string(rows) + "_cols" + std::to_string(cols)); });
     CUDA_TRY(launch_bias_add(a, c->stream));
     c->note_output(out, (size_t)rows * cols * 2);
     c->launches++;
@@ -764,7 +765,7 @@ extern "C" int nn_rmsnorm(nn_context* c, int rows, int cols, nn_buf x, nn_buf we
     if (!c || !x || !weight || !out) return NN_FAIL(NN_ERR_ARG, "nn_rmsnorm: null argument");
     if (rows < 0 || cols <= 0) return NN_FAIL(NN_ERR_ARG, "nn_rmsnorm: bad shape rows=%d cols=%d", rows, cols);
     if (rows == 0) return NN_OK;
-    ProfScope prof(c, "rmsnorm_rows" + std::to_string(rows) + "_cols" + std::to_string(cols));
+    ProfScope prof(c, [&] { return std::string("rmsnorm_rows" + std::to_string(rows) + "_cols" + std::to_string(cols)); });
     CUDA_TRY(launch_rmsnorm((const uint16_t*)x, (const uint16_t*)weight, (uint16_t*)out, rows, cols, eps, c->stream, c->use_pdl));
     c->note_output(out, (size_t)rows * cols * 2);
     c->launches++;
@@ -844,7 +845,7 @@ int nnb::linear_argmax(nn_context* c, int N, int K, nn_buf x, nn_buf W, nn_buf l
         if (rc) return rc;
         return nn_argmax(c, N, logits, out_idx);
     }
-    ProfScope prof(c, op_label(1, N, K, r.fmt, "_argmax"));
+    ProfScope prof(c, [&] { return std::string(op_label(1, N, K, r.fmt, "_argmax")); });
     a.argmax_slot = c->argmax_slot + 1;
     a.argmax_done = reinterpret_cast<unsigned*>(c->argmax_slot + 2);
     a.argmax_out = (int*)out_idx;
@@ -860,7 +861,7 @@ int nnb::linear_argmax(nn_context* c, int N, int K, nn_buf x, nn_buf W, nn_buf l
 extern "C" int nn_argmax(nn_context* c, int n, nn_buf logits, nn_buf out_idx) {
     if (!c || !logits || !out_idx) return NN_FAIL(NN_ERR_ARG, "nn_argmax: null argument");
     if (n < 0) return NN_FAIL(NN_ERR_ARG, "nn_argmax: n=%d", n);
-    ProfScope prof(c, "argmax_n" + std::to_string(n));
+    ProfScope prof(c, [&] { return std::string("argmax_n" + std::to_string(n)); });
     CUDA_TRY(launch_argmax_half((const uint16_t*)logits, n, (int*)out_idx, c->argmax_slot, c->stream));
     c->launches += n > 0 ? 3 : 2;
     return NN_OK;
@@ -1058,7 +1059,7 @@ extern "C" int nn_plan_end(nn_context* c, nn_plan** out) {
 
 extern "C" int nn_plan_launch(nn_context* c, nn_plan* p) {
     if (!c || !p || !p->exec) return NN_FAIL(NN_ERR_ARG, "nn_plan_launch: null argument");
-    ProfScope prof(c, "plan_replay_" + std::to_string(p->recorded) + "ops_" + std::to_string(p->kernels) + "launches");
+    ProfScope prof(c, [&] { return std::string("plan_replay_" + std::to_string(p->recorded) + "ops_" + std::to_string(p->kernels) + "launches"); });
     CUDA_TRY(cudaGraphLaunch(p->exec, c->stream));
     c->launches += p->kernels;
     return NN_OK;
