@@ -117,6 +117,7 @@ template <> struct KArgsFor<FMT_Q4> { typedef KArgsQ4 type; };
 template <int FMT, int NT, bool DUAL, int VAR, bool ONE>
 __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_constant__ typename KMapsFor<FMT>::type km, const KScal ka) {
     constexpr bool EXT = VAR == 2;
+    constexpr int RED_WORDS = NCW * 8 * NT * RED_TS;   // one reduction buffer
     extern __shared__ __align__(128) uint8_t smem[];
     const LinArgs& a = ka.a;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -284,60 +285,43 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
 
     float acc[2][2][NT][4];      // [accumulator set][row block][n tile][frag]
     int iacc[FMT == FMT_INT8 ? 3 : 1][2][NT][4];  // int8: exact integer sums per activation limb
-    // Prefetched epilogue operands stay as raw fp16 bits until they are used, so that the
-    // loads' latency is not waited for where they are issued.
-    uint16_t sc_reg[2][2];          // int8: row scales of the current tile (rows g, g+8 of each block)
+    // Prefetched epilogue operands stay as raw fp16 bits until they are used, so that the loads' latency is not waited for
+    // where they are issued.
     // Single-token launches (one weight): lane L of a warp finishes row L of the warp's 32 rows, so
     // it prefetches one scale and one residual value and the tile leaves in one 64-byte store.
-    const bool lane_rows = !DUAL && aM == 1;
+    // Batched launches: a thread finishes pairs of neighbouring rows, one pair of one token at a time (see the finish below).
     uint16_t sc1 = 0, res1 = 0, bias1 = 0;
-    uint16_t bias_reg[2][2];        // q/k/v bias of the same rows
-    uint32_t res_reg[2][2][NT][2];  // in-place epilogues: the values to be updated
+    uint16_t p_sc[2] = {0, 0}, p_sc2[2] = {0, 0}, p_bias[2] = {0, 0}, p_res[2][2];
     bool failed = false;
     unsigned long long am_best = 0ull;  // fused arg-max: best key among this thread's rows
+    // batched: pairs of output rows of the finishing group (a warp with rows of its own, or all four that split K)
+    const bool coop = ksplit && !(EXT && a.streamk != 0);
+    const int f_idx = coop ? tid : lane, f_log = DUAL ? 3 : 4, f_pair = f_idx & ((1 << f_log) - 1), f_m0 = f_idx >> f_log,
+              f_step = (coop ? NCW * 32 : 32) >> f_log;
+    const bool finisher = ONE ? writer : (coop || writer);
 
     // Per-row scales and biases do not depend on the previous launch: fetch them ahead of use.
     auto prefetch_scales = [&](int tile) {
-        if (VAR >= 1 && !DUAL) {
-            const LinSeg sg = seg_at(tile_segment(tile));
-            const int row0 = (tile - sg.tile0) * tile_rows + wrow_off;
-            if (sg.bias) {
-                if (lane_rows) {
-                    bias1 = sg.bias[min(row0 + lane, sg.N - 1)];
-                } else {
+        const LinSeg sg = seg_at(DUAL ? 0 : tile_segment(tile));
+        const int row0 = (tile - (DUAL ? 0 : sg.tile0)) * tile_rows + wrow_off;
+        if (!ONE) {
 #pragma unroll
-                    for (int rb = 0; rb < 2; ++rb)
-#pragma unroll
-                        for (int i2 = 0; i2 < 2; ++i2) bias_reg[rb][i2] = sg.bias[min(row0 + rb * 16 + g + i2 * 8, sg.N - 1)];
-                }
+            for (int i = 0; i < 2; ++i) {
+                const int n = min(row0 + 2 * f_pair + i, sg.N - 1);
+                if (FMT == FMT_INT8) p_sc[i] = sg.scale[n];
+                if (FMT == FMT_INT8 && DUAL) p_sc2[i] = a.scale2[n];
+                if (VAR >= 1 && !DUAL && sg.bias) p_bias[i] = sg.bias[n];
             }
+            return;
         }
+        if (VAR >= 1 && !DUAL && sg.bias) bias1 = sg.bias[min(row0 + lane, sg.N - 1)];
         if (FMT != FMT_INT8) return;
-        if (DUAL) {
-            if (aM == 1) {   // lane L (< 16) finishes row L of the warp's 16 rows
-                const int n = min(tile * tile_rows + wrow_off + (lane & 15), a.seg[0].N - 1);
-                sc1 = a.seg[0].scale[n];
-                res1 = a.scale2[n];   // the up weight's scale rides in the spare register
-                return;
-            }
-#pragma unroll
-            for (int i2 = 0; i2 < 2; ++i2) {
-                const int n = min(tile * tile_rows + wrow_off + g + i2 * 8, a.seg[0].N - 1);
-                sc_reg[0][i2] = a.seg[0].scale[n];
-                sc_reg[1][i2] = a.scale2[n];
-            }
+        if (DUAL) {   // lane L (< 16) finishes row L of the warp's 16 rows
+            const int n = min(row0 + (lane & 15), sg.N - 1);
+            sc1 = sg.scale[n];
+            res1 = a.scale2[n];   // the up weight's scale rides in the spare register
         } else {
-            const LinSeg sg = seg_at(tile_segment(tile));
-            const int row0 = (tile - sg.tile0) * tile_rows + wrow_off;
-            if (lane_rows) {
-                sc1 = sg.scale[min(row0 + lane, sg.N - 1)];
-                return;
-            }
-#pragma unroll
-            for (int rb = 0; rb < 2; ++rb)
-#pragma unroll
-                for (int i2 = 0; i2 < 2; ++i2)
-                    sc_reg[rb][i2] = sg.scale[min(row0 + rb * 16 + g + i2 * 8, sg.N - 1)];
+            sc1 = sg.scale[min(row0 + lane, sg.N - 1)];
         }
     };
     // Q4: this lane's row of block scales for pipeline item `j` travels by cp.async and
@@ -372,37 +356,35 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
         cp_async_mbar_arrive_noinc(bar);
     };
 
-    // In-place epilogues read the values they update; issued early, used at the tile's end.
+    // In-place epilogues read the values they update; issued early, used at the tile's end (batched: the first two of a thread's
+    // tokens).
+    const bool inplace = !DUAL && (a_epi == EPI_RESIDUAL || a_epi == EPI_SILU_GATE);
     auto prefetch_residual = [&](int tile) {
-        if (DUAL || !(a_epi == EPI_RESIDUAL || a_epi == EPI_SILU_GATE)) return;
+        if (!inplace) return;
         const LinSeg sg = seg_at(tile_segment(tile));
         const int row0 = (tile - sg.tile0) * tile_rows + wrow_off;
-        if (lane_rows) {
+        if (ONE) {
             res1 = (row0 + lane < sg.N) ? sg.out[row0 + lane] : (uint16_t)0;
             return;
         }
 #pragma unroll
-        for (int rb = 0; rb < 2; ++rb)
+        for (int k = 0; k < 2; ++k)
 #pragma unroll
-            for (int i2 = 0; i2 < 2; ++i2)
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const int n = row0 + rb * 16 + g + i2 * 8, m = nt * 8 + 2 * t + j;
-                        res_reg[rb][i2][nt][j] = (n < sg.N && m < aM) ? (uint32_t)sg.out[(size_t)m * sg.ld_out + n] : 0u;
-                    }
+            for (int i = 0; i < 2; ++i) {
+                const int n = row0 + 2 * f_pair + i, m = f_m0 + k * f_step;
+                p_res[k][i] = (n < sg.N && m < aM) ? sg.out[(size_t)m * sg.ld_out + n] : (uint16_t)0;
+            }
     };
 
     if (FMT == FMT_Q4 && !ka.scale_tma) {
         const int pre = min(stages - 1, n_items);
         for (int j = 0; j < pre; ++j) issue_scales(j);
     }
-    if (n_items > 0 && writer) prefetch_scales(tile_first);
+    if (n_items > 0 && finisher) prefetch_scales(tile_first);
 
     pdl_launch_dependents();
     pdl_wait_prior_grid();
-    if (n_items > 0 && writer) prefetch_residual(tile_first);
+    if (n_items > 0 && finisher) prefetch_residual(tile_first);
     const uint16_t* x_src = a.x;
     if (!ONE && a.staged != nullptr) {
         // the launch before this one (stage_image_kernel) wrote the staged form of all M rows in this
@@ -453,7 +435,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
 #pragma unroll
                             for (int i = 0; i < 4; ++i) iacc[l % (FMT == FMT_INT8 ? 3 : 1)][rb][nt][i] = 0;
             }
-            if (writer && it > 0) {
+            if (finisher && it > 0) {
                 prefetch_scales(tile);
                 prefetch_residual(tile);
             }
@@ -506,10 +488,10 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
             for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc[0][rb][nt][i] += acc[1][rb][nt][i];
-        if (ksplit) {
+        if (ksplit && !(!ONE && coop)) {
             // partial sums meet in shared memory; the buffer alternates between tiles so one
             // barrier per tile is enough
-            float* buf = red + (ti & 1) * (NCW * 32 * 2 * NT * 4);
+            float* buf = red + (ti & 1) * RED_WORDS;
             if (warp != 0) {
                 float* mine = buf + (warp * 32 + lane) * (2 * NT * 4);
 #pragma unroll
@@ -584,128 +566,149 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
                 }
             }
         }
-        if (!writer) continue;
-
-        if (DUAL) {
-            const int seg_n = a.seg[0].N, seg_ld = a.seg[0].ld_out, m_count = aM;
-            uint16_t* const seg_out = a.seg[0].out;
-            if (m_count == 1) {
-                // single token: rows g, g + 8 of the warp's 16 gate / up rows sit in lanes 0, 4, .. 28;
-                // lane L < 16 takes row L and the 16 rows leave in one 32-byte store
-                const int src = (lane & 7) * 4, hi = (lane >> 3) & 1;
-                const float g0 = __shfl_sync(0xffffffffu, acc[0][0][0][0], src), g1 = __shfl_sync(0xffffffffu, acc[0][0][0][2], src);
-                const float u0 = __shfl_sync(0xffffffffu, acc[0][1][0][0], src), u1 = __shfl_sync(0xffffffffu, acc[0][1][0][2], src);
-                float gv = hi ? g1 : g0, uv = hi ? u1 : u0;
-                const int n = tile * tile_rows + wrow_off + lane;
-                if (lane < 16 && n < seg_n) {
-                    if (FMT == FMT_INT8) {
-                        gv *= __half2float(__ushort_as_half(sc1));
-                        uv *= __half2float(__ushort_as_half(res1));
-                    }
-                    const float r = (gv / (1.0f + expf(-gv))) * uv;
-                    seg_out[n] = __half_as_ushort(__float2half_rn(r));
-                }
-                continue;
-            }
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int n = tile * tile_rows + wrow_off + g + (i >> 1) * 8;
-                    const int m = nt * 8 + 2 * t + (i & 1);
-                    if (n < seg_n && m < m_count) {
-                        float gv = acc[0][0][nt][i], uv = acc[0][1][nt][i];
-                        if (FMT == FMT_INT8) {
-                            gv *= __half2float(__ushort_as_half(sc_reg[0][i >> 1]));
-                            uv *= __half2float(__ushort_as_half(sc_reg[1][i >> 1]));
-                        }
-                        const float r = (gv / (1.0f + expf(-gv))) * uv;
-                        seg_out[(size_t)m * seg_ld + n] = __half_as_ushort(__float2half_rn(r));
-                    }
-                }
-        } else {
-            // Everything the store loop needs is copied into registers first: the segment lives in
-            // kernel-parameter memory reached through a run-time index, and a 16-bit store may alias
-            // it as far as the compiler can tell, so every field read after a store would be a fresh
-            // (slow) load.
-            const LinSeg sg = seg_at(tile_segment(tile));
-            const int seg_n = sg.N, seg_ld = sg.ld_out, seg_tile0 = sg.tile0;
-            uint16_t* const seg_out = sg.out;
-            const bool biased = sg.bias != nullptr;
-            const int m_count = aM, epi = a_epi;
-            const int npeer = EXT ? a.npeer : 0;
-            unsigned long long* const am_slot = EXT ? a.argmax_slot : nullptr;
-            const int am_base = EXT ? a.argmax_base : 0;
-            uint16_t* peer[7];
-#pragma unroll
-            for (int p = 0; p < 7; ++p) peer[p] = (EXT && p < npeer) ? a.peer_out[p] : nullptr;
-            const int row0 = (tile - seg_tile0) * tile_rows + wrow_off;
-            if (lane_rows) {
-                // the token's 32 results sit in lanes 0, 4, .. 28 (rows g, g + 8 of each row block):
-                // bring row L to lane L, finish it there and store the 32 rows with one instruction
-                const int src = (lane & 7) * 4, sel = lane >> 3;
-                const float v00 = __shfl_sync(0xffffffffu, acc[0][0][0][0], src), v01 = __shfl_sync(0xffffffffu, acc[0][0][0][2], src);
-                const float v10 = __shfl_sync(0xffffffffu, acc[0][1][0][0], src), v11 = __shfl_sync(0xffffffffu, acc[0][1][0][2], src);
-                float v = sel == 0 ? v00 : sel == 1 ? v01 : sel == 2 ? v10 : v11;
-                const int n = row0 + lane;
-                if (n < seg_n) {
-                    if (FMT == FMT_INT8) v = __fmul_rn(v, __half2float(__ushort_as_half(sc1)));  // roundings as in finish_row
-                    if (VAR >= 1 && biased) v = __fadd_rn(__half2float(__float2half_rn(v)), __half2float(__ushort_as_half(bias1)));
-                    if (epi == EPI_RESIDUAL) {
-                        v = __fadd_rn(__half2float(__ushort_as_half(res1)), v);
-                    } else if (epi == EPI_SILU_GATE) {
-                        const float gt = __half2float(__ushort_as_half(res1));
-                        v = gt * (1.0f / (1.0f + expf(-gt))) * v;
-                    }
-                    const uint16_t hv = __half_as_ushort(__float2half_rn(v));
-                    if (!EXT || seg_out) seg_out[n] = hv;
-                    if (EXT) {
-#pragma unroll
-                        for (int p = 0; p < 7; ++p)
-                            if (p < npeer) peer[p][n] = hv;
-                    }
-                    if (EXT && am_slot && (hv & 0x7FFFu) <= 0x7C00u) {  // NaNs never win
-                        const unsigned long long key = argmax_key_half(hv, am_base + n);
-                        am_best = key > am_best ? key : am_best;
-                    }
-                }
-                continue;
-            }
+        if (!finisher) continue;
+        // Everything the store loop needs is copied into registers first: a 16-bit store may alias the parameter block as far as
+        // the compiler can tell, so every field read after a store would be a fresh (slow) load.
+        const LinSeg sg = seg_at(DUAL ? 0 : tile_segment(tile));
+        const int seg_n = sg.N, seg_ld = sg.ld_out;
+        uint16_t* const seg_out = sg.out;
+        const bool biased = !DUAL && sg.bias != nullptr;
+        const int epi = a_epi, npeer = EXT ? a.npeer : 0;
+        const int row0 = (tile - (DUAL ? 0 : sg.tile0)) * tile_rows + wrow_off;
+        if constexpr (!ONE) {
+            // ---- batched finish.  The parts of the tile go to shared memory as [part][token][row] and come back as pairs of
+            //      neighbouring rows, one pair of one token per step of a rolled loop.  Finishing the fragments where they lie
+            //      takes sixteen unrolled copies of the epilogue, straight-line code that every launch fetches anew: with it an
+            //      896 x 896 projection of 16 rows took 7.5 us; and its stores were two bytes each. ----
+            float* const buf = red + (ti & 1) * RED_WORDS;
+            float* const mine = buf + warp * (8 * NT * RED_TS) + (2 * t) * RED_TS + g;
 #pragma unroll
             for (int rb = 0; rb < 2; ++rb)
 #pragma unroll
-                for (int i2 = 0; i2 < 2; ++i2) {
-                    const int n = row0 + rb * 16 + g + i2 * 8;
-                    if (n >= seg_n) continue;
+                for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-                    for (int nt = 0; nt < NT; ++nt)
+                    for (int i = 0; i < 4; ++i) mine[(nt * 8 + (i & 1)) * RED_TS + rb * 16 + (i >> 1) * 8] = acc[0][rb][nt][i];
+            if (coop) asm volatile("bar.sync 1, %0;" ::"n"(NCW * 32) : "memory");
+            else __syncwarp();
+            const int n = row0 + 2 * f_pair;
+            const bool two = n + 1 < seg_n;
+            const float* const src = buf + (coop ? 0 : warp * (8 * NT * RED_TS)) + 2 * f_pair;
+            if (n < seg_n) {
+                int k = 0;
+#pragma unroll 1
+                for (int m = f_m0; m < aM; m += f_step, ++k) {
+                    auto sum = [&](int up) {   // K parts in consumer order
+                        const float* s = src + m * RED_TS + up;
+                        float2 v = *reinterpret_cast<const float2*>(s);
+                        if (coop) {
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) {
-                            const int m = nt * 8 + 2 * t + j;
-                            if (m >= m_count) continue;
-                            float v = acc[0][rb][nt][i2 * 2 + j];
-                            if (FMT == FMT_INT8) v = __fmul_rn(v, __half2float(__ushort_as_half(sc_reg[rb][i2])));  // roundings as in finish_row
-                            if (VAR >= 1 && biased) v = __fadd_rn(__half2float(__float2half_rn(v)), __half2float(__ushort_as_half(bias_reg[rb][i2])));
-                            if (epi == EPI_RESIDUAL) {
-                                v = __fadd_rn(__half2float(__ushort_as_half((uint16_t)res_reg[rb][i2][nt][j])), v);
-                            } else if (epi == EPI_SILU_GATE) {
-                                const float gt = __half2float(__ushort_as_half((uint16_t)res_reg[rb][i2][nt][j]));
-                                v = gt * (1.0f / (1.0f + expf(-gt))) * v;
-                            }
-                            const uint16_t hv = __half_as_ushort(__float2half_rn(v));
-                            const size_t o = (size_t)m * seg_ld + n;
-                            if (!EXT || seg_out) seg_out[o] = hv;
-                            if (EXT) {
-#pragma unroll
-                                for (int p = 0; p < 7; ++p)
-                                    if (p < npeer) peer[p][o] = hv;
-                            }
-                            if (EXT && am_slot && m == 0 && (hv & 0x7FFFu) <= 0x7C00u) {  // NaNs never win
-                                const unsigned long long key = argmax_key_half(hv, am_base + n);
-                                am_best = key > am_best ? key : am_best;
+                            for (int p = 1; p < NCW; ++p) {
+                                const float2 o = *reinterpret_cast<const float2*>(s + p * (8 * NT * RED_TS));
+                                v.x += o.x;
+                                v.y += o.y;
                             }
                         }
+                        return v;
+                    };
+                    const float2 s0 = sum(0);
+                    const float2 s1 = DUAL ? sum(16) : make_float2(0.f, 0.f);
+                    uint16_t old[2] = {p_res[0][0], p_res[0][1]};
+                    if (inplace && k > 0) {
+                        old[0] = p_res[1][0];
+                        old[1] = p_res[1][1];
+                        if (k > 1) {
+                            old[0] = seg_out[(size_t)m * seg_ld + n];
+                            old[1] = two ? seg_out[(size_t)m * seg_ld + n + 1] : (uint16_t)0;
+                        }
+                    }
+                    uint16_t hv[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        float v = i ? s0.y : s0.x;
+                        if (DUAL) {
+                            float uv = i ? s1.y : s1.x;
+                            if (FMT == FMT_INT8) {
+                                v *= __half2float(__ushort_as_half(p_sc[i]));
+                                uv *= __half2float(__ushort_as_half(p_sc2[i]));
+                            }
+                            v = (v / (1.0f + expf(-v))) * uv;
+                        } else {
+                            if (FMT == FMT_INT8) v = __fmul_rn(v, __half2float(__ushort_as_half(p_sc[i])));  // roundings as in finish_row
+                            if (VAR >= 1 && biased) v = __fadd_rn(__half2float(__float2half_rn(v)), __half2float(__ushort_as_half(p_bias[i])));
+                            const float gt = __half2float(__ushort_as_half(old[i]));
+                            if (epi == EPI_RESIDUAL) v = __fadd_rn(gt, v);
+                            else if (epi == EPI_SILU_GATE) v = gt * (1.0f / (1.0f + expf(-gt))) * v;
+                        }
+                        hv[i] = __half_as_ushort(__float2half_rn(v));
+                    }
+                    const size_t o = (size_t)m * seg_ld + n;
+                    auto put = [&](uint16_t* dst) {
+                        if (two && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
+                            *reinterpret_cast<uint32_t*>(dst) = (uint32_t)hv[0] | (uint32_t)hv[1] << 16;
+                        } else {
+                            dst[0] = hv[0];
+                            if (two) dst[1] = hv[1];
+                        }
+                    };
+                    put(seg_out + o);
+                    if (EXT) {
+#pragma unroll 1
+                        for (int p = 0; p < npeer; ++p) put(a.peer_out[p] + o);
+                    }
                 }
+            }
+            continue;
+        }
+        if (DUAL) {
+            // single token: rows g, g + 8 of the warp's 16 gate / up rows sit in lanes 0, 4, .. 28;
+            // lane L < 16 takes row L and the 16 rows leave in one 32-byte store
+            const int src = (lane & 7) * 4, hi = (lane >> 3) & 1;
+            const float g0 = __shfl_sync(0xffffffffu, acc[0][0][0][0], src), g1 = __shfl_sync(0xffffffffu, acc[0][0][0][2], src);
+            const float u0 = __shfl_sync(0xffffffffu, acc[0][1][0][0], src), u1 = __shfl_sync(0xffffffffu, acc[0][1][0][2], src);
+            float gv = hi ? g1 : g0, uv = hi ? u1 : u0;
+            const int n = tile * tile_rows + wrow_off + lane;
+            if (lane < 16 && n < seg_n) {
+                if (FMT == FMT_INT8) {
+                    gv *= __half2float(__ushort_as_half(sc1));
+                    uv *= __half2float(__ushort_as_half(res1));
+                }
+                const float r = (gv / (1.0f + expf(-gv))) * uv;
+                seg_out[n] = __half_as_ushort(__float2half_rn(r));
+            }
+        } else {
+            const int am_base = EXT ? a.argmax_base : 0;
+            unsigned long long* const am_slot = EXT ? a.argmax_slot : nullptr;
+            uint16_t* peer[7];
+#pragma unroll
+            for (int p = 0; p < 7; ++p) peer[p] = (EXT && p < npeer) ? a.peer_out[p] : nullptr;
+            // the token's 32 results sit in lanes 0, 4, .. 28 (rows g, g + 8 of each row block):
+            // bring row L to lane L, finish it there and store the 32 rows with one instruction
+            const int src = (lane & 7) * 4, sel = lane >> 3;
+            const float v00 = __shfl_sync(0xffffffffu, acc[0][0][0][0], src), v01 = __shfl_sync(0xffffffffu, acc[0][0][0][2], src);
+            const float v10 = __shfl_sync(0xffffffffu, acc[0][1][0][0], src), v11 = __shfl_sync(0xffffffffu, acc[0][1][0][2], src);
+            float v = sel == 0 ? v00 : sel == 1 ? v01 : sel == 2 ? v10 : v11;
+            const int n = row0 + lane;
+            if (n < seg_n) {
+                if (FMT == FMT_INT8) v = __fmul_rn(v, __half2float(__ushort_as_half(sc1)));  // roundings as in finish_row
+                if (VAR >= 1 && biased) v = __fadd_rn(__half2float(__float2half_rn(v)), __half2float(__ushort_as_half(bias1)));
+                if (epi == EPI_RESIDUAL) {
+                    v = __fadd_rn(__half2float(__ushort_as_half(res1)), v);
+                } else if (epi == EPI_SILU_GATE) {
+                    const float gt = __half2float(__ushort_as_half(res1));
+                    v = gt * (1.0f / (1.0f + expf(-gt))) * v;
+                }
+                const uint16_t hv = __half_as_ushort(__float2half_rn(v));
+                if (!EXT || seg_out) seg_out[n] = hv;
+                if (EXT) {
+#pragma unroll
+                    for (int p = 0; p < 7; ++p)
+                        if (p < npeer) peer[p][n] = hv;
+                }
+                if (EXT && am_slot && (hv & 0x7FFFu) <= 0x7C00u) {  // NaNs never win
+                    const unsigned long long key = argmax_key_half(hv, am_base + n);
+                    am_best = key > am_best ? key : am_best;
+                }
+            }
         }
     }
     if (EXT && a.argmax_slot) {

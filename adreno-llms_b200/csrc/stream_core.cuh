@@ -42,8 +42,10 @@ __host__ __device__ inline int x_bytes_of(int fmt, int M, int K) {
 // Q4: per 32-weight block and token pair one float4 (c0, c1, c0, c1) with c = -72 * (sum of the
 // block's activations), the value the block's accumulator starts from
 __host__ __device__ inline int ctab_bytes_of(int fmt, int M, int K) { return fmt == FMT_Q4 ? (K / 32) * ((M + 1) / 2) * 16 : 0; }
-// two reduction buffers for the consumers that split K of one tile
-__host__ __device__ inline int red_bytes_of(int nt) { return 2 * NCW * 32 * 2 * nt * 4 * 4; }
+// two reduction buffers, [consumer][token][its 32 rows] with RED_TS words from token to token (padded: the fragments' stores and
+// the finish's reads of two neighbouring rows are conflict-free)
+constexpr int RED_TS = 36;
+__host__ __device__ inline int red_bytes_of(int nt) { return 2 * NCW * 8 * nt * RED_TS * 4; }
 // K parts of a tile whose K is split over the consumers (see "K parts" below)
 constexpr int KPARTS = 2 * NCW;
 
