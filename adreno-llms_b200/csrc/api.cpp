@@ -197,8 +197,7 @@ extern "C" int nn_init(int device, nn_context** out) {
     }
     // normalised activations for the norm-then-project calls that cannot fuse the norm: sized for the
     // decode shapes up front so that such calls also work inside a recording (it grows outside one)
-    // the staged activations of a batched call never exceed the shared memory of one block
-    c->stage_img_bytes = (size_t)256 << 10;
+    c->stage_img_bytes = STAGE_IMG_BYTES;   // the staged activations of a batched call
     if (cudaMalloc(&c->stage_img, c->stage_img_bytes) != cudaSuccess || cudaMemset(c->stage_img, 0, c->stage_img_bytes) != cudaSuccess) {
         delete c;
         return NN_FAIL(NN_ERR_CUDA, "nn_init: cudaMalloc failed");

@@ -52,22 +52,25 @@ struct Geo {  // shared-memory geometry, computed identically on host and device
     int nbox;         // 128-byte column boxes per stage
     int sstride;      // bytes between Q4 scale rows in a stage
     int stage_bytes;  // one stage (multiple of 1024)
+    int off_sx;       // activations that travel with the weights: their place in a stage
     int xstride;      // bytes between activation rows
     int off_bar, off_x, off_ctab, off_norm, off_red, off_ring;
     int total;
 };
 
-__host__ __device__ inline Geo make_geo(int fmt, int M, int K, int kcb, int stages, int nt, bool norm) {
+// xcols > 0: the activations are not resident but travel with the weights, xcols bytes of every row per stage.
+__host__ __device__ inline Geo make_geo(int fmt, int M, int K, int kcb, int stages, int nt, bool norm, int xcols) {
     Geo g;
     g.nbox = stage_nbox(kcb);
     g.sstride = stage_sstride(kcb);
-    g.stage_bytes = stage_bytes_of(fmt, kcb);
-    g.xstride = x_stride_of(fmt, K);
+    g.off_sx = stage_bytes_of(fmt, kcb);
+    g.xstride = xcols ? xcols + 16 : x_stride_of(fmt, K);
+    g.stage_bytes = g.off_sx + (xcols ? ((fmt == FMT_INT8 ? 3 : 1) * M * g.xstride + 1023) / 1024 * 1024 : 0);
     g.off_bar = 64;  // full[stages], empty[stages]
     g.off_x = HDR_BYTES + ((stages * 16 + 127) / 128) * 128;
-    g.off_ctab = g.off_x + x_bytes_of(fmt, M, K);
+    g.off_ctab = g.off_x + (xcols ? 256 : x_bytes_of(fmt, M, K));   // (travelling int8 rows: their scales stay)
     // fused RMSNorm: the normalised fp16 activations [M][K], from which the staging then reads
-    g.off_norm = g.off_ctab + ctab_bytes_of(fmt, M, K);
+    g.off_norm = g.off_ctab + (xcols ? 0 : ctab_bytes_of(fmt, M, K));
     g.off_red = g.off_norm + (norm ? ((M * K * 2 + 127) / 128) * 128 : 0);
     g.off_ring = ((g.off_red + red_bytes_of(nt) + 1023) / 1024) * 1024;  // two reduction buffers
     g.total = g.off_ring + stages * g.stage_bytes + 1024;  // slack to align the ring to 1 KB
@@ -108,7 +111,7 @@ template <> struct KArgsFor<FMT_Q4> { typedef KArgsQ4 type; };
 // VAR selects how much of the kernel is compiled in: 0 = the plain projection, 1 = plus the RMSNorm
 // prologue and the bias (an int8 1152 x 896 projection of 16 rows with its bias: 17.3 us in the full
 // variant, 13.2 here), 2 = plus the rarer features (balanced item dealing, peer stores, the gather signal,
-// the fused arg-max).  The plain instantiation carries none of that code: the per-layer operators
+// the fused arg-max), 3 = 1 with activations that travel with the weights.  The plain instantiation carries none of that code: the per-layer operators
 // are launch-latency-bound, and every instruction-cache line their blocks have to fetch shows up
 // in the step time (the full variant is 0.5 us slower per small launch with nothing switched on).
 // ONE: the launch has a single activation row (decode).  The row count then is a compile-time
@@ -131,7 +134,8 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     const bool ksplit = a.kw > 1;  // the four consumers split K of one 32-row tile
     const int rowbytes = ka.rowbytes, nchunks = ka.nchunks;
     const bool a_norm = VAR >= 1 && a.norm_w != nullptr;
-    const Geo geo = make_geo(FMT, aM, aK, kcb, stages, NT, a_norm);
+    const int xcols = VAR == 3 ? a.xcols : 0;
+    const Geo geo = make_geo(FMT, aM, aK, kcb, stages, NT, a_norm, xcols);
     const int warp_rows = DUAL ? 16 : WARP_ROWS;                       // rows of each weight per warp
     const int tile_rows = ksplit ? warp_rows : NCW * warp_rows;        // rows of each weight per block tile
     const int groups = ksplit ? (nchunks + NCW - 1) / NCW : nchunks;   // pipeline items per tile
@@ -144,7 +148,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     const uint32_t ring = (s_base + geo.off_ring + 1023u) & ~1023u;
 
     if (tid < 16) reinterpret_cast<uint32_t*>(smem)[tid] = 0u;
-    if (FMT == FMT_INT8 && tid >= 32 && tid < 48) reinterpret_cast<uint32_t*>(xs + 3 * aM * geo.xstride)[tid - 32] = 0u;  // per-row max words
+    if (FMT == FMT_INT8 && !xcols && tid >= 32 && tid < 48) reinterpret_cast<uint32_t*>(xs + 3 * aM * geo.xstride)[tid - 32] = 0u;  // per-row max words
     const uint32_t xbar = s_base + geo.off_x - 8;  // batched calls: the staged activations have landed
     if (tid == 0) {
         for (int s = 0; s < stages; ++s) {
@@ -195,77 +199,109 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     // ================= producer warp: one elected lane feeds the TMA unit =================
     if (warp == NCW) {
         pdl_launch_dependents();
-        if (lane == 0) {
-            const uint64_t policy = ka.evict_first ? l2_policy_evict_first() : l2_policy_evict_normal();
+        const uint64_t policy = ka.evict_first ? l2_policy_evict_first() : l2_policy_evict_normal();
+        // one pipeline item's weights (and Q4 scales), by one lane; `more` = bytes that others will add to the stage
+        auto send_weights = [&](int tile, int cg, int stage, uint32_t more) {
+            const uint32_t dst = ring + stage * geo.stage_bytes, bar = full0 + stage * 8;
+            const int sg = DUAL ? 0 : tile_segment(tile);
+            const int row0 = (tile - (DUAL ? 0 : seg_at(sg).tile0)) * tile_rows;
+            if (!ksplit) {
+                // one copy per 128-byte column covers the rows of all four consumers
+                const int cb = min(kcb, rowbytes - cg * kcb);
+                const int nb = (cb + 127) >> 7;
+                const bool stma = FMT == FMT_Q4 && ka.scale_tma;
+                const int bw = kcb / 8;  // bytes of block scales per row and stage
+                mbar_arrive_expect_tx(bar, (uint32_t)(nb * CTA_BOX + (stma ? NCW * WARP_ROWS * bw : 0)) + more);
+                if (stma) {
+                    const uint32_t sdst = dst + geo.nbox * CTA_BOX;
+                    if (DUAL) {
+                        tma_load_2d(sdst, scale_map(km, 0), cg * bw, row0, bar, policy);
+                        tma_load_2d(sdst + (NCW * WARP_ROWS / 2) * bw, scale_map(km, 3), cg * bw, row0, bar, policy);
+                    } else {
+                        tma_load_2d(sdst, scale_map(km, sg), cg * bw, row0, bar, policy);
+                    }
+                }
+                for (int b = 0; b < nb; ++b) {
+                    const int x = cg * kcb + b * 128;
+                    if (DUAL) {
+                        tma_load_2d(dst + b * CTA_BOX, &km.tm[0], x, row0, bar, policy);
+                        tma_load_2d(dst + b * CTA_BOX + CTA_BOX / 2, &km.tm[3], x, row0, bar, policy);
+                    } else {
+                        tma_load_2d(dst + b * CTA_BOX, &km.tm[sg], x, row0, bar, policy);
+                    }
+                }
+            } else {
+                // the consumers take consecutive K chunks of the same rows
+                const bool stma = FMT == FMT_Q4 && ka.scale_tma;
+                const int bw = kcb / 8;
+                uint32_t bytes = 0;
+                for (int w = 0; w < NCW; ++w) {
+                    const int c = cg * NCW + w;
+                    if (c < nchunks) bytes += (uint32_t)(((min(kcb, rowbytes - c * kcb) + 127) >> 7) * BOX_BYTES + (stma ? WARP_ROWS * bw : 0));
+                }
+                mbar_arrive_expect_tx(bar, bytes + more);
+                for (int w = 0; w < NCW; ++w) {
+                    const int c = cg * NCW + w;
+                    if (c >= nchunks) break;
+                    if (stma) {
+                        const uint32_t sdst = dst + geo.nbox * CTA_BOX;
+                        if (DUAL) {
+                            tma_load_2d(sdst + w * (WARP_ROWS / 2) * bw, scale_map(km, 0), c * bw, row0, bar, policy);
+                            tma_load_2d(sdst + (NCW * WARP_ROWS / 2 + w * (WARP_ROWS / 2)) * bw, scale_map(km, 3), c * bw, row0, bar, policy);
+                        } else {
+                            tma_load_2d(sdst + w * WARP_ROWS * bw, scale_map(km, sg), c * bw, row0, bar, policy);
+                        }
+                    }
+                    const int nb = (min(kcb, rowbytes - c * kcb) + 127) >> 7;
+                    for (int b = 0; b < nb; ++b) {
+                        const int x = c * kcb + b * 128;
+                        if (DUAL) {
+                            tma_load_2d(dst + b * CTA_BOX + w * (BOX_BYTES / 2), &km.tm[0], x, row0, bar, policy);
+                            tma_load_2d(dst + b * CTA_BOX + CTA_BOX / 2 + w * (BOX_BYTES / 2), &km.tm[3], x, row0, bar, policy);
+                        } else {
+                            tma_load_2d(dst + b * CTA_BOX + w * BOX_BYTES, &km.tm[sg], x, row0, bar, policy);
+                        }
+                    }
+                }
+            }
+        };
+        if constexpr (VAR == 3) {
+            // The staged activations travel with the weights, the columns of the stage's K range of every row: the whole warp
+            // copies rows, once the launch that staged them is over; the weights of the first stages do not wait for that.
+            const int xrows = (FMT == FMT_INT8 ? 3 : 1) * aM, ximg = x_stride_of(FMT, aK);
+            auto cols = [&](int cg) { return min(xcols, rowbytes - cg * xcols); };
+            int tile_s = tile_first, cg = 0, stage = 0, tile_w = tile_first, cg_w = 0;
+            for (int it = 0; it < n_items; ++it) {
+                if (it == 0) {
+                    const int ahead = min(stages, n_items);
+                    for (int j = 0; j < ahead; ++j) {
+                        if (lane == 0) send_weights(tile_w, cg_w, j, (uint32_t)(xrows * cols(cg_w)));
+                        if (++cg_w == groups) { cg_w = 0; tile_w += tile_step; }
+                    }
+                    __syncwarp();
+                    pdl_wait_prior_grid();
+                } else if (it >= stages) {
+                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(empty0 + stage * 8, (uint32_t)(((it / stages) - 1) & 1)))) {
+                        *reinterpret_cast<volatile int*>(a_status) = 2;
+                        break;
+                    }
+                    if (lane == 0) send_weights(tile_s, cg, stage, (uint32_t)(xrows * cols(cg)));
+                    __syncwarp();
+                }
+                const uint32_t dst = ring + stage * geo.stage_bytes + geo.off_sx, n = (uint32_t)cols(cg);
+                for (int r = lane; r < xrows; r += 32)
+                    bulk_g2s(dst + r * geo.xstride, a.staged + (size_t)r * ximg + (size_t)cg * xcols, n, full0 + stage * 8, l2_policy_evict_normal());
+                if (++cg == groups) { cg = 0; tile_s += tile_step; }
+                if (++stage == stages) stage = 0;
+            }
+        } else if (lane == 0) {
             int tile_s = tile_first, cg = cg_first, stage = 0;
             for (int it = 0; it < n_items; ++it) {
-                const int tile = tile_s;
                 if (it >= stages && !mbar_wait_bounded(empty0 + stage * 8, (uint32_t)(((it / stages) - 1) & 1))) {
                     *reinterpret_cast<volatile int*>(a_status) = 2;
                     break;
                 }
-                const uint32_t dst = ring + stage * geo.stage_bytes, bar = full0 + stage * 8;
-                const int sg = DUAL ? 0 : tile_segment(tile);
-                const int row0 = (tile - (DUAL ? 0 : seg_at(sg).tile0)) * tile_rows;
-                if (!ksplit) {
-                    // one copy per 128-byte column covers the rows of all four consumers
-                    const int cb = min(kcb, rowbytes - cg * kcb);
-                    const int nb = (cb + 127) >> 7;
-                    const bool stma = FMT == FMT_Q4 && ka.scale_tma;
-                    const int bw = kcb / 8;  // bytes of block scales per row and stage
-                    mbar_arrive_expect_tx(bar, (uint32_t)(nb * CTA_BOX + (stma ? NCW * WARP_ROWS * bw : 0)));
-                    if (stma) {
-                        const uint32_t sdst = dst + geo.nbox * CTA_BOX;
-                        if (DUAL) {
-                            tma_load_2d(sdst, scale_map(km, 0), cg * bw, row0, bar, policy);
-                            tma_load_2d(sdst + (NCW * WARP_ROWS / 2) * bw, scale_map(km, 3), cg * bw, row0, bar, policy);
-                        } else {
-                            tma_load_2d(sdst, scale_map(km, sg), cg * bw, row0, bar, policy);
-                        }
-                    }
-                    for (int b = 0; b < nb; ++b) {
-                        const int x = cg * kcb + b * 128;
-                        if (DUAL) {
-                            tma_load_2d(dst + b * CTA_BOX, &km.tm[0], x, row0, bar, policy);
-                            tma_load_2d(dst + b * CTA_BOX + CTA_BOX / 2, &km.tm[3], x, row0, bar, policy);
-                        } else {
-                            tma_load_2d(dst + b * CTA_BOX, &km.tm[sg], x, row0, bar, policy);
-                        }
-                    }
-                } else {
-                    // the consumers take consecutive K chunks of the same rows
-                    const bool stma = FMT == FMT_Q4 && ka.scale_tma;
-                    const int bw = kcb / 8;
-                    uint32_t bytes = 0;
-                    for (int w = 0; w < NCW; ++w) {
-                        const int c = cg * NCW + w;
-                        if (c < nchunks) bytes += (uint32_t)(((min(kcb, rowbytes - c * kcb) + 127) >> 7) * BOX_BYTES + (stma ? WARP_ROWS * bw : 0));
-                    }
-                    mbar_arrive_expect_tx(bar, bytes);
-                    for (int w = 0; w < NCW; ++w) {
-                        const int c = cg * NCW + w;
-                        if (c >= nchunks) break;
-                        if (stma) {
-                            const uint32_t sdst = dst + geo.nbox * CTA_BOX;
-                            if (DUAL) {
-                                tma_load_2d(sdst + w * (WARP_ROWS / 2) * bw, scale_map(km, 0), c * bw, row0, bar, policy);
-                                tma_load_2d(sdst + (NCW * WARP_ROWS / 2 + w * (WARP_ROWS / 2)) * bw, scale_map(km, 3), c * bw, row0, bar, policy);
-                            } else {
-                                tma_load_2d(sdst + w * WARP_ROWS * bw, scale_map(km, sg), c * bw, row0, bar, policy);
-                            }
-                        }
-                        const int nb = (min(kcb, rowbytes - c * kcb) + 127) >> 7;
-                        for (int b = 0; b < nb; ++b) {
-                            const int x = c * kcb + b * 128;
-                            if (DUAL) {
-                                tma_load_2d(dst + b * CTA_BOX + w * (BOX_BYTES / 2), &km.tm[0], x, row0, bar, policy);
-                                tma_load_2d(dst + b * CTA_BOX + CTA_BOX / 2 + w * (BOX_BYTES / 2), &km.tm[3], x, row0, bar, policy);
-                            } else {
-                                tma_load_2d(dst + b * CTA_BOX + w * BOX_BYTES, &km.tm[sg], x, row0, bar, policy);
-                            }
-                        }
-                    }
-                }
+                send_weights(tile_s, cg, stage, 0u);
                 if (++cg == groups) { cg = 0; tile_s += tile_step; }
                 if (++stage == stages) stage = 0;
             }
@@ -277,7 +313,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     const int g = lane >> 2, t = lane & 3;
     LaneGeo<NT> lg;
     lane_geo_init<FMT, NT>(lg, DUAL, warp, lane, aM, smem_u32(xs), geo.xstride, zero_addr, smem + geo.off_ctab);
-    const float* rowscale = reinterpret_cast<const float*>(xs + 3 * aM * geo.xstride + 64);
+    const float* rowscale = reinterpret_cast<const float*>(xs + (xcols ? 0 : 3 * aM * geo.xstride) + 64);
 
     // rows of this warp inside its tile, and which warp writes results
     const int wrow_off = ksplit ? 0 : warp * warp_rows;
@@ -389,11 +425,14 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     if (!ONE && a.staged != nullptr) {
         // the launch before this one (stage_image_kernel) wrote the staged form of all M rows in this
         // kernel's shared-memory layout: one bulk copy instead of M rows converted by every block
-        if (tid == 0) {
-            mbar_arrive_expect_tx(xbar, a.staged_bytes);
-            bulk_g2s(smem_u32(xs), a.staged, a.staged_bytes, xbar, l2_policy_evict_normal());
+        // (rows that travel with the weights: only the int8 row scales behind them)
+        const uint32_t skip = xcols ? (uint32_t)(3 * aM * x_stride_of(FMT, aK)) : 0u, bytes = xcols ? 192u : a.staged_bytes;
+        const bool some = !xcols || FMT == FMT_INT8;
+        if (tid == 0 && some) {
+            mbar_arrive_expect_tx(xbar, bytes);
+            bulk_g2s(smem_u32(xs), a.staged + skip, bytes, xbar, l2_policy_evict_normal());
         }
-        if (!mbar_wait_bounded(xbar, 0u)) *reinterpret_cast<volatile int*>(a_status) = 5;
+        if (some && !mbar_wait_bounded(xbar, 0u)) *reinterpret_cast<volatile int*>(a_status) = 5;
     } else {
     if (a_norm) {
         // RMSNorm prologue: the normalised fp16 rows go to shared memory and the staging below
@@ -451,6 +490,13 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
             if (lane == 0) *reinterpret_cast<volatile int*>(a_status) = 1;
         }
         const uint32_t sw = ring + stage * geo.stage_bytes;
+        if constexpr (VAR == 3) {   // this stage's activations begin at its first column
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                const int n = (lane & 7) + nt * 8;
+                if (n < aM) lg.b_base[nt] = sw + geo.off_sx + n * geo.xstride + (lane >> 3) * 16 - (uint32_t)(cg * xcols);
+            }
+        }
         const int cb = (failed || !active) ? 0 : min(kcb, rowbytes - c * kcb);
 
         if constexpr (FMT == FMT_FP16) {
@@ -786,6 +832,8 @@ cudaError_t launch_t(const typename KArgsFor<FMT>::type& ka, const StreamPlan& p
     const bool ext = a.streamk || a.npeer > 0 || a.sig.world > 0 || a.argmax_slot != nullptr || a.seg[0].out == nullptr;
     const bool bias = a.seg[0].bias != nullptr || a.seg[1].bias != nullptr || a.seg[2].bias != nullptr;
     if (ext) return launch_e<FMT, NT, DUAL, 2>(ka, p, st, pdl);
+    if constexpr (FMT != FMT_Q4)
+        if (p.xcols) return launch_o<FMT, NT, DUAL, 3, false>(ka, p, st, pdl);
     if (a.norm_w || bias) return launch_e<FMT, NT, DUAL, 1>(ka, p, st, pdl);
     return launch_e<FMT, NT, DUAL, 0>(ka, p, st, pdl);
 }
@@ -848,6 +896,7 @@ cudaError_t configure_one() {
 #define SET_SMEM(V, O)                                                                                                                       \
     if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_stream_kernel<FMT, NT, DUAL, V, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     SET_SMEM(0, false) SET_SMEM(1, false) SET_SMEM(2, false)
+    if constexpr (FMT != FMT_Q4) { SET_SMEM(3, false) }
     if (NT == 1) { SET_SMEM(0, true) SET_SMEM(1, true) SET_SMEM(2, true) }
 #undef SET_SMEM
     return e;
@@ -975,8 +1024,16 @@ StreamPlan stream_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limi
         if (kcb > 384) kcb = 256;
     }
     if (kcb > rb_cols) kcb = rb_cols;
-    while ((size_t)make_geo(fmt, M, K, kcb, 2, nt, norm).total > smem_limit && kcb > 128) kcb -= 128;
-    if ((size_t)make_geo(fmt, M, K, kcb, 2, nt, norm).total > smem_limit) { p.ok = false; return p; }
+    // Rows too many or too long to be resident beside two stages (int8, 16 rows of 4864 values: 234 KB of limbs) travel with the
+    // weights instead of being walked in slices that stream the weights again.
+    int xcols = 0;
+    if (M > 1 && fmt != FMT_Q4 && !norm && a.npeer == 0 && a.sig.world == 0 && stage_image_bytes(fmt, M, K) <= STAGE_IMG_BYTES &&
+        (size_t)make_geo(fmt, M, K, kcb, 2, nt, norm, 0).total > smem_limit) {
+        xcols = (kw == 1 ? 1 : NCW) * kcb;
+        if ((size_t)make_geo(fmt, M, K, kcb, 2, nt, norm, xcols).total > smem_limit) xcols = 0;
+    }
+    while ((size_t)make_geo(fmt, M, K, kcb, 2, nt, norm, xcols).total > smem_limit && kcb > 128) kcb -= 128;
+    if ((size_t)make_geo(fmt, M, K, kcb, 2, nt, norm, xcols).total > smem_limit) { p.ok = false; return p; }
     const int ntiles = count_tiles(a, kw == 1 ? NCW * warp_rows : warp_rows);
     const int nchunks = (rb + kcb - 1) / kcb;
     const int groups = kw == 1 ? nchunks : (nchunks + NCW - 1) / NCW;
@@ -987,8 +1044,8 @@ StreamPlan stream_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limi
     for (int ps = 2; ps >= 1 && !per_sm; --ps) {
         const size_t budget = (smem_limit + 1024) / ps - 1024;
         int st = ps >= 2 ? 4 : 6;
-        while (st > 2 && (size_t)make_geo(fmt, M, K, kcb, st, nt, norm).total > budget) --st;
-        if ((size_t)make_geo(fmt, M, K, kcb, st, nt, norm).total > budget) continue;
+        while (st > 2 && (size_t)make_geo(fmt, M, K, kcb, st, nt, norm, xcols).total > budget) --st;
+        if ((size_t)make_geo(fmt, M, K, kcb, st, nt, norm, xcols).total > budget) continue;
         const int resident = sm_count * ps;
         const int items = ((ntiles + resident - 1) / resident) * groups;  // pipeline items of the busiest block
         if (items <= st) st = items < 2 ? 2 : items;
@@ -998,7 +1055,7 @@ StreamPlan stream_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limi
     }
     if (per_sm == 0) { p.ok = false; return p; }
     const int stages = p.stages;
-    Geo g = make_geo(fmt, M, K, kcb, stages, nt, norm);
+    Geo g = make_geo(fmt, M, K, kcb, stages, nt, norm, xcols);
     const int resident = sm_count * per_sm;
     const int waves = (ntiles + resident - 1) / resident;
     p.grid = waves > 0 ? (ntiles + waves - 1) / waves : 1;
@@ -1024,6 +1081,7 @@ StreamPlan stream_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limi
             p.grid = resident;
         }
     }
+    p.xcols = xcols;
     p.kcb = kcb;
     p.kw = kw;
     p.warps = NCW;
@@ -1037,6 +1095,7 @@ cudaError_t launch_stream(int fmt, const LinArgs& a, const StreamPlan& p, cudaSt
     KArgsQ4 ka;  // sliced to KArgs for the formats without block scales
     ka.a = a;
     ka.a.kcb = p.kcb;
+    ka.a.xcols = p.xcols;
     ka.a.kw = p.kw;
     ka.a.ntiles = p.ntiles;
     ka.a.streamk = p.streamk ? 1 : 0;

@@ -80,6 +80,7 @@ struct LinArgs {
     // stage_image_kernel in the kernel's own shared-memory layout; every block copies it in
     const uint8_t* staged;
     unsigned staged_bytes;
+    int xcols;       // > 0: the staged rows travel with the weights, this many bytes of each per stage (StreamPlan)
     // host side only: Q4 scales with rows padded to a multiple of 16 bytes (seg[0..2], then the second weight of the
     // two-weight form), for the tensor copies when K / 16 is not such a multiple; all null otherwise
     const uint16_t* scale_pad[4];
@@ -95,6 +96,7 @@ struct StreamPlan {  // launch geometry chosen on the host
     int kw;      // warps splitting K of one tile
     int warps;   // warps per block
     int stages;  // ring depth
+    int xcols;   // > 0: batched activations travel with the weights, this many bytes of every row per stage
     int ntiles;  // block tiles over all segments
     size_t smem;
     bool ok;
@@ -176,6 +178,7 @@ inline bool q4_scale_views(const LinArgs& a, const uint16_t* base[4], int* pitch
 }
 cudaError_t launch_l2_flush(void* buf, size_t bytes, cudaStream_t st);
 // the staged activations of a batched call (layout of the streaming kernel's shared memory), with the optional RMSNorm
+constexpr size_t STAGE_IMG_BYTES = (size_t)1 << 20;   // the context's room for them (int8: 16 rows of 21 000 values)
 size_t stage_image_bytes(int fmt, int M, int K);
 cudaError_t launch_stage_image(int fmt, const uint16_t* x, int M, int K, const uint16_t* norm_w, float eps, uint8_t* img, cudaStream_t st,
                                bool pdl);
