@@ -184,7 +184,7 @@ extern "C" int nn_init(int device, nn_context** out) {
         return NN_FAIL(NN_ERR_CUDA, "nn_init: status word allocation failed");
     }
     *c->status_host = 0;
-    // [0] nn_argmax's reduction word, [1] the fused arg-max's word, [2] its block counter
+    // [0] nn_argmax's reduction word, [3] its block counter; [1] and [2] the fused arg-max's
     if (cudaMalloc((void**)&c->argmax_slot, 32) != cudaSuccess || cudaMemset(c->argmax_slot, 0, 32) != cudaSuccess) {
         delete c;
         return NN_FAIL(NN_ERR_CUDA, "nn_init: cudaMalloc failed");
@@ -861,8 +861,8 @@ extern "C" int nn_argmax(nn_context* c, int n, nn_buf logits, nn_buf out_idx) {
     if (!c || !logits || !out_idx) return NN_FAIL(NN_ERR_ARG, "nn_argmax: null argument");
     if (n < 0) return NN_FAIL(NN_ERR_ARG, "nn_argmax: n=%d", n);
     ProfScope prof(c, [&] { return std::string("argmax_n" + std::to_string(n)); });
-    CUDA_TRY(launch_argmax_half((const uint16_t*)logits, n, (int*)out_idx, c->argmax_slot, c->stream));
-    c->launches += n > 0 ? 3 : 2;
+    CUDA_TRY(launch_argmax_half((const uint16_t*)logits, n, (int*)out_idx, c->argmax_slot, reinterpret_cast<unsigned*>(c->argmax_slot + 3), c->stream, c->use_pdl));
+    c->launches++;
     return NN_OK;
 }
 

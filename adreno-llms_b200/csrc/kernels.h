@@ -154,9 +154,8 @@ cudaError_t launch_comm_pick(const unsigned* my_flags, int world, unsigned* pick
 // Multiprocessors of the current device (cached per device; allocates nothing).
 int current_sm_count();
 cudaError_t launch_dequant(int fmt, int N, int K, const void* W, const uint16_t* scale, float* out, cudaStream_t st);
-cudaError_t launch_argmax_half(const uint16_t* v, int n, int* out_idx, unsigned long long* slot, cudaStream_t st);
-cudaError_t launch_fill_u64(unsigned long long* p, unsigned long long v, cudaStream_t st);
-cudaError_t launch_argmax_finish(const unsigned long long* slot, int* out_idx, cudaStream_t st);
+// slot and done: 0 before and after the launch
+cudaError_t launch_argmax_half(const uint16_t* v, int n, int* out_idx, unsigned long long* slot, unsigned* done, cudaStream_t st, bool pdl);
 // Q4 block scales by tensor copy: from the weight's own scale array when its rows (K / 16 bytes) are a multiple of 16 bytes
 // and 16-byte aligned, else from the padded copy made at registration.  False: neither is there (per-lane copies then).
 inline bool q4_scale_views(const LinArgs& a, const uint16_t* base[4], int* pitch) {

@@ -42,39 +42,53 @@ __device__ __forceinline__ unsigned long long argmax_key(float v, int idx) {
     return ((unsigned long long)b << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned int)idx);
 }
 
-__global__ void argmax_half_kernel(const uint16_t* __restrict__ v, int n, unsigned long long* slot) {
+// One launch: every block folds its values into `slot` (0 between launches) and the block that finishes last writes the index and
+// clears the words.  (Clearing, folding and finishing as three launches cost a step of one token 6 us on a 151936-entry
+// vocabulary, most of it launches.)
+__global__ void __launch_bounds__(256) argmax_half_kernel(const uint16_t* __restrict__ v, int n, unsigned long long* slot, unsigned* done, int* out_idx) {
+    pdl_launch_dependents();
+    pdl_wait_prior_grid();
     unsigned long long best = 0ull;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float f = h2f(v[i]);
+    auto take = [&](uint16_t h, int i) {
+        const float f = h2f(h);
         if (f == f) {  // NaNs never win
             const unsigned long long k = argmax_key(f, i);
             best = k > best ? k : best;
         }
+    };
+    const int stride = gridDim.x * blockDim.x, at = blockIdx.x * blockDim.x + threadIdx.x;
+    const int pieces = (reinterpret_cast<uintptr_t>(v) & 15) == 0 ? n / 8 : 0;
+    for (int p = at; p < pieces; p += stride) {
+        const uint4 q = reinterpret_cast<const uint4*>(v)[p];
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            take((uint16_t)(w[j] & 0xFFFFu), p * 8 + 2 * j);
+            take((uint16_t)(w[j] >> 16), p * 8 + 2 * j + 1);
+        }
     }
+    for (int i = pieces * 8 + at; i < n; i += stride) take(v[i], i);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
         best = other > best ? other : best;
     }
-    __shared__ unsigned long long sm[32];
+    __shared__ unsigned long long sm[8];
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = best;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        best = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0ull;
+    if (threadIdx.x == 0) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-            best = other > best ? other : best;
+        for (int i = 1; i < 8; ++i) best = sm[i] > best ? sm[i] : best;
+        if (best) atomicMax(slot, best);
+        __threadfence();
+        if (atomicAdd(done, 1u) == gridDim.x - 1u) {
+            __threadfence();
+            const unsigned long long k = *reinterpret_cast<volatile unsigned long long*>(slot);
+            *reinterpret_cast<volatile unsigned long long*>(slot) = 0ull;
+            *reinterpret_cast<volatile unsigned*>(done) = 0u;
+            *out_idx = k ? (int)(0xFFFFFFFFu - (unsigned int)(k & 0xFFFFFFFFull)) : -1;
         }
-        if (threadIdx.x == 0 && best) atomicMax(slot, best);
     }
-}
-
-__global__ void fill_u64_kernel(unsigned long long* p, unsigned long long v) { *p = v; }
-
-__global__ void argmax_finish_kernel(const unsigned long long* slot, int* out_idx) {
-    const unsigned long long k = *slot;
-    *out_idx = k ? (int)(0xFFFFFFFFu - (unsigned int)(k & 0xFFFFFFFFull)) : -1;
 }
 
 // RMSNorm on fp16 storage, one block per row: out = half((x * rsqrt(mean(x^2) + eps)) * weight)
@@ -257,27 +271,21 @@ cudaError_t launch_dequant(int fmt, int N, int K, const void* W, const uint16_t*
     return cudaGetLastError();
 }
 
-cudaError_t launch_fill_u64(unsigned long long* p, unsigned long long v, cudaStream_t st) {
-    fill_u64_kernel<<<1, 1, 0, st>>>(p, v);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_argmax_finish(const unsigned long long* slot, int* out_idx, cudaStream_t st) {
-    argmax_finish_kernel<<<1, 1, 0, st>>>(slot, out_idx);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_argmax_half(const uint16_t* v, int n, int* out_idx, unsigned long long* slot, cudaStream_t st) {
-    cudaError_t e = launch_fill_u64(slot, 0ull, st);
-    if (e != cudaSuccess) return e;
-    if (n > 0) {
-        int blocks = (n + 1023) / 1024;
-        const int cap = current_sm_count() * 4;
-        if (blocks > cap) blocks = cap;
-        argmax_half_kernel<<<blocks, 256, 0, st>>>(v, n, slot);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
-    return launch_argmax_finish(slot, out_idx, st);
+cudaError_t launch_argmax_half(const uint16_t* v, int n, int* out_idx, unsigned long long* slot, unsigned* done, cudaStream_t st, bool pdl) {
+    int blocks = (n + 2047) / 2048;   // one 16-byte piece per thread, up to one block per SM
+    const int cap = current_sm_count();
+    if (blocks > cap) blocks = cap;
+    if (blocks < 1) blocks = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, argmax_half_kernel, v, n, slot, done, out_idx);
 }
 
 cudaError_t launch_rmsnorm(const uint16_t* x, const uint16_t* w, uint16_t* out, int rows, int cols, float eps, cudaStream_t st, bool pdl) {
