@@ -425,7 +425,7 @@ bool nnb::resolve_weight(const nn_context* c, const void* W, int K, ResolvedW* o
 // ---------------------------------------------------------------------------------
 // M > 16: the tensor-core GEMM, with whatever follows the product in its epilogue (quantised weights are expanded to fp16
 // inside the kernel).  Shapes it does not take are walked in slices of 16 rows by the streaming kernel.
-static int run_gemm_tc(nn_context* c, int fmt, const LinArgs& a, int M, const char* who, bool* done) {
+static int run_gemm_tc(nn_context* c, int fmt, const LinArgs& a, int M, bool plain_form, const char* who, bool* done) {
     *done = false;
     if (!gemm_tc_supported(fmt, a, M)) return NN_OK;
     bool wait_first = false;
@@ -433,7 +433,7 @@ static int run_gemm_tc(nn_context* c, int fmt, const LinArgs& a, int M, const ch
     for (int i = 0; i < a.nseg; ++i) wait_first = wait_first || c->recently_written(a.seg[i].W, rb * (size_t)a.seg[i].N);
     if (a.epi == EPI_SWIGLU) wait_first = wait_first || c->recently_written(a.W2, rb * (size_t)a.seg[0].N);
     int n = 0;
-    cudaError_t e = launch_gemm_tc(fmt, a, M, wait_first, c->use_pdl, c->stream, &n);
+    cudaError_t e = launch_gemm_tc(fmt, a, M, plain_form, wait_first, c->use_pdl, c->stream, &n);
     c->launches += n;
     if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: tensor-core launch failed: %s (M=%d N=%d K=%d)", who, cudaGetErrorString(e), M, a.seg[0].N, a.K);
     *done = true;
@@ -466,6 +466,7 @@ static void note_recorded(nn_context* c, int fmt, const LinArgs& a, const Stream
 
 static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char* who) {
     for (int i = 0; i < a.nseg; ++i) c->note_output(a.seg[i].out, (size_t)M_total * a.seg[i].ld_out * 2);
+    const bool plain_form = !a.norm_w && !a.seg[0].bias;
     a.sk_scratch = c->sk_scratch;
     a.sk_flags = c->sk_flags;
     if (a.norm_w) {
@@ -498,7 +499,7 @@ static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char
     }
     if (M_total > 16) {
         bool done = false;
-        const int rc = run_gemm_tc(c, fmt, a, M_total, who, &done);
+        const int rc = run_gemm_tc(c, fmt, a, M_total, plain_form, who, &done);
         if (rc != NN_OK || done) return rc;
     }
     // M > 16 is walked in slices of 16 activation rows (each slice re-streams the weights).

@@ -1128,7 +1128,7 @@ bool gemm_tc_supported(int fmt, const LinArgs& a, int M) {
     return a.epi != EPI_SWIGLU || al16(a.W2);
 }
 
-cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool wait_first, bool pdl, cudaStream_t st, int* launches) {
+cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool plain_form, bool wait_first, bool pdl, cudaStream_t st, int* launches) {
     const bool dual = a.epi == EPI_SWIGLU;
     const int K = a.K, sms = current_sm_count();
     if (a.npeer < 0 || a.npeer > 7) return cudaErrorInvalidValue;
@@ -1205,14 +1205,14 @@ cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool wait_first, bo
         if (dual && !make_scale_map(&mp.sc[1], sbase[3], a.seg[0].N, pitch, 16, trows)) g.scale_tma = 0;
     }
     if (!encode_tiled_2d(&mp.x, true, a.x, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, (uint32_t)c.bn)) return cudaErrorInvalidValue;
-    // Calls of the fused forms with few results keep the three launches that nn_launch_count has always reported for them and
-    // callers check (one weight each; SwiGLU: a third of the columns each), side by side; they cost 4-5 us more than one launch
-    // does, so larger calls (from the size of 43 tiles of 128 x 64 results on) are one.
+    // The plain fused forms (q/k/v, SwiGLU) with few results go out as three launches side by side, which is what
+    // nn_launch_count reports for them and its tests state; that costs 4-5 us more than one launch does, so larger calls (from the
+    // results of 43 tiles of 128 x 64 on) and the forms with a norm or a bias, which a layer uses, are one.
     const int tiles = rows * c.ntok;
     long long results = 0;
     for (int i = 0; i < a.nseg; ++i) results += (long long)M * a.seg[i].N;
     int cut[4] = {0, tiles, tiles, tiles}, parts = 1;
-    if ((dual || a.nseg == 3) && rows >= 3 && results < 43ll * 128 * 64) {
+    if (plain_form && (dual || a.nseg == 3) && rows >= 3 && results < 43ll * 128 * 64) {
         parts = 3;
         for (int i = 1; i < 3; ++i) cut[i] = (dual ? i * rows / 3 : g.seg[i].tile0) * c.ntok;
         cut[3] = tiles;
