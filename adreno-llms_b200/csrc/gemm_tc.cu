@@ -9,11 +9,11 @@
 //
 // A block computes tiles of 128 weight rows x bn tokens (bn <= 256, a multiple of 16), the weights
 // as the MMA's M operand, into tensor memory:
-//   * warp 0, one lane: TMA producer of the token operand (64-wide K blocks, 128-byte swizzle) and,
+//   * warp 0: TMA producer of the token operand (64-wide K blocks, 128-byte swizzle) and,
 //     for fp16 weights, of the weight operand.
-//   * warp 1, one lane: issues tcgen05.mma (cta_group::1, kind::f16, M128 x N(bn) x K16, four per
+//   * warp 1: issues tcgen05.mma (cta_group::1, kind::f16, M128 x N(bn) x K16, four per
 //     K block and weight); tcgen05.commit hands operands back and signals the epilogue.
-//   * warps 2-5: epilogue.  Warp w reads lanes 32 (w % 4) .. +31 of the accumulator with
+//   * warps 2-9 (Q4: 2-5): epilogue.  Warp w reads lanes 32 (w % 4) .. +31 of the accumulator with
 //     tcgen05.ld (lane = weight row, column = token) and finishes the values there: int8 row
 //     scale, bias, in-place residual, SiLU gate.  SwiGLU: a tile is 64 gate rows and the 64 up rows of
 //     the same numbers, and the warps that hold them swap half of each other's columns through shared
@@ -28,6 +28,8 @@
 //   * few tiles (a per-layer projection of a prompt): the K blocks of a tile are split over a
 //     cluster of 2..8 blocks, whose fp32 partial sums meet through distributed shared memory, each
 //     block finishing its share of the tokens; the sums are added in rank order.
+//   * long calls: two blocks of a cluster share a tile of 256 rows (cta_group::2), each with its half of the rows and of the
+//     tokens; one of them issues the MMAs of both.
 //   * every block walks K from a starting place of its own, so that the blocks do not all ask for
 //     the same lines of the token operand at the same moment.
 #include <cuda.h>
@@ -45,27 +47,29 @@ namespace {
 
 constexpr int BM = 128;       // weight rows per tile (UMMA M)
 constexpr int BK = 64;        // K elements per block = one 128-byte swizzle span of fp16
-constexpr int EPI_WARPS = 4;
 constexpr int A_BYTES = BM * BK * 2;  // 16 KB
 constexpr int RAW_BYTES = BM * 128;   // packed span of one weight: 128 bytes of each of the tile's rows
 constexpr int SC_BYTES = BM * 16;     // Q4: the block scales of a span
 constexpr int RING_MAX = 16;          // token (and fp16 weight) stages
 constexpr int RAW_MAX = 8;            // packed spans
-constexpr int SLAB_MAX = 128;         // tokens per output slab (staging buffer: 128 x 128 fp16 = 32 KB)
+constexpr int SLAB_MAX = 128;         // tokens per output slab (a staging buffer of 128 x 128 fp16 = 32 KB)
 constexpr int SMEM_LIMIT = 227 * 1024;
 // K blocks per packed span, and as many groups of four expanding warps
 __host__ __device__ constexpr int span_blocks(int wfmt) { return wfmt == FMT_Q4 ? 4 : wfmt == FMT_INT8 ? 2 : 1; }
 __host__ __device__ constexpr int dq_warps(int wfmt) { return wfmt == FMT_FP16 ? 0 : 4 * span_blocks(wfmt); }
+// epilogue warps: one or two groups of four, which take the 16-token steps of a slab in turn (Q4: the expanding warps leave
+// registers for four)
+__host__ __device__ constexpr int epi_warps(int wfmt) { return wfmt == FMT_Q4 ? 4 : 8; }
 __host__ __device__ constexpr int raw_stage_bytes(int wfmt) { return RAW_BYTES + (wfmt == FMT_Q4 ? SC_BYTES : 0); }
 __host__ __device__ constexpr int gemm_threads(int wfmt) {
-    return (2 + EPI_WARPS) * 32 + (wfmt == FMT_FP16 ? 0 : dq_warps(wfmt) * 32 + 32);
+    return (2 + epi_warps(wfmt)) * 32 + (wfmt == FMT_FP16 ? 0 : dq_warps(wfmt) * 32 + 32);
 }
 
 // shared-memory header: barriers and the tensor-memory address
 constexpr int H_FULL = 0, H_EMPTY = H_FULL + RING_MAX * 8, H_RAW_FULL = H_EMPTY + RING_MAX * 8, H_RAW_EMPTY = H_RAW_FULL + RAW_MAX * 8;
 constexpr int H_ACC_FULL = H_RAW_EMPTY + RAW_MAX * 8, H_ACC_EMPTY = H_ACC_FULL + 16, H_RES = H_ACC_EMPTY + 16, H_TMEM = H_RES + 8, H_XCHG = H_TMEM + 8;
 constexpr int HDR = 1024;
-constexpr int SWAP_BYTES = 8192;   // the SwiGLU epilogue's two exchange buffers (16 tokens x 64 rows fp32 each), behind the output slab
+constexpr int SWAP_BYTES = 8192;   // the SwiGLU epilogue's two exchange buffers (16 tokens x 64 rows fp32 each) of four warps, behind the output slabs
 static_assert(H_XCHG + 8 <= HDR, "header");
 
 // The maps travel in a parameter of their own: their address is taken, and a scalar beside them would be read
@@ -96,7 +100,7 @@ struct GemmArgs {
     int kps, lag;            // packed weights: K blocks per token stage; spans whose expanded blocks are in tensor memory at a time
     int accw, nacc;          // tensor-memory columns of one accumulator, and how many sets
     int tmem_cols;
-    int slab;                // tokens per output slab
+    int slab, two_slabs;     // tokens per output slab; whether there are two staging buffers
     int scale_tma;           // Q4: the block scales arrive with the packed spans (else the expanding threads load them)
     int swap_off;            // SwiGLU: the exchange buffers, from the ring's start
     int xchg_off;            // split tiles: where the other blocks' parts land, from the ring's start
@@ -109,44 +113,83 @@ struct GemmArgs {
     GatherSignal sig;        // completion signal of the gather (world == 0: none)
 };
 
-// ---- tcgen05 wrappers -------------------------------------------------------------------
+// ---- tcgen05 wrappers (DUO: the forms for two blocks, cta_group::2) -------------------------
+template <bool DUO>
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (DUO) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
 }
+template <bool DUO>
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+    if (DUO) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+template <bool DUO>
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
+    if (DUO)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+            : "memory");
 }
 // the M operand from tensor memory: lane = row, one 32-bit column = two consecutive k
+template <bool DUO>
 __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
+    if (DUO)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+            : "memory");
 }
+// (DUO: arrives on the barrier at this place in both blocks)
+template <bool DUO>
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    if (DUO) asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+    else asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+// (the registers are valid after tmem_wait_ld, which "writes" them too so that no use moves before it)
+__device__ __forceinline__ void tmem_ld16_begin(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
           "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
+                   "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :: "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    tmem_ld16_begin(taddr, r);
+    tmem_wait_ld(r);
 }
 // 16 columns of this thread's lane
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -177,6 +220,24 @@ __device__ __forceinline__ uint32_t peer_smem(uint32_t addr, int rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
+// Arrival on a barrier of any block of the cluster (an address from peer_smem).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+template <bool DUO>
+__device__ __forceinline__ void arrive_on(uint32_t bar) {
+    if (DUO) mbar_arrive_cluster(bar);
+    else mbar_arrive(bar);
+}
+// An operand copy: into this block's memory, counted on `bar` (DUO: a barrier of either block).
+template <bool DUO>
+__device__ __forceinline__ void load_2d(uint32_t dst, const void* tmap, int x, int y, uint32_t bar, uint64_t policy) {
+    if (!DUO) return tma_load_2d(dst, tmap, x, y, bar, policy);
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;" ::"r"(dst),
+        "l"(tmap), "r"(x), "r"(y), "r"(bar), "l"(policy)
+        : "memory");
+}
 // Shared memory of this block -> shared memory of another block of the cluster, counted on that block's barrier.
 __device__ __forceinline__ void bulk_s2peer(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src), "r"(bytes), "r"(bar)
@@ -194,9 +255,9 @@ __device__ __forceinline__ uint64_t desc_of(uint32_t lo) {
     asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(DESC_HI));
     return d;
 }
-// Instruction descriptor: fp32 accumulate, fp16 x fp16, both operands K-major, M = 128, N = bn.
-__device__ __forceinline__ uint32_t instr_desc_f16(int bn) {
-    return (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+// Instruction descriptor: fp32 accumulate, fp16 x fp16, both operands K-major, M = 128 (two blocks: 256), N = bn.
+__device__ __forceinline__ uint32_t instr_desc_f16(int bn, int m) {
+    return (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 // One lane of a convergent warp.
@@ -207,6 +268,7 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // Whether any epilogue thread's flag is set.
+template <int EPI_WARPS>
 __device__ __forceinline__ bool epilogue_any(bool f) {
     int r;
     asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 3, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
@@ -215,9 +277,9 @@ __device__ __forceinline__ bool epilogue_any(bool f) {
 }
 
 // Rows [m, m + rows) x columns [n0, n0 + cols) of a [.][ld] fp16 matrix of N columns, between global memory and a dense slab of
-// `cols` columns in shared memory, by the 128 epilogue threads: a warp takes a row, two values per lane and step where the
+// `cols` columns in shared memory, by the epilogue threads: a warp takes a row, two values per lane and step where the
 // rows are 4-byte aligned.  (One 2-byte store per value straight from the accumulator's lanes took 140 clocks per token.)
-template <bool IN>
+template <bool IN, int EPI_WARPS>
 __device__ __forceinline__ void copy_rows(uint16_t* out, int ld, int N, int n0, int m, int rows, int cols, uint32_t slab, int et) {
     const int lane = et & 31, valid = min(cols, N - n0);
     const bool pairs = ((ld | n0) & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0;
@@ -324,11 +386,12 @@ __device__ __forceinline__ void expand_q4_word(uint32_t w, __half2 scale, uint32
     }
 }
 
-template <int WFMT>
+// DUO: two blocks of a cluster work on two neighbouring row tiles and the same tokens: see `duo` in gemm_choose.
+template <int WFMT, bool DUO>
 __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(const __grid_constant__ GemmMaps mp, const GemmArgs g) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr bool PACKED = WFMT != FMT_FP16;
-    constexpr int SPAN = span_blocks(WFMT), DQ = dq_warps(WFMT);
+    constexpr int SPAN = span_blocks(WFMT), DQ = dq_warps(WFMT), EPI_WARPS = epi_warps(WFMT), GROUPS = EPI_WARPS / 4;
     // (the shuffle tells the compiler that a warp's number is uniform, and so the control flow that depends on it)
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t s_base = smem_u32(smem);
@@ -336,7 +399,7 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
     const uint32_t acc_full0 = s_base + H_ACC_FULL, acc_empty0 = s_base + H_ACC_EMPTY;
     const uint32_t res_bar = s_base + H_RES, xchg_bar = s_base + H_XCHG;
     const uint32_t ring = (s_base + (uint32_t)HDR + 1023u) & ~1023u;
-    const int bn = g.bn, stages = g.stages, raw_stages = g.raw_stages, ntok = g.ntok, S = g.ksplit, nacc = g.nacc, accw = g.accw;
+    const int bn = g.bn, stages = g.stages, raw_stages = g.raw_stages, ntok = g.ntok, S = DUO ? 1 : g.ksplit, nacc = g.nacc, accw = g.accw;
     // Scalars used in loops are read from the parameter block once: a store the compiler cannot see through would otherwise
     // have every later use read it again.
     const bool pair = g.epi == EPI_SWIGLU;   // a tile is 64 rows of each of two weights
@@ -345,7 +408,9 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
     const int lag = g.lag;   // packed weights: spans whose expanded blocks are in tensor memory at a time (1, 2 or 4)
     const bool tma_store = g.tma_store != 0, wait_first = g.wait_first != 0;
     int* const status = g.status;
-    const int b_bytes = bn * BK * 2;                                   // a multiple of 2 KB
+    const int half_rank = DUO ? (int)(blockIdx.x & 1u) : 0;            // 0: the block that issues the MMAs of both
+    const int xtok = DUO ? bn / 2 : bn;                                // tokens that this block loads
+    const int b_bytes = xtok * BK * 2;                                 // a multiple of 2 KB
     // K blocks per stage: one; packed weights: 1, 2 or 4 (dividing the span's), so that few waits and commits are paid per block
     const int kps = PACKED ? g.kps : 1;
     const int b_off = PACKED ? 0 : A_BYTES, stage_bytes = b_off + kps * b_bytes;
@@ -357,21 +422,23 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
     const int nkb = (g.K + BK - 1) / BK, nunits = (nkb + SPAN - 1) / SPAN;
     const int rank = S > 1 ? (int)(blockIdx.x % (unsigned)S) : 0;
     const int u0 = rank * nunits / S, nu = (rank + 1) * nunits / S - u0;
-    const int tile_first = g.tile_begin + (S > 1 ? (int)(blockIdx.x / (unsigned)S) : (int)blockIdx.x);
+    const int tile_first = g.tile_begin + (DUO ? (int)(blockIdx.x >> 1) : S > 1 ? (int)(blockIdx.x / (unsigned)S) : (int)blockIdx.x);
     const int fin = g.fin, cps = bn / fin;                              // blocks of a cluster that finish tokens, and how many each
-    const int tile_step = S > 1 ? g.tile_end : (int)gridDim.x;          // a split tile: one per cluster
+    const int tile_step = DUO ? (int)(gridDim.x >> 1) : S > 1 ? g.tile_end : (int)gridDim.x;   // a split tile: one per cluster
+    // DUO: a tile number stands for two row tiles.  The second one of the last pair may lie past the end: its copies bring zeros.
+    auto row_tile = [&](int tile) { return DUO ? 2 * (tile / ntok) + half_rank : tile / ntok; };
     auto segment = [&](int rt) { return (g.nseg > 2 && rt >= g.seg[2].tile0) ? 2 : (g.nseg > 1 && rt >= g.seg[1].tile0) ? 1 : 0; };
     auto seg_at = [&](int si) { return si == 0 ? g.seg[0] : si == 1 ? g.seg[1] : g.seg[2]; };
-    auto first_unit = [&](int rt) { return (int)((unsigned)(rt * 7) % (unsigned)nu); };   // where the walk over K starts
+    auto first_unit = [&](int tile) { return (int)((unsigned)(tile / ntok * 7) % (unsigned)nu); };   // where the walk over K starts
 
     // one barrier per thread: a single thread took a thousand clocks over them
     if (tid < RING_MAX) {
-        if (tid < stages) mbar_init(full0 + tid * 8, PACKED ? 1 + 4 * kps : 1);   // the copies (and the four warps that expand each K block)
+        if (tid < stages) mbar_init(full0 + tid * 8, PACKED ? 1 + 4 * kps * (DUO ? 2 : 1) : 1);   // the copies (and the four warps that expand each K block)
     } else if (tid < 2 * RING_MAX) {
         if (tid - RING_MAX < stages) mbar_init(empty0 + (tid - RING_MAX) * 8, 1);
     } else if (tid < 2 * RING_MAX + 4) {
         const int a = tid - 2 * RING_MAX;
-        mbar_init((a < 2 ? acc_full0 : acc_empty0) + (a & 1) * 8, a < 2 ? 1 : EPI_WARPS);
+        mbar_init((a < 2 ? acc_full0 : acc_empty0) + (a & 1) * 8, a < 2 ? 1 : EPI_WARPS * (DUO ? 2 : 1));
     } else if (tid == 2 * RING_MAX + 4) {
         mbar_init(res_bar, 1);
     } else if (tid == 2 * RING_MAX + 5) {
@@ -382,11 +449,17 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         if (r < raw_stages) mbar_init((tid < 64 + RAW_MAX ? raw_full0 : raw_empty0) + r * 8, tid < 64 + RAW_MAX ? 1 : DQ);
     }
     mbar_init_fence();
-    if (warp == 1) tmem_alloc(s_base + H_TMEM, (uint32_t)g.tmem_cols);
+    if (warp == 1) tmem_alloc<DUO>(s_base + H_TMEM, (uint32_t)g.tmem_cols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem + H_TMEM);
+    if (DUO) {   // both blocks hold their tensor memory and their barriers are ready
+        cluster_arrive();
+        cluster_wait();
+    }
+    // where operands and expanded blocks are announced, and accumulators given back: the issuing block
+    const uint32_t full_at = DUO ? peer_smem(full0, 0) : full0, acc_empty_at = DUO ? peer_smem(acc_empty0, 0) : acc_empty0;
     const uint32_t at_base = tmem_base + (uint32_t)(nacc * accw);
     // The launch after this one may begin (its prologue, and weights that no launch writes) once every block of this one
     // holds its tensor memory: a later block must never take columns that an earlier launch still has to get.
@@ -397,20 +470,23 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
     }
 
     // ---- the finish of a tile, by the epilogue warps: columns [col0, col0 + ncols) of the accumulators at `acc_col` ----
-    const int q = warp & 3;
+    const int q = warp & 3, group = (warp - 2) >> 2 & 1;
     int n_slabs = 0;
     const bool inplace = epi == EPI_RESIDUAL || epi == EPI_SILU_GATE;
     constexpr int CH = 16;   // columns read at a time
-    auto prefetch_slab = [&](int tile, int col) {   // in-place epilogues: the values to be updated, into the staging buffer
-        const int rt = tile / ntok, tt = tile - rt * ntok, si = segment(rt);
+    const bool two_slabs = DUO && !PACKED && g.two_slabs;
+    const uint32_t stage_step = two_slabs ? (uint32_t)((slab + 15) / 16 * 16 * trows * 2) : 0u;
+    auto stage_of = [&](int n) { return out_stage + (uint32_t)(n & 1) * stage_step; };
+    auto prefetch_slab = [&](int tile, int col) {   // in-place epilogues: the values to be updated, into the next staging buffer
+        const int rt = row_tile(tile), tt = tile % ntok, si = segment(rt);
         if (warp == 2 && lane == 0) {
-            if (n_slabs > 0) bulk_wait_read0();
+            if (!two_slabs && n_slabs > 0) bulk_wait_read0();
             mbar_arrive_expect_tx(res_bar, (uint32_t)(slab * BM * 2));   // (SwiGLU is not in place: tiles of 128 rows here)
-            tma_load_2d(out_stage, &mp.out[si], (rt - seg_at(si).tile0) * BM, tt * bn + col, res_bar, l2_policy_evict_normal());
+            tma_load_2d(stage_of(n_slabs), &mp.out[si], (rt - seg_at(si).tile0) * BM, tt * bn + col, res_bar, l2_policy_evict_normal());
         }
     };
-    auto finish_tile = [&](int tile, uint32_t acc_col, int col0, int ncols, bool& failed, uint32_t release_bar) {
-        const int rt = tile / ntok, tt = tile - rt * ntok, si = segment(rt);
+    auto finish_tile = [&](int tile, uint32_t acc_col, int col0, int ncols, bool& failed, uint32_t ready_bar, uint32_t ready_ph, uint32_t release_bar) __attribute__((always_inline)) {
+        const int rt = row_tile(tile), tt = tile % ntok, si = segment(rt);
         const GemmSeg sg = seg_at(si);
         // row: this thread's accumulator lane; orow: the output column (within the tile) it finishes
         const int n0 = (rt - sg.tile0) * trows, row = q * 32 + lane, orow = pair ? row & 63 : row, n = n0 + orow, m0 = tt * bn;
@@ -419,11 +495,26 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         if (WFMT == FMT_INT8 && row_ok) rs = __half2float(__ushort_as_half((pair && row >= 64 ? g.scale2 : sg.scale)[n]));
         const bool biased = sg.bias != nullptr;
         if (biased && row_ok) bias = __half2float(__ushort_as_half(sg.bias[n]));
+        if (ready_bar) {   // (the scale and the bias are on their way by now)
+            if (!failed && !wait_asleep(ready_bar, ready_ph)) {
+                failed = true;
+                if (lane == 0) *reinterpret_cast<volatile int*>(status) = 5;
+            }
+            failed = epilogue_any<EPI_WARPS>(failed);   // (the warps meet at barriers below: all of them take the same way)
+            tc_fence_after();
+        }
         const uint32_t tm = tmem_base + acc_col + ((uint32_t)(q * 32) << 16);
-        // the sums of columns c .. c + CH - 1 (a split tile: all ranks' parts, in rank order), times the int8 row scale
-        auto sums = [&](int c, float (&v)[CH]) {
-            uint32_t r[CH];
-            tmem_ld16(tm + (uint32_t)c, r);
+        // the accumulator is free as soon as this warp's last columns have been read
+        bool released = release_bar == 0u;
+        auto release = [&]() {
+            released = true;
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) arrive_on<DUO>(release_bar);
+        };
+        // the sums of columns c .. c + CH - 1 (a split tile: all ranks' parts, in rank order), times the int8 row scale, from the
+        // accumulator's columns in r
+        auto sums = [&](int c, const uint32_t (&r)[CH], float (&v)[CH]) __attribute__((always_inline)) {
 #pragma unroll
             for (int j = 0; j < CH; ++j) v[j] = __uint_as_float(r[j]);
             if (S > 1) {
@@ -455,9 +546,9 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         // SwiGLU: the gate row's thread finishes the first half of the columns, the up row's thread the second; each hands the
         // other its values of the other half through shared memory (two buffers in turn, so one barrier per CH columns).
         int swaps = 0;
-        auto swap_halves = [&](float (&v)[CH]) {
+        auto swap_halves = [&](float (&v)[CH]) __attribute__((always_inline)) {
             const int up = row >> 6;
-            const uint32_t buf = swap_base + (uint32_t)((swaps++ & 1) * 4096), at = buf + (uint32_t)(orow * 16);
+            const uint32_t buf = swap_base + (uint32_t)(group * SWAP_BYTES + (swaps++ & 1) * 4096), at = buf + (uint32_t)(orow * 16);
             const uint32_t mine = at + (uint32_t)(up * 2048), theirs = at + (uint32_t)((up ^ 1) * 2048);
 #pragma unroll
             for (int j = 0; j < CH / 2; j += 4) {
@@ -465,7 +556,7 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
                 const float c = up ? v[j + 2] : v[CH / 2 + j + 2], d = up ? v[j + 3] : v[CH / 2 + j + 3];
                 asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(mine + (uint32_t)(j / 4 * 1024)), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
             }
-            asm volatile("bar.sync 3, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+            asm volatile("bar.sync %0, 128;" ::"r"(4 + group) : "memory");
 #pragma unroll
             for (int j = 0; j < CH / 2; j += 4) {
                 float o[4];
@@ -502,33 +593,45 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
             // row by row, and for the in-place forms in.)  Two columns of one token per 32-bit store: neighbouring lanes swap
             // halves, the even lane then holds token j of both columns and the odd lane token j + 1.
             const uint32_t pick = (lane & 1) ? 0x3276u : 0x5410u, pitch = (uint32_t)(trows * 2);
-            const uint32_t pair0 = out_stage + (uint32_t)((orow & ~1) * 2) + (lane & 1) * pitch, mine0 = out_stage + (uint32_t)(orow * 2);
+            // The next columns are on their way out of tensor memory while these are finished.
+            uint32_t r[CH];
+            constexpr bool AHEAD = WFMT != FMT_Q4;   // (Q4's epilogue has no registers left for it)
+            if (AHEAD && group * CH < slab) tmem_ld16_begin(tm + (uint32_t)(col0 + group * CH), r);
             for (int h0 = 0; h0 < ncols; h0 += slab) {
                 const int hrows = min(slab, ncols - h0);
                 if (!tma_store) {
                     asm volatile("bar.sync 2, %0;" ::"n"(EPI_WARPS * 32) : "memory");   // the previous slab has been copied out
                     if (inplace) {
-                        copy_rows<true>(sg.out, sg.ld, sg.N, n0, m0 + col0 + h0, min(hrows, gM - m0 - col0 - h0), trows, out_stage, tid - 64);
+                        copy_rows<true, EPI_WARPS>(sg.out, sg.ld, sg.N, n0, m0 + col0 + h0, min(hrows, gM - m0 - col0 - h0), trows, out_stage, tid - 64);
                         asm volatile("bar.sync 2, %0;" ::"n"(EPI_WARPS * 32) : "memory");
                     }
                 } else if (inplace) {
-                    if (h0 > 0) prefetch_slab(tile, col0 + h0);   // (the first slab of a tile was asked for at its start)
                     if (!mbar_wait_bounded_warp(res_bar, (uint32_t)(n_slabs & 1))) {
                         failed = true;
                         if (lane == 0) *reinterpret_cast<volatile int*>(status) = 9;
                     }
-                } else if (n_slabs > 0) {
+                } else if (!two_slabs && n_slabs > 0) {
                     // the previous slab's store must have finished reading the staging buffer
                     if (warp == 2 && lane == 0) bulk_wait_read0();
                     asm volatile("bar.sync 2, %0;" ::"n"(EPI_WARPS * 32) : "memory");
                 }
+                const uint32_t buf = tma_store ? stage_of(n_slabs) : out_stage;
+                const uint32_t pair0 = buf + (uint32_t)((orow & ~1) * 2) + (lane & 1) * pitch, mine0 = buf + (uint32_t)(orow * 2);
                 // (a slab's last columns may be fewer than CH: the buffer has room for the rest, which no store reads)
-                by_mode([&](auto mode) {
+                by_mode([&](auto mode) __attribute__((always_inline)) {
                     constexpr int MODE = decltype(mode)::value, NC = MODE == 4 ? CH / 2 : CH;
                     const int half = MODE == 4 && row >= 64 ? CH / 2 : 0;
-                    for (int c = 0; c < hrows; c += CH) {
+                    for (int c = group * CH; c < hrows; c += GROUPS * CH) {
                         float v[CH];
-                        sums(col0 + h0 + c, v);
+                        if (AHEAD) tmem_wait_ld(r);
+                        else tmem_ld16(tm + (uint32_t)(col0 + h0 + c), r);
+                        sums(col0 + h0 + c, r, v);
+                        const int after = c + GROUPS * CH < hrows ? h0 + c + GROUPS * CH : h0 + slab + group * CH;
+                        if (after >= ncols) {
+                            if (!released) release();
+                        } else if (AHEAD) {
+                            tmem_ld16_begin(tm + (uint32_t)(col0 + after), r);
+                        }
                         if (MODE == 4) swap_halves(v);
                         const uint32_t off = (uint32_t)(c + half) * pitch;
                         uint16_t old[CH];
@@ -538,31 +641,34 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
                                 asm volatile("ld.shared.u16 %0, [%1];" : "=h"(old[j]) : "r"(mine0 + off + (uint32_t)(j * (BM * 2))) : "memory");
                             __syncwarp();   // the neighbour writes where this lane has read
                         }
+                        // (all exchanges before the first store: one at a time, a value pair takes the latency of its exchange)
+                        uint32_t own[NC / 2], other[NC / 2];
 #pragma unroll
                         for (int j = 0; j < NC; j += 2) {
                             const __half2 h2 = __floats2half2_rn(value(mode, v[j], MODE == 2 || MODE == 3 ? old[j] : (uint16_t)0),
                                                                  value(mode, v[j + 1], MODE == 2 || MODE == 3 ? old[j + 1] : (uint16_t)0));
-                            const uint32_t h = *reinterpret_cast<const uint32_t*>(&h2), o = __shfl_xor_sync(0xffffffffu, h, 1);
-                            asm volatile("st.shared.u32 [%0], %1;" ::"r"(pair0 + off + (uint32_t)j * (MODE == 4 ? 128u : 256u)), "r"(__byte_perm(h, o, pick)) : "memory");
+                            own[j / 2] = *reinterpret_cast<const uint32_t*>(&h2);
                         }
+#pragma unroll
+                        for (int j = 0; j < NC / 2; ++j) other[j] = __shfl_xor_sync(0xffffffffu, own[j], 1);
+#pragma unroll
+                        for (int j = 0; j < NC; j += 2)
+                            asm volatile("st.shared.u32 [%0], %1;" ::"r"(pair0 + off + (uint32_t)j * (MODE == 4 ? 128u : 256u)), "r"(__byte_perm(own[j / 2], other[j / 2], pick)) : "memory");
                     }
                 });
-                if (h0 + slab >= ncols && release_bar) {
-                    // the accumulator is free as soon as its last columns have been read
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(release_bar);
-                }
                 fence_async_smem();
+                // two buffers: the store before this one has read its own, which past the barrier is the next slab's
+                if (two_slabs && warp == 2 && lane == 0) bulk_wait_read0();
                 asm volatile("bar.sync 2, %0;" ::"n"(EPI_WARPS * 32) : "memory");
                 const int rows_out = min(hrows, gM - m0 - col0 - h0);
                 if (!tma_store) {
-                    copy_rows<false>(sg.out, sg.ld, sg.N, n0, m0 + col0 + h0, rows_out, trows, out_stage, tid - 64);
-                    for (int p = 0; p < npeer; ++p) copy_rows<false>(g.peer_out[p], sg.ld, sg.N, n0, m0 + col0 + h0, rows_out, trows, out_stage, tid - 64);
+                    copy_rows<false, EPI_WARPS>(sg.out, sg.ld, sg.N, n0, m0 + col0 + h0, rows_out, trows, out_stage, tid - 64);
+                    for (int p = 0; p < npeer; ++p) copy_rows<false, EPI_WARPS>(g.peer_out[p], sg.ld, sg.N, n0, m0 + col0 + h0, rows_out, trows, out_stage, tid - 64);
                     continue;
                 }
-                if (warp == 2 && lane == 0) tma_store_2d(&mp.out[si], out_stage, n0, m0 + col0 + h0);
+                if (warp == 2 && lane == 0 && (!DUO || n0 < sg.N)) tma_store_2d(&mp.out[si], buf, n0, m0 + col0 + h0);
                 ++n_slabs;
+                if (inplace && h0 + slab < ncols) prefetch_slab(tile, col0 + h0 + slab);   // (the first slab of a tile was asked for at its start)
                 if (npeer > 0) {
                     // peers get the slab in 16-byte pieces, 256 contiguous bytes per token row (a plain store: tiles of 128 columns)
                     const int et = (warp - 2) * 32 + lane;
@@ -571,7 +677,7 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
                         if (n0 + ch * 8 >= sg.N) continue;
                         uint4 v;
                         asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                                     : "r"(out_stage + (uint32_t)(mr * (BM * 2) + ch * 16)) : "memory");
+                                     : "r"(buf + (uint32_t)(mr * (BM * 2) + ch * 16)) : "memory");
                         const size_t o = (size_t)(m0 + col0 + h0 + mr) * sg.ld + n0 + ch * 8;
 #pragma unroll
                         for (int p = 0; p < 7; ++p)
@@ -579,13 +685,8 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
                     }
                 }
             }
-            return;
         }
-        if (release_bar) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(release_bar);
-        }
+        if (!released) release();
     };
 
     bool failed = false;
@@ -599,14 +700,14 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         int ahead = 0;
         if (!PACKED && tile_first < tile_end && !wait_first) {
             // fp16 weights of the ring's first pass: they do not depend on the launch before this one
-            const int rt = tile_first / ntok, f = first_unit(rt), si = segment(rt), row0 = (rt - seg_at(si).tile0) * trows;
+            const int rt = row_tile(tile_first), f = first_unit(tile_first), si = segment(rt), row0 = (rt - seg_at(si).tile0) * trows;
             ahead = min(stages, nu);
             if (elect_one()) {
                 for (int j = 0; j < ahead; ++j) {
                     const int kb = u0 + (f + j < nu ? f + j : f + j - nu);
-                    mbar_arrive_expect_tx(full0 + j * 8, (uint32_t)stage_bytes);
-                    tma_load_2d(ring + j * stage_bytes, &mp.w[si], kb * BK, row0, full0 + j * 8, policy);
-                    if (pair) tma_load_2d(ring + j * stage_bytes + A_BYTES / 2, &mp.w[1], kb * BK, row0, full0 + j * 8, policy);
+                    if (half_rank == 0) mbar_arrive_expect_tx(full0 + j * 8, (uint32_t)(stage_bytes * (DUO ? 2 : 1)));   // both blocks' copies
+                    load_2d<DUO>(ring + j * stage_bytes, &mp.w[si], kb * BK, row0, full_at + j * 8, policy);
+                    if (pair) load_2d<DUO>(ring + j * stage_bytes + A_BYTES / 2, &mp.w[1], kb * BK, row0, full_at + j * 8, policy);
                 }
             }
             __syncwarp();
@@ -617,9 +718,9 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         int it = 0;
         bool ok = true;
         for (int tile = tile_first; tile < tile_end && ok; tile += tile_step) {
-            const int rt = tile / ntok, tt = tile - rt * ntok, si = segment(rt), row0 = (rt - seg_at(si).tile0) * trows;
+            const int rt = row_tile(tile), x0 = tile % ntok * bn + half_rank * xtok, si = segment(rt), row0 = (rt - seg_at(si).tile0) * trows;
             const CUtensorMap* const mw = &mp.w[si];
-            int u = first_unit(rt);
+            int u = first_unit(tile);
             for (int j = 0; j < nu && ok; ++j, u = (u + 1 == nu ? 0 : u + 1)) {
                 const int kb0 = (u0 + u) * SPAN, nb = min(SPAN, nkb - kb0);
                 for (int p = 0; p < nb; p += kps, ++it, r.next(stages)) {   // (kps divides SPAN: a stage never crosses a span)
@@ -629,18 +730,18 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
                         break;
                     }
                     if (elect_one()) {
-                        const uint32_t dst = ring + r.s * stage_bytes, bar = full0 + r.s * 8;
+                        const uint32_t dst = ring + r.s * stage_bytes, own = full0 + r.s * 8, bar = full_at + r.s * 8;
                         if (PACKED) {
                             const int n = min(kps, nb - p);
-                            mbar_arrive_expect_tx(bar, (uint32_t)(n * b_bytes));
-                            for (int i = 0; i < n; ++i) tma_load_2d(dst + i * b_bytes, &mp.x, (kb0 + p + i) * BK, tt * bn, bar, policy);
+                            if (half_rank == 0) mbar_arrive_expect_tx(own, (uint32_t)(n * b_bytes * (DUO ? 2 : 1)));
+                            for (int i = 0; i < n; ++i) load_2d<DUO>(dst + i * b_bytes, &mp.x, (kb0 + p + i) * BK, x0, bar, policy);
                         } else {
                             if (it >= ahead) {
-                                mbar_arrive_expect_tx(bar, (uint32_t)stage_bytes);
-                                tma_load_2d(dst, mw, kb0 * BK, row0, bar, policy);
-                                if (pair) tma_load_2d(dst + A_BYTES / 2, &mp.w[1], kb0 * BK, row0, bar, policy);
+                                if (half_rank == 0) mbar_arrive_expect_tx(own, (uint32_t)(stage_bytes * (DUO ? 2 : 1)));
+                                load_2d<DUO>(dst, mw, kb0 * BK, row0, bar, policy);
+                                if (pair) load_2d<DUO>(dst + A_BYTES / 2, &mp.w[1], kb0 * BK, row0, bar, policy);
                             }
-                            tma_load_2d(dst + b_off, &mp.x, kb0 * BK, tt * bn, bar, policy);
+                            load_2d<DUO>(dst + b_off, &mp.x, kb0 * BK, x0, bar, policy);
                         }
                     }
                     __syncwarp();
@@ -649,12 +750,12 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         }
     } else if (warp == 1) {
         // ---- MMA issuer ----
-        const uint32_t idesc = instr_desc_f16(bn);
+        const uint32_t idesc = instr_desc_f16(bn, DUO ? 2 * BM : BM);
         const uint32_t lo_step = (uint32_t)stage_bytes >> 4, lo0 = smem_desc_lo(ring), b_lo_off = (uint32_t)b_off >> 4, blk_step = (uint32_t)b_bytes >> 4;
         uint32_t lo = lo0, at = at_base;   // descriptor of the stage; this span's expanded blocks
         RingPos r;
         int tl = 0, nspan = 0;
-        bool ok = true;
+        bool ok = half_rank == 0;
         for (int tile = tile_first; tile < tile_end && ok; tile += tile_step, ++tl) {
             const int acc = nacc == 2 ? (tl & 1) : 0, pass = nacc == 2 ? tl >> 1 : tl;
             if (pass >= 1 && !wait_parked(acc_empty0 + acc * 8, (uint32_t)((pass - 1) & 1))) {
@@ -664,7 +765,7 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
             tc_fence_after();
             const uint32_t tmem_d = tmem_base + (uint32_t)(acc * accw);
             uint32_t accumulate = 0u;
-            int u = PACKED ? first_unit(tile / ntok) : 0;
+            int u = PACKED ? first_unit(tile) : 0;
             for (int j = 0; j < nu && ok; ++j) {
                 const int nb = PACKED ? min(SPAN, nkb - (u0 + u) * SPAN) : 1;
                 for (int p = 0; p < nb; p += kps) {
@@ -681,12 +782,12 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
 #pragma unroll
                             for (int k = 0; k < BK / 16; ++k) {
                                 const uint32_t acc_in = (k || i) ? 1u : accumulate;
-                                if (PACKED) umma_f16_ts(tmem_d, a_tm + (uint32_t)(k * 8), desc_of(b_lo + 2 * k), idesc, acc_in);
-                                else umma_f16(tmem_d, desc_of(lo + 2 * k), desc_of(b_lo + 2 * k), idesc, acc_in);
+                                if (PACKED) umma_f16_ts<DUO>(tmem_d, a_tm + (uint32_t)(k * 8), desc_of(b_lo + 2 * k), idesc, acc_in);
+                                else umma_f16<DUO>(tmem_d, desc_of(lo + 2 * k), desc_of(b_lo + 2 * k), idesc, acc_in);
                             }
                         }
-                        umma_commit(empty0 + r.s * 8);  // the operands are free once these MMAs have read them
-                        if (j + 1 == nu && p + kps >= nb) umma_commit(acc_full0 + acc * 8);  // this tile's accumulators are complete
+                        umma_commit<DUO>(empty0 + r.s * 8);  // the operands are free once these MMAs have read them
+                        if (j + 1 == nu && p + kps >= nb) umma_commit<DUO>(acc_full0 + acc * 8);  // this tile's accumulators are complete
                     }
                     __syncwarp();
                     accumulate = 1u;
@@ -713,9 +814,9 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         int it = 0;
         bool ok = true;
         for (int tile = tile_first; tile < tile_end && ok; tile += tile_step) {
-            const int rt = tile / ntok, si = segment(rt), n0 = (rt - seg_at(si).tile0) * trows;
+            const int rt = row_tile(tile), si = segment(rt), n0 = (rt - seg_at(si).tile0) * trows;
             const CUtensorMap *const mw = &mp.w[si], *const ms = &mp.sc[si];
-            int u = first_unit(rt);
+            int u = first_unit(tile);
             for (int j = 0; j < nu; ++j, ++it, r.next(raw_stages), u = (u + 1 == nu ? 0 : u + 1)) {
                 if (it >= raw_stages && !wait_parked(raw_empty0 + r.s * 8, r.ph ^ 1u)) {
                     if (lane == 0) *reinterpret_cast<volatile int*>(status) = 11;
@@ -762,7 +863,8 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         constexpr int NP = WFMT == FMT_INT8 ? 4 : 2;   // 16-byte pieces of a row per K block
         const int kps_log = kps == 4 ? 2 : kps - 1, sub = grp >> kps_log;
         // A store to tensor memory takes some 500 clocks to complete.  With two buffers per group the arrival for a block is
-        // left until the next block's codes are converted (or no next span is there yet), so that nobody waits for it.
+        // left until the next block's codes are converted, or until this group would have to wait (for the next span, or for the
+        // MMAs that free its buffer: left pending through that wait the arrival would hold up the MMAs of its own span as well).
         const bool defer = lag >= 2;
         uint32_t at = at_base + (uint32_t)(grp * 32) + lane_off, at_end = at + (uint32_t)(lag * SPAN * 32);
         const uint32_t at_first = at;
@@ -770,11 +872,11 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(pending);
+            if (lane == 0) arrive_on<DUO>(pending);
             pending = 0;
         };
         for (int tile = tile_first; tile < tile_end && ok; tile += tile_step) {
-            int u = first_unit(tile / ntok);
+            int u = first_unit(tile);
             for (int j = 0; j < nu; ++j) {
                 const uint32_t rbar = raw_full0 + r.s * 8;
                 const int kb0 = (u0 + u) * SPAN, nb = min(SPAN, nkb - kb0), nsub = (nb + kps - 1) >> kps_log;
@@ -782,8 +884,9 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
                 RingPos mine = t;
                 mine.advance(min(sub, nsub - 1), stages);
                 t.advance(nsub, stages);
-                if (pending && !__all_sync(0xffffffffu, mbar_try_wait(rbar, r.ph) != 0)) flush();
                 const RingPos free_at = lag == 4 ? old[3] : lag == 2 ? old[1] : old[0];
+                if (pending && !__all_sync(0xffffffffu, mbar_test_wait(rbar, r.ph) != 0 && (n < lag || mbar_test_wait(empty0 + free_at.s * 8, free_at.ph) != 0)))
+                    flush();
                 if (!wait_parked(rbar, r.ph) || (n >= lag && !wait_parked(empty0 + free_at.s * 8, free_at.ph))) {
                     if (lane == 0) *reinterpret_cast<volatile int*>(status) = 10;
                     ok = false;
@@ -799,7 +902,7 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
                                      : "=r"(c[i][0]), "=r"(c[i][1]), "=r"(c[i][2]), "=r"(c[i][3])
                                      : "r"(span + rbase + (((uint32_t)(grp * (8 / SPAN) + i) ^ x7) << 4)));
                     if (scale_tma) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sc) : "r"(span + RAW_BYTES + row * 16 + grp * 4));
-                    else if (WFMT == FMT_Q4) sc = load_scales(tile / ntok, kb0 + grp);
+                    else if (WFMT == FMT_Q4) sc = load_scales(row_tile(tile), kb0 + grp);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         uint32_t o[16];
@@ -814,11 +917,11 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
                         if (h == 0 && pending) flush();
                         tmem_st16(at + (uint32_t)(h * 16), o);
                     }
-                    pending = full0 + mine.s * 8;
+                    pending = full_at + mine.s * 8;
                     if (!defer) flush();
                 } else {
                     if (pending) flush();
-                    if (sub < nsub && lane == 0) mbar_arrive(full0 + mine.s * 8);
+                    if (sub < nsub && lane == 0) arrive_on<DUO>(full_at + mine.s * 8);
                 }
                 if ((at += SPAN * 32) == at_end) at = at_first;
                 old[3] = old[2];
@@ -840,13 +943,16 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         for (int tile = tile_first; tile < tile_end; tile += tile_step, ++tl) {
             const int acc = nacc == 2 ? (tl & 1) : 0, pass = nacc == 2 ? tl >> 1 : tl;
             if (inplace && tma_store && rank < fin) prefetch_slab(tile, rank * cps);
-            if (!failed && !wait_asleep(acc_full0 + acc * 8, (uint32_t)(pass & 1))) {
-                failed = true;
-                if (lane == 0) *reinterpret_cast<volatile int*>(status) = 5;
+            if (S > 1) {
+                if (!wait_asleep(acc_full0, 0u)) {
+                    failed = true;
+                    if (lane == 0) *reinterpret_cast<volatile int*>(status) = 5;
+                }
+                failed = epilogue_any<EPI_WARPS>(failed);
+                tc_fence_after();
+            } else {
+                finish_tile(tile, (uint32_t)(acc * accw), 0, bn, failed, acc_full0 + acc * 8, (uint32_t)(pass & 1), acc_empty_at + acc * 8);
             }
-            failed = epilogue_any(failed);   // (the warps meet at barriers below: all of them take the same way)
-            tc_fence_after();
-            if (S == 1) finish_tile(tile, (uint32_t)(acc * accw), 0, bn, failed, acc_empty0 + acc * 8);
         }
     }
     if (S > 1) {
@@ -861,7 +967,7 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
             const uint32_t tm = tmem_base + ((uint32_t)(q * 32) << 16), part = (uint32_t)(cps * BM * 4);
             for (int d = 0; d < fin; ++d) {
                 if (d == rank) continue;
-                for (int c = 0; c < cps; c += CH) {
+                for (int c = group * CH; c < cps; c += GROUPS * CH) {
                     uint32_t r[CH];
                     tmem_ld16(tm + (uint32_t)(d * cps + c), r);
 #pragma unroll
@@ -885,8 +991,8 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
                     failed = true;
                     if (lane == 0) *reinterpret_cast<volatile int*>(status) = 12;
                 }
-                failed = epilogue_any(failed);
-                finish_tile(tile_first, 0u, rank * cps, cps, failed, 0u);
+                failed = epilogue_any<EPI_WARPS>(failed);
+                finish_tile(tile_first, 0u, rank * cps, cps, failed, 0u, 0u, 0u);
             }
         }
         __syncwarp();
@@ -900,43 +1006,54 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         __syncwarp();
         cluster_wait();
     }
+    if (DUO) {   // neither block goes while the other's MMAs, commits or arrivals may still reach it
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+    }
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, (uint32_t)g.tmem_cols);
+    if (warp == 1) tmem_dealloc<DUO>(tmem_base, (uint32_t)g.tmem_cols);
     if (tid == 0 && g.sig.world > 0) gather_signal_block_done(g.sig);
 }
 
 // ---- launch configuration ------------------------------------------------------------------
 struct GemmConfig {
     int bn, ntok, ksplit, fin;
-    int stages, raw_stages, kps, lag, accw, nacc, tmem_cols, slab;
+    int stages, raw_stages, kps, lag, accw, nacc, tmem_cols, slab, two_slabs;
     int swap_off, xchg_off;
     size_t smem;
-    bool ok;
+    bool duo, ok;
 };
 
 // Shared and tensor memory of one (bn, ksplit) choice.
-GemmConfig gemm_geometry(int fmt, int trows, int M, int K, int bn, int ksplit) {
+GemmConfig gemm_geometry(int fmt, int trows, int M, int K, int bn, int ksplit, bool duo) {
     GemmConfig c = {};
     const bool packed = fmt != FMT_FP16;
     c.bn = bn;
     c.ntok = (M + bn - 1) / bn;
     c.ksplit = ksplit;
+    c.duo = duo;
     c.fin = 1;
     for (int f = ksplit; f > 1; --f)
         if (bn % (16 * f) == 0) { c.fin = f; break; }
     c.accw = (bn + 31) / 32 * 32;
     const int cps = bn / c.fin;
+    // One slab of up to SLAB_MAX tokens, or two halves: a slab costs its fence, barrier and store (some 800 clocks) beside 300 per
+    // 16 tokens.  Two buffers, where the pace of the tensor core is otherwise the epilogue's and the ring can spare the second one.
     c.slab = cps <= SLAB_MAX ? cps : cps / 2;
+    c.two_slabs = duo && !packed ? 1 : 0;
+    if (ksplit > 1 && c.slab % 16 != 0) return c;   // (whole steps: the other blocks' parts end with the last token)
     // the output slab (the epilogue writes 16 tokens at a time), and what the SwiGLU epilogue swaps through
-    const int slab_only = (c.slab + 15) / 16 * 16 * trows * 2, slab_bytes = slab_only + (trows < BM ? SWAP_BYTES : 0);
-    const int b_bytes = bn * BK * 2;
+    const int slab_only = (1 + c.two_slabs) * ((c.slab + 15) / 16 * 16) * trows * 2, slab_bytes = slab_only + (trows < BM ? epi_warps(fmt) / 4 * SWAP_BYTES : 0);
+    const int b_bytes = (duo ? bn / 2 : bn) * BK * 2;
     const int span = span_blocks(fmt), nkb = (K + BK - 1) / BK, units = (nkb + span - 1) / span, my_units = (units + ksplit - 1) / ksplit;
     const int room = SMEM_LIMIT - HDR - 1024 - slab_bytes;
     int stage_bytes = b_bytes + A_BYTES;
     c.kps = 1;
     if (packed) {
         // The packed spans cover the HBM latency (half of the room, as far as that is of use), the token stages that of L2.
-        // As many K blocks per token stage as leave at least three stages (and two spans in all).
+        // As many K blocks per token stage as leave at least three stages (and two spans in all).  Whole tiles of int8
+        // have the tokens of four spans: the MMAs of one, the expansion of the next and the barriers between them then overlap.
         const int rs = raw_stage_bytes(fmt);
         c.raw_stages = room / 2 / rs;
         if (c.raw_stages > RAW_MAX) c.raw_stages = RAW_MAX;
@@ -949,6 +1066,7 @@ GemmConfig gemm_geometry(int fmt, int trows, int M, int K, int bn, int ksplit) {
         stage_bytes = c.kps * b_bytes;
         // a wide token tile: fewer spans in flight, so that the tokens of two spans fit
         while (c.raw_stages > 2 && (room - c.raw_stages * rs) / stage_bytes * c.kps < 2 * span) --c.raw_stages;
+        while (ksplit == 1 && fmt == FMT_INT8 && c.raw_stages > 3 && (room - c.raw_stages * rs) / stage_bytes * c.kps < 4 * span) --c.raw_stages;
     }
     c.stages = (room - c.raw_stages * (packed ? raw_stage_bytes(fmt) : 0)) / stage_bytes;
     if (c.stages > RING_MAX) c.stages = RING_MAX;
@@ -959,8 +1077,8 @@ GemmConfig gemm_geometry(int fmt, int trows, int M, int K, int bn, int ksplit) {
     if (ksplit > 1) {
         // the parts to send lie in the ring, the parts to receive behind everything else
         const size_t send = (size_t)bn * BM * 4, recv = (size_t)(ksplit - 1) * cps * BM * 4;
-        const int least = packed ? (2 * span / c.kps > 2 ? 2 * span / c.kps : 2) : 2;
-        while (c.stages > least && HDR + 1024 + (size_t)c.stages * stage_bytes + raws + slab_bytes + recv > (size_t)SMEM_LIMIT) --c.stages;
+        const int least_stages = packed ? (2 * span / c.kps > 2 ? 2 * span / c.kps : 2) : 2;
+        while (c.stages > least_stages && HDR + 1024 + (size_t)c.stages * stage_bytes + raws + slab_bytes + recv > (size_t)SMEM_LIMIT) --c.stages;
         const size_t rings = (size_t)c.stages * stage_bytes + raws;
         c.xchg_off = (int)(rings + slab_bytes);
         c.smem = HDR + 1024 + rings + slab_bytes + recv;
@@ -1003,7 +1121,7 @@ int max_clusters(int size, int sms) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, linear_gemm_tc_kernel<FMT_FP16>, &cfg) != cudaSuccess || n < 1) {
+        if (cudaOccupancyMaxActiveClusters(&n, linear_gemm_tc_kernel<FMT_FP16, false>, &cfg) != cudaSuccess || n < 1) {
             cudaGetLastError();
             n = sms / (2 * size);
         }
@@ -1019,7 +1137,7 @@ int max_clusters(int size, int sms) {
 double gemm_cost(int fmt, const GemmConfig& c, int row_tiles, int K, int sms) {
     const int nkb = (K + BK - 1) / BK;
     const double blocks = (double)((nkb + c.ksplit - 1) / c.ksplit);
-    double per = (c.bn * 128.0 + (fmt == FMT_FP16 ? 16384.0 : fmt == FMT_INT8 ? 8192.0 : 4608.0)) / 58.0;
+    double per = ((c.duo ? c.bn / 2 : c.bn) * 128.0 + (fmt == FMT_FP16 ? 16384.0 : fmt == FMT_INT8 ? 8192.0 : 4608.0)) / 58.0;
     if (2.0 * c.bn > per) per = 2.0 * c.bn;
     const double least = fmt == FMT_FP16 ? 360.0 : c.lag >= 2 ? 420.0 : 700.0;
     if (per < least) per = least;
@@ -1028,11 +1146,11 @@ double gemm_cost(int fmt, const GemmConfig& c, int row_tiles, int K, int sms) {
     // (a launch of at most half the SMs starts on the ones that the launch before it leaves free)
     const double fixed = tiles * c.ksplit <= sms / 2 ? 4000.0 : 6500.0;
     if (c.ksplit > 1) return tiles > max_clusters(c.ksplit, sms) ? 1e30 : fixed + 3000.0 + 14.0 * c.bn + tile + epi;
-    const int waves = (tiles + sms - 1) / sms;
+    const int at_a_time = c.duo ? max_clusters(2, sms) : sms, waves = ((c.duo ? (row_tiles + 1) / 2 * c.ntok : tiles) + at_a_time - 1) / at_a_time;
     return fixed + (c.nacc == 2 ? waves * (tile > epi ? tile : epi) + epi : waves * (tile + epi));
 }
 
-GemmConfig gemm_choose(int fmt, int trows, int M, int row_tiles, int K, int sms, bool may_split) {
+GemmConfig gemm_choose(int fmt, int trows, int M, int row_tiles, int K, int sms, bool may_split, bool may_duo) {
     const int units = ((K + BK - 1) / BK + span_blocks(fmt) - 1) / span_blocks(fmt);
     GemmConfig best = {};
     double best_cost = 1e30;
@@ -1043,14 +1161,21 @@ GemmConfig gemm_choose(int fmt, int trows, int M, int row_tiles, int K, int sms,
             const int bn = ((M + ntok - 1) / ntok + 15) / 16 * 16;
             if (bn == last) continue;
             last = bn;
-            const GemmConfig c = gemm_geometry(fmt, trows, M, K, bn, ks);
-            if (!c.ok) continue;
-            const double cost = gemm_cost(fmt, c, row_tiles, K, sms);
-            if (cost < best_cost) {
-                best_cost = cost;
-                best = c;
+            // Two blocks on one 256-row tile (cta_group::2): each loads half of the tile's tokens, so a K block of 256 tokens is 32 KB
+            // per SM instead of 48 and the tensor core sets the pace instead of the copies: 2048 x 151936 x 896 in fp16 576 -> 500 us,
+            // 256 x 151936 x 896 in int8 101 -> 92.  Starting and ending in pairs costs some 3 us (the gate and up of a 512-token
+            // prompt, one wave of pairs: 14 -> 17 us), which long calls only, from four waves on, win back.
+            const bool long_call = (row_tiles + 1) / 2 * ntok >= 4 * max_clusters(2, sms);
+            for (int duo = 0; duo <= (may_duo && ks == 1 && bn % 32 == 0 && long_call ? 1 : 0); ++duo) {
+                const GemmConfig c = gemm_geometry(fmt, trows, M, K, bn, ks, duo != 0);
+                if (!c.ok) continue;
+                const double cost = gemm_cost(fmt, c, row_tiles, K, sms);
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    best = c;
+                }
             }
-            if (row_tiles * c.ntok > 4 * sms && best.ok) break;   // more tiles only re-read the weights
+            if (row_tiles * ntok > 4 * sms && best.ok) break;   // more tiles only re-read the weights
         }
     }
     return best;
@@ -1058,7 +1183,7 @@ GemmConfig gemm_choose(int fmt, int trows, int M, int row_tiles, int K, int sms,
 
 // The choice for a shape, kept (a choice is a function of its arguments alone): trying all tilings takes the host microseconds,
 // and a model asks for the same few shapes over and over.
-GemmConfig gemm_config(int fmt, int trows, int M, int row_tiles, int K, int sms, bool may_split) {
+GemmConfig gemm_config(int fmt, int trows, int M, int row_tiles, int K, int sms, bool may_split, bool may_duo) {
     struct Slot {
         int key[7];
         GemmConfig c;
@@ -1066,18 +1191,18 @@ GemmConfig gemm_config(int fmt, int trows, int M, int row_tiles, int K, int sms,
     constexpr int SLOTS = 256;
     static thread_local Slot* slots = nullptr;
     if (!slots) slots = new Slot[SLOTS]();
-    const int key[7] = {fmt + 1, trows, M, row_tiles, K, sms, may_split ? 1 : 0};
+    const int key[7] = {fmt + 1, trows, M, row_tiles, K, sms, (may_split ? 1 : 0) + (may_duo ? 2 : 0)};
     uint32_t h = 0;
     for (int v : key) h = (h ^ (uint32_t)v) * 0x9E3779B1u, h ^= h >> 15;
     Slot& s = slots[h % SLOTS];
     if (memcmp(s.key, key, sizeof(key)) != 0) {
-        s.c = gemm_choose(fmt, trows, M, row_tiles, K, sms, may_split);
+        s.c = gemm_choose(fmt, trows, M, row_tiles, K, sms, may_split, may_duo);
         memcpy(s.key, key, sizeof(key));
     }
     return s.c;
 }
 
-template <int WFMT>
+template <int WFMT, bool DUO>
 cudaError_t launch_one(const GemmMaps& mp, const GemmArgs& g, int grid, size_t smem, bool pdl, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
@@ -1089,19 +1214,19 @@ cudaError_t launch_one(const GemmMaps& mp, const GemmArgs& g, int grid, size_t s
     attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (g.ksplit > 1) {
+    if (DUO || g.ksplit > 1) {
         attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = (unsigned)g.ksplit;
+        attr[1].val.clusterDim.x = DUO ? 2u : (unsigned)g.ksplit;
         attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
         cfg.numAttrs = 2;
     }
-    return cudaLaunchKernelEx(&cfg, linear_gemm_tc_kernel<WFMT>, mp, g);
+    return cudaLaunchKernelEx(&cfg, linear_gemm_tc_kernel<WFMT, DUO>, mp, g);
 }
 
-cudaError_t launch_fmt(int fmt, const GemmMaps& mp, const GemmArgs& g, int grid, size_t smem, bool pdl, cudaStream_t st) {
-    if (fmt == FMT_FP16) return launch_one<FMT_FP16>(mp, g, grid, smem, pdl, st);
-    if (fmt == FMT_INT8) return launch_one<FMT_INT8>(mp, g, grid, smem, pdl, st);
-    return launch_one<FMT_Q4>(mp, g, grid, smem, pdl, st);
+cudaError_t launch_fmt(int fmt, bool duo, const GemmMaps& mp, const GemmArgs& g, int grid, size_t smem, bool pdl, cudaStream_t st) {
+    if (fmt == FMT_FP16) return duo ? launch_one<FMT_FP16, true>(mp, g, grid, smem, pdl, st) : launch_one<FMT_FP16, false>(mp, g, grid, smem, pdl, st);
+    if (fmt == FMT_INT8) return duo ? launch_one<FMT_INT8, true>(mp, g, grid, smem, pdl, st) : launch_one<FMT_INT8, false>(mp, g, grid, smem, pdl, st);
+    return duo ? launch_one<FMT_Q4, true>(mp, g, grid, smem, pdl, st) : launch_one<FMT_Q4, false>(mp, g, grid, smem, pdl, st);
 }
 
 }  // namespace
@@ -1109,7 +1234,8 @@ cudaError_t launch_fmt(int fmt, const GemmMaps& mp, const GemmArgs& g, int grid,
 cudaError_t gemm_tc_configure() {
     cudaError_t e = cudaSuccess;
 #define CFG(F) \
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_gemm_tc_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_gemm_tc_kernel<F, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT); \
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_gemm_tc_kernel<F, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
     CFG(FMT_FP16) CFG(FMT_INT8) CFG(FMT_Q4)
 #undef CFG
     return e;
@@ -1165,7 +1291,13 @@ cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool plain_form, bo
     g.tma_store = aligned ? 1 : 0;
     g.wait_first = wait_first ? 1 : 0;
     const bool may_split = a.npeer == 0 && a.sig.world == 0;
-    GemmConfig c = gemm_config(fmt, trows, M, rows, K, sms, may_split);
+    // The plain fused forms (q/k/v, SwiGLU) with few results go out as three launches side by side, which is what
+    // nn_launch_count reports for them and its tests state; that costs 4-5 us more than one launch does, so larger calls (from the
+    // results of 43 tiles of 128 x 64 on) and the forms with a norm or a bias, which a layer uses, are one.
+    long long results = 0;
+    for (int i = 0; i < a.nseg; ++i) results += (long long)M * a.seg[i].N;
+    const bool three = plain_form && (dual || a.nseg == 3) && rows >= 3 && results < 43ll * 128 * 64;
+    const GemmConfig c = gemm_config(fmt, trows, M, rows, K, sms, may_split, may_split && !three);
     if (!c.ok) return cudaErrorInvalidValue;
     g.bn = c.bn;
     g.ntok = c.ntok;
@@ -1179,6 +1311,7 @@ cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool plain_form, bo
     g.nacc = c.nacc;
     g.tmem_cols = c.tmem_cols;
     g.slab = c.slab;
+    g.two_slabs = c.two_slabs;
     g.swap_off = c.swap_off;
     g.xchg_off = c.xchg_off;
     size_t wbytes = 0;
@@ -1204,15 +1337,10 @@ cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool plain_form, bo
             if (!make_scale_map(&mp.sc[i], sbase[i], a.seg[i].N, pitch, 16, trows)) g.scale_tma = 0;
         if (dual && !make_scale_map(&mp.sc[1], sbase[3], a.seg[0].N, pitch, 16, trows)) g.scale_tma = 0;
     }
-    if (!encode_tiled_2d(&mp.x, true, a.x, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, (uint32_t)c.bn)) return cudaErrorInvalidValue;
-    // The plain fused forms (q/k/v, SwiGLU) with few results go out as three launches side by side, which is what
-    // nn_launch_count reports for them and its tests state; that costs 4-5 us more than one launch does, so larger calls (from the
-    // results of 43 tiles of 128 x 64 on) and the forms with a norm or a bias, which a layer uses, are one.
-    const int tiles = rows * c.ntok;
-    long long results = 0;
-    for (int i = 0; i < a.nseg; ++i) results += (long long)M * a.seg[i].N;
+    if (!encode_tiled_2d(&mp.x, true, a.x, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, (uint32_t)(c.duo ? c.bn / 2 : c.bn))) return cudaErrorInvalidValue;
+    const int tiles = (c.duo ? (rows + 1) / 2 : rows) * c.ntok;
     int cut[4] = {0, tiles, tiles, tiles}, parts = 1;
-    if (plain_form && (dual || a.nseg == 3) && rows >= 3 && results < 43ll * 128 * 64) {
+    if (three) {
         parts = 3;
         for (int i = 1; i < 3; ++i) cut[i] = (dual ? i * rows / 3 : g.seg[i].tile0) * c.ntok;
         cut[3] = tiles;
@@ -1222,8 +1350,10 @@ cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool plain_form, bo
         g.tile_end = cut[i + 1];
         g.chain = parts == 1 ? 0 : i == 0 ? 1 : 2;
         int grid = (g.tile_end - g.tile_begin) * c.ksplit;
-        if (c.ksplit == 1 && grid > sms) grid = sms;   // persistent: one block per SM walks the tiles
-        cudaError_t e = launch_fmt(fmt, mp, g, grid, c.smem, pdl, st);
+        const int at_a_time = c.duo ? max_clusters(2, sms) : sms;
+        if (c.ksplit == 1 && grid > at_a_time) grid = at_a_time;   // persistent: one block (pair) per SM (pair) walks the tiles
+        if (c.duo) grid *= 2;
+        cudaError_t e = launch_fmt(fmt, c.duo, mp, g, grid, c.smem, pdl, st);
         if (e != cudaSuccess) return e;
         ++*launches;
     }

@@ -54,6 +54,27 @@ def test_tiles_and_epilogues(nnb, ctx, fmt, N, K, M):
 
 
 @pytest.mark.parametrize("fmt", ["fp16", "int8", "q4"])
+def test_pairs_of_blocks(nnb, ctx, fmt):
+    """Enough tiles for two blocks on each: an odd number of row tiles, remainders in rows, tokens and K."""
+    M, N, K = 1000, 128 * 146 + 8, 544
+    x, r = make_x(M, K, 61), make_x(M, N, 62)
+    (W, s), (W2, s2) = make_weight(fmt, N, K, 63), make_weight(fmt, N, K, 64)
+    q, q2 = nnb.QuantWeight(ctx, fmt, W, s), nnb.QuantWeight(ctx, fmt, W2, s2)
+    xb, ob = ctx.upload(x.view(np.uint16)), alloc_with_canary(ctx, M * N * 2)
+    y, y2 = _want(fmt, x, W, s), _want(fmt, x, W2, s2)
+    ctx.upload(r.view(np.uint16), ob)
+    ctx.linear_add(M, N, K, xb, q.buf, ob)
+    check_close(ctx.download(ob, (M, N), np.uint16).view(np.float16), r.astype(np.float64) + y, what=f"residual {fmt}")
+    ctx.fused_gate_up_silu(M, N, K, xb, q.buf, q2.buf, ob)
+    check_close(ctx.download(ob, (M, N), np.uint16).view(np.float16), _silu(y) * y2, what=f"swiglu {fmt}")
+    check_canary(ctx, ob, M * N * 2, fmt)
+    for w in (q, q2):
+        w.release()
+    for b in (xb, ob):
+        ctx.free(b)
+
+
+@pytest.mark.parametrize("fmt", ["fp16", "int8", "q4"])
 @pytest.mark.parametrize("M,Ns", [(33, (200, 72, 65)), (600, (896, 128, 128))])
 def test_three_weights_with_bias(nnb, ctx, fmt, M, Ns):
     """Three launches side by side, and (many results) one launch over all three weights."""
