@@ -127,7 +127,11 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     // Scalars used all over the kernel are read from the parameter block once.  The block's
     // address is taken (the tensor maps in it are handed to the TMA unit), so the compiler must
     // assume that any store may change it and would otherwise re-read a field after every store.
-    const int aM = ONE ? 1 : a.M, aK = a.K, a_epi = a.epi, a_nseg = a.nseg;
+    // Token halves (int8, 9..16 rows; see stream_plan): blocks 2 i and 2 i + 1 share the tiles of block i, eight rows each.
+    const bool halves = !ONE && !EXT && FMT == FMT_INT8 && NT == 1 && a.halves;
+    const int M_all = ONE ? 1 : a.M, m_first = halves ? (int)(blockIdx.x & 1u) * 8 : 0, gM = ONE ? 1 : halves ? 8 : M_all;   // gM: rows the layout has room for
+    const int bx = halves ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, gx = halves ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+    const int aM = ONE ? 1 : halves ? min(8, M_all - m_first) : M_all, aK = a.K, a_epi = a.epi, a_nseg = a.nseg;
     int* const a_status = a.status;
     const int seg1_tile0 = a.seg[1].tile0, seg2_tile0 = a.seg[2].tile0;
     const int stages = ka.stages, kcb = a.kcb;
@@ -135,7 +139,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     const int rowbytes = ka.rowbytes, nchunks = ka.nchunks;
     const bool a_norm = VAR >= 1 && a.norm_w != nullptr;
     const int xcols = VAR == 3 ? a.xcols : 0;
-    const Geo geo = make_geo(FMT, aM, aK, kcb, stages, NT, a_norm, xcols);
+    const Geo geo = make_geo(FMT, gM, aK, kcb, stages, NT, a_norm, xcols);
     const int warp_rows = DUAL ? 16 : WARP_ROWS;                       // rows of each weight per warp
     const int tile_rows = ksplit ? warp_rows : NCW * warp_rows;        // rows of each weight per block tile
     const int groups = ksplit ? (nchunks + NCW - 1) / NCW : nchunks;   // pipeline items per tile
@@ -148,7 +152,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     const uint32_t ring = (s_base + geo.off_ring + 1023u) & ~1023u;
 
     if (tid < 16) reinterpret_cast<uint32_t*>(smem)[tid] = 0u;
-    if (FMT == FMT_INT8 && !xcols && tid >= 32 && tid < 48) reinterpret_cast<uint32_t*>(xs + 3 * aM * geo.xstride)[tid - 32] = 0u;  // per-row max words
+    if (FMT == FMT_INT8 && !xcols && tid >= 32 && tid < 48) reinterpret_cast<uint32_t*>(xs + 3 * gM * geo.xstride)[tid - 32] = 0u;  // per-row max words
     const uint32_t xbar = s_base + geo.off_x - 8;  // batched calls: the staged activations have landed
     if (tid == 0) {
         for (int s = 0; s < stages; ++s) {
@@ -172,12 +176,12 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
         tile_first = (int)(i0 / groups);
         cg_first = (int)(i0 - (long long)tile_first * groups);
     } else {
-        const int my_tiles = (int)blockIdx.x < a.ntiles ? (a.ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+        const int my_tiles = bx < a.ntiles ? (a.ntiles - bx + gx - 1) / gx : 0;
         n_items = my_tiles * groups;
-        tile_first = (int)blockIdx.x;
+        tile_first = bx;
         cg_first = 0;
     }
-    const int tile_step = sk ? 1 : (int)gridDim.x;
+    const int tile_step = sk ? 1 : gx;
 
     auto tile_segment = [&](int tile) {
         int si = 0;
@@ -289,8 +293,11 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
                     __syncwarp();
                 }
                 const uint32_t dst = ring + stage * geo.stage_bytes + geo.off_sx, n = (uint32_t)cols(cg);
-                for (int r = lane; r < xrows; r += 32)
-                    bulk_g2s(dst + r * geo.xstride, a.staged + (size_t)r * ximg + (size_t)cg * xcols, n, full0 + stage * 8, l2_policy_evict_normal());
+                for (int r = lane; r < xrows; r += 32) {
+                    // (halves: rows m_first .. of every plane)
+                    const int l = halves ? r / aM : 0, to = halves ? l * gM + r - l * aM : r, from = halves ? l * M_all + m_first + r - l * aM : r;
+                    bulk_g2s(dst + to * geo.xstride, a.staged + (size_t)from * ximg + (size_t)cg * xcols, n, full0 + stage * 8, l2_policy_evict_normal());
+                }
                 if (++cg == groups) { cg = 0; tile_s += tile_step; }
                 if (++stage == stages) stage = 0;
             }
@@ -312,8 +319,8 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     // ================= consumer warps =================
     const int g = lane >> 2, t = lane & 3;
     LaneGeo<NT> lg;
-    lane_geo_init<FMT, NT>(lg, DUAL, warp, lane, aM, smem_u32(xs), geo.xstride, zero_addr, smem + geo.off_ctab);
-    const float* rowscale = reinterpret_cast<const float*>(xs + (xcols ? 0 : 3 * aM * geo.xstride) + 64);
+    lane_geo_init<FMT, NT>(lg, DUAL, warp, lane, gM, smem_u32(xs), geo.xstride, zero_addr, smem + geo.off_ctab);
+    const float* rowscale = reinterpret_cast<const float*>(xs + (xcols ? 0 : 3 * gM * geo.xstride) + 64) + m_first;
 
     // rows of this warp inside its tile, and which warp writes results
     const int wrow_off = ksplit ? 0 : warp * warp_rows;
@@ -408,7 +415,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int n = row0 + 2 * f_pair + i, m = f_m0 + k * f_step;
-                p_res[k][i] = (n < sg.N && m < aM) ? sg.out[(size_t)m * sg.ld_out + n] : (uint16_t)0;
+                p_res[k][i] = (n < sg.N && m < aM) ? sg.out[(size_t)(m_first + m) * sg.ld_out + n] : (uint16_t)0;
             }
     };
 
@@ -426,11 +433,15 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
         // the launch before this one (stage_image_kernel) wrote the staged form of all M rows in this
         // kernel's shared-memory layout: one bulk copy instead of M rows converted by every block
         // (rows that travel with the weights: only the int8 row scales behind them)
-        const uint32_t skip = xcols ? (uint32_t)(3 * aM * x_stride_of(FMT, aK)) : 0u, bytes = xcols ? 192u : a.staged_bytes;
+        const uint32_t row = (uint32_t)x_stride_of(FMT, aK), skip = xcols || halves ? 3u * (uint32_t)M_all * row : 0u, bytes = xcols || halves ? 192u : a.staged_bytes;
         const bool some = !xcols || FMT == FMT_INT8;
         if (tid == 0 && some) {
-            mbar_arrive_expect_tx(xbar, bytes);
-            bulk_g2s(smem_u32(xs), a.staged + skip, bytes, xbar, l2_policy_evict_normal());
+            const bool planes = halves && !xcols;
+            mbar_arrive_expect_tx(xbar, bytes + (planes ? 3u * (uint32_t)aM * row : 0u));
+            if (planes)
+                for (int l = 0; l < 3; ++l)
+                    bulk_g2s(smem_u32(xs) + (uint32_t)(l * gM) * row, a.staged + (size_t)(l * M_all + m_first) * row, (uint32_t)aM * row, xbar, l2_policy_evict_normal());
+            bulk_g2s(smem_u32(xs) + (planes ? 3u * (uint32_t)gM * row : 0u), a.staged + skip, bytes, xbar, l2_policy_evict_normal());
         }
         if (some && !mbar_wait_bounded(xbar, 0u)) *reinterpret_cast<volatile int*>(a_status) = 5;
     } else {
@@ -494,7 +505,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 const int n = (lane & 7) + nt * 8;
-                if (n < aM) lg.b_base[nt] = sw + geo.off_sx + n * geo.xstride + (lane >> 3) * 16 - (uint32_t)(cg * xcols);
+                if (n < gM) lg.b_base[nt] = sw + geo.off_sx + n * geo.xstride + (lane >> 3) * 16 - (uint32_t)(cg * xcols);
             }
         }
         const int cb = (failed || !active) ? 0 : min(kcb, rowbytes - c * kcb);
@@ -663,8 +674,8 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
                         old[0] = p_res[1][0];
                         old[1] = p_res[1][1];
                         if (k > 1) {
-                            old[0] = seg_out[(size_t)m * seg_ld + n];
-                            old[1] = two ? seg_out[(size_t)m * seg_ld + n + 1] : (uint16_t)0;
+                            old[0] = seg_out[(size_t)(m_first + m) * seg_ld + n];
+                            old[1] = two ? seg_out[(size_t)(m_first + m) * seg_ld + n + 1] : (uint16_t)0;
                         }
                     }
                     uint16_t hv[2];
@@ -687,7 +698,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
                         }
                         hv[i] = __half_as_ushort(__float2half_rn(v));
                     }
-                    const size_t o = (size_t)m * seg_ld + n;
+                    const size_t o = (size_t)(m_first + m) * seg_ld + n;
                     auto put = [&](uint16_t* dst) {
                         if (two && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
                             *reinterpret_cast<uint32_t*>(dst) = (uint32_t)hv[0] | (uint32_t)hv[1] << 16;
@@ -1002,9 +1013,16 @@ bool stream_supported(int fmt, int M, int K, const LinArgs& a) {
 //   * the grid is sized so that every block gets the same number of tiles.
 StreamPlan stream_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit) {
     StreamPlan p = {};
-    const int M = a.M, K = a.K;
+    const int K = a.K;
     const bool dual = a.epi == EPI_SWIGLU, norm = a.norm_w != nullptr;
     const int rb = fmt_row_bytes(fmt, K);
+    // int8, 9..16 staged rows, an operator whose 32-row tiles take at most half the SMs: two blocks per tile, eight rows each.
+    // The integer MMAs set the pace (60 % of the SM's cycles on 896 x 4864, 28 blocks), and the weights come from L2 twice for
+    // little: that operator 19.0 -> 9.5 us, a 16-row step of a 24-layer, 896-wide model 999 -> 783 us.  Beyond half of the SMs the
+    // second block would only queue.
+    p.halves = fmt == FMT_INT8 && a.M > 8 && a.staged && !norm && a.npeer == 0 && a.sig.world == 0 && !a.argmax_slot && a.seg[0].out &&
+               count_tiles(a, dual ? 16 : WARP_ROWS) * 2 <= sm_count;
+    const int M = p.halves ? 8 : a.M;
     const int nt = M > 8 ? 2 : 1;
     const int rb_cols = ((rb + 127) / 128) * 128;
     const int warp_rows = dual ? 16 : WARP_ROWS;
@@ -1027,7 +1045,7 @@ StreamPlan stream_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limi
     // Rows too many or too long to be resident beside two stages (int8, 16 rows of 4864 values: 234 KB of limbs) travel with the
     // weights instead of being walked in slices that stream the weights again.
     int xcols = 0;
-    if (M > 1 && fmt != FMT_Q4 && !norm && a.npeer == 0 && a.sig.world == 0 && stage_image_bytes(fmt, M, K) <= STAGE_IMG_BYTES &&
+    if (M > 1 && fmt != FMT_Q4 && !norm && a.npeer == 0 && a.sig.world == 0 && stage_image_bytes(fmt, a.M, K) <= STAGE_IMG_BYTES &&
         (size_t)make_geo(fmt, M, K, kcb, 2, nt, norm, 0).total > smem_limit) {
         xcols = (kw == 1 ? 1 : NCW) * kcb;
         if ((size_t)make_geo(fmt, M, K, kcb, 2, nt, norm, xcols).total > smem_limit) xcols = 0;
@@ -1081,6 +1099,7 @@ StreamPlan stream_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limi
             p.grid = resident;
         }
     }
+    if (p.halves) p.grid *= 2;
     p.xcols = xcols;
     p.kcb = kcb;
     p.kw = kw;
@@ -1096,6 +1115,7 @@ cudaError_t launch_stream(int fmt, const LinArgs& a, const StreamPlan& p, cudaSt
     ka.a = a;
     ka.a.kcb = p.kcb;
     ka.a.xcols = p.xcols;
+    ka.a.halves = p.halves ? 1 : 0;
     ka.a.kw = p.kw;
     ka.a.ntiles = p.ntiles;
     ka.a.streamk = p.streamk ? 1 : 0;
@@ -1106,7 +1126,7 @@ cudaError_t launch_stream(int fmt, const LinArgs& a, const StreamPlan& p, cudaSt
     for (int i = 0; i < a.nseg; ++i) wbytes += (size_t)a.seg[i].N * ka.rowbytes;
     ka.evict_first = wbytes > ((size_t)96 << 20) ? 1 : 0;  // weights that cannot stay in L2 anyway are streamed evict-first
     const bool dual = a.epi == EPI_SWIGLU;
-    const int nt = a.M > 8 ? 2 : 1;
+    const int nt = a.M > 8 && !p.halves ? 2 : 1;
     const int warp_rows = dual ? 16 : WARP_ROWS;
     const int tile_rows = p.kw == 1 ? NCW * warp_rows : warp_rows;
     int t0 = 0;

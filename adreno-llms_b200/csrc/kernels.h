@@ -80,6 +80,7 @@ struct LinArgs {
     // stage_image_kernel in the kernel's own shared-memory layout; every block copies it in
     const uint8_t* staged;
     unsigned staged_bytes;
+    int halves;      // two blocks per tile, eight rows each (StreamPlan)
     int xcols;       // > 0: the staged rows travel with the weights, this many bytes of each per stage (StreamPlan)
     // host side only: Q4 scales with rows padded to a multiple of 16 bytes (seg[0..2], then the second weight of the
     // two-weight form), for the tensor copies when K / 16 is not such a multiple; all null otherwise
@@ -96,6 +97,7 @@ struct StreamPlan {  // launch geometry chosen on the host
     int kw;      // warps splitting K of one tile
     int warps;   // warps per block
     int stages;  // ring depth
+    bool halves; // 9..16 rows: two blocks per tile, eight rows each (grid counts both)
     int xcols;   // > 0: batched activations travel with the weights, this many bytes of every row per stage
     int ntiles;  // block tiles over all segments
     size_t smem;
