@@ -101,8 +101,6 @@ struct CState {            // consumer-side state carried from operator to opera
     unsigned st_epoch;
     int st_fmt;
     const void* st_norm;
-    const void* st_gamma;  // the norm weight held in shared memory
-    uint32_t st_xrow;      // shared-memory address of the staged activations
 };
 
 __device__ __noinline__ void report_failure(int* status, unsigned* state, int code) {
@@ -237,6 +235,231 @@ __device__ __forceinline__ uint16_t poll_row(const PlanParams& P, CState& S, con
     return (uint16_t)((n & 1) ? (w >> 16) : w);
 }
 
+// Whether a wait has lasted too long (recorded) or another block has given up.  Out of line: taken every 64th look.
+__device__ __noinline__ bool waited_too_long(const PlanParams& P, long long t0) {
+    if (clock64() - t0 > P.wait_cycles) {
+        report_failure(P.status, P.state, 4);
+        return true;
+    }
+    return ld_relaxed_u32(P.state + 2) != 0u;
+}
+
+// Eight values of the row as published: four words, each with its epoch.  Two 16-byte loads; every 8-byte word is looked at on
+// its own, so it does not matter that a 16-byte load is not one access.
+__device__ __forceinline__ bool fetch_piece(const unsigned long long* ll, int p, unsigned epoch, uint32_t (&w)[4]) {
+    unsigned e[4];
+    const unsigned long long* a = ll + (size_t)p * 4;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(e[0]), "=r"(w[1]), "=r"(e[1]) : "l"(a) : "memory");
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[2]), "=r"(e[2]), "=r"(w[3]), "=r"(e[3]) : "l"(a + 2) : "memory");
+    return e[0] == epoch && e[1] == epoch && e[2] == epoch && e[3] == epoch;
+}
+
+// The operator's activation row, from the other blocks' words (or memory) to its staged form, with the RMSNorm when asked: the
+// row stays in registers from the first look at the words to the staged stores, so that one barrier (fp16), two (int8: the
+// row's largest magnitude) or one more (the norm's sum of squares) are all that stands between the arrival of the last word and
+// the first matrix instruction.  Rows of up to PIECES pieces per thread (plan_stage_fast); longer ones take stage_general.
+//
+// This is the step's critical path, and it runs once per operator: what it costs is its instruction count, cold.  The version
+// that went through shared memory between fetch, norm, maximum and split (five barriers, 54 KB of code for one operator body)
+// took 2 700 of an operator's 7 000 clocks on the 135M shape (chained int8 step with its norms 413 -> 381 us; 500M fp16 532 -> 516).
+// The sums are taken in the order of rmsnorm_rows and stage_x (stream_core.cuh), for the same bits.
+constexpr int PIECES = PLAN_STAGE_PIECES;
+template <int FMT>
+__device__ __forceinline__ bool stage_fast(const PlanParams& P, const PlanOpScalars& D, uint8_t* smem, unsigned x_epoch, bool failed, int tid, int lane,
+                                           int warp) {
+    const int per = D.K / 8;
+    const bool norm = D.norm_w != nullptr;
+    const int nthr = norm ? NCW * 32 : PTHREADS;   // (the norm's sums are those of four warps)
+    uint8_t* xs = smem + P.off_xs;
+    float* red = reinterpret_cast<float*>(smem + P.off_red);
+    uint32_t w[PIECES][4], gm[PIECES][4];
+    unsigned pending = 0u;
+#pragma unroll
+    for (int j = 0; j < PIECES; ++j) {
+        const int p = tid + j * nthr;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[j][i] = gm[j][i] = 0u;
+        if (tid < nthr && p < per) {
+            pending |= 1u << j;
+            if (norm) {
+                const uint4 g = *reinterpret_cast<const uint4*>(D.norm_w + p * 8);
+                gm[j][0] = g.x; gm[j][1] = g.y; gm[j][2] = g.z; gm[j][3] = g.w;
+            }
+        }
+    }
+    const unsigned have = pending;
+    if (D.x_ll) {
+        long long t0 = 0;
+        unsigned looks = 0;
+        while (pending) {
+#pragma unroll
+            for (int j = 0; j < PIECES; ++j)
+                if ((pending >> j) & 1u) {
+                    if (fetch_piece(D.x_ll, tid + j * nthr, x_epoch, w[j])) pending &= ~(1u << j);
+                }
+            if (!pending || failed) break;   // after an earlier wait of this launch ran out: take what is there
+            if ((++looks & 63u) == 0u) {
+                if (looks == 64u) t0 = clock64();
+                else if (waited_too_long(P, t0)) failed = true;
+            }
+        }
+        failed = __any_sync(0xffffffffu, failed) != 0;
+    } else {
+#pragma unroll
+        for (int j = 0; j < PIECES; ++j)
+            if ((have >> j) & 1u) {
+                const uint4 v = *reinterpret_cast<const uint4*>(D.x + (tid + j * nthr) * 8);
+                w[j][0] = v.x; w[j][1] = v.y; w[j][2] = v.z; w[j][3] = v.w;
+            }
+    }
+    if (norm && warp < NCW) {
+        float ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < PIECES; ++j) {
+            if (!((have >> j) & 1u)) continue;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j][q]));
+                ss += f.x * f.x;
+                ss += f.y * f.y;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) red[warp] = ss;
+        asm volatile("bar.sync 2, %0;" ::"n"(NCW * 32) : "memory");
+        float tot = 0.f;
+#pragma unroll
+        for (int w2 = 0; w2 < NCW; ++w2) tot += red[w2];
+        const float inv = 1.0f / sqrtf(tot / (float)D.K + D.norm_eps);
+#pragma unroll
+        for (int j = 0; j < PIECES; ++j) {
+            if (!((have >> j) & 1u)) continue;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float2 fx = __half22float2(*reinterpret_cast<const __half2*>(&w[j][q])), fg = __half22float2(*reinterpret_cast<const __half2*>(&gm[j][q]));
+                const __half2 h = __floats2half2_rn((fx.x * inv) * fg.x, (fx.y * inv) * fg.y);
+                w[j][q] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+        }
+    }
+    if (FMT == FMT_INT8) {
+        // 24-bit fixed point in three 8-bit limbs, scaled by the row's largest magnitude (see stage_x_int8)
+        const int xstride = x_stride_of(FMT_INT8, D.K);
+        unsigned mx = 0u;
+#pragma unroll
+        for (int j = 0; j < PIECES; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) mx = max(mx, max(w[j][q] & 0x7FFFu, (w[j][q] >> 16) & 0x7FFFu));
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        unsigned* wmax = reinterpret_cast<unsigned*>(red) + 16;
+        if (lane == 0) wmax[warp] = mx;
+        consumers_sync();
+        const uint4 m0 = *reinterpret_cast<const uint4*>(wmax), m1 = *reinterpret_cast<const uint4*>(wmax + 4);
+        mx = max(max(max(m0.x, m0.y), max(m0.z, m0.w)), max(max(m1.x, m1.y), max(m1.z, m1.w)));
+        const bool bad = mx >= 0x7C00u;
+        const int e = (int)(mx >> 10) > 0 ? (int)(mx >> 10) - 15 : -14;
+        const int pw = (mx == 0u || bad) ? 0 : 22 - e;
+        const float up = __int_as_float((127 + pw) << 23);
+        if (tid == 0) *reinterpret_cast<float*>(xs + 3 * xstride + 64) = bad ? __int_as_float(0x7FC00000) : __int_as_float((127 - pw) << 23);
+#pragma unroll
+        for (int j = 0; j < PIECES; ++j) {
+            if (!((have >> j) & 1u)) continue;
+            uint32_t l[3][2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                int f[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t v = w[j][h * 2 + (i >> 1)];
+                    f[i] = bad ? 0 : __float2int_rn(__half2float(__ushort_as_half((uint16_t)(i & 1 ? v >> 16 : v & 0xFFFFu))) * up);
+                }
+                // bytes b of the four values side by side
+#pragma unroll
+                for (int b = 0; b < 3; ++b)
+                    l[b][h] = __byte_perm(__byte_perm((uint32_t)f[0], (uint32_t)f[1], (uint32_t)(b | ((b + 4) << 4))),
+                                          __byte_perm((uint32_t)f[2], (uint32_t)f[3], (uint32_t)(b | ((b + 4) << 4))), 0x5410u);
+            }
+            uint8_t* dst = xs + (tid + j * nthr) * 8;
+            *reinterpret_cast<uint2*>(dst) = make_uint2(l[2][0], l[2][1]);
+            *reinterpret_cast<uint2*>(dst + xstride) = make_uint2(l[1][0], l[1][1]);
+            *reinterpret_cast<uint2*>(dst + 2 * xstride) = make_uint2(l[0][0], l[0][1]);
+        }
+    } else {
+        uint8_t* row = FMT == FMT_FP16 ? xs : smem + P.off_xraw;
+#pragma unroll
+        for (int j = 0; j < PIECES; ++j)
+            if ((have >> j) & 1u) *reinterpret_cast<uint4*>(row + (tid + j * nthr) * 16) = make_uint4(w[j][0], w[j][1], w[j][2], w[j][3]);
+        if (FMT == FMT_Q4) {
+            // per 32 k, piece j holds the pairs (k 8t+j, k 8t+j+4), t = 0..3; the block's accumulator start goes to the table
+            consumers_sync();
+            float4* ctab = reinterpret_cast<float4*>(smem + P.off_ctab);
+#pragma unroll 1
+            for (int b = tid; b < D.K / 32; b += PTHREADS) {
+                uint32_t o[4][4];
+                float bsum = 0.f;
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(row + b * 64 + t * 16);
+                    const uint32_t vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&vv[q]));
+                        bsum += f.x;
+                        bsum += f.y;
+                    }
+                    o[0][t] = __byte_perm(v.x, v.z, 0x5410);
+                    o[1][t] = __byte_perm(v.x, v.z, 0x7632);
+                    o[2][t] = __byte_perm(v.y, v.w, 0x5410);
+                    o[3][t] = __byte_perm(v.y, v.w, 0x7632);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(xs + b * 64 + j * 16) = make_uint4(o[j][0], o[j][1], o[j][2], o[j][3]);
+                const float nc = -Q4_BIAS * bsum;
+                ctab[b] = make_float4(nc, 0.f, nc, 0.f);
+            }
+        }
+    }
+    consumers_sync();
+    return failed;
+}
+
+// The same for rows of any length: through shared memory, loop by loop.  Returns the failure flag.
+template <int FMT>
+__device__ __noinline__ bool stage_general(const PlanParams& P, const PlanOpScalars& D, uint8_t* smem, unsigned x_epoch, bool failed, int tid, int lane,
+                                           int warp) {
+    CState S;
+    S.failed = failed;
+    const int aK = D.K, xstride = x_stride_of(FMT, aK);
+    uint8_t* xs = smem + P.off_xs;
+    float* red = reinterpret_cast<float*>(smem + P.off_red);
+    const uint16_t* x_src = D.x;
+    uint16_t* gamma_s = reinterpret_cast<uint16_t*>(smem + P.off_gamma);
+    if (D.norm_w) {
+        for (int p = tid; p < aK / 8; p += PTHREADS) cp_async_16(smem_u32(gamma_s) + p * 16, D.norm_w + p * 8);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    if (D.x_ll) {
+        uint32_t* xraw = reinterpret_cast<uint32_t*>(smem + P.off_xraw);
+        poll_words(P, S, D.x_ll, (aK + 1) >> 1, x_epoch, xraw, tid);
+        S.failed = __any_sync(0xffffffffu, S.failed) != 0;  // (some lanes may have learnt of a failure, others not)
+        x_src = reinterpret_cast<const uint16_t*>(xraw);
+    }
+    if (FMT == FMT_INT8 && tid < 16) reinterpret_cast<uint32_t*>(xs + 3 * xstride)[tid] = 0u;  // the row-maximum words
+    if (D.norm_w) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    consumers_sync();
+    if (D.norm_w) {
+        uint16_t* xn = reinterpret_cast<uint16_t*>(smem + P.off_norm);
+        if (warp < NCW) rmsnorm_row_smem(x_src, gamma_s, D.norm_eps, aK, xn, red, tid, lane, warp);
+        consumers_sync();
+        x_src = xn;
+    }
+    if (FMT == FMT_INT8) stage_x_int8(x_src, 1, aK, xs, xstride, tid, PTHREADS);
+    else stage_x<FMT>(x_src, 1, aK, xs, xstride, reinterpret_cast<float*>(smem + P.off_ctab), tid, PTHREADS);
+    consumers_sync();
+    return S.failed;
+}
+
 // One operator on the consumer warps.  D lives in shared memory.
 // WIDE: the operator's tiles split K (few rows): eight K parts per tile, one per consumer warp
 // (stream_core.cuh: "K parts").  Otherwise the first NCW warps each stream whole rows of a tile,
@@ -302,12 +525,13 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
     unsigned long long am_best = 0ull;
     uint16_t sc1 = 0, res1 = 0;
     PlanSeg sg = D.seg[0];
-    int row0 = 0;
+    int row0 = 0, seg_i = 0;
     bool scales_ride = false;
     auto tile_prologue = [&](int tile, bool first) {
         sc1 = 0;
         res1 = 0;
-        sg = D.seg[DUAL ? 0 : tile_segment(tile)];
+        seg_i = DUAL ? 0 : tile_segment(tile);
+        sg = D.seg[seg_i];
         row0 = (tile - sg.tile0) * tile_rows + wrow_off;
         // int8 row scales: with the tile's last item when its rows allow a bulk copy, else from memory now
         scales_ride = FMT == FMT_INT8 && row_scales && plan_rows_bulk_ok(min(tile_rows, sg.N - (tile - sg.tile0) * tile_rows));
@@ -359,59 +583,19 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
     if (tile_first < ntiles) claim_item(off_first, slot_first);
 
     // ---------------- activations: fetch (poll the producer's words), normalise, stage ----------------
-    // fp16 weights multiply the activations as a plain fp16 row: when the row is in shared memory already
-    // (fetched from another operator, or normalised) it is used where it lies and nothing is staged.
-    constexpr bool plain = FMT == FMT_FP16;
-    constexpr int mode = FMT;
     const void* src_id = D.x_ll ? (const void*)D.x_ll : (const void*)D.x;
     const unsigned x_epoch = D.x_ll ? S.ebase + (unsigned)D.x_epoch : 0u;
-    const bool reuse = S.st_src == src_id && S.st_epoch == x_epoch && S.st_fmt == mode && S.st_norm == (const void*)D.norm_w;
-    // where the row will be read from is known before it arrives
-    const uint32_t x_addr = reuse ? S.st_xrow
-                                  : s_base + (uint32_t)(!plain ? P.off_xs : D.norm_w ? P.off_norm : D.x_ll ? P.off_xraw : P.off_xs);
+    const bool reuse = S.st_src == src_id && S.st_epoch == x_epoch && S.st_fmt == FMT && S.st_norm == (const void*)D.norm_w;
     LaneGeo<1> lg;
-    lane_geo_init<FMT, 1>(lg, DUAL, quarter, lane, 1, x_addr, xstride, s_base, smem + P.off_ctab);
+    lane_geo_init<FMT, 1>(lg, DUAL, quarter, lane, 1, s_base + (uint32_t)P.off_xs, xstride, s_base, smem + P.off_ctab);
     const float* rowscale = reinterpret_cast<const float*>(xs + 3 * xstride + 64);
     if (!reuse) {
-        const uint16_t* x_src = D.x;
-        // ... and the norm weight, which goes to shared memory
-        uint16_t* gamma_s = reinterpret_cast<uint16_t*>(smem + P.off_gamma);
-        const bool gamma_fresh = D.norm_w && S.st_gamma != (const void*)D.norm_w;
-        if (gamma_fresh) {
-            for (int p = tid; p < aK / 8; p += PTHREADS) cp_async_16(smem_u32(gamma_s) + p * 16, D.norm_w + p * 8);
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            S.st_gamma = (const void*)D.norm_w;
-        }
-        if (D.x_ll) {
-            uint32_t* xraw = reinterpret_cast<uint32_t*>(smem + P.off_xraw);
-            poll_words(P, S, D.x_ll, (aK + 1) >> 1, x_epoch, xraw, tid);
-            S.failed = __any_sync(0xffffffffu, S.failed) != 0;  // (some lanes may have learnt of a failure, others not)
-            x_src = reinterpret_cast<const uint16_t*>(xraw);
-        }
-        if (IMMA && tid < 16) reinterpret_cast<uint32_t*>(xs + 3 * xstride)[tid] = 0u;  // the row-maximum words
-        if (gamma_fresh) asm volatile("cp.async.wait_group 0;" ::: "memory");
-        // everyone is done with the previous staging and reduction buffers; the fetched row is complete
-        consumers_sync();
-        if (D.norm_w) {
-            uint16_t* xn = reinterpret_cast<uint16_t*>(smem + P.off_norm);
-            if (warp < NCW) rmsnorm_row_smem(x_src, gamma_s, D.norm_eps, aK, xn, red, tid, lane, warp);
-            consumers_sync();
-            x_src = xn;
-        }
-        if (plain) {
-            if (!D.x_ll && !D.norm_w) {  // a row in global memory: bring it in
-                stage_x<FMT_FP16>(x_src, 1, aK, xs, aK * 2 + 16, nullptr, tid, PTHREADS);
-                consumers_sync();
-            }
-        } else {
-            if (IMMA) stage_x_int8(x_src, 1, aK, xs, xstride, tid, PTHREADS);
-            else stage_x<FMT>(x_src, 1, aK, xs, xstride, reinterpret_cast<float*>(smem + P.off_ctab), tid, PTHREADS);
-            consumers_sync();
-        }
-        S.st_xrow = x_addr;
+        // (everyone is done with the previous staging and reduction buffers: the consumers met at this operator's start)
+        S.failed = plan_stage_fast(aK, D.norm_w != nullptr) ? stage_fast<FMT>(P, D, smem, x_epoch, S.failed, tid, lane, warp)
+                                                            : stage_general<FMT>(P, D, smem, x_epoch, S.failed, tid, lane, warp);
         S.st_src = src_id;
         S.st_epoch = x_epoch;
-        S.st_fmt = mode;
+        S.st_fmt = FMT;
         S.st_norm = (const void*)D.norm_w;
     }
 
@@ -437,6 +621,7 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
             if constexpr (FMT == FMT_FP16) {
                 if constexpr (WIDE) {
                     const int s0 = (c * kcb) / 64;
+#pragma unroll 1
                     for (int u = set; u < cb / 64; u += 2) step_fp16<1>(lg, sw, s0 + u, u, acc[0]);
                 } else {
                     chunk_fp16<1>(lg, sw, c, kcb, cb, acc);
@@ -444,6 +629,7 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
             } else if constexpr (FMT == FMT_INT8) {
                 if constexpr (WIDE) {
                     const int s0 = (c * kcb) / 64;
+#pragma unroll 1
                     for (int u = set; u < cb / 64; u += 2) step_int8<1>(lg, sw, s0 + u, u, iacc);
                 } else {
                     chunk_int8<1>(lg, sw, c, kcb, cb, iacc);
@@ -457,6 +643,7 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
                 const uint8_t* scb = smem + ring_off + off + nbox * CTA_BOX;
                 const uint8_t* const sc_rb[2] = {scb + (srow0 + g) * sstr, scb + (srow1 + g) * sstr};
                 if constexpr (WIDE) {
+#pragma unroll 1
                     for (int u = set; u < cb / 16; u += 2) block_q4_at<1>(lg, sw, c, kcb, u, acc[0], sc_rb, sstr);
                 } else {
                     chunk_q4<1>(lg, sw, c, kcb, cb, acc, sc_rb, sstr);
@@ -488,6 +675,11 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
                     }
                 }
                 consumers_sync();
+                tile += G;
+                if (warp != 0) {   // the first warp finishes the tile; the others go on to the block's next one
+                    if (tile < ntiles) tile_prologue(tile, false);
+                    continue;
+                }
                 auto quarter_sum = [&](int q, int r) {
                     const int* a = ibuf + (2 * q) * 3 * 32 + r;
                     const int* b2 = a + 3 * 32;
@@ -512,6 +704,11 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
                     mine[24] = acc[0][1][0][2];
                 }
                 consumers_sync();
+                tile += G;
+                if (warp != 0) {
+                    if (tile < ntiles) tile_prologue(tile, false);
+                    continue;
+                }
                 v0 = buf[r0] + buf[32 + r0];
 #pragma unroll
                 for (int q = 1; q < NCW; ++q) v0 += buf[(2 * q) * 32 + r0] + buf[(2 * q + 1) * 32 + r0];
@@ -552,7 +749,7 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
                 hv = finish_row<FMT>(v0, sc1, epi, res1);
                 if (bias_on) {
                     // the reference adds the bias to the stored fp16 result, in fp32, and rounds again
-                    const uint16_t* bp = P.bias[op * 3 + tile_segment(tile)];
+                    const uint16_t* bp = P.bias[op * 3 + seg_i];
                     if (bp) hv = __half_as_ushort(__float2half_rn(__fadd_rn(__half2float(__ushort_as_half(hv)), __half2float(__ushort_as_half(bp[n])))));
                 }
             }
@@ -570,7 +767,7 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
             const unsigned long long key = argmax_key_half(hv, D.argmax_base + n);
             am_best = key > am_best ? key : am_best;
         }
-        tile += G;
+        if (!WIDE) tile += G;
         if (tile < ntiles) tile_prologue(tile, false);
     }
 
@@ -775,8 +972,6 @@ __global__ void __launch_bounds__(PLAN_BLOCK, 1) decode_plan_kernel(const __grid
         S.st_epoch = 0u;
         S.st_fmt = -1;
         S.st_norm = nullptr;
-        S.st_gamma = nullptr;
-        S.st_xrow = 0u;
         *reinterpret_cast<CState*>(smem + PLAN_HDR_STATE) = S;
     }
 

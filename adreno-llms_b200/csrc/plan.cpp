@@ -241,7 +241,6 @@ cudaError_t build_run(const std::vector<RecordedOp>& rec, const std::vector<OpDe
             s.x = nullptr;
             s.x_ll = run->d_ll + ll_off[(size_t)d.x_dep * 3 + d.x_dep_seg];
             s.x_epoch = d.x_dep + 1;
-            if (a.K > k_ll) k_ll = a.K;
         } else {
             s.x = a.x;
         }
@@ -255,7 +254,10 @@ cudaError_t build_run(const std::vector<RecordedOp>& rec, const std::vector<OpDe
         }
         s.norm_w = a.norm_w;
         s.norm_eps = a.norm_eps;
-        if (a.norm_w && a.K > k_norm) k_norm = a.K;
+        // the row as it was fetched: Q4 permutes it from there; rows too long for registers pass through it
+        const bool fast = plan_stage_fast(a.K, a.norm_w != nullptr);
+        if ((r.fmt == FMT_Q4 || !fast) && a.K > k_ll) k_ll = a.K;
+        if (a.norm_w && !fast && a.K > k_norm) k_norm = a.K;
         s.argmax_slot = a.argmax_slot;
         s.argmax_done = a.argmax_done;
         s.argmax_out = a.argmax_out;

@@ -64,6 +64,11 @@ constexpr int PLAN_ROW_SCALE_BYTES = 1024;  // room for them at the end of an it
 // Bulk copies move multiples of 16 bytes: a tile's row scales travel with it when its valid rows are a multiple of 8.
 __host__ __device__ inline bool plan_rows_bulk_ok(int rows_valid) { return rows_valid > 0 && (rows_valid & 7) == 0; }
 
+// An activation row of at most this many 16-byte pieces per consumer thread (of all 256, or of the 128 that take a norm's sums) is
+// staged from registers; longer rows go through shared memory, which then holds the fetched row, the norm weight and the result.
+constexpr int PLAN_STAGE_PIECES = 3;
+__host__ __device__ inline bool plan_stage_fast(int K, bool norm) { return K / 8 <= PLAN_STAGE_PIECES * (norm ? 128 : 256); }
+
 constexpr int PLAN_SLOTS = 16;        // ring items in flight per block
 constexpr int PLAN_MAX_OPS = 1024;    // operators per run (their tile table sits in shared memory)
 // head of the kernel's shared memory: 64 bytes of zeros, full[] and empty[] barriers, the producer's
