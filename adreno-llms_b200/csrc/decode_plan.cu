@@ -244,14 +244,21 @@ __device__ __noinline__ bool waited_too_long(const PlanParams& P, long long t0) 
     return ld_relaxed_u32(P.state + 2) != 0u;
 }
 
-// Eight values of the row as published: four words, each with its epoch.  Two 16-byte loads; every 8-byte word is looked at on
-// its own, so it does not matter that a 16-byte load is not one access.
+// Eight values of the row as published: four words, each with its epoch.  Two 16-byte loads of two 64-bit elements: a vector
+// access is a set of accesses of its element type, and a word is value and epoch at once only if it is read as one element (its
+// writer stores it as one).  In what order the elements are read does not matter, since every word is looked at on its own.
 __device__ __forceinline__ bool fetch_piece(const unsigned long long* ll, int p, unsigned epoch, uint32_t (&w)[4]) {
-    unsigned e[4];
+    unsigned long long v[4];
     const unsigned long long* a = ll + (size_t)p * 4;
-    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(e[0]), "=r"(w[1]), "=r"(e[1]) : "l"(a) : "memory");
-    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[2]), "=r"(e[2]), "=r"(w[3]), "=r"(e[3]) : "l"(a + 2) : "memory");
-    return e[0] == epoch && e[1] == epoch && e[2] == epoch && e[3] == epoch;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v[0]), "=l"(v[1]) : "l"(a) : "memory");
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v[2]), "=l"(v[3]) : "l"(a + 2) : "memory");
+    bool all = true;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        w[i] = (uint32_t)v[i];
+        all = all && (unsigned)(v[i] >> 32) == epoch;
+    }
+    return all;
 }
 
 // The operator's activation row, from the other blocks' words (or memory) to its staged form, with the RMSNorm when asked: the

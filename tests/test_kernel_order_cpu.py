@@ -1,0 +1,35 @@
+"""Orderings inside the kernels that no run can show to be missing (a race that is nearly always won, a wait that is nearly always
+short), stated over the kernels' source."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "adreno-llms_b200", "csrc")
+
+
+def source(name):
+    """The file without its comments."""
+    with open(os.path.join(CSRC, name)) as f:
+        s = f.read()
+    return re.sub(r"//[^\n]*|/\*.*?\*/", "", s, flags=re.S)
+
+
+def block_after(s, start):
+    """From `start` (a text that occurs once, up to a body's opening brace or before it) to the end of that body."""
+    assert s.count(start) == 1, start
+    i = s.index("{", s.index(start))
+    depth = 0
+    for j in range(i, len(s)):
+        depth += {"{": 1, "}": -1}.get(s[j], 0)
+        if depth == 0:
+            return s[i:j + 1]
+    raise AssertionError(start)
+
+
+def test_published_words_are_read_whole():
+    """A published word is value and epoch in 64 bits, stored as one; a vector load reads it as one only with 64-bit elements."""
+    s = source("decode_plan.cu")
+    assert "st.relaxed.gpu.global.u64" in s
+    for body in ("bool fetch_piece(", "void poll_batch(", "uint16_t poll_row("):
+        loads = re.findall(r"ld\.[a-z0-9_.]+", block_after(s, body)) + re.findall(r"\bld_relaxed_u64\b", block_after(s, body))
+        assert loads, body
+        assert all(l.endswith("u64") for l in loads), (body, loads)
