@@ -639,6 +639,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
             //      896 x 896 projection of 16 rows took 7.5 us; and its stores were two bytes each. ----
             float* const buf = red + (ti & 1) * RED_WORDS;
             float* const mine = buf + warp * (8 * NT * RED_TS) + (2 * t) * RED_TS + g;
+            __syncwarp();   // (balanced launch with a K split: the lanes have read the other warps' parts, into which this layout reaches)
 #pragma unroll
             for (int rb = 0; rb < 2; ++rb)
 #pragma unroll

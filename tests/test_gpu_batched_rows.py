@@ -3,7 +3,8 @@ counts: every row carries the bits of the single-token call, whichever way it wa
 import numpy as np
 import pytest
 
-from helpers import alloc_with_canary, check_canary, make_weight, make_x
+from helpers import alloc_with_canary, check_canary, check_close, make_weight, make_x
+from oracle import cpu
 
 pytestmark = pytest.mark.gpu
 
@@ -38,4 +39,27 @@ def test_rows_of_a_batch_are_the_single_calls(nnb, ctx, fmt, N, K):
         check_canary(ctx, ob, 16 * N * 2, f"{fmt} {N}x{K} M={M}")
     qw.release()
     for b in (xb, ob, rb):
+        ctx.free(b)
+
+
+@pytest.mark.parametrize("M", [4, 9])
+def test_balanced_launch_with_split_k(nnb, ctx, M):
+    """Q4, long rows, 500 tiles of 32 rows dealt out as pipeline items: warp 0 adds the K parts of a tile and finishes it."""
+    N, K = 16000, 8192
+    W, s = make_weight("q4", 1000, K, 311)
+    qw = nnb.QuantWeight(ctx, "q4", np.tile(W, (16, 1)), np.tile(s, (16, 1)))
+    x, r = make_x(M, K, 312), make_x(M, N, 313)
+    xb, ob = ctx.upload(x.view(np.uint16)), alloc_with_canary(ctx, M * N * 2)
+    want = np.tile(x.astype(np.float64) @ cpu.dequant("q4", W, s).astype(np.float64).T, (1, 16))
+    seen = None
+    for rep in range(6):
+        ctx.upload(r.view(np.uint16), ob)
+        ctx.linear_add(M, N, K, xb, qw.buf, ob)
+        got = ctx.download(ob, (M, N), np.uint16)
+        check_close(got.view(np.float16), r.astype(np.float64) + want, what=f"q4 {N}x{K} M={M}")
+        assert seen is None or np.array_equal(got, seen)
+        seen = got
+    check_canary(ctx, ob, M * N * 2, f"q4 {N}x{K} M={M}")
+    qw.release()
+    for b in (xb, ob):
         ctx.free(b)

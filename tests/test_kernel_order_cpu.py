@@ -33,3 +33,12 @@ def test_published_words_are_read_whole():
         loads = re.findall(r"ld\.[a-z0-9_.]+", block_after(s, body)) + re.findall(r"\bld_relaxed_u64\b", block_after(s, body))
         assert loads, body
         assert all(l.endswith("u64") for l in loads), (body, loads)
+
+
+def test_batched_finish_waits_for_the_reads_of_its_buffer():
+    """Where one warp has added up the K parts, it writes its finish layout (8 * NT rows of RED_TS words) over the place of the
+    parts it has just read (32 * 8 * NT words each): the lanes meet in between."""
+    red_ts = int(re.search(r"constexpr int RED_TS = (\d+);", source("stream_core.cuh")).group(1))
+    assert 8 * red_ts > 32 * 8, "the layouts no longer overlap: the meeting is not needed for this"
+    _, finish = source("gemv_stream.cu").split("float* const mine = buf + warp * (8 * NT * RED_TS)")
+    assert "__syncwarp();" in finish[:finish.index("mine[")]
