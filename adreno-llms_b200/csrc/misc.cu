@@ -122,11 +122,10 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) rmsnorm_rows_kernel(const uin
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, r = blockIdx.x * NORM_WARPS + (threadIdx.x >> 5), pieces = cols / 8;
     const uint4* gw = reinterpret_cast<const uint4*>(w);
-    uint4 g0 = make_uint4(0, 0, 0, 0);
-    if (lane < pieces) g0 = gw[lane];   // the norm weight does not depend on the launch before
-    pdl_wait_prior_grid();
+    pdl_wait_prior_grid();   // the rows, and as far as is known the norm weight, may come from the launch before
     if (r >= rows) return;
     const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)r * cols);
+    const uint4 g0 = lane < pieces ? gw[lane] : make_uint4(0, 0, 0, 0);   // (asked for with the row)
     uint4* orow = reinterpret_cast<uint4*>(out + (size_t)r * cols);
     uint4 v[NORM_PIECES];
 #pragma unroll

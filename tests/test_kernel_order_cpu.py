@@ -42,3 +42,10 @@ def test_batched_finish_waits_for_the_reads_of_its_buffer():
     assert 8 * red_ts > 32 * 8, "the layouts no longer overlap: the meeting is not needed for this"
     _, finish = source("gemv_stream.cu").split("float* const mine = buf + warp * (8 * NT * RED_TS)")
     assert "__syncwarp();" in finish[:finish.index("mine[")]
+
+
+def test_norm_weight_is_read_after_the_launch_before():
+    """nn_rmsnorm takes any buffer as its weight, so also one that the call before has written."""
+    body = block_after(source("misc.cu"), "rmsnorm_rows_kernel(const uint16_t* __restrict__ x")
+    early = body[:body.index("pdl_wait_prior_grid()")]
+    assert not re.search(r"\b(gw|xr|orow)\[", early), early
