@@ -251,6 +251,7 @@ extern "C" void* nn_stream(nn_context* c) { return c ? (void*)c->stream : nullpt
 extern "C" int nn_sync(nn_context* c) {
     if (!c) return NN_FAIL(NN_ERR_ARG, "nn_sync: null context");
     CUDA_TRY(cudaStreamSynchronize(c->stream));
+    c->in_flight.ordered();
     if (*c->status_host != 0) {
         const int s = *c->status_host;
         *c->status_host = 0;
@@ -314,12 +315,14 @@ extern "C" int nn_buf_copy(nn_context* c, nn_buf dst, nn_buf src, size_t bytes) 
     if (!c || !dst || !src) return NN_FAIL(NN_ERR_ARG, "nn_buf_copy: null argument");
     if (!bytes) return NN_OK;
     CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, c->stream));
+    c->in_flight.ordered();
     return NN_OK;
 }
 extern "C" int nn_buf_fill(nn_context* c, nn_buf dst, int v, size_t bytes) {
     if (!c || !dst) return NN_FAIL(NN_ERR_ARG, "nn_buf_fill: null argument");
     if (!bytes) return NN_OK;
     CUDA_TRY(cudaMemsetAsync(dst, v, bytes, c->stream));
+    c->in_flight.ordered();
     return NN_OK;
 }
 extern "C" void* nn_host_alloc(size_t bytes) {
@@ -423,19 +426,30 @@ bool nnb::resolve_weight(const nn_context* c, const void* W, int K, ResolvedW* o
 // ---------------------------------------------------------------------------------
 // operator dispatch
 // ---------------------------------------------------------------------------------
+// Weights are fetched before a launch waits for the one before it: whether a launch that may still run could be writing one.
+static bool weights_in_flight(const nn_context* c, int fmt, const LinArgs& a) {
+    const size_t rb = fmt_rowbytes(fmt, a.K);
+    bool hit = false;
+    for (int i = 0; i < a.nseg; ++i) hit |= c->in_flight.may_write(a.seg[i].W, rb * (size_t)a.seg[i].N);
+    if (a.epi == EPI_SWIGLU) hit |= c->in_flight.may_write(a.W2, rb * (size_t)a.seg[0].N);
+    return hit;
+}
+static void note_outputs(nn_context* c, const LinArgs& a, int rows) {
+    for (int i = 0; i < a.nseg; ++i) c->in_flight.wrote(a.seg[i].out, (size_t)rows * a.seg[i].ld_out * 2);
+}
+
 // M > 16: the tensor-core GEMM, with whatever follows the product in its epilogue (quantised weights are expanded to fp16
 // inside the kernel).  Shapes it does not take are walked in slices of 16 rows by the streaming kernel.
 static int run_gemm_tc(nn_context* c, int fmt, const LinArgs& a, int M, bool plain_form, const char* who, bool* done) {
     *done = false;
     if (!gemm_tc_supported(fmt, a, M)) return NN_OK;
-    bool wait_first = false;
-    const size_t rb = fmt_rowbytes(fmt, a.K);
-    for (int i = 0; i < a.nseg; ++i) wait_first = wait_first || c->recently_written(a.seg[i].W, rb * (size_t)a.seg[i].N);
-    if (a.epi == EPI_SWIGLU) wait_first = wait_first || c->recently_written(a.W2, rb * (size_t)a.seg[0].N);
+    const bool overlap = !weights_in_flight(c, fmt, a);
     int n = 0;
-    cudaError_t e = launch_gemm_tc(fmt, a, M, plain_form, wait_first, c->use_pdl, c->stream, &n);
+    cudaError_t e = launch_gemm_tc(fmt, a, M, plain_form, c->use_pdl && overlap, c->stream, &n);
     c->launches += n;
     if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: tensor-core launch failed: %s (M=%d N=%d K=%d)", who, cudaGetErrorString(e), M, a.seg[0].N, a.K);
+    if (!overlap) c->in_flight.ordered();
+    note_outputs(c, a, M);
     *done = true;
     return NN_OK;
 }
@@ -465,7 +479,6 @@ static void note_recorded(nn_context* c, int fmt, const LinArgs& a, const Stream
 }
 
 static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char* who) {
-    for (int i = 0; i < a.nseg; ++i) c->note_output(a.seg[i].out, (size_t)M_total * a.seg[i].ld_out * 2);
     const bool plain_form = !a.norm_w && !a.seg[0].bias;
     a.sk_scratch = c->sk_scratch;
     a.sk_flags = c->sk_flags;
@@ -550,6 +563,8 @@ static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char
         if (!p.ok && stream_supported(fmt, a.M, a.K, a)) p = stream_plan(fmt, a, c->sm_count, c->smem_limit);
         if (p.ok) {
             e = launch_stream(fmt, b, p, c->stream, c->use_pdl);
+            if (e == cudaSuccess)
+                for (int i = 0; i < a.nseg; ++i) c->in_flight.wrote(out0[i], (size_t)M_total * a.seg[i].ld_out * 2);
             if (e == cudaSuccess && M_total == 1) note_recorded(c, fmt, a, p);
         } else {
             if (a.npeer > 0)
@@ -726,6 +741,7 @@ static int linear_qkv(nn_context* c, int M, int K, nn_buf x, nn_buf Wq, int Nq, 
         ba.nseg = 3;
         ProfScope prof(c, [&] { return std::string("bias_add_qkv_rows" + std::to_string(M)); });
         CUDA_TRY(launch_bias_add(ba, c->stream));
+        c->in_flight.ordered();
         c->launches++;
         return NN_OK;
     }
@@ -750,7 +766,7 @@ extern "C" int nn_bias_add(nn_context* c, int rows, int cols, nn_buf out, nn_buf
     a.nseg = 1;
     ProfScope prof(c, [&] { return std::string("bias_add_rows" + std::to_string(rows) + "_cols" + std::to_string(cols)); });
     CUDA_TRY(launch_bias_add(a, c->stream));
-    c->note_output(out, (size_t)rows * cols * 2);
+    c->in_flight.ordered();   // (neither this launch nor one behind it overlaps)
     c->launches++;
     return NN_OK;
 }
@@ -767,7 +783,7 @@ extern "C" int nn_rmsnorm(nn_context* c, int rows, int cols, nn_buf x, nn_buf we
     if (rows == 0) return NN_OK;
     ProfScope prof(c, [&] { return std::string("rmsnorm_rows" + std::to_string(rows) + "_cols" + std::to_string(cols)); });
     CUDA_TRY(launch_rmsnorm((const uint16_t*)x, (const uint16_t*)weight, (uint16_t*)out, rows, cols, eps, c->stream, c->use_pdl));
-    c->note_output(out, (size_t)rows * cols * 2);
+    c->in_flight.wrote(out, (size_t)rows * cols * 2);
     c->launches++;
     return NN_OK;
 }
@@ -853,6 +869,8 @@ int nnb::linear_argmax(nn_context* c, int N, int K, nn_buf x, nn_buf W, nn_buf l
     if (sig) a.sig = *sig;
     cudaError_t e = launch_stream(r.fmt, a, p, c->stream, c->use_pdl);
     if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: launch failed: %s (N=%d K=%d)", who, cudaGetErrorString(e), N, K);
+    note_outputs(c, a, 1);
+    c->in_flight.wrote(out_idx, 4);
     note_recorded(c, r.fmt, a, p);
     c->launches++;
     return NN_OK;
@@ -863,6 +881,7 @@ extern "C" int nn_argmax(nn_context* c, int n, nn_buf logits, nn_buf out_idx) {
     if (n < 0) return NN_FAIL(NN_ERR_ARG, "nn_argmax: n=%d", n);
     ProfScope prof(c, [&] { return std::string("argmax_n" + std::to_string(n)); });
     CUDA_TRY(launch_argmax_half((const uint16_t*)logits, n, (int*)out_idx, c->argmax_slot, reinterpret_cast<unsigned*>(c->argmax_slot + 3), c->stream, c->use_pdl));
+    c->in_flight.wrote(out_idx, 4);
     c->launches++;
     return NN_OK;
 }
@@ -889,6 +908,7 @@ extern "C" int nn_plan_begin(nn_context* c) {
     if (c->capturing) return NN_FAIL(NN_ERR_ARG, "nn_plan_begin: already recording");
     CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     c->capturing = true;
+    c->in_flight.ordered();   // a replay starts after everything before it
     c->rec.clear();
     c->launches_at_capture = c->launches;
     return NN_OK;
@@ -1033,6 +1053,7 @@ extern "C" int nn_plan_end(nn_context* c, nn_plan** out) {
     if (!c || !out) return NN_FAIL(NN_ERR_ARG, "nn_plan_end: null argument");
     if (!c->capturing) return NN_FAIL(NN_ERR_ARG, "nn_plan_end: not recording");
     c->capturing = false;
+    c->in_flight.wrote_unknown();   // what was in flight when the recording began, for the calls that follow it outside
     nn_plan* p = new nn_plan();
     p->device = c->device;
     cudaError_t e = cudaStreamEndCapture(c->stream, &p->graph);
@@ -1061,6 +1082,7 @@ extern "C" int nn_plan_launch(nn_context* c, nn_plan* p) {
     if (!c || !p || !p->exec) return NN_FAIL(NN_ERR_ARG, "nn_plan_launch: null argument");
     ProfScope prof(c, [&] { return std::string("plan_replay_" + std::to_string(p->recorded) + "ops_" + std::to_string(p->kernels) + "launches"); });
     CUDA_TRY(cudaGraphLaunch(p->exec, c->stream));
+    c->in_flight.wrote_unknown();
     c->launches += p->kernels;
     return NN_OK;
 }

@@ -105,7 +105,6 @@ struct GemmArgs {
     int swap_off;            // SwiGLU: the exchange buffers, from the ring's start
     int xchg_off;            // split tiles: where the other blocks' parts land, from the ring's start
     int epi, tma_store, evict_first;
-    int wait_first;          // the weights may be the output of a launch still in flight: nothing is fetched before the wait
     int chain;               // 0: waits for the launch before it; 1: first of several launches that run side by side; 2: a later one of them
     int* status;
     uint16_t* peer_out[7];   // the same output block in the other ranks' gather buffers
@@ -406,7 +405,7 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
     const int trows = g.rows;
     const int epi = g.epi, slab = g.slab, gM = g.M, npeer = g.npeer, tile_end = g.tile_end;
     const int lag = g.lag;   // packed weights: spans whose expanded blocks are in tensor memory at a time (1, 2 or 4)
-    const bool tma_store = g.tma_store != 0, wait_first = g.wait_first != 0;
+    const bool tma_store = g.tma_store != 0;
     int* const status = g.status;
     const int half_rank = DUO ? (int)(blockIdx.x & 1u) : 0;            // 0: the block that issues the MMAs of both
     const int xtok = DUO ? bn / 2 : bn;                                // tokens that this block loads
@@ -698,7 +697,7 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         // ---- TMA producer: walks (tile, K block) and keeps the ring full ----
         const uint64_t policy = l2_policy_evict_normal();
         int ahead = 0;
-        if (!PACKED && tile_first < tile_end && !wait_first) {
+        if (!PACKED && tile_first < tile_end) {
             // fp16 weights of the ring's first pass: they do not depend on the launch before this one
             const int rt = row_tile(tile_first), f = first_unit(tile_first), si = segment(rt), row0 = (rt - seg_at(si).tile0) * trows;
             ahead = min(stages, nu);
@@ -807,7 +806,6 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         }
     } else if (PACKED && warp == 2 + EPI_WARPS + DQ) {
         // ---- packed-weight producer: runs raw_stages spans ahead of the expanding warps ----
-        if (wait_first) pdl_wait_prior_grid();
         const bool scale_tma = WFMT == FMT_Q4 && g.scale_tma;
         const uint64_t policy = g.evict_first ? l2_policy_evict_first() : l2_policy_evict_normal();
         RingPos r;
@@ -1254,7 +1252,7 @@ bool gemm_tc_supported(int fmt, const LinArgs& a, int M) {
     return a.epi != EPI_SWIGLU || al16(a.W2);
 }
 
-cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool plain_form, bool wait_first, bool pdl, cudaStream_t st, int* launches) {
+cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool plain_form, bool overlap, cudaStream_t st, int* launches) {
     const bool dual = a.epi == EPI_SWIGLU;
     const int K = a.K, sms = current_sm_count();
     if (a.npeer < 0 || a.npeer > 7) return cudaErrorInvalidValue;
@@ -1289,7 +1287,6 @@ cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool plain_form, bo
     g.epi = a.epi;
     g.status = a.status;
     g.tma_store = aligned ? 1 : 0;
-    g.wait_first = wait_first ? 1 : 0;
     const bool may_split = a.npeer == 0 && a.sig.world == 0;
     // The plain fused forms (q/k/v, SwiGLU) with few results go out as three launches side by side, which is what
     // nn_launch_count reports for them and its tests state; that costs 4-5 us more than one launch does, so larger calls (from the
@@ -1353,7 +1350,7 @@ cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool plain_form, bo
         const int at_a_time = c.duo ? max_clusters(2, sms) : sms;
         if (c.ksplit == 1 && grid > at_a_time) grid = at_a_time;   // persistent: one block (pair) per SM (pair) walks the tiles
         if (c.duo) grid *= 2;
-        cudaError_t e = launch_fmt(fmt, c.duo, mp, g, grid, c.smem, pdl, st);
+        cudaError_t e = launch_fmt(fmt, c.duo, mp, g, grid, c.smem, overlap, st);
         if (e != cudaSuccess) return e;
         ++*launches;
     }

@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 
+#include "in_flight.h"
 #include "plan.h"
 
 struct QuantEntry {
@@ -54,20 +55,7 @@ struct nn_context {
     void* flush_buf = nullptr;
     size_t flush_bytes = 0;
     bool use_pdl = true;
-    // outputs of the last calls (address ranges, oldest overwritten): launches overlap, so a "weight" that is one of these
-    // may still be in the making
-    uintptr_t recent_lo[16] = {}, recent_hi[16] = {};
-    unsigned recent_n = 0;
-    void note_output(const void* p, size_t bytes) {
-        recent_lo[recent_n % 16] = (uintptr_t)p;
-        recent_hi[recent_n % 16] = (uintptr_t)p + bytes;
-        ++recent_n;
-    }
-    bool recently_written(const void* p, size_t bytes) const {
-        for (int i = 0; i < 16; ++i)
-            if ((uintptr_t)p < recent_hi[i] && recent_lo[i] < (uintptr_t)p + bytes) return true;
-        return false;
-    }
+    nnb::InFlight in_flight;       // outputs of the launches that the next one may overlap
     bool capturing = false;
     std::vector<nnb::RecordedOp> rec;  // streamed single-token operators of the recording in progress
     bool profiling = false;

@@ -49,3 +49,28 @@ def test_norm_weight(nnb, ctx):
     free()
     for b in (xb, g, out):
         ctx.free(b)
+
+
+@pytest.mark.parametrize("between", [0, 6])
+def test_gemm_weight(nnb, ctx, between):
+    """Keys projected from a prompt, any number of small calls, then scores against the keys."""
+    M, T, H = 48, 640, 512
+    call, want_k, free = _producers(nnb, ctx, T, H)
+    x = make_x(M, H, 91)
+    W, _ = make_weight("fp16", 64, H, 92)
+    q = nnb.QuantWeight(ctx, "fp16", W, None)
+    xb, keys, out = ctx.upload(x.view(np.uint16)), ctx.alloc(T * H * 2), ctx.alloc(M * T * 2)
+    small = [[ctx.alloc(M * 64 * 2) for _ in range(3)] for _ in range(between)]
+    for _ in range(4):
+        _poison(ctx, keys, T * H * 2)
+        call(keys)
+        for o in small:
+            ctx.linear_qkv(M, H, xb, q.buf, 64, q.buf, 64, q.buf, 64, *o)
+        ctx.linear(M, T, H, xb, keys, out)
+        k = _f16(ctx, keys, (T, H)).astype(np.float64)
+        check_close(k, want_k, what="projected keys")
+        check_close(_f16(ctx, out, (M, T)), x.astype(np.float64) @ k.T, what=f"scores, {between} calls between")
+    free()
+    q.release()
+    for b in [xb, keys, out] + sum(small, []):
+        ctx.free(b)
