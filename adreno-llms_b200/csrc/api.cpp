@@ -426,12 +426,16 @@ bool nnb::resolve_weight(const nn_context* c, const void* W, int K, ResolvedW* o
 // ---------------------------------------------------------------------------------
 // operator dispatch
 // ---------------------------------------------------------------------------------
-// Weights are fetched before a launch waits for the one before it: whether a launch that may still run could be writing one.
-static bool weights_in_flight(const nn_context* c, int fmt, const LinArgs& a) {
+// Weights (and by the streaming kernel biases) are fetched before a launch waits for the one before it: whether a launch that may
+// still run could be writing one.
+static bool read_ahead_in_flight(const InFlight& f, int fmt, const LinArgs& a) {
     const size_t rb = fmt_rowbytes(fmt, a.K);
     bool hit = false;
-    for (int i = 0; i < a.nseg; ++i) hit |= c->in_flight.may_write(a.seg[i].W, rb * (size_t)a.seg[i].N);
-    if (a.epi == EPI_SWIGLU) hit |= c->in_flight.may_write(a.W2, rb * (size_t)a.seg[0].N);
+    for (int i = 0; i < a.nseg; ++i) {
+        hit |= f.may_write(a.seg[i].W, rb * (size_t)a.seg[i].N);
+        if (a.seg[i].bias) hit |= f.may_write(a.seg[i].bias, (size_t)a.seg[i].N * 2);
+    }
+    if (a.epi == EPI_SWIGLU) hit |= f.may_write(a.W2, rb * (size_t)a.seg[0].N);
     return hit;
 }
 static void note_outputs(nn_context* c, const LinArgs& a, int rows) {
@@ -443,7 +447,7 @@ static void note_outputs(nn_context* c, const LinArgs& a, int rows) {
 static int run_gemm_tc(nn_context* c, int fmt, const LinArgs& a, int M, bool plain_form, const char* who, bool* done) {
     *done = false;
     if (!gemm_tc_supported(fmt, a, M)) return NN_OK;
-    const bool overlap = !weights_in_flight(c, fmt, a);
+    const bool overlap = !read_ahead_in_flight(c->in_flight, fmt, a);
     int n = 0;
     cudaError_t e = launch_gemm_tc(fmt, a, M, plain_form, c->use_pdl && overlap, c->stream, &n);
     c->launches += n;
@@ -456,7 +460,7 @@ static int run_gemm_tc(nn_context* c, int fmt, const LinArgs& a, int M, bool pla
 
 // While a step is being recorded, every launch of the streaming kernel is also noted with its
 // arguments and its graph node, so that nn_plan_end can hand runs of them to the resident kernel.
-static void note_recorded(nn_context* c, int fmt, const LinArgs& a, const StreamPlan& p) {
+static void note_recorded(nn_context* c, int fmt, const LinArgs& a, const StreamPlan& p, bool overlap) {
     if (!c->capturing) return;
     RecordedOp r;
     r.fmt = fmt;
@@ -474,7 +478,7 @@ static void note_recorded(nn_context* c, int fmt, const LinArgs& a, const Stream
         int pitch = 0;
         q4_ok = q4_scale_views(a, base, &pitch);
     }
-    r.eligible = r.node && a.M == 1 && !p.streamk && a.npeer == 0 && a.sig.world == 0 && q4_ok;
+    r.eligible = r.node && a.M == 1 && !p.streamk && a.npeer == 0 && a.sig.world == 0 && q4_ok && overlap;
     c->rec.push_back(r);
 }
 
@@ -533,6 +537,7 @@ static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char
             slice >>= 1;
         }
     }
+    const bool overlap = !read_ahead_in_flight(c->in_flight, fmt, a);
     for (int m0 = 0; m0 < M_total; m0 += slice) {
         a.sig = sig0;
         if (m0 + slice < M_total) a.sig.world = 0;  // the last slice sends the gather's signal
@@ -562,10 +567,11 @@ static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char
         }
         if (!p.ok && stream_supported(fmt, a.M, a.K, a)) p = stream_plan(fmt, a, c->sm_count, c->smem_limit);
         if (p.ok) {
-            e = launch_stream(fmt, b, p, c->stream, c->use_pdl);
+            e = launch_stream(fmt, b, p, c->stream, c->use_pdl && overlap);
+            if (e == cudaSuccess && !overlap) c->in_flight.ordered();
             if (e == cudaSuccess)
                 for (int i = 0; i < a.nseg; ++i) c->in_flight.wrote(out0[i], (size_t)M_total * a.seg[i].ld_out * 2);
-            if (e == cudaSuccess && M_total == 1) note_recorded(c, fmt, a, p);
+            if (e == cudaSuccess && M_total == 1) note_recorded(c, fmt, a, p, overlap);
         } else {
             if (a.npeer > 0)
                 return NN_FAIL(NN_ERR_UNSUPPORTED, "%s: this shape takes the any-shape kernel, which does not write to peer ranks (K=%d)", who, a.K);
@@ -867,11 +873,13 @@ int nnb::linear_argmax(nn_context* c, int N, int K, nn_buf x, nn_buf W, nn_buf l
     a.argmax_out = (int*)out_idx;
     a.argmax_base = row_base;
     if (sig) a.sig = *sig;
-    cudaError_t e = launch_stream(r.fmt, a, p, c->stream, c->use_pdl);
+    const bool overlap = !read_ahead_in_flight(c->in_flight, r.fmt, a);
+    cudaError_t e = launch_stream(r.fmt, a, p, c->stream, c->use_pdl && overlap);
     if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: launch failed: %s (N=%d K=%d)", who, cudaGetErrorString(e), N, K);
+    if (!overlap) c->in_flight.ordered();
     note_outputs(c, a, 1);
     c->in_flight.wrote(out_idx, 4);
-    note_recorded(c, r.fmt, a, p);
+    note_recorded(c, r.fmt, a, p, overlap);
     c->launches++;
     return NN_OK;
 }
@@ -909,6 +917,7 @@ extern "C" int nn_plan_begin(nn_context* c) {
     CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     c->capturing = true;
     c->in_flight.ordered();   // a replay starts after everything before it
+    c->in_flight.limit = (size_t)-1;
     c->rec.clear();
     c->launches_at_capture = c->launches;
     return NN_OK;
@@ -969,20 +978,15 @@ static cudaGraph_t consolidate_runs(nn_context* c, nn_plan* p, cudaGraph_t g) {
     }
     std::vector<HazardOp> hz(rec.size());
     for (size_t i = 0; i < rec.size(); ++i) hz[i] = hazard_view(rec[i]);
-    // bias rows are read like weights, with no ordering of their own: an operator whose bias any recorded operator writes
-    // keeps its own launch
+    // weights, biases and norm weights are read with no ordering of their own inside a run: an operator for which any recorded
+    // operator writes one keeps its own launch
+    InFlight written;
+    written.limit = (size_t)-1;
+    for (const HazardOp& h : hz)
+        for (int o = 0; o < h.nout; ++o) written.wrote((const void*)h.out[o], h.out_bytes[o]);
     std::vector<char> elig(rec.size());
-    for (size_t i = 0; i < rec.size(); ++i) {
-        elig[i] = rec[i].eligible ? 1 : 0;
-        for (int k = 0; k < rec[i].a.nseg && elig[i]; ++k) {
-            const uint16_t* bp = rec[i].a.seg[k].bias;
-            if (!bp) continue;
-            const uintptr_t b0 = (uintptr_t)bp, b1 = b0 + (size_t)rec[i].a.seg[k].N * 2;
-            for (size_t j = 0; j < rec.size() && elig[i]; ++j)
-                for (int o = 0; o < hz[j].nout; ++o)
-                    if (b0 < hz[j].out[o] + hz[j].out_bytes[o] && hz[j].out[o] < b1) elig[i] = 0;
-        }
-    }
+    for (size_t i = 0; i < rec.size(); ++i)
+        elig[i] = rec[i].eligible && !read_ahead_in_flight(written, rec[i].fmt, rec[i].a) && !written.may_write(rec[i].a.norm_w, (size_t)rec[i].a.K * 2);
     cudaGraph_t g2 = nullptr;
     if (cudaGraphClone(&g2, g) != cudaSuccess) return g;
     auto give_up = [&]() {
@@ -1053,6 +1057,7 @@ extern "C" int nn_plan_end(nn_context* c, nn_plan** out) {
     if (!c || !out) return NN_FAIL(NN_ERR_ARG, "nn_plan_end: null argument");
     if (!c->capturing) return NN_FAIL(NN_ERR_ARG, "nn_plan_end: not recording");
     c->capturing = false;
+    c->in_flight.limit = InFlight::MAX;
     c->in_flight.wrote_unknown();   // what was in flight when the recording began, for the calls that follow it outside
     nn_plan* p = new nn_plan();
     p->device = c->device;

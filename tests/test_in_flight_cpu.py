@@ -17,18 +17,18 @@ int main() {
     f.wrote(at(4096), 64);
     for (int rep = 0; rep < 50; ++rep)   // six q/k/v calls, then fifty: the first output stays known
         for (int i = 0; i < 20; ++i) f.wrote(at(1 << 20) + i * 4096, 4096);
-    CHECK(f.n == 21 && !f.more);
-    CHECK(f.may_write(at(4096), 64) && f.may_write(at(4096 + 63), 1) && f.may_write(at(0), 4097));
-    CHECK(!f.may_write(at(4096 + 64), 64) && !f.may_write(at(0), 4096));
+    CHECK(f.out.size() == 21 && !f.more);
+    CHECK(f.may_write(at(4096), 64) && f.may_write(at(4096 + 63), 1) && f.may_write(at(1), 4096));
+    CHECK(!f.may_write(at(4096 + 64), 64) && !f.may_write(at(1), 4095));
     f.wrote(at(4096 + 16), 16);          // inside a known one
     f.wrote(at(4000), 400);              // around it
-    CHECK(f.n == 21 && f.may_write(at(4000), 1) && f.may_write(at(4399), 1) && !f.may_write(at(4400), 1));
+    CHECK(f.out.size() == 21 && f.may_write(at(4000), 1) && f.may_write(at(4399), 1) && !f.may_write(at(4400), 1));
     f.wrote(nullptr, 64);
     f.wrote(at(64), 0);
-    CHECK(f.n == 21);
+    CHECK(f.out.size() == 21 && !f.may_write(nullptr, 64));
     f.ordered();
     CHECK(!f.may_write(at(4096), 64));
-    for (int i = 0; i < InFlight::MAX; ++i) f.wrote(at(4096) + i * 128, 64);
+    for (size_t i = 0; i < InFlight::MAX; ++i) f.wrote(at(4096) + i * 128, 64);
     CHECK(!f.more && !f.may_write(at(1 << 30), 64));
     f.wrote(at(1 << 20), 64);            // one more than fit: everything may be in flight
     CHECK(f.may_write(at(1 << 30), 64) && f.may_write(at(4096), 64));
@@ -36,6 +36,10 @@ int main() {
     CHECK(!f.may_write(at(1 << 30), 64));
     f.wrote_unknown();
     CHECK(f.may_write(at(1 << 30), 64));
+    f.ordered();
+    f.limit = (size_t)-1;                // a recording
+    for (size_t i = 0; i < 10 * InFlight::MAX; ++i) f.wrote(at(4096) + i * 128, 64);
+    CHECK(!f.more && f.may_write(at(4096), 64) && f.may_write(at(4096 + 639 * 128), 1) && !f.may_write(at(4096 + 64), 64));
     return 0;
 }
 """

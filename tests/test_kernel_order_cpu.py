@@ -49,3 +49,11 @@ def test_norm_weight_is_read_after_the_launch_before():
     body = block_after(source("misc.cu"), "rmsnorm_rows_kernel(const uint16_t* __restrict__ x")
     early = body[:body.index("pdl_wait_prior_grid()")]
     assert not re.search(r"\b(gw|xr|orow)\[", early), early
+
+
+def test_launches_that_read_ahead_ask_first():
+    """The streaming kernel and the GEMM fetch weights (and biases) before they wait for the launch before: each call site has asked
+    whether a launch in flight may be writing one."""
+    calls = re.findall(r"launch_(?:stream|gemm_tc)\(([^;]*)\);", source("api.cpp"))
+    assert len(calls) >= 3
+    assert all("c->use_pdl && overlap" in c for c in calls), calls
