@@ -444,16 +444,15 @@ static void note_outputs(nn_context* c, const LinArgs& a, int rows) {
 
 // M > 16: the tensor-core GEMM, with whatever follows the product in its epilogue (quantised weights are expanded to fp16
 // inside the kernel).  Shapes it does not take are walked in slices of 16 rows by the streaming kernel.
-static int run_gemm_tc(nn_context* c, int fmt, const LinArgs& a, int M, bool plain_form, const char* who, bool* done) {
+static int run_gemm_tc(nn_context* c, int fmt, const LinArgs& a, int M, const char* who, bool* done) {
     *done = false;
     if (!gemm_tc_supported(fmt, a, M)) return NN_OK;
     const bool overlap = !read_ahead_in_flight(c->in_flight, fmt, a);
-    int n = 0;
-    cudaError_t e = launch_gemm_tc(fmt, a, M, plain_form, c->use_pdl && overlap, c->stream, &n);
-    c->launches += n;
+    cudaError_t e = launch_gemm_tc(fmt, a, M, c->use_pdl && overlap, c->stream);
     if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: tensor-core launch failed: %s (M=%d N=%d K=%d)", who, cudaGetErrorString(e), M, a.seg[0].N, a.K);
     if (!overlap) c->in_flight.ordered();
     note_outputs(c, a, M);
+    c->launches++;
     *done = true;
     return NN_OK;
 }
@@ -483,7 +482,6 @@ static void note_recorded(nn_context* c, int fmt, const LinArgs& a, const Stream
 }
 
 static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char* who) {
-    const bool plain_form = !a.norm_w && !a.seg[0].bias;
     a.sk_scratch = c->sk_scratch;
     a.sk_flags = c->sk_flags;
     if (a.norm_w) {
@@ -516,7 +514,7 @@ static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char
     }
     if (M_total > 16) {
         bool done = false;
-        const int rc = run_gemm_tc(c, fmt, a, M_total, plain_form, who, &done);
+        const int rc = run_gemm_tc(c, fmt, a, M_total, who, &done);
         if (rc != NN_OK || done) return rc;
     }
     // M > 16 is walked in slices of 16 activation rows (each slice re-streams the weights).

@@ -94,7 +94,7 @@ struct GemmArgs {
     int nseg, M, K;
     int rows;                // output columns per tile: 128, SwiGLU 64
     int bn, ntok;            // tokens per tile, token tiles
-    int tile_begin, tile_end;  // this launch's tiles (row tile * ntok + token tile)
+    int tiles;               // row tile * ntok + token tile
     int ksplit, fin;         // blocks of a cluster that share a tile's K, and how many of them finish tokens
     int stages, raw_stages;
     int kps, lag;            // packed weights: K blocks per token stage; spans whose expanded blocks are in tensor memory at a time
@@ -105,7 +105,6 @@ struct GemmArgs {
     int swap_off;            // SwiGLU: the exchange buffers, from the ring's start
     int xchg_off;            // split tiles: where the other blocks' parts land, from the ring's start
     int epi, tma_store, evict_first;
-    int chain;               // 0: waits for the launch before it; 1: first of several launches that run side by side; 2: a later one of them
     int* status;
     uint16_t* peer_out[7];   // the same output block in the other ranks' gather buffers
     int npeer;
@@ -403,7 +402,7 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
     // have every later use read it again.
     const bool pair = g.epi == EPI_SWIGLU;   // a tile is 64 rows of each of two weights
     const int trows = g.rows;
-    const int epi = g.epi, slab = g.slab, gM = g.M, npeer = g.npeer, tile_end = g.tile_end;
+    const int epi = g.epi, slab = g.slab, gM = g.M, npeer = g.npeer, tile_end = g.tiles;
     const int lag = g.lag;   // packed weights: spans whose expanded blocks are in tensor memory at a time (1, 2 or 4)
     const bool tma_store = g.tma_store != 0;
     int* const status = g.status;
@@ -421,9 +420,9 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
     const int nkb = (g.K + BK - 1) / BK, nunits = (nkb + SPAN - 1) / SPAN;
     const int rank = S > 1 ? (int)(blockIdx.x % (unsigned)S) : 0;
     const int u0 = rank * nunits / S, nu = (rank + 1) * nunits / S - u0;
-    const int tile_first = g.tile_begin + (DUO ? (int)(blockIdx.x >> 1) : S > 1 ? (int)(blockIdx.x / (unsigned)S) : (int)blockIdx.x);
+    const int tile_first = DUO ? (int)(blockIdx.x >> 1) : S > 1 ? (int)(blockIdx.x / (unsigned)S) : (int)blockIdx.x;
     const int fin = g.fin, cps = bn / fin;                              // blocks of a cluster that finish tokens, and how many each
-    const int tile_step = DUO ? (int)(gridDim.x >> 1) : S > 1 ? g.tile_end : (int)gridDim.x;   // a split tile: one per cluster
+    const int tile_step = DUO ? (int)(gridDim.x >> 1) : S > 1 ? g.tiles : (int)gridDim.x;   // a split tile: one per cluster
     // DUO: a tile number stands for two row tiles.  The second one of the last pair may lie past the end: its copies bring zeros.
     auto row_tile = [&](int tile) { return DUO ? 2 * (tile / ntok) + half_rank : tile / ntok; };
     auto segment = [&](int rt) { return (g.nseg > 2 && rt >= g.seg[2].tile0) ? 2 : (g.nseg > 1 && rt >= g.seg[1].tile0) ? 1 : 0; };
@@ -462,7 +461,7 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
     const uint32_t at_base = tmem_base + (uint32_t)(nacc * accw);
     // The launch after this one may begin (its prologue, and weights that no launch writes) once every block of this one
     // holds its tensor memory: a later block must never take columns that an earlier launch still has to get.
-    if (g.chain != 1 && tid == 0) pdl_launch_dependents();
+    if (tid == 0) pdl_launch_dependents();
     if (S > 1) {   // the other blocks' memory may be written once they run: their arrivals are awaited before anything is sent
         __syncwarp();
         cluster_arrive();
@@ -711,8 +710,7 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
             }
             __syncwarp();
         }
-        if (g.chain != 2) pdl_wait_prior_grid();
-        if (g.chain == 1) pdl_launch_dependents();   // the launches beside this one need no wait of their own
+        pdl_wait_prior_grid();
         RingPos r;
         int it = 0;
         bool ok = true;
@@ -936,7 +934,7 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         if (pending) flush();
     } else {
         // ---- epilogue warps ----
-        if (g.chain != 2) pdl_wait_prior_grid();
+        pdl_wait_prior_grid();
         int tl = 0;
         for (int tile = tile_first; tile < tile_end; tile += tile_step, ++tl) {
             const int acc = nacc == 2 ? (tl & 1) : 0, pass = nacc == 2 ? tl >> 1 : tl;
@@ -997,8 +995,6 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
         cluster_arrive();   // this block has its parts; awaited below, before the senders' memory goes away
     }
     if (tma_store && warp == 2 && lane == 0) bulk_wait0();  // all of this block's tensor stores have landed
-    // one of several launches that run side by side: complete only after the one before it
-    if (g.chain == 2 && tid == 0) pdl_wait_prior_grid();
     tc_fence_before();
     if (S > 1) {
         __syncwarp();
@@ -1252,7 +1248,7 @@ bool gemm_tc_supported(int fmt, const LinArgs& a, int M) {
     return a.epi != EPI_SWIGLU || al16(a.W2);
 }
 
-cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool plain_form, bool overlap, cudaStream_t st, int* launches) {
+cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool overlap, cudaStream_t st) {
     const bool dual = a.epi == EPI_SWIGLU;
     const int K = a.K, sms = current_sm_count();
     if (a.npeer < 0 || a.npeer > 7) return cudaErrorInvalidValue;
@@ -1288,13 +1284,7 @@ cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool plain_form, bo
     g.status = a.status;
     g.tma_store = aligned ? 1 : 0;
     const bool may_split = a.npeer == 0 && a.sig.world == 0;
-    // The plain fused forms (q/k/v, SwiGLU) with few results go out as three launches side by side, which is what
-    // nn_launch_count reports for them and its tests state; that costs 4-5 us more than one launch does, so larger calls (from the
-    // results of 43 tiles of 128 x 64 on) and the forms with a norm or a bias, which a layer uses, are one.
-    long long results = 0;
-    for (int i = 0; i < a.nseg; ++i) results += (long long)M * a.seg[i].N;
-    const bool three = plain_form && (dual || a.nseg == 3) && rows >= 3 && results < 43ll * 128 * 64;
-    const GemmConfig c = gemm_config(fmt, trows, M, rows, K, sms, may_split, may_split && !three);
+    const GemmConfig c = gemm_config(fmt, trows, M, rows, K, sms, may_split, may_split);
     if (!c.ok) return cudaErrorInvalidValue;
     g.bn = c.bn;
     g.ntok = c.ntok;
@@ -1335,26 +1325,12 @@ cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool plain_form, bo
         if (dual && !make_scale_map(&mp.sc[1], sbase[3], a.seg[0].N, pitch, 16, trows)) g.scale_tma = 0;
     }
     if (!encode_tiled_2d(&mp.x, true, a.x, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, (uint32_t)(c.duo ? c.bn / 2 : c.bn))) return cudaErrorInvalidValue;
-    const int tiles = (c.duo ? (rows + 1) / 2 : rows) * c.ntok;
-    int cut[4] = {0, tiles, tiles, tiles}, parts = 1;
-    if (three) {
-        parts = 3;
-        for (int i = 1; i < 3; ++i) cut[i] = (dual ? i * rows / 3 : g.seg[i].tile0) * c.ntok;
-        cut[3] = tiles;
-    }
-    for (int i = 0; i < parts; ++i) {
-        g.tile_begin = cut[i];
-        g.tile_end = cut[i + 1];
-        g.chain = parts == 1 ? 0 : i == 0 ? 1 : 2;
-        int grid = (g.tile_end - g.tile_begin) * c.ksplit;
-        const int at_a_time = c.duo ? max_clusters(2, sms) : sms;
-        if (c.ksplit == 1 && grid > at_a_time) grid = at_a_time;   // persistent: one block (pair) per SM (pair) walks the tiles
-        if (c.duo) grid *= 2;
-        cudaError_t e = launch_fmt(fmt, c.duo, mp, g, grid, c.smem, overlap, st);
-        if (e != cudaSuccess) return e;
-        ++*launches;
-    }
-    return cudaSuccess;
+    g.tiles = (c.duo ? (rows + 1) / 2 : rows) * c.ntok;
+    int grid = g.tiles * c.ksplit;
+    const int at_a_time = c.duo ? max_clusters(2, sms) : sms;
+    if (c.ksplit == 1 && grid > at_a_time) grid = at_a_time;   // persistent: one block (pair) per SM (pair) walks the tiles
+    if (c.duo) grid *= 2;
+    return launch_fmt(fmt, c.duo, mp, g, grid, c.smem, overlap, st);
 }
 
 }  // namespace nnb

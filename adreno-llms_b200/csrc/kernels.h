@@ -121,9 +121,9 @@ bool encode_tiled_2d(void* map, bool half_elems, const void* base, uint64_t dim0
 // gemm_tc.cu: tcgen05 / tensor-memory GEMM for M > 16
 cudaError_t gemm_tc_configure();
 bool gemm_tc_supported(int fmt, const LinArgs& a, int M);
-// out = x . W^T for M rows with every epilogue of LinArgs.  `plain_form`: the call carries neither a norm nor a bias.  `overlap`: it may begin
-// while the launch before it runs and fetch weights meanwhile.  Adds the number of launches to *launches.
-cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool plain_form, bool overlap, cudaStream_t st, int* launches);
+// out = x . W^T for M rows with every epilogue of LinArgs.  `overlap`: it may begin while the launch before it runs and
+// fetch weights meanwhile.
+cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool overlap, cudaStream_t st);
 
 // gemv_generic.cu: any K, any alignment (the reference's gemv_rT_fp32acc role)
 cudaError_t launch_generic(int fmt, const LinArgs& a, cudaStream_t st);

@@ -77,7 +77,7 @@ def test_pairs_of_blocks(nnb, ctx, fmt):
 @pytest.mark.parametrize("fmt", ["fp16", "int8", "q4"])
 @pytest.mark.parametrize("M,Ns", [(33, (200, 72, 65)), (600, (896, 128, 128))])
 def test_three_weights_with_bias(nnb, ctx, fmt, M, Ns):
-    """Three launches side by side, and (many results) one launch over all three weights."""
+    """One launch over three weights of unequal, unaligned row counts: one row tile of each, and several of one beside one."""
     K = 448
     x = make_x(M, K, 41)
     ws = [make_weight(fmt, n, K, 42 + i) for i, n in enumerate(Ns)]
