@@ -883,8 +883,9 @@ __global__ void __launch_bounds__(PLAN_BLOCK, 1) decode_plan_kernel(const __grid
                     if (n - oldest == (unsigned)PLAN_SLOTS && need == oldest) need = oldest + 1u;  // the new item's own slot
                     while (oldest != need) {
                         // (four times the consumers' limit: a consumer that gives up on its own wait
-                        // releases its items right after, and the producer should still be there)
-                        if (!mbar_wait_bounded(empty0 + (oldest % PLAN_SLOTS) * 8, (oldest / PLAN_SLOTS) & 1u, 4 * P.wait_cycles)) {
+                        // releases its items right after, and the producer should still be there; the first item is
+                        // released only after the launch before this one)
+                        if (!mbar_wait_bounded(empty0 + (oldest % PLAN_SLOTS) * 8, (oldest / PLAN_SLOTS) & 1u, oldest == 0u ? WAIT_CYCLES + 4 * P.wait_cycles : 4 * P.wait_cycles)) {
                             *reinterpret_cast<volatile int*>(P.status) = 2;
                             atomicExch(P.state + 2, 1u);
                             *s_issued = n;

@@ -341,7 +341,7 @@ __device__ __forceinline__ bool wait_asleep(uint32_t bar, uint32_t parity) {
         const long long t0 = clock64();
         while (!mbar_try_wait(bar, parity)) {
             __nanosleep(100);
-            if (clock64() - t0 > 200000000ll) {
+            if (clock64() - t0 > WAIT_CYCLES) {
                 ok = 0;
                 break;
             }
@@ -364,7 +364,7 @@ __device__ __forceinline__ bool wait_parked(uint32_t bar, uint32_t parity) {
                 "selp.u32 %0, 1, 0, p;\n\t}"
                 : "=r"(done) : "r"(bar), "r"(parity), "r"(1000000u) : "memory");
             ok = done != 0;
-        } while (!ok && clock64() - t0 < 200000000ll);
+        } while (!ok && clock64() - t0 < WAIT_CYCLES);
     }
     return __all_sync(0xffffffffu, ok) != 0;
 }

@@ -49,9 +49,14 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
         : "memory");
     return ok;
 }
-// Bounded wait: gives up after about a tenth of a second of SM clocks and returns false
+// Bounded wait: gives up after about two seconds of SM clocks and returns false
 // (the caller records an error status and carries on; nothing spins forever).
-__device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, long long limit_cycles = 200000000ll) {
+// Why so long: a launch may begin while the one before it runs, and the activations, or the room that their use frees, come only
+// after that launch, so a wait's time includes what is left of it.  The limit is beyond any launch of this library (all of the
+// device's memory read once takes 28 ms).  Waiting for that launch first, in every warp, has the copies start later: Q4
+// 28672 x 8192, 32 rows 66.5 -> 67.7 us; a limit of its own for each first wait costs the expanding warps registers (69.1 us).
+constexpr long long WAIT_CYCLES = 4000000000ll;
+__device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, long long limit_cycles = WAIT_CYCLES) {
     if (mbar_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
     for (;;) {
@@ -63,7 +68,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 // Warp-wide form for long waits (a whole K loop): one lane polls, with a suspend-time hint so that
 // the hardware parks it between polls, and the result is shared by shuffle.  Thirty-two lanes
 // spinning on the same barrier would only take issue slots from the warps that do the work.
-__device__ __forceinline__ bool mbar_wait_bounded_warp(uint32_t bar, uint32_t parity, long long limit_cycles = 200000000ll) {
+__device__ __forceinline__ bool mbar_wait_bounded_warp(uint32_t bar, uint32_t parity, long long limit_cycles = WAIT_CYCLES) {
     int ok = 1;
     if ((threadIdx.x & 31) == 0) {
         const long long t0 = clock64();

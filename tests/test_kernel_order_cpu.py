@@ -57,3 +57,15 @@ def test_launches_that_read_ahead_ask_first():
     calls = re.findall(r"launch_(?:stream|gemm_tc)\(([^;]*)\);", source("api.cpp"))
     assert len(calls) >= 3
     assert all("c->use_pdl && overlap" in c for c in calls), calls
+
+
+def test_waits_have_time_for_the_launch_before():
+    """Launches begin while the one before them runs, and what they wait for (tokens, or room that the use of tokens frees) comes
+    only after it: every limit on such a wait is far above the longest launch, and none is written out by itself."""
+    limit = int(re.search(r"constexpr long long WAIT_CYCLES = (\d+)ll;", source("ptx.cuh")).group(1))
+    assert limit >= 2 * 1_900_000_000          # two seconds at the highest clock
+    for name in ("gemm_tc.cu", "gemv_stream.cu", "ptx.cuh"):
+        s = source(name)
+        assert not re.search(r"clock64\(\) - t0 [<>] 200000000ll", s) and "limit_cycles = 200000000ll" not in s, name
+    ring = block_after(source("decode_plan.cu"), "if (warp == PCW) {")
+    assert "oldest == 0u ? WAIT_CYCLES + 4 * P.wait_cycles" in ring
