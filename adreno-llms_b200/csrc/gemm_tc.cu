@@ -1144,12 +1144,12 @@ double gemm_cost(int fmt, const GemmConfig& c, int row_tiles, int K, int sms) {
     return fixed + (c.nacc == 2 ? waves * (tile > epi ? tile : epi) + epi : waves * (tile + epi));
 }
 
-GemmConfig gemm_choose(int fmt, int trows, int M, int row_tiles, int K, int sms, bool may_split, bool may_duo) {
+GemmConfig gemm_choose(int fmt, int trows, int M, int row_tiles, int K, int sms) {
     const int units = ((K + BK - 1) / BK + span_blocks(fmt) - 1) / span_blocks(fmt);
     GemmConfig best = {};
     double best_cost = 1e30;
     for (int ks = 1; ks <= 8; ks *= 2) {
-        if (ks > 1 && (!may_split || ks > units || row_tiles * ks > sms)) break;
+        if (ks > 1 && (ks > units || row_tiles * ks > sms)) break;
         int last = 0;
         for (int ntok = (M + 255) / 256; ntok <= (M + 15) / 16; ++ntok) {
             const int bn = ((M + ntok - 1) / ntok + 15) / 16 * 16;
@@ -1160,7 +1160,7 @@ GemmConfig gemm_choose(int fmt, int trows, int M, int row_tiles, int K, int sms,
             // 256 x 151936 x 896 in int8 101 -> 92.  Starting and ending in pairs costs some 3 us (the gate and up of a 512-token
             // prompt, one wave of pairs: 14 -> 17 us), which long calls only, from four waves on, win back.
             const bool long_call = (row_tiles + 1) / 2 * ntok >= 4 * max_clusters(2, sms);
-            for (int duo = 0; duo <= (may_duo && ks == 1 && bn % 32 == 0 && long_call ? 1 : 0); ++duo) {
+            for (int duo = 0; duo <= (ks == 1 && bn % 32 == 0 && long_call ? 1 : 0); ++duo) {
                 const GemmConfig c = gemm_geometry(fmt, trows, M, K, bn, ks, duo != 0);
                 if (!c.ok) continue;
                 const double cost = gemm_cost(fmt, c, row_tiles, K, sms);
@@ -1177,20 +1177,20 @@ GemmConfig gemm_choose(int fmt, int trows, int M, int row_tiles, int K, int sms,
 
 // The choice for a shape, kept (a choice is a function of its arguments alone): trying all tilings takes the host microseconds,
 // and a model asks for the same few shapes over and over.
-GemmConfig gemm_config(int fmt, int trows, int M, int row_tiles, int K, int sms, bool may_split, bool may_duo) {
+GemmConfig gemm_config(int fmt, int trows, int M, int row_tiles, int K, int sms) {
     struct Slot {
-        int key[7];
+        int key[6];
         GemmConfig c;
     };
     constexpr int SLOTS = 256;
     static thread_local Slot* slots = nullptr;
     if (!slots) slots = new Slot[SLOTS]();
-    const int key[7] = {fmt + 1, trows, M, row_tiles, K, sms, (may_split ? 1 : 0) + (may_duo ? 2 : 0)};
+    const int key[6] = {fmt + 1, trows, M, row_tiles, K, sms};
     uint32_t h = 0;
     for (int v : key) h = (h ^ (uint32_t)v) * 0x9E3779B1u, h ^= h >> 15;
     Slot& s = slots[h % SLOTS];
     if (memcmp(s.key, key, sizeof(key)) != 0) {
-        s.c = gemm_choose(fmt, trows, M, row_tiles, K, sms, may_split, may_duo);
+        s.c = gemm_choose(fmt, trows, M, row_tiles, K, sms);
         memcpy(s.key, key, sizeof(key));
     }
     return s.c;
@@ -1283,8 +1283,7 @@ cudaError_t launch_gemm_tc(int fmt, const LinArgs& a, int M, bool overlap, cudaS
     g.epi = a.epi;
     g.status = a.status;
     g.tma_store = aligned ? 1 : 0;
-    const bool may_split = a.npeer == 0 && a.sig.world == 0;
-    const GemmConfig c = gemm_config(fmt, trows, M, rows, K, sms, may_split, may_split);
+    const GemmConfig c = gemm_config(fmt, trows, M, rows, K, sms);   // the same for a call with peers: the same order of the sums
     if (!c.ok) return cudaErrorInvalidValue;
     g.bn = c.bn;
     g.ntok = c.ntok;

@@ -1,5 +1,6 @@
 """Multi-GPU parity of the row-sharded projections (needs at least two GPUs; skipped otherwise)
 and the single-rank behaviour of the gather entry points, including a wait that runs out."""
+import ctypes
 import os
 import socket
 import subprocess
@@ -8,7 +9,7 @@ import sys
 import numpy as np
 import pytest
 
-from helpers import TOL, make_weight, make_x
+from helpers import TOL, alloc_with_canary, check_canary, make_weight, make_x
 from oracle import cpu
 
 REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -56,6 +57,53 @@ def test_single_rank_gather_is_linear(nnb, ctx, fmt, N, K, M):
     finally:
         ctx.sync()
         comm.close()
+
+
+# shapes whose K the plain call splits over 2 .. 8 blocks (one with unaligned rows), and one whose tiles it gives to pairs of blocks
+GEMM_SHAPES = [("q4", 512, 2048, 40), ("q4", 1024, 2048, 40), ("int8", 384, 896, 256), ("fp16", 257, 4864, 33), ("fp16", 18696, 544, 1000)]
+
+
+@pytest.mark.parametrize("fmt,N,K,M", GEMM_SHAPES)
+def test_gather_of_many_rows_has_the_bits_of_linear(nnb, ctx, fmt, N, K, M):
+    """A gather adds in the order of the plain call, whatever tiles and splits that takes."""
+    comm = nnb.Comm(ctx, None, 0, 1)
+    try:
+        W, s = make_weight(fmt, N, K, 33)
+        qw, dx = nnb.QuantWeight(ctx, fmt, W, s), ctx.upload(make_x(M, K, 34).view(np.uint16))
+        g, out = comm.symm_alloc(M * N * 2), ctx.alloc(M * N * 2)
+        ctx.linear(M, N, K, dx, qw.buf, out)
+        for _ in range(3):
+            ctx.L.nn_buf_fill(ctx.h, g, 0x7E, M * N * 2)
+            comm.linear_gather(M, N, K, dx, qw.buf, g)
+            assert np.array_equal(ctx.download(g, (M, N), np.uint16), ctx.download(out, (M, N), np.uint16))
+        qw.release()
+        ctx.free(dx)
+        ctx.free(out)
+    finally:
+        ctx.sync()
+        comm.close()
+
+
+@pytest.mark.parametrize("fmt,N,K,M", GEMM_SHAPES)
+def test_peer_copies_of_many_rows(nnb, ctx, fmt, N, K, M):
+    """What the kernel stores to peers, with buffers of this GPU in the peers' place: whole, nothing past the end."""
+    W, s = make_weight(fmt, N, K, 35)
+    qw, dx = nnb.QuantWeight(ctx, fmt, W, s), ctx.upload(make_x(M, K, 36).view(np.uint16))
+    own = ctx.alloc(M * N * 2)
+    peers = [alloc_with_canary(ctx, M * N * 2) for _ in range(3)]
+    to_peers = ctx.L._ZN3nnb15linear_to_peersEP10nn_contextiiiPvS2_S2_PKPtiPKNS_12GatherSignalEPKc
+    vp, i = ctypes.c_void_p, ctypes.c_int
+    to_peers.argtypes, to_peers.restype = [vp, i, i, i, vp, vp, vp, vp, i, vp, ctypes.c_char_p], i
+    assert to_peers(ctx.h, M, N, K, dx, qw.buf, own, (vp * 3)(*peers), 3, None, b"test") == 0
+    want = ctx.download(own, (M, N), np.uint16)
+    for p in peers:
+        assert np.array_equal(ctx.download(p, (M, N), np.uint16), want)
+        check_canary(ctx, p, M * N * 2, f"{fmt} {N}x{K} M={M}")
+    ctx.linear(M, N, K, dx, qw.buf, own)
+    assert np.array_equal(ctx.download(own, (M, N), np.uint16), want)
+    qw.release()
+    for b in [dx, own] + peers:
+        ctx.free(b)
 
 
 @pytest.mark.parametrize("fmt,N,K", [("int8", 49152, 576), ("q4", 4096, 1024), ("fp16", 1536, 896)])
