@@ -384,6 +384,20 @@ __device__ __forceinline__ void expand_q4_word(uint32_t w, __half2 scale, uint32
     }
 }
 
+// x / (1 + exp(-x)) with the division's rounding: a quotient by the approximate reciprocal (1 ulp), corrected by its remainder, which
+// the fused multiply-add gives exactly (P. Markstein, IBM J. Res. Dev. 34, 1990).  Outside (-86, 32) the first quotient
+// stays: x itself above, where the denominator is 1, and below it less than 2^-117, -0 at the end, NaN for -inf.  For no fp32 x does it
+// differ from the division where that is 1e-30 or more; the two-ulp __fdividef differs for 1.1e8 of them, which shows in fp16
+// results, and is 0 to 0.2 us per call faster.  The division itself took a 512-token prompt (24 layers with gate and up of
+// 4864 x 896, fp16) from 1.28 to 1.41 ms.
+__device__ __forceinline__ float silu(float x) {
+    const float d = 1.0f + expf(-x);
+    float y;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(d));
+    const float q = x * y, r = fmaf(fmaf(-q, d, x), y, q);
+    return fabsf(x + 27.0f) < 59.0f ? r : q;
+}
+
 // DUO: two blocks of a cluster work on two neighbouring row tiles and the same tokens: see `duo` in gemm_choose.
 template <int WFMT, bool DUO>
 __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(const __grid_constant__ GemmMaps mp, const GemmArgs g) {
@@ -562,7 +576,7 @@ __global__ void __launch_bounds__(gemm_threads(WFMT), 1) linear_gemm_tc_kernel(c
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const float gt = up ? o[i] : v[j + i], u = up ? v[CH / 2 + j + i] : o[i];
-                    v[j + i] = __fdividef(gt, 1.0f + expf(-gt)) * u;
+                    v[j + i] = silu(gt) * u;
                 }
             }
         };

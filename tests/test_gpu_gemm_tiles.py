@@ -97,6 +97,52 @@ def test_three_weights_with_bias(nnb, ctx, fmt, M, Ns):
         ctx.free(b)
 
 
+@pytest.mark.parametrize("N", [4096, 2051])
+def test_swiglu_has_the_bits_of_few_rows(nnb, ctx, N):
+    """One-hot activations: gate and up are single weights, exact in both kernels, and what is left is SiLU(gate) * up.  Gates: at
+    N = 4096 every fp16 value, infinities and NaNs too, with ups of every magnitude; else the usual range."""
+    M, K = 64, 64
+    rng = np.random.default_rng(65)
+    if N * K == 1 << 18:
+        # column m of the weights holds the values of row m; rows of x pick one column, so no infinity meets a zero of another
+        Wg = np.tile(np.arange(1 << 16, dtype=np.uint16), 4).reshape(K, N)
+        Wu = rng.integers(0, 0x7C00, (K, N)).astype(np.uint16) | (rng.integers(0, 2, (K, N)) << 15).astype(np.uint16)
+        Wg, Wu = Wg.view(np.float16), Wu.view(np.float16)
+    else:
+        Wg, Wu = rng.uniform(-14.0, 14.0, (K, N)).astype(np.float16), rng.standard_normal((K, N)).astype(np.float16)
+    special = ~np.isfinite(Wg.astype(np.float32))
+    xb, ob = ctx.upload(np.eye(M, K, dtype=np.float16).view(np.uint16)), ctx.alloc(M * N * 2)
+
+    def both(wg):
+        qg, qu = (nnb.QuantWeight(ctx, "fp16", np.ascontiguousarray(w.T), None) for w in (wg, Wu))
+        ctx.fused_gate_up_silu(M, N, K, xb, qg.buf, qu.buf, ob)
+        many = ctx.download(ob, (M, N), np.uint16)
+        few = []
+        for m in range(0, M, 16):
+            ctx.fused_gate_up_silu(16, N, K, xb + m * K * 2, qg.buf, qu.buf, ob)
+            few.append(ctx.download(ob, (16, N), np.uint16))
+        qg.release()
+        qu.release()
+        return many, np.concatenate(few)
+
+    finite = np.where(special, np.float16(0), Wg)
+    many, few = both(finite)
+    assert np.array_equal(many, few), f"{(many != few).sum()} of {many.size} values"
+    g, u = finite.astype(np.float64), Wu.astype(np.float64)
+    with np.errstate(over="ignore"):
+        want = (g / (1.0 + np.exp(-g)) * u).astype(np.float16)
+    got = many.view(np.float16)
+    near = np.isfinite(want) & np.isfinite(got)
+    assert (~near).sum() == (~np.isfinite(want)).sum() == (~np.isfinite(got)).sum()
+    check_close(got[near], want[near], what="swiglu of single weights")
+    if special.any():   # a whole column of them, so that every row meets one: an infinity times zero is a NaN in both kernels
+        many, few = both(np.where(special, Wg, np.float16(1)))
+        nan = np.isnan(few.view(np.float16))
+        assert np.array_equal(np.isnan(many.view(np.float16)), nan) and np.array_equal(many[~nan], few[~nan])
+    for b in (xb, ob):
+        ctx.free(b)
+
+
 def test_weight_written_by_the_call_before(nnb, ctx):
     """A weight may be another call's result (scores against keys just projected): nothing of it is fetched early."""
     M, T, H = 48, 640, 512
