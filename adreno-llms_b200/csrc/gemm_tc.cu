@@ -36,6 +36,7 @@
 #include <cuda_fp16.h>
 
 #include <cstring>
+#include <memory>
 #include <type_traits>
 
 #include "kernels.h"
@@ -1197,8 +1198,8 @@ GemmConfig gemm_config(int fmt, int trows, int M, int row_tiles, int K, int sms)
         GemmConfig c;
     };
     constexpr int SLOTS = 256;
-    static thread_local Slot* slots = nullptr;
-    if (!slots) slots = new Slot[SLOTS]();
+    static thread_local std::unique_ptr<Slot[]> slots;   // given back when the thread ends
+    if (!slots) slots = std::make_unique<Slot[]>(SLOTS);
     const int key[6] = {fmt + 1, trows, M, row_tiles, K, sms};
     uint32_t h = 0;
     for (int v : key) h = (h ^ (uint32_t)v) * 0x9E3779B1u, h ^= h >> 15;

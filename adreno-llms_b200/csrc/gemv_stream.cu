@@ -36,6 +36,7 @@
 #include <cuda_fp16.h>
 #include <cstdio>
 #include <cstdlib>
+#include <memory>
 
 #include "kernels.h"
 #include "plan.h"
@@ -872,11 +873,11 @@ struct MapSlot {
     CUtensorMap map;
 };
 constexpr int MAP_SLOTS = 2048;
-thread_local MapSlot* t_map_cache = nullptr;
+thread_local std::unique_ptr<MapSlot[]> t_map_cache;   // given back when the thread ends
 
 bool cached_map(CUtensorMap* m, const MapKey& k) {
     if (!g_encode_tiled) return false;
-    if (!t_map_cache) t_map_cache = new MapSlot[MAP_SLOTS]();
+    if (!t_map_cache) t_map_cache = std::make_unique<MapSlot[]>(MAP_SLOTS);
     uint64_t h = reinterpret_cast<uintptr_t>(k.base) >> 4;
     h ^= k.dim1 * 0x9E3779B97F4A7C15ull + k.dim0 * 0xC2B2AE3D27D4EB4Full + (uint64_t)(k.box1 * 16 + k.box0 * 32 + k.kind);
     MapSlot& s = t_map_cache[(h ^ (h >> 17) ^ (h >> 31)) % MAP_SLOTS];
