@@ -35,6 +35,7 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <atomic>
 #include <cstring>
 #include <memory>
 #include <type_traits>
@@ -1114,11 +1115,12 @@ GemmConfig gemm_geometry(int fmt, int trows, int M, int K, int bn, int ksplit, b
 // Clusters of `size` blocks that can run at a time (one block per SM): the SMs of a cluster lie in one GPC, so fewer than
 // sms / size.  Asked of the driver once per device.
 int max_clusters(int size, int sms) {
-    static int cached[64][4] = {};
+    static std::atomic<int> cached[64][4] = {};   // (any thread; all find the same number)
     int dev = 0;
     const int k = size == 2 ? 1 : size == 4 ? 2 : 3;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sms / (2 * size);
-    if (!cached[dev][k]) {
+    int n = cached[dev][k].load(std::memory_order_relaxed);
+    if (!n) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(size * (sms / size)));
         cfg.blockDim = dim3((unsigned)gemm_threads(FMT_FP16));
@@ -1129,14 +1131,13 @@ int max_clusters(int size, int sms) {
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, linear_gemm_tc_kernel<FMT_FP16, false>, &cfg) != cudaSuccess || n < 1) {
             cudaGetLastError();
             n = sms / (2 * size);
         }
-        cached[dev][k] = n;
+        cached[dev][k].store(n, std::memory_order_relaxed);
     }
-    return cached[dev][k];
+    return n;
 }
 
 // What a choice costs, in SM clocks, to compare choices with.  Fitted to timings of tiles between 64 x 896 x 896 and

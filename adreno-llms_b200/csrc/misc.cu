@@ -3,6 +3,8 @@
 #include <cuda_fp16.h>
 #include <float.h>
 
+#include <atomic>
+
 #include "kernels.h"
 #include "ptx.cuh"
 
@@ -245,15 +247,15 @@ __global__ void l2_flush_kernel(uint4* buf, size_t n16) {
 }  // namespace
 
 int current_sm_count() {
-    static int cached[64] = {};
+    static std::atomic<int> cached[64] = {};   // (any thread; all find the same number)
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 132;
-    if (!cached[dev]) {
-        int n = 0;
+    int n = cached[dev].load(std::memory_order_relaxed);
+    if (!n) {
         if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 132;
-        cached[dev] = n;
+        cached[dev].store(n, std::memory_order_relaxed);
     }
-    return cached[dev];
+    return n;
 }
 
 cudaError_t launch_dequant(int fmt, int N, int K, const void* W, const uint16_t* scale, float* out, cudaStream_t st) {

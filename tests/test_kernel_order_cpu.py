@@ -69,3 +69,12 @@ def test_waits_have_time_for_the_launch_before():
         assert not re.search(r"clock64\(\) - t0 [<>] 200000000ll", s) and "limit_cycles = 200000000ll" not in s, name
     ring = block_after(source("decode_plan.cu"), "if (warp == PCW) {")
     assert "oldest == 0u ? WAIT_CYCLES + 4 * P.wait_cycles" in ring
+
+
+def test_tables_that_any_thread_fills_are_atomic():
+    """What a device's properties give is kept in static tables, which calls of any thread read and fill."""
+    tables = []
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cpp", ".h", ".cuh")):
+            tables += [(name, t.strip()) for t in re.findall(r"\bstatic ([^;(={]*\bcached\b)", source(name))]
+    assert len(tables) >= 2 and all(t.startswith("std::atomic<") for _, t in tables), tables
