@@ -115,15 +115,15 @@ __device__ __forceinline__ void record_failure(const PlanParams& P, CState& S, i
 __device__ __noinline__ bool wait_full_slow(uint32_t bar, uint32_t parity, long long limit) { return mbar_wait_bounded(bar, parity, limit); }
 
 // Poll published words until each carries `epoch`, and leave their fp16 pairs in dst.  Thread tid
-// takes words base + tid + j * PTHREADS, j < B; all of a thread's loads are in flight together, and a
-// word is asked for again only while it has not arrived.
-template <int B>
+// takes words base + tid + j * PTHREADS, j < POLL_WORDS; all of a thread's loads are in flight together, and a
+// word is asked for again only while it has not arrived.  (Rows that come this way have at least 1536 words.)
+constexpr int POLL_WORDS = 4;
 __device__ __forceinline__ void poll_batch(const PlanParams& P, CState& S, const unsigned long long* ll, int base, int nw, unsigned epoch,
                                            uint32_t* dst, int tid) {
-    unsigned long long w[B];
+    unsigned long long w[POLL_WORDS];
     unsigned pending = 0u;
 #pragma unroll
-    for (int j = 0; j < B; ++j) {
+    for (int j = 0; j < POLL_WORDS; ++j) {
         w[j] = 0ull;
         if (base + j * PTHREADS + tid < nw) pending |= 1u << j;
     }
@@ -131,10 +131,10 @@ __device__ __forceinline__ void poll_batch(const PlanParams& P, CState& S, const
     unsigned spins = 0;
     while (pending) {
 #pragma unroll
-        for (int j = 0; j < B; ++j)
+        for (int j = 0; j < POLL_WORDS; ++j)
             if (pending & (1u << j)) w[j] = ld_relaxed_u64(ll + base + j * PTHREADS + tid);
 #pragma unroll
-        for (int j = 0; j < B; ++j)
+        for (int j = 0; j < POLL_WORDS; ++j)
             if ((unsigned)(w[j] >> 32) == epoch) pending &= ~(1u << j);
         if (pending) {
             if (S.failed) break;  // an earlier wait of this launch ran out: take what is there
@@ -151,20 +151,14 @@ __device__ __forceinline__ void poll_batch(const PlanParams& P, CState& S, const
         }
     }
 #pragma unroll
-    for (int j = 0; j < B; ++j) {
+    for (int j = 0; j < POLL_WORDS; ++j) {
         const int idx = base + j * PTHREADS + tid;
         if (idx < nw) dst[idx] = (uint32_t)w[j];
     }
 }
 __device__ __forceinline__ void poll_words(const PlanParams& P, CState& S, const unsigned long long* ll, int nw, unsigned epoch, uint32_t* dst,
                                            int tid) {
-    if (nw <= PTHREADS) {
-        poll_batch<1>(P, S, ll, 0, nw, epoch, dst, tid);
-    } else if (nw <= 2 * PTHREADS) {
-        poll_batch<2>(P, S, ll, 0, nw, epoch, dst, tid);
-    } else {
-        for (int base = 0; base < nw; base += 4 * PTHREADS) poll_batch<4>(P, S, ll, base, nw, epoch, dst, tid);
-    }
+    for (int base = 0; base < nw; base += POLL_WORDS * PTHREADS) poll_batch(P, S, ll, base, nw, epoch, dst, tid);
 }
 
 // RMSNorm of the single row x (in shared or global memory) with the norm weight gw (in shared
