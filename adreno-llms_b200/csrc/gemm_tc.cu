@@ -1173,7 +1173,7 @@ GemmConfig gemm_choose(int fmt, int trows, int M, int row_tiles, int K, int sms)
             last = bn;
             // Two blocks on one 256-row tile (cta_group::2): each loads half of the tile's tokens, so a K block of 256 tokens is 32 KB
             // per SM instead of 48 and the tensor core sets the pace instead of the copies: 2048 x 151936 x 896 in fp16 576 -> 500 us,
-            // 256 x 151936 x 896 in int8 101 -> 92.  Starting and ending in pairs costs some 3 us (the gate and up of a 512-token
+            // 256 x 151936 x 896 in int8 101 -> 90.  Starting and ending in pairs costs some 3 us (the gate and up of a 512-token
             // prompt, one wave of pairs: 14 -> 17 us), which long calls only, from four waves on, win back.
             const bool long_call = (row_tiles + 1) / 2 * ntok >= 4 * max_clusters(2, sms);
             for (int duo = 0; duo <= (ks == 1 && bn % 32 == 0 && long_call ? 1 : 0); ++duo) {
