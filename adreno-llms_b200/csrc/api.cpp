@@ -339,7 +339,7 @@ extern "C" int nn_host_free(void* p) {
 // ---------------------------------------------------------------------------------
 // registry
 // ---------------------------------------------------------------------------------
-static size_t fmt_rowbytes(int fmt, int K) { return fmt == FMT_FP16 ? (size_t)K * 2 : fmt == FMT_INT8 ? (size_t)K : (size_t)K / 2; }
+static size_t fmt_rowbytes(int fmt, int K) { return fmt == FMT_FP16 ? (size_t)K * 2 : fmt == FMT_Q4 ? (size_t)K / 2 : (size_t)K; }
 
 static int register_weight(nn_context* c, int fmt, nn_buf W, nn_buf scale, int N, int K, const char* who) {
     if (!c) return NN_FAIL(NN_ERR_ARG, "%s: null context", who);
@@ -481,9 +481,10 @@ static void note_recorded(nn_context* c, int fmt, const LinArgs& a, const Stream
     c->rec.push_back(r);
 }
 
-static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char* who) {
+static int run_linear(nn_context* c, int weight_fmt, LinArgs a, int M_total, const char* who) {
     a.sk_scratch = c->sk_scratch;
     a.sk_flags = c->sk_flags;
+    int fmt = M_total <= 16 ? stream_format(weight_fmt, a, c->sm_count) : weight_fmt;
     if (a.norm_w) {
         // the prologue is fused into the streaming kernel; every other route normalises into
         // context scratch first
@@ -516,6 +517,7 @@ static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char
         bool done = false;
         const int rc = run_gemm_tc(c, fmt, a, M_total, who, &done);
         if (rc != NN_OK || done) return rc;
+        fmt = stream_format(weight_fmt, a, c->sm_count);
     }
     // M > 16 is walked in slices of 16 activation rows (each slice re-streams the weights).
     const uint16_t* x0 = a.x;
@@ -573,7 +575,7 @@ static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char
         } else {
             if (a.npeer > 0)
                 return NN_FAIL(NN_ERR_UNSUPPORTED, "%s: this shape takes the any-shape kernel, which does not write to peer ranks (K=%d)", who, a.K);
-            e = launch_generic(fmt, a, c->stream);
+            e = launch_generic(weight_fmt, a, c->stream);
         }
         if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: launch failed: %s (M=%d K=%d)", who, cudaGetErrorString(e), a.M, a.K);
         c->launches++;
@@ -856,7 +858,8 @@ int nnb::linear_argmax(nn_context* c, int N, int K, nn_buf x, nn_buf W, nn_buf l
     a.sk_scratch = c->sk_scratch;
     a.sk_flags = c->sk_flags;
     StreamPlan p = {};
-    if (stream_supported(r.fmt, 1, K, a)) p = stream_plan(r.fmt, a, c->sm_count, c->smem_limit);
+    const int fmt = stream_format(r.fmt, a, c->sm_count);
+    if (stream_supported(fmt, 1, K, a)) p = stream_plan(fmt, a, c->sm_count, c->smem_limit);
     if (!p.ok) {
         // shapes the streaming kernel does not take: projection, then the separate arg-max
         if (sig) return NN_FAIL(NN_ERR_UNSUPPORTED, "%s: this shape (K=%d) is not taken by the streaming kernel", who, K);
@@ -871,13 +874,13 @@ int nnb::linear_argmax(nn_context* c, int N, int K, nn_buf x, nn_buf W, nn_buf l
     a.argmax_out = (int*)out_idx;
     a.argmax_base = row_base;
     if (sig) a.sig = *sig;
-    const bool overlap = !read_ahead_in_flight(c->in_flight, r.fmt, a);
-    cudaError_t e = launch_stream(r.fmt, a, p, c->stream, c->use_pdl && overlap);
+    const bool overlap = !read_ahead_in_flight(c->in_flight, fmt, a);
+    cudaError_t e = launch_stream(fmt, a, p, c->stream, c->use_pdl && overlap);
     if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: launch failed: %s (N=%d K=%d)", who, cudaGetErrorString(e), N, K);
     if (!overlap) c->in_flight.ordered();
     note_outputs(c, a, 1);
     c->in_flight.wrote(out_idx, 4);
-    note_recorded(c, r.fmt, a, p, overlap);
+    note_recorded(c, fmt, a, p, overlap);
     c->launches++;
     return NN_OK;
 }

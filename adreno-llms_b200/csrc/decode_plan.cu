@@ -26,7 +26,7 @@
 //   * the arithmetic is the separate launch's (stream_core.cuh), on the same K partition and in the
 //     same order, so a run gives the same bits as the operators launched one by one.  A per-layer
 //     operator is bound by latency, not by its weight stream, so a block has eight consumer warps: a
-//     tile whose K is split has sixteen K parts and every warp takes two of them; int8 weights of such
+//     tile whose K is split has eight K parts and every warp takes one of them; int8 weights of such
 //     tiles are multiplied with the fp16 activations as they are (no fixed-point copy to build once the
 //     activations arrive).  What does not depend on the activations (descriptor, norm weight, row
 //     scales, the values an in-place epilogue updates, the tile's weights) is fetched or waited for
@@ -256,8 +256,8 @@ __device__ __forceinline__ bool fetch_piece(const unsigned long long* ll, int p,
 }
 
 // The operator's activation row, from the other blocks' words (or memory) to its staged form, with the RMSNorm when asked: the
-// row stays in registers from the first look at the words to the staged stores, so that one barrier (fp16), two (int8: the
-// row's largest magnitude) or one more (the norm's sum of squares) are all that stands between the arrival of the last word and
+// row stays in registers from the first look at the words to the staged stores, so that one barrier, two (whole-row int8
+// tiles: the row's largest magnitude) or one more (the norm's sum of squares) are all that stands between the arrival of the last word and
 // the first matrix instruction.  Rows of up to PIECES pieces per thread (plan_stage_fast); longer ones take stage_general.
 //
 // This is the step's critical path, and it runs once per operator: what it costs is its instruction count, cold.  The version
@@ -387,7 +387,7 @@ __device__ __forceinline__ bool stage_fast(const PlanParams& P, const PlanOpScal
             *reinterpret_cast<uint2*>(dst + 2 * xstride) = make_uint2(l[0][0], l[0][1]);
         }
     } else {
-        uint8_t* row = FMT == FMT_FP16 ? xs : smem + P.off_xraw;
+        uint8_t* row = FMT != FMT_Q4 ? xs : smem + P.off_xraw;
 #pragma unroll
         for (int j = 0; j < PIECES; ++j)
             if ((have >> j) & 1u) *reinterpret_cast<uint4*>(row + (tid + j * nthr) * 16) = make_uint4(w[j][0], w[j][1], w[j][2], w[j][3]);
@@ -535,8 +535,8 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
         sg = D.seg[seg_i];
         row0 = (tile - sg.tile0) * tile_rows + wrow_off;
         // int8 row scales: with the tile's last item when its rows allow a bulk copy, else from memory now
-        scales_ride = FMT == FMT_INT8 && row_scales && plan_rows_bulk_ok(min(tile_rows, sg.N - (tile - sg.tile0) * tile_rows));
-        if (writer && FMT == FMT_INT8 && !scales_ride) {
+        scales_ride = int8_weights(FMT) && row_scales && plan_rows_bulk_ok(min(tile_rows, sg.N - (tile - sg.tile0) * tile_rows));
+        if (writer && int8_weights(FMT) && !scales_ride) {
             if (DUAL) {
                 const int n = min(row0 + (lane & 15), sg.N - 1);
                 sc1 = sg.scale[n];
@@ -610,7 +610,7 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
             if (tile != tile_first || cg != 0) claim_item(off, slot);
             const uint32_t sw = ring + (uint32_t)off;
             const int cb = (S.failed || !active) ? 0 : min(kcb, rowbytes - c * kcb);
-            if (FMT == FMT_INT8 && scales_ride && writer && cg == groups - 1) {
+            if (int8_weights(FMT) && scales_ride && writer && cg == groups - 1) {
                 const uint16_t* sc = reinterpret_cast<const uint16_t*>(smem + ring_off + off + scale_off);
                 if (DUAL) {
                     sc1 = sc[wrow_off + (lane & 15)];
@@ -628,13 +628,11 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
                     chunk_fp16<1>(lg, sw, c, kcb, cb, acc);
                 }
             } else if constexpr (FMT == FMT_INT8) {
-                if constexpr (WIDE) {
-                    const int s0 = (c * kcb) / 64;
+                chunk_int8<1>(lg, sw, c, kcb, cb, iacc);
+            } else if constexpr (FMT == FMT_INT8H) {
+                const int s0 = (c * kcb) / 64;
 #pragma unroll 1
-                    for (int u = set; u < cb / 64; u += 2) step_int8<1>(lg, sw, s0 + u, u, iacc);
-                } else {
-                    chunk_int8<1>(lg, sw, c, kcb, cb, iacc);
-                }
+                for (int u = set; u < cb / 64; u += 2) step_int8h<1>(lg, sw, s0 + u, u, acc[0]);
             } else {
                 // block scales arrive by tensor copies: whole boxes, which for two weights means all
                 // gate rows first, then all up rows
@@ -660,64 +658,29 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
         float v0, v1 = 0.f;  // v1: the second weight's sum (two-weight epilogue)
         if constexpr (WIDE) {
             // The eight K parts meet in shared memory.  Per consumer of the separate launch (quarter) the
-            // two sets are added first, then the quarters in order; int8 parts are exact integer limb
-            // sums, added as integers and turned into a float once per quarter, as that consumer does.
+            // two sets are added first, then the quarters in order.
             const int r0 = DUAL ? (lane & 15) : lane;
-            if constexpr (IMMA) {
-                int* ibuf = reinterpret_cast<int*>(red) + (S.ti & 1) * (KPARTS * 3 * 32);
-                if (t == 0) {
+            float* buf = red + (S.ti & 1) * (KPARTS * 32);
+            if (t == 0) {
+                float* mine = buf + warp * 32 + g;
+                mine[0] = acc[0][0][0][0];
+                mine[8] = acc[0][0][0][2];
+                mine[16] = acc[0][1][0][0];
+                mine[24] = acc[0][1][0][2];
+            }
+            consumers_sync();
+            tile += G;
+            if (warp != 0) {
+                if (tile < ntiles) tile_prologue(tile, false);
+                continue;
+            }
+            v0 = buf[r0] + buf[32 + r0];
 #pragma unroll
-                    for (int l = 0; l < 3; ++l) {
-                        int* mine = ibuf + (warp * 3 + l) * 32 + g;
-                        mine[0] = iacc[l][0][0][0];
-                        mine[8] = iacc[l][0][0][2];
-                        mine[16] = iacc[l][1][0][0];
-                        mine[24] = iacc[l][1][0][2];
-                    }
-                }
-                consumers_sync();
-                tile += G;
-                if (warp != 0) {   // the first warp finishes the tile; the others go on to the block's next one
-                    if (tile < ntiles) tile_prologue(tile, false);
-                    continue;
-                }
-                auto quarter_sum = [&](int q, int r) {
-                    const int* a = ibuf + (2 * q) * 3 * 32 + r;
-                    const int* b2 = a + 3 * 32;
-                    const float f = fmaf((float)(a[0] + b2[0]), 65536.f, fmaf((float)(a[32] + b2[32]), 256.f, (float)(a[64] + b2[64])));
-                    return f * rowscale[0] + 0.f;  // (+ 0: the consumer adds its empty second set)
-                };
-                v0 = quarter_sum(0, r0);
+            for (int q = 1; q < NCW; ++q) v0 += buf[(2 * q) * 32 + r0] + buf[(2 * q + 1) * 32 + r0];
+            if (DUAL) {
+                v1 = buf[16 + r0] + buf[32 + 16 + r0];
 #pragma unroll
-                for (int q = 1; q < NCW; ++q) v0 += quarter_sum(q, r0);
-                if (DUAL) {
-                    v1 = quarter_sum(0, 16 + r0);
-#pragma unroll
-                    for (int q = 1; q < NCW; ++q) v1 += quarter_sum(q, 16 + r0);
-                }
-            } else {
-                float* buf = red + (S.ti & 1) * (KPARTS * 32);
-                if (t == 0) {
-                    float* mine = buf + warp * 32 + g;
-                    mine[0] = acc[0][0][0][0];
-                    mine[8] = acc[0][0][0][2];
-                    mine[16] = acc[0][1][0][0];
-                    mine[24] = acc[0][1][0][2];
-                }
-                consumers_sync();
-                tile += G;
-                if (warp != 0) {
-                    if (tile < ntiles) tile_prologue(tile, false);
-                    continue;
-                }
-                v0 = buf[r0] + buf[32 + r0];
-#pragma unroll
-                for (int q = 1; q < NCW; ++q) v0 += buf[(2 * q) * 32 + r0] + buf[(2 * q + 1) * 32 + r0];
-                if (DUAL) {
-                    v1 = buf[16 + r0] + buf[32 + 16 + r0];
-#pragma unroll
-                    for (int q = 1; q < NCW; ++q) v1 += buf[(2 * q) * 32 + 16 + r0] + buf[(2 * q + 1) * 32 + 16 + r0];
-                }
+                for (int q = 1; q < NCW; ++q) v1 += buf[(2 * q) * 32 + 16 + r0] + buf[(2 * q + 1) * 32 + 16 + r0];
             }
         } else {
             if constexpr (IMMA) int8_recombine<1>(iacc, acc[0], rowscale, 1, t);
@@ -810,7 +773,7 @@ __global__ void __launch_bounds__(PLAN_BLOCK, 1) decode_plan_kernel(const __grid
     const int nops = P.nops;
     const int ring_off = (int)(((s_base + (uint32_t)P.off_ring + 1023u) & ~1023u) - s_base);
 
-    if (tid < 16) reinterpret_cast<uint32_t*>(smem)[tid] = 0u;  // 64 bytes of zeros: B operand of absent token rows
+    if (tid < HDR_BYTES / 4) reinterpret_cast<uint32_t*>(smem)[tid] = 0u;  // B operand of absent token rows
     if (tid == 0) {
         *s_issued = 0xFFFFFFFFu;
         for (int s = 0; s < PLAN_SLOTS; ++s) {
@@ -1006,7 +969,7 @@ __global__ void __launch_bounds__(PLAN_BLOCK, 1) decode_plan_kernel(const __grid
             case FMT_FP16 * 2: run_op<FMT_FP16, false>(P, D, op, smem, tid, lane, warp); break;
             case FMT_FP16 * 2 + 1: run_op<FMT_FP16, true>(P, D, op, smem, tid, lane, warp); break;
             case FMT_INT8 * 2: run_op<FMT_INT8, false>(P, D, op, smem, tid, lane, warp); break;
-            case FMT_INT8 * 2 + 1: run_op<FMT_INT8, true>(P, D, op, smem, tid, lane, warp); break;
+            case FMT_INT8H * 2 + 1: run_op<FMT_INT8H, true>(P, D, op, smem, tid, lane, warp); break;
             case FMT_Q4 * 2: run_op<FMT_Q4, false>(P, D, op, smem, tid, lane, warp); break;
             default: run_op<FMT_Q4, true>(P, D, op, smem, tid, lane, warp); break;
         }
