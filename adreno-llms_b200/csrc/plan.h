@@ -146,5 +146,6 @@ void free_run(PlanRun* run);
 // gemv_stream.cu: tensor maps of a streamed operator (weights: 128-byte swizzled boxes of `box_rows`
 // rows; Q4 scales: dense boxes of `box_bytes` x `box_rows`).
 bool make_weight_map(CUtensorMap* m, const void* W, int rows, int rowbytes, int box_rows);
+bool make_scale_map(CUtensorMap* m, const void* S, int rows, int rowbytes, int box_bytes, int box_rows);
 
 }  // namespace nnb
