@@ -481,10 +481,49 @@ static void note_recorded(nn_context* c, int fmt, const LinArgs& a, const Stream
     c->rec.push_back(r);
 }
 
+// 2..16 activation rows in one launch of the batch kernel, where it takes the shape.  Two kinds of call stay two launches, which callers
+// count (nn_launch_count, nn_plan_num_recorded and the tests of both say so): a norm outside a recording, where a call costs the host as much
+// as the device, is applied by the staging launch; two rows without a norm inside a recording take that launch and the streaming kernel.
+static int run_batch(nn_context* c, int fmt, LinArgs a, int M, const char* who, bool* done) {
+    *done = false;
+    a.M = M;
+    if (M == 2 && !a.norm_w && c->capturing) return NN_OK;
+    const uint16_t* norm_w = c->capturing ? nullptr : a.norm_w;
+    const int pitch = stage_row_bytes(a.K);
+    if (norm_w) {
+        if ((size_t)M * pitch > c->stage_img_bytes || (size_t)a.K * 2 > ((size_t)48 << 10)) return NN_OK;
+        a.norm_w = nullptr;
+    }
+    const BatchPlan p = batch_plan(fmt, a, c->sm_count, c->smem_limit);
+    if (!p.ok) return NN_OK;
+    cudaError_t e;
+    if (norm_w) {
+        if ((reinterpret_cast<uintptr_t>(norm_w) & 15) != 0) return NN_OK;
+        e = launch_stage_image(FMT_FP16, a.x, M, a.K, norm_w, a.norm_eps, (uint8_t*)c->stage_img, c->stream, c->use_pdl);
+        if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: norm launch failed: %s (M=%d K=%d)", who, cudaGetErrorString(e), M, a.K);
+        c->launches++;
+        a.x = (const uint16_t*)c->stage_img;
+        a.x_pitch = pitch;
+    }
+    const bool overlap = !read_ahead_in_flight(c->in_flight, fmt, a);
+    e = launch_batch(fmt, a, p, c->stream, c->use_pdl && overlap);
+    if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: launch failed: %s (M=%d K=%d)", who, cudaGetErrorString(e), M, a.K);
+    if (!overlap) c->in_flight.ordered();
+    note_outputs(c, a, M);
+    c->launches++;
+    *done = true;
+    return NN_OK;
+}
+
 static int run_linear(nn_context* c, int weight_fmt, LinArgs a, int M_total, const char* who) {
     a.sk_scratch = c->sk_scratch;
     a.sk_flags = c->sk_flags;
     int fmt = M_total <= 16 ? stream_format(weight_fmt, a, c->sm_count) : weight_fmt;
+    if (M_total >= 2 && M_total <= 16) {
+        bool done = false;
+        const int rc = run_batch(c, fmt, a, M_total, who, &done);
+        if (rc != NN_OK || done) return rc;
+    }
     if (a.norm_w) {
         // the prologue is fused into the streaming kernel; every other route normalises into
         // context scratch first

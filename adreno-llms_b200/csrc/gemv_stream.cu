@@ -856,7 +856,7 @@ EncodeTiledFn g_encode_tiled = nullptr;
 struct MapKey {
     const void* base;
     uint64_t dim0, dim1, stride1;
-    uint32_t box0, box1, kind;  // kind: fp16 elements | 128-byte swizzle << 1 | 256-byte L2 promotion << 2 | 8
+    uint32_t box0, box1, kind;  // kind: fp16 elements | 128-byte swizzle << 1 | 256-byte L2 promotion << 2 | 8; three dimensions: 16 or 32
     bool operator==(const MapKey& o) const {
         return base == o.base && dim0 == o.dim0 && dim1 == o.dim1 && stride1 == o.stride1 && box0 == o.box0 && box1 == o.box1 && kind == o.kind;
     }
@@ -878,11 +878,14 @@ bool cached_map(CUtensorMap* m, const MapKey& k) {
         *m = s.map;
         return true;
     }
-    const cuuint64_t dims[2] = {k.dim0, k.dim1};
-    const cuuint64_t strides[1] = {k.stride1};
-    const cuuint32_t box[2] = {k.box0, k.box1};
-    const cuuint32_t estr[2] = {1u, 1u};
-    if (g_encode_tiled(m, (k.kind & 1u) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(k.base), dims, strides,
+    // (three dimensions: 128-byte columns behind the rows, or the columns of a row before the rows)
+    const bool cols_last = (k.kind & 16u) != 0, cols_first = (k.kind & 32u) != 0;
+    const cuuint64_t cols = k.dim0 / 128;
+    const cuuint64_t dims[3] = {cols_last || cols_first ? 128 : k.dim0, cols_first ? cols : k.dim1, cols_first ? k.dim1 : cols};
+    const cuuint64_t strides[2] = {cols_first ? 128 : k.stride1, cols_first ? k.stride1 : 128};
+    const cuuint32_t box[3] = {cols_last || cols_first ? 128u : k.box0, cols_first ? k.box0 : k.box1, cols_first ? k.box1 : k.box0};
+    const cuuint32_t estr[3] = {1u, 1u, 1u};
+    if (g_encode_tiled(m, (k.kind & 1u) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, cols_last || cols_first ? 3 : 2, const_cast<void*>(k.base), dims, strides,
                        box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, (k.kind & 2u) ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                        (k.kind & 4u) ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
@@ -948,6 +951,15 @@ bool make_weight_map(CUtensorMap* m, const void* W, int rows, int rowbytes, int 
     return cached_byte_map(m, W, rows, rowbytes, 128, box_rows, true);
 }
 
+bool make_columns_map(CUtensorMap* m, const void* W, int rows, int rowbytes, int box_rows, int cols) {
+    if (rowbytes % 128 || cols > 256 || box_rows > 256) return false;
+    return cached_map(m, MapKey{W, (uint64_t)rowbytes, (uint64_t)rows, (uint64_t)rowbytes, (uint32_t)cols, (uint32_t)box_rows, 8u | 6u | 16u});
+}
+bool make_rows_map(CUtensorMap* m, const void* x, int rows, int rowbytes, int pitch, int cols, int box_rows) {
+    if (rowbytes % 128 || pitch % 16 || cols > 256 || box_rows > 256) return false;
+    return cached_map(m, MapKey{x, (uint64_t)rowbytes, (uint64_t)rows, (uint64_t)pitch, (uint32_t)cols, (uint32_t)box_rows, 8u | 6u | 32u});
+}
+
 // 2-D byte view of a Q4 scale tensor: [rows][rowbytes], dense box of box_bytes x box_rows.
 bool make_scale_map(CUtensorMap* m, const void* S, int rows, int rowbytes, int box_bytes, int box_rows) {
     if (box_bytes % 16 || box_bytes > 256 || box_rows > 256) return false;
@@ -976,6 +988,7 @@ cudaError_t stream_configure() {
     CFG(FMT_Q4, 1, false) CFG(FMT_Q4, 2, false) CFG(FMT_Q4, 1, true) CFG(FMT_Q4, 2, true)
 #undef CFG
     if ((e = decode_plan_configure()) != cudaSuccess) return e;
+    if ((e = batch_configure()) != cudaSuccess) return e;
     return gemm_tc_configure();
 }
 

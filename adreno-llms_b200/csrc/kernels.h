@@ -51,6 +51,7 @@ struct LinArgs {
     const uint8_t* W2;       // EPI_SWIGLU: the "up" weight (seg[0] is the gate)
     const uint16_t* scale2;  // EPI_SWIGLU: its scales
     const uint16_t* x;       // [M, K] fp16
+    int x_pitch;             // batched calls: bytes from row to row of x when they are not K * 2 (0: they are)
     int M, K;
     int ntiles;      // row tiles over all segments
     int epi;         // Epi
@@ -105,6 +106,17 @@ struct StreamPlan {  // launch geometry chosen on the host
 };
 
 struct StreamPart { int kw, kcb; };   // warps that split K of a tile, bytes of a row per K chunk
+
+// gemv_batch.cu: 2..16 activation rows, one launch per operator
+struct BatchPlan {
+    int grid, kcb, tile_rows, cols, xcols, stages, stage_bytes, ntiles;
+    int off_ctab, off_red, off_ring;   // shared memory
+    size_t smem;
+    bool ok;
+};
+BatchPlan batch_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit);
+cudaError_t launch_batch(int fmt, const LinArgs& a, const BatchPlan& p, cudaStream_t st, bool pdl);
+cudaError_t batch_configure();
 
 // gemv_stream.cu
 int count_tiles(const LinArgs& a, int tile_rows);
@@ -189,6 +201,7 @@ cudaError_t launch_l2_flush(void* buf, size_t bytes, cudaStream_t st);
 // the staged activations of a batched call (layout of the streaming kernel's shared memory), with the optional RMSNorm
 constexpr size_t STAGE_IMG_BYTES = (size_t)1 << 20;   // the context's room for them (16 rows of 32 000 values)
 size_t stage_image_bytes(int fmt, int M, int K);
+int stage_row_bytes(int K);   // of a row of fp16 values in such an image
 cudaError_t launch_stage_image(int fmt, const uint16_t* x, int M, int K, const uint16_t* norm_w, float eps, uint8_t* img, cudaStream_t st,
                                bool pdl);
 // read-bandwidth probes over `bytes` (a multiple of 16 KiB) at src; sink: 256 floats; status: one word, set on a timed-out wait

@@ -146,6 +146,11 @@ void free_run(PlanRun* run);
 // gemv_stream.cu: tensor maps of a streamed operator (weights: 128-byte swizzled boxes of `box_rows`
 // rows; Q4 scales: dense boxes of `box_bytes` x `box_rows`).
 bool make_weight_map(CUtensorMap* m, const void* W, int rows, int rowbytes, int box_rows);
+// The same weight (rows of whole 128-byte columns) with a box of `cols` columns one after another, each `box_rows` rows of 128 bytes; and
+// rows of `rowbytes` bytes, `pitch` from one to the next, with a box of `box_rows` rows of `cols` columns.  Swizzled as above; columns
+// and rows past the end come as zeros.
+bool make_columns_map(CUtensorMap* m, const void* W, int rows, int rowbytes, int box_rows, int cols);
+bool make_rows_map(CUtensorMap* m, const void* x, int rows, int rowbytes, int pitch, int cols, int box_rows);
 bool make_scale_map(CUtensorMap* m, const void* S, int rows, int rowbytes, int box_bytes, int box_rows);
 
 }  // namespace nnb

@@ -136,6 +136,8 @@ __global__ void __launch_bounds__(ST_MAX) stage_image_kernel(const uint16_t* __r
 }  // namespace
 
 size_t stage_image_bytes(int fmt, int M, int K) { return (size_t)x_bytes_of(fmt, M, K) + (size_t)ctab_bytes_of(fmt, M, K); }
+int stage_row_bytes(int K) { return x_stride_of(FMT_FP16, K); }
+
 cudaError_t launch_stage_image(int fmt, const uint16_t* x, int M, int K, const uint16_t* norm_w, float eps, uint8_t* img, cudaStream_t st,
                                bool pdl) {
     cudaLaunchConfig_t cfg = {};
