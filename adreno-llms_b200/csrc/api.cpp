@@ -898,7 +898,7 @@ int nnb::linear_argmax(nn_context* c, int N, int K, nn_buf x, nn_buf W, nn_buf l
     a.sk_flags = c->sk_flags;
     StreamPlan p = {};
     const int fmt = stream_format(r.fmt, a, c->sm_count);
-    if (stream_supported(fmt, 1, K, a)) p = stream_plan(fmt, a, c->sm_count, c->smem_limit);
+    if (stream_supported(fmt, 1, K, a) && (stream_whole_steps(fmt, K) || (logits && !sig))) p = stream_plan(fmt, a, c->sm_count, c->smem_limit);
     if (!p.ok) {
         // shapes the streaming kernel does not take: projection, then the separate arg-max
         if (sig) return NN_FAIL(NN_ERR_UNSUPPORTED, "%s: this shape (K=%d) is not taken by the streaming kernel", who, K);

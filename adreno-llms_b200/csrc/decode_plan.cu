@@ -391,6 +391,7 @@ __device__ __forceinline__ bool stage_fast(const PlanParams& P, const PlanOpScal
 #pragma unroll
         for (int j = 0; j < PIECES; ++j)
             if ((have >> j) & 1u) *reinterpret_cast<uint4*>(row + (tid + j * nthr) * 16) = make_uint4(w[j][0], w[j][1], w[j][2], w[j][3]);
+        if (FMT == FMT_INT8H && per + tid < x_values_of(FMT, D.K) / 8) *reinterpret_cast<uint4*>(row + (per + tid) * 16) = make_uint4(0, 0, 0, 0);
         if (FMT == FMT_Q4) {
             // per 32 k, piece j holds the pairs (k 8t+j, k 8t+j+4), t = 0..3; the block's accumulator start goes to the table
             consumers_sync();
@@ -632,7 +633,7 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
             } else if constexpr (FMT == FMT_INT8H) {
                 const int s0 = (c * kcb) / 64;
 #pragma unroll 1
-                for (int u = set; u < cb / 64; u += 2) step_int8h<1>(lg, sw, s0 + u, u, acc[0]);
+                for (int u = set; u < (cb + 63) / 64; u += 2) step_int8h<1>(lg, sw, s0 + u, u, acc[0]);
             } else {
                 // block scales arrive by tensor copies: whole boxes, which for two weights means all
                 // gate rows first, then all up rows

@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
             // copies rows, once the launch that staged them is over; the weights of the first stages do not wait for that.
             const int xrows = (FMT == FMT_INT8 ? 3 : 1) * aM, ximg = x_stride_of(FMT, aK);
             constexpr int XB = FMT == FMT_INT8 ? 1 : 2;   // bytes per value
-            auto cols = [&](int cg) { return min(xcols, aK - cg * xcols) * XB; };
+            auto cols = [&](int cg) { return min(xcols, x_values_of(FMT, aK) - cg * xcols) * XB; };
             int tile_s = tile_first, cg = 0, stage = 0, tile_w = tile_first, cg_w = 0;
             for (int it = 0; it < n_items; ++it) {
                 if (it == 0) {
@@ -992,15 +992,20 @@ cudaError_t stream_configure() {
     return gemm_tc_configure();
 }
 
-// Shapes the streaming kernel takes: 1 <= M <= 16, rows of at least 128 bytes whose
-// length is a multiple of 64 bytes (fp16: K % 32, int8: K % 64; Q4: a multiple of 32 bytes,
-// K % 64), and 16-byte aligned operands.  Everything else goes to the generic kernel.
+// Shapes the streaming kernel takes: 1 <= M <= 16, rows of at least 128 bytes, K a multiple of 32, and 16-byte aligned operands.
+// Everything else goes to the generic kernel.  (int8 and Q4 rows of an odd number of 32 values went there too: one row of 108592 x 736 in int8
+// 80.6 us, here 17.5.  Forms whose results other ranks are sent still want whole 64-byte steps or pairs of blocks.)
 bool stream_supported(int fmt, int M, int K, const LinArgs& a) {
     if (M < 1 || M > 16) return false;
     const int rb = fmt_row_bytes(fmt, K);
-    // fp16 / int8 consume a row in 64-byte steps; a Q4 step is one 16-byte block, and its scale
-    // rows are copied in 4-byte pieces (two blocks), so Q4 rows only have to be whole pairs of blocks
-    if (rb < 128 || (rb % (fmt == FMT_Q4 ? 32 : 64)) != 0) return false;
+    // fp16 and int8 rows are consumed in 64-byte steps, of which int8 may leave the last half empty; a Q4 step is one 16-byte block,
+    // whose scales are copied in pairs unless tensor copies bring them
+    if (rb < 128 || K % 32 != 0) return false;
+    if (!stream_whole_steps(fmt, K)) {
+        const uint16_t* base[4];
+        int pitch = 0;
+        if (a.npeer > 0 || a.sig.world > 0 || (fmt == FMT_Q4 && !q4_scale_views(a, base, &pitch))) return false;
+    }
     // int8: the limb sums are 32-bit; |code| <= 128 times a limb <= 255 over K terms must stay below 2^31
     if (int8_weights(fmt) && K > 65536) return false;
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
@@ -1161,6 +1166,7 @@ cudaError_t launch_stream(int fmt, const LinArgs& a, const StreamPlan& p, cudaSt
         if (ok && dual) ok = make_scale_map(&ka.tm_s[3], sbase[3], a.seg[0].N, srow, bw, tile_rows);
         ka.scale_tma = ok ? 1 : 0;
     }
+    if (fmt == FMT_Q4 && !ka.scale_tma && !stream_whole_steps(fmt, a.K)) return cudaErrorInvalidValue;
 #define GO(F)                                                                                                  \
     if (fmt == F) {                                                                                            \
         if (dual) return nt == 2 ? launch_t<F, 2, true>(ka, p, st, pdl) : launch_t<F, 1, true>(ka, p, st, pdl); \

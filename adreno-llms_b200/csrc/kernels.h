@@ -129,6 +129,8 @@ inline int stream_format(int fmt, const LinArgs& a, int sm_count) { return fmt =
 constexpr int SK_MAX_BLOCKS = 1024;                         // grid limit of a balanced launch (sizes its scratch)
 constexpr size_t SK_SCRATCH_BYTES = (size_t)SK_MAX_BLOCKS * 128 * 16 * sizeof(float);
 bool stream_supported(int fmt, int M, int K, const LinArgs& a);
+// K a multiple of a step of 64 values (fp16: 32)
+inline bool stream_whole_steps(int fmt, int K) { return K % (fmt == FMT_FP16 ? 32 : 64) == 0; }
 StreamPlan stream_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit);
 cudaError_t launch_stream(int fmt, const LinArgs& a, const StreamPlan& p, cudaStream_t st, bool pdl);
 cudaError_t stream_configure();  // opt in to large dynamic shared memory, once per device

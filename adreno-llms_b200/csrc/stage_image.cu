@@ -45,7 +45,8 @@ __global__ void __launch_bounds__(ST_MAX) stage_image_kernel(const uint16_t* __r
     const int xstride = x_stride_of(FMT, K);
     if (FMT == FMT_FP16 || FMT == FMT_INT8H) {
         uint8_t* dst = img + (size_t)m * xstride;
-        for (int p = tid; p < K / 8; p += nthr) *reinterpret_cast<uint4*>(dst + p * 16) = *reinterpret_cast<const uint4*>(row + p * 8);
+        for (int p = tid; p < x_values_of(FMT, K) / 8; p += nthr)
+            *reinterpret_cast<uint4*>(dst + p * 16) = p < K / 8 ? *reinterpret_cast<const uint4*>(row + p * 8) : make_uint4(0, 0, 0, 0);
     } else if (FMT == FMT_INT8) {
         // the row's largest magnitude, then 24-bit fixed point in three 8-bit limbs (see stage_x_int8)
         const int per_row = K / 8;

@@ -37,7 +37,12 @@ __host__ __device__ inline int stage_bytes_of(int fmt, int kcb) {
 // Staged activations.  fp16, Q4, int8 as fp16 (FMT_INT8H, whose 8-byte loads want rows 32 bytes apart modulo 128 where ldmatrix wants
 // 16): fp16 rows; int8: three 8-bit limb planes of a 24-bit fixed-point
 // copy (row stride K + 16 bytes) followed by 192 bytes of per-row maximum and scale words.
-__host__ __device__ inline int x_stride_of(int fmt, int K) { return fmt == FMT_INT8 ? K + 16 : K * 2 + (fmt == FMT_INT8H ? 32 : 16); }
+// The values of a staged row.  An int8 step is 64 values: the second half of a row's last step may lie past the row's end, where the
+// weights are zeros (the tensor copy's fill) and the activations must be numbers: zeros, in the fp16 form (in the integer form any bytes are).
+__host__ __device__ inline int x_values_of(int fmt, int K) { return fmt == FMT_INT8H ? (K + 63) / 64 * 64 : K; }
+__host__ __device__ inline int x_stride_of(int fmt, int K) {
+    return fmt == FMT_INT8 ? K + 16 : fmt == FMT_INT8H ? x_values_of(fmt, K) * 2 + 32 : K * 2 + 16;
+}
 __host__ __device__ inline int x_bytes_of(int fmt, int M, int K) {
     return (((fmt == FMT_INT8 ? 3 * M * x_stride_of(fmt, K) + 192 : M * x_stride_of(fmt, K)) + 127) / 128) * 128;
 }
@@ -178,6 +183,10 @@ __device__ __forceinline__ void stage_x(const uint16_t* __restrict__ x, int M, i
                     *reinterpret_cast<uint4*>(xs + m * xstride + p * 16) = v[j];
                 }
             }
+        }
+        if (FMT == FMT_INT8H) {
+            const int tail = x_values_of(FMT, K) / 8 - per_row;
+            for (int i = tid; i < M * tail; i += nthreads) *reinterpret_cast<uint4*>(xs + i / tail * xstride + (per_row + i % tail) * 16) = make_uint4(0, 0, 0, 0);
         }
     } else {
         const int per_row = K / 32;
@@ -466,7 +475,7 @@ __device__ __forceinline__ void step_int8(const LaneGeo<NT>& L, uint32_t sw, int
 template <int NT>
 __device__ __forceinline__ void chunk_int8(const LaneGeo<NT>& L, uint32_t sw, int c, int kcb, int cb, int (&iacc)[3][2][NT][4]) {
     const int s0 = (c * kcb) / 64;
-    for (int s = 0; s < cb / 64; ++s) step_int8<NT>(L, sw, s0 + s, s, iacc);
+    for (int s = 0; s < (cb + 63) / 64; ++s) step_int8<NT>(L, sw, s0 + s, s, iacc);
 }
 
 // int8: recombine the limb sums, (hi * 2^16 + mid * 2^8 + lo) * 2^-p, in fp32, into acc
@@ -540,7 +549,7 @@ __device__ __forceinline__ void step_int8h(const LaneGeo<NT>& L, uint32_t sw, in
 // K chunk c.  The next unit's operands are on their way while this one's codes are converted.
 template <int NT>
 __device__ __forceinline__ void chunk_int8h(const LaneGeo<NT>& L, uint32_t sw, int c, int kcb, int cb, float (&acc)[2][2][NT][4]) {
-    const int s0 = (c * kcb) / 64, ns = cb / 64;
+    const int s0 = (c * kcb) / 64, ns = (cb + 63) / 64;
     if (ns <= 0) return;
     FragInt8H<NT> f[2];
     load_int8h<NT>(L, sw, s0, 0, f[0]);
