@@ -483,11 +483,11 @@ static void note_recorded(nn_context* c, int fmt, const LinArgs& a, const Stream
 
 // 2..16 activation rows in one launch of the batch kernel, where it takes the shape.  Two kinds of call stay two launches, which callers
 // count (nn_launch_count, nn_plan_num_recorded and the tests of both say so): a norm outside a recording, where a call costs the host as much
-// as the device, is applied by the staging launch; two rows without a norm inside a recording take that launch and the streaming kernel.
+// as the device, is applied by the staging launch; a plain projection of two rows inside a recording takes that launch and the streaming kernel.
 static int run_batch(nn_context* c, int fmt, LinArgs a, int M, const char* who, bool* done) {
     *done = false;
     a.M = M;
-    if (M == 2 && !a.norm_w && c->capturing) return NN_OK;
+    if (M == 2 && !a.norm_w && a.epi == EPI_STORE && c->capturing) return NN_OK;
     const uint16_t* norm_w = c->capturing ? nullptr : a.norm_w;
     const int pitch = stage_row_bytes(a.K);
     if (norm_w) {

@@ -357,6 +357,9 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
     else if (tid < 2 * BATCH_STAGES) mbar_init(full0 + tid * 8, (uint32_t)BCW);
     else if (tid == 2 * BATCH_STAGES) mbar_init(xbar, 1u);
     mbar_init_fence();
+    // Absent rows are zeros, but not by the copy: 128 bytes past the end take it five times as long as those that are there (9 rows of a
+    // 24-layer, 896-wide int8 model 613 us with boxes of 16 rows, 493 so; 2 rows of a 16-layer, 1024-wide Q4 one 440 and 316).
+    for (uint32_t i = (uint32_t)(M * xpitch + tid * 16); i < (uint32_t)(8 * NT * xpitch); i += BATCH_THREADS * 16) *reinterpret_cast<uint4*>(sm + OFF_X + i) = make_uint4(0, 0, 0, 0);
     __syncthreads();
 
     auto segment = [&](int tile) { return (a.nseg > 2 && tile >= a.seg[2].tile0) ? 2 : (a.nseg > 1 && tile >= a.seg[1].tile0) ? 1 : 0; };
@@ -377,9 +380,9 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
             if (it == ahead) {
                 pdl_wait_prior_grid();
                 if (lane == 0) {
-                    // One copy for all rows, absent ones as zeros.  A copy takes some 50 clocks to issue, whatever its size: 16 rows of
+                    // One copy for all rows.  A copy takes some 50 clocks to issue, whatever its size: 16 rows of
                     // 896 values are there after 1330 clocks, as pieces of 1 KB after 2900 (155 KB: 2600 and 10000).
-                    mbar_arrive_expect_tx(xbar, (uint32_t)(8 * NT * xpitch + (a.norm_w ? K * 2 : 0)));
+                    mbar_arrive_expect_tx(xbar, (uint32_t)(M * xpitch + (a.norm_w ? K * 2 : 0)));
                     tma_load_3d(base + OFF_X, &km.x, 0, 0, 0, xbar, l2_policy_evict_normal());
                     if (a.norm_w) bulk_g2s(base + a.off_red, a.norm_w, (uint32_t)K * 2u, xbar, l2_policy_evict_normal());   // (the sums come later)
                 }
@@ -668,7 +671,7 @@ cudaError_t launch_f(const LinArgs& a, const BatchPlan& p, cudaStream_t st, bool
         if (!weight_map(&km.tm[i], a.seg[i].W, a.seg[i].N)) return cudaErrorInvalidValue;
     }
     if (dual && !weight_map(&km.tm[3], a.W2, a.seg[0].N)) return cudaErrorInvalidValue;
-    if (!make_rows_map(&km.x, a.x, a.M, a.K * 2, a.x_pitch ? a.x_pitch : a.K * 2, p.xcols, a.M > 8 ? 16 : 8)) return cudaErrorInvalidValue;
+    if (!make_rows_map(&km.x, a.x, a.M, a.K * 2, a.x_pitch ? a.x_pitch : a.K * 2, p.xcols, a.M)) return cudaErrorInvalidValue;
     if (!fill_scale_maps(km, a, p.cols * 16, tile_rows)) return cudaErrorInvalidValue;
     b.scale2 = a.scale2;
     b.norm_w = a.norm_w;
@@ -730,7 +733,7 @@ BatchPlan batch_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit)
     // 1024 x 4608, 8 rows, 8.4 -> 7.4 us.  Rows of one stage gain nothing (1024 x 1024: 3.3 against 3.5 us).
     if (!dual && groups > 1 && count_tiles(a, WARP_ROWS) * 2 <= sm_count) p.tile_rows = 16;
     p.ntiles = count_tiles(a, p.tile_rows);
-    p.cols = NCW * (p.kcb / 128);
+    p.cols = groups == 1 ? (rb + 127) / 128 : NCW * (p.kcb / 128);   // (not more than there are: what lies past the end takes a copy long)
     p.xcols = batch_xcols(fmt, a.K);
     if (a.K % 64 != 0 || p.xcols > 256 || p.cols * 16 > 256) return p;   // one copy's reach
     if (a.norm_w && a.K * 2 > BCW * 8 * nt * RED_TS * 4) return p;       // the norm weight lies where the sums will
