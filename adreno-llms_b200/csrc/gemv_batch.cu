@@ -711,9 +711,10 @@ cudaError_t batch_configure() {
 
 // Which batched calls this kernel takes: those that the streaming kernel takes with K split, whose activations are whole 128-byte columns and fit
 // in shared memory beside two stages of weights, and (Q4) whose block scales can be reached by tensor copies.  The K parts are the single call's.
-// Not Q4 above 8 rows: a block's two token tiles make its chain of loads and MMAs the longer one (9 rows of a 17-layer, 1216-wide
-// model 792 us here, 584 with the staging launch; 12 rows of 768: 215 and 206).  Nor whole-row tiles (an lm_head): the finish there needs
-// no meeting of warps in the streaming kernel (16 rows of 151936 x 896: fp16 48 us in both; 8 rows of 65536 x 1024 in Q4 20.6 against 16.5).
+// Not Q4 gate and up of more than 8 rows without a norm (12 rows of 3000 x 2048: 8.9 us here, 8.4 with the staging launch; in steps, with the
+// norm, they are better here: 9 rows of a 16-layer, 1024-wide model 414 us, 432 with the staging launch for normed operators).
+// Nor whole-row tiles (an lm_head): the finish there needs no meeting of warps in the streaming kernel (16 rows of 151936 x 896 in fp16: 48 us in
+// both; 8 rows of 65536 x 1024 in Q4 20.6 against 16.5).
 BatchPlan batch_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit) {
     BatchPlan p = {};
     if (a.M < 2 || a.npeer > 0 || a.sig.world > 0 || a.argmax_slot || !stream_supported(fmt, a.M, a.K, a)) return p;
@@ -723,7 +724,11 @@ BatchPlan batch_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit)
     int pitch = 0;
     if (fmt == FMT_Q4 && !q4_scale_views(a, base, &pitch)) return p;
     const StreamPart part = stream_part(fmt, a, sm_count);
-    if (part.kw == 1 || (fmt == FMT_Q4 && a.M > 8)) return p;
+    if (part.kw == 1) return p;
+    if (fmt == FMT_Q4 && a.M > 8 && !a.norm_w && a.epi == EPI_SWIGLU) {
+        const StreamPlan sp = stream_plan(fmt, a, sm_count, smem_limit);
+        if (sp.ok && sp.kcb == part.kcb) return p;   // (rows so long that it takes smaller chunks, and so other sums, stay here)
+    }
     const bool dual = a.epi == EPI_SWIGLU;
     const int rb = fmt_row_bytes(fmt, a.K), nt = a.M > 8 ? 2 : 1, warp_rows = dual ? 16 : WARP_ROWS;
     p.kcb = part.kcb;
