@@ -391,7 +391,7 @@ __device__ __forceinline__ bool stage_fast(const PlanParams& P, const PlanOpScal
 #pragma unroll
         for (int j = 0; j < PIECES; ++j)
             if ((have >> j) & 1u) *reinterpret_cast<uint4*>(row + (tid + j * nthr) * 16) = make_uint4(w[j][0], w[j][1], w[j][2], w[j][3]);
-        if (FMT == FMT_INT8H && per + tid < x_values_of(FMT, D.K) / 8) *reinterpret_cast<uint4*>(row + (per + tid) * 16) = make_uint4(0, 0, 0, 0);
+    if (FMT == FMT_INT8H && (D.K & 63) != 0 && tid < 4) *reinterpret_cast<uint4*>(row + (per + tid) * 16) = make_uint4(0, 0, 0, 0);   // (half a step)
         if (FMT == FMT_Q4) {
             // per 32 k, piece j holds the pairs (k 8t+j, k 8t+j+4), t = 0..3; the block's accumulator start goes to the table
             consumers_sync();

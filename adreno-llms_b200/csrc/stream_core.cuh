@@ -497,7 +497,7 @@ __device__ __forceinline__ void int8_recombine(const int (&iacc)[3][2][NT][4], f
 // 16-byte piece of rows g and g + 8; as fp16 (exact) they are its two A registers per row of a k16 step whose k order is (4t, 4t+1)
 // for the first pairs and (4t+2, 4t+3) for the second, so the B registers are four neighbouring activations: one 8-byte load.
 // Against integer MMAs with limbs (above) there is no copy of the row to build (its maximum, the split: two barriers) and two bytes of
-// shared memory per activation instead of three: a recorded token of a 30-layer, 576-wide model 370 -> 319 us.
+// shared memory per activation instead of three: a recorded token of a 30-layer, 576-wide model 370 -> 324 us.
 //
 // The four MMAs of a unit start from zero and their sum is added in fp32: the tensor core cuts off what lies below its running sum
 // instead of rounding, so a chain over a long row would lose more than the additions do.
