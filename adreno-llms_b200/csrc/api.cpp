@@ -515,10 +515,9 @@ static int run_batch(nn_context* c, int fmt, LinArgs a, int M, const char* who, 
     return NN_OK;
 }
 
-static int run_linear(nn_context* c, int weight_fmt, LinArgs a, int M_total, const char* who) {
+static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char* who) {
     a.sk_scratch = c->sk_scratch;
     a.sk_flags = c->sk_flags;
-    int fmt = M_total <= 16 ? stream_format(weight_fmt, a, c->sm_count) : weight_fmt;
     if (M_total >= 2 && M_total <= 16) {
         bool done = false;
         const int rc = run_batch(c, fmt, a, M_total, who, &done);
@@ -556,7 +555,6 @@ static int run_linear(nn_context* c, int weight_fmt, LinArgs a, int M_total, con
         bool done = false;
         const int rc = run_gemm_tc(c, fmt, a, M_total, who, &done);
         if (rc != NN_OK || done) return rc;
-        fmt = stream_format(weight_fmt, a, c->sm_count);
     }
     // M > 16 is walked in slices of 16 activation rows (each slice re-streams the weights).
     const uint16_t* x0 = a.x;
@@ -614,7 +612,7 @@ static int run_linear(nn_context* c, int weight_fmt, LinArgs a, int M_total, con
         } else {
             if (a.npeer > 0)
                 return NN_FAIL(NN_ERR_UNSUPPORTED, "%s: this shape takes the any-shape kernel, which does not write to peer ranks (K=%d)", who, a.K);
-            e = launch_generic(weight_fmt, a, c->stream);
+            e = launch_generic(fmt, a, c->stream);
         }
         if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: launch failed: %s (M=%d K=%d)", who, cudaGetErrorString(e), a.M, a.K);
         c->launches++;
@@ -897,7 +895,7 @@ int nnb::linear_argmax(nn_context* c, int N, int K, nn_buf x, nn_buf W, nn_buf l
     a.sk_scratch = c->sk_scratch;
     a.sk_flags = c->sk_flags;
     StreamPlan p = {};
-    const int fmt = stream_format(r.fmt, a, c->sm_count);
+    const int fmt = r.fmt;
     if (stream_supported(fmt, 1, K, a) && (stream_whole_steps(fmt, K) || (logits && !sig))) p = stream_plan(fmt, a, c->sm_count, c->smem_limit);
     if (!p.ok) {
         // shapes the streaming kernel does not take: projection, then the separate arg-max

@@ -26,9 +26,7 @@
 //   * the arithmetic is the separate launch's (stream_core.cuh), on the same K partition and in the
 //     same order, so a run gives the same bits as the operators launched one by one.  A per-layer
 //     operator is bound by latency, not by its weight stream, so a block has eight consumer warps: a
-//     tile whose K is split has eight K parts and every warp takes one of them; int8 weights of such
-//     tiles are multiplied with the fp16 activations as they are (no fixed-point copy to build once the
-//     activations arrive).  What does not depend on the activations (descriptor, norm weight, row
+//     tile whose K is split has eight K parts and every warp takes one of them.  What does not depend on the activations (descriptor, norm weight, row
 //     scales, the values an in-place epilogue updates, the tile's weights) is fetched or waited for
 //     before the wait for them, so that little is left to do once they are there;
 //   * every wait (ring slot, weights, activations) is bounded; when one runs out the block records
@@ -256,8 +254,8 @@ __device__ __forceinline__ bool fetch_piece(const unsigned long long* ll, int p,
 }
 
 // The operator's activation row, from the other blocks' words (or memory) to its staged form, with the RMSNorm when asked: the
-// row stays in registers from the first look at the words to the staged stores, so that one barrier, two (whole-row int8
-// tiles: the row's largest magnitude) or one more (the norm's sum of squares) are all that stands between the arrival of the last word and
+// row stays in registers from the first look at the words to the staged stores, so that one barrier (fp16), two (int8: the
+// row's largest magnitude) or one more (the norm's sum of squares) are all that stands between the arrival of the last word and
 // the first matrix instruction.  Rows of up to PIECES pieces per thread (plan_stage_fast); longer ones take stage_general.
 //
 // This is the step's critical path, and it runs once per operator: what it costs is its instruction count, cold.  The version
@@ -351,47 +349,31 @@ __device__ __forceinline__ bool stage_fast(const PlanParams& P, const PlanOpScal
 #pragma unroll
         for (int j = 0; j < PIECES; ++j)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) mx = max(mx, max(w[j][q] & 0x7FFFu, (w[j][q] >> 16) & 0x7FFFu));
-        mx = __reduce_max_sync(0xffffffffu, mx);
+            for (int q = 0; q < 4; ++q) mx = half2_magnitude_max(mx, w[j][q]);
+        mx = __reduce_max_sync(0xffffffffu, max(mx & 0xFFFFu, mx >> 16));
         unsigned* wmax = reinterpret_cast<unsigned*>(red) + 16;
         if (lane == 0) wmax[warp] = mx;
         consumers_sync();
         const uint4 m0 = *reinterpret_cast<const uint4*>(wmax), m1 = *reinterpret_cast<const uint4*>(wmax + 4);
         mx = max(max(max(m0.x, m0.y), max(m0.z, m0.w)), max(max(m1.x, m1.y), max(m1.z, m1.w)));
-        const bool bad = mx >= 0x7C00u;
-        const int e = (int)(mx >> 10) > 0 ? (int)(mx >> 10) - 15 : -14;
-        const int pw = (mx == 0u || bad) ? 0 : 22 - e;
-        const float up = __int_as_float((127 + pw) << 23);
-        if (tid == 0) *reinterpret_cast<float*>(xs + 3 * xstride + 64) = bad ? __int_as_float(0x7FC00000) : __int_as_float((127 - pw) << 23);
+        float up, down;
+        int8_row_scale(mx, up, down);
+        if (tid == 0) *reinterpret_cast<float*>(xs + 3 * xstride + 64) = down;
 #pragma unroll
         for (int j = 0; j < PIECES; ++j) {
             if (!((have >> j) & 1u)) continue;
-            uint32_t l[3][2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                int f[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint32_t v = w[j][h * 2 + (i >> 1)];
-                    f[i] = bad ? 0 : __float2int_rn(__half2float(__ushort_as_half((uint16_t)(i & 1 ? v >> 16 : v & 0xFFFFu))) * up);
-                }
-                // bytes b of the four values side by side
-#pragma unroll
-                for (int b = 0; b < 3; ++b)
-                    l[b][h] = __byte_perm(__byte_perm((uint32_t)f[0], (uint32_t)f[1], (uint32_t)(b | ((b + 4) << 4))),
-                                          __byte_perm((uint32_t)f[2], (uint32_t)f[3], (uint32_t)(b | ((b + 4) << 4))), 0x5410u);
-            }
+            uint32_t a[3], b[3];
+            int8_limbs(w[j][0], w[j][1], up, a);
+            int8_limbs(w[j][2], w[j][3], up, b);
             uint8_t* dst = xs + (tid + j * nthr) * 8;
-            *reinterpret_cast<uint2*>(dst) = make_uint2(l[2][0], l[2][1]);
-            *reinterpret_cast<uint2*>(dst + xstride) = make_uint2(l[1][0], l[1][1]);
-            *reinterpret_cast<uint2*>(dst + 2 * xstride) = make_uint2(l[0][0], l[0][1]);
+#pragma unroll
+            for (int l = 0; l < 3; ++l) *reinterpret_cast<uint2*>(dst + l * xstride) = make_uint2(a[l], b[l]);
         }
     } else {
-        uint8_t* row = FMT != FMT_Q4 ? xs : smem + P.off_xraw;
+        uint8_t* row = FMT == FMT_FP16 ? xs : smem + P.off_xraw;
 #pragma unroll
         for (int j = 0; j < PIECES; ++j)
             if ((have >> j) & 1u) *reinterpret_cast<uint4*>(row + (tid + j * nthr) * 16) = make_uint4(w[j][0], w[j][1], w[j][2], w[j][3]);
-    if (FMT == FMT_INT8H && (D.K & 63) != 0 && tid < 4) *reinterpret_cast<uint4*>(row + (per + tid) * 16) = make_uint4(0, 0, 0, 0);   // (half a step)
         if (FMT == FMT_Q4) {
             // per 32 k, piece j holds the pairs (k 8t+j, k 8t+j+4), t = 0..3; the block's accumulator start goes to the table
             consumers_sync();
@@ -536,8 +518,8 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
         sg = D.seg[seg_i];
         row0 = (tile - sg.tile0) * tile_rows + wrow_off;
         // int8 row scales: with the tile's last item when its rows allow a bulk copy, else from memory now
-        scales_ride = int8_weights(FMT) && row_scales && plan_rows_bulk_ok(min(tile_rows, sg.N - (tile - sg.tile0) * tile_rows));
-        if (writer && int8_weights(FMT) && !scales_ride) {
+        scales_ride = FMT == FMT_INT8 && row_scales && plan_rows_bulk_ok(min(tile_rows, sg.N - (tile - sg.tile0) * tile_rows));
+        if (writer && FMT == FMT_INT8 && !scales_ride) {
             if (DUAL) {
                 const int n = min(row0 + (lane & 15), sg.N - 1);
                 sc1 = sg.scale[n];
@@ -611,7 +593,7 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
             if (tile != tile_first || cg != 0) claim_item(off, slot);
             const uint32_t sw = ring + (uint32_t)off;
             const int cb = (S.failed || !active) ? 0 : min(kcb, rowbytes - c * kcb);
-            if (int8_weights(FMT) && scales_ride && writer && cg == groups - 1) {
+            if (FMT == FMT_INT8 && scales_ride && writer && cg == groups - 1) {
                 const uint16_t* sc = reinterpret_cast<const uint16_t*>(smem + ring_off + off + scale_off);
                 if (DUAL) {
                     sc1 = sc[wrow_off + (lane & 15)];
@@ -629,11 +611,13 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
                     chunk_fp16<1>(lg, sw, c, kcb, cb, acc);
                 }
             } else if constexpr (FMT == FMT_INT8) {
-                chunk_int8<1>(lg, sw, c, kcb, cb, iacc);
-            } else if constexpr (FMT == FMT_INT8H) {
-                const int s0 = (c * kcb) / 64;
+                if constexpr (WIDE) {
+                    const int s0 = (c * kcb) / 64;
 #pragma unroll 1
-                for (int u = set; u < (cb + 63) / 64; u += 2) step_int8h<1>(lg, sw, s0 + u, u, acc[0]);
+                    for (int u = set; u < (cb + 63) / 64; u += 2) step_int8<1>(lg, sw, s0 + u, u, iacc);
+                } else {
+                    chunk_int8<1>(lg, sw, c, kcb, cb, iacc);
+                }
             } else {
                 // block scales arrive by tensor copies: whole boxes, which for two weights means all
                 // gate rows first, then all up rows
@@ -659,29 +643,42 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
         float v0, v1 = 0.f;  // v1: the second weight's sum (two-weight epilogue)
         if constexpr (WIDE) {
             // The eight K parts meet in shared memory.  Per consumer of the separate launch (quarter) the
-            // two sets are added first, then the quarters in order.
+            // two sets are added first, then the quarters in order; int8 parts are exact integer limb
+            // sums, added as integers and turned into a float once per quarter, as that consumer does.
             const int r0 = DUAL ? (lane & 15) : lane;
-            float* buf = red + (S.ti & 1) * (KPARTS * 32);
+            constexpr int LIMBS = IMMA ? 3 : 1;
+            float* buf = red + (S.ti & 1) * (KPARTS * LIMBS * 32);
             if (t == 0) {
-                float* mine = buf + warp * 32 + g;
-                mine[0] = acc[0][0][0][0];
-                mine[8] = acc[0][0][0][2];
-                mine[16] = acc[0][1][0][0];
-                mine[24] = acc[0][1][0][2];
+#pragma unroll
+                for (int l = 0; l < LIMBS; ++l) {
+                    float* mine = buf + (warp * LIMBS + l) * 32 + g;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) mine[i * 8] = IMMA ? __int_as_float(iacc[l][i >> 1][0][2 * (i & 1)]) : acc[0][i >> 1][0][2 * (i & 1)];
+                }
             }
             consumers_sync();
             tile += G;
-            if (warp != 0) {
+            if (warp != 0) {   // the first warp finishes the tile; the others go on to the block's next one
                 if (tile < ntiles) tile_prologue(tile, false);
                 continue;
             }
-            v0 = buf[r0] + buf[32 + r0];
+            auto quarter_sum = [&](int q, int r) {
+                const float* a = buf + 2 * q * LIMBS * 32 + r;
+                const float* b2 = a + LIMBS * 32;
+                if constexpr (IMMA) {
+                    auto limb = [&](int l) { return (float)(__float_as_int(a[l * 32]) + __float_as_int(b2[l * 32])); };
+                    return fmaf(limb(0), 65536.f, fmaf(limb(1), 256.f, limb(2))) * rowscale[0] + 0.f;  // (+ 0: the consumer adds its empty second set)
+                } else {
+                    return a[0] + b2[0];
+                }
+            };
+            v0 = quarter_sum(0, r0);
 #pragma unroll
-            for (int q = 1; q < NCW; ++q) v0 += buf[(2 * q) * 32 + r0] + buf[(2 * q + 1) * 32 + r0];
+            for (int q = 1; q < NCW; ++q) v0 += quarter_sum(q, r0);
             if (DUAL) {
-                v1 = buf[16 + r0] + buf[32 + 16 + r0];
+                v1 = quarter_sum(0, 16 + r0);
 #pragma unroll
-                for (int q = 1; q < NCW; ++q) v1 += buf[(2 * q) * 32 + 16 + r0] + buf[(2 * q + 1) * 32 + 16 + r0];
+                for (int q = 1; q < NCW; ++q) v1 += quarter_sum(q, 16 + r0);
             }
         } else {
             if constexpr (IMMA) int8_recombine<1>(iacc, acc[0], rowscale, 1, t);
@@ -964,13 +961,13 @@ __global__ void __launch_bounds__(PLAN_BLOCK, 1) decode_plan_kernel(const __grid
         const PlanOpScalars& D = dbuf[cur];
         const int nxt = next_op(op);
         if (nxt < nops) fetch_desc(nxt, cur ^ 1);
-        // tiles that split K take the sixteen-part path, as in the separate launch
+        // tiles that split K take the eight-part path, with the sums of the separate launch
         const int sel = D.fmt * 2 + (D.ksplit ? 1 : 0);
         switch (sel) {
             case FMT_FP16 * 2: run_op<FMT_FP16, false>(P, D, op, smem, tid, lane, warp); break;
             case FMT_FP16 * 2 + 1: run_op<FMT_FP16, true>(P, D, op, smem, tid, lane, warp); break;
             case FMT_INT8 * 2: run_op<FMT_INT8, false>(P, D, op, smem, tid, lane, warp); break;
-            case FMT_INT8H * 2 + 1: run_op<FMT_INT8H, true>(P, D, op, smem, tid, lane, warp); break;
+            case FMT_INT8 * 2 + 1: run_op<FMT_INT8, true>(P, D, op, smem, tid, lane, warp); break;
             case FMT_Q4 * 2: run_op<FMT_Q4, false>(P, D, op, smem, tid, lane, warp); break;
             default: run_op<FMT_Q4, true>(P, D, op, smem, tid, lane, warp); break;
         }

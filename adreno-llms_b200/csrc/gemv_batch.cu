@@ -12,10 +12,11 @@
 //     per warp (16 rows of 896 values: 2500 clocks), and the accumulator starts of Q4 blocks are summed there;
 //   * eight consumer warps, one per K part of a tile: a warp multiplies every second unit of its K chunks;
 //   * a stage's weights are one copy too where the rows are whole columns (a copy takes some 50 clocks to issue);
-//   * what the waits do not hold up (places of operands, scales, biases) is worked out before them, and no register is spilled: with
-//     100 bytes of spills the 16-row step of a 24-layer, 896-wide int8 model took 880 us instead of 540.
-// Steps of 16 rows of that model (staging launch + streaming kernel before): int8 774 -> 540 us, fp16 1063 -> 610; 8 rows of a 16-layer,
-// 1024-wide Q4 model 396 -> 364; 4 rows of a 30-layer, 576-wide int8 model 543 -> 400.
+//   * what the waits do not hold up (places of operands, scales, biases) is worked out before them, and no register is spilled;
+//   * int8 has eight rows of activations per block at most, and two blocks per tile for 9..16: its exact sums are 24 registers per
+//     lane and eight rows (with 16 rows in a block, 48 registers of sums and some spills, the step below took 830 us).
+// Steps of 16 rows of a 24-layer, 896-wide model (staging launch + streaming kernel before): int8 771 -> 620 us, fp16 1063 -> 610; 8 rows
+// of a 16-layer, 1024-wide Q4 model 396 -> 364; 4 rows of a 30-layer, 576-wide int8 model 540 -> 449.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -32,8 +33,19 @@ constexpr int BCW = KPARTS;                  // consumer warps
 constexpr int BATCH_THREADS = BCW * 32 + 32; // + the producer warp
 constexpr int BATCH_STAGES = 6;              // ring stages at most
 constexpr int OFF_BARS = HDR_BYTES;          // full[], empty[], and one for the activations
+constexpr int OFF_SCALE = 512;               // int8: 2^p of the 16 rows, then 2^-p
+constexpr int OFF_ROW = 640;                 // int8: a tile's 32 weight-row scales, then what is added or the second weight's scales
 constexpr int OFF_X = 1024;                  // (128-byte swizzle: 1 KB boundaries)
-static_assert(OFF_BARS + (2 * BATCH_STAGES + 1) * 8 <= OFF_X, "barriers");
+static_assert(OFF_BARS + (2 * BATCH_STAGES + 1) * 8 <= OFF_SCALE && OFF_SCALE + 128 <= OFF_ROW && OFF_ROW + 256 <= OFF_X, "header");
+
+// Where the parts of a tile meet: fp32 sums as [part][token][row].  int8: a chunk's pair of warps adds its limb sums first, 24 (times NT)
+// integers per lane in the region that then takes the pair's fp32 sums.
+constexpr int PAIR_INTS = 3 * 2 * 4 * 32;    // (times NT)
+__host__ __device__ constexpr int batch_part_words(int fmt, int nt) { return fmt == FMT_INT8 ? PAIR_INTS / 2 * nt : 8 * nt * RED_TS; }
+__host__ __device__ constexpr int batch_red_bytes(int fmt, int nt) { return BCW * batch_part_words(fmt, nt) * 4; }
+static_assert(2 * batch_part_words(FMT_INT8, 1) >= 8 * RED_TS, "a pair's sums fit where its integers were");
+// (the norm weight lies there first, and is read in whole passes of 32 pieces)
+static_assert(batch_red_bytes(FMT_FP16, 1) % 512 == 0 && batch_red_bytes(FMT_INT8, 1) % 512 == 0, "norm weight");
 
 struct BatchSeg {
     const uint16_t* scale;
@@ -49,6 +61,7 @@ struct BatchArgs {
     float norm_eps;
     int M, K, epi, nseg, ntiles, tile_rows;
     int kcb, nchunks, groups, rowbytes;
+    int halves;                   // blocks 2 i and 2 i + 1 share the tiles of block i, eight activation rows each
     int cols, wide;               // columns of 128 bytes of a weight's rows in a stage; whether one copy brings them all
     int xcols;                    // columns of 128 bytes of an activation row in shared memory
     int stages, stage_bytes, evict_first;
@@ -69,7 +82,7 @@ __device__ __forceinline__ const CUtensorMap* batch_scale_map(const BatchMapsQ4&
 __host__ __device__ inline int batch_xcols(int fmt, int K) {
     const int n = K / 64;
     if (fmt == FMT_FP16) return n | 1;
-    if (fmt == FMT_INT8H) return (n + 1) / 4 * 4 + 2;
+    if (fmt == FMT_INT8) return (n + 1) / 4 * 4 + 2;
     return (n + 3) / 8 * 8 + 4;
 }
 
@@ -238,14 +251,32 @@ struct BatchGeo {
     bool two;              // both row blocks
 };
 
-// One unit (stream_core.cuh: step_fp16, step_int8, block_q4; the same products in the same order): i counts the warp's units of the chunk,
+// int8: the scales 2^p and 2^-p of one row from its largest magnitude (stream_core.cuh), by one warp; the row is `bytes` long at `row`.
+__device__ __forceinline__ void batch_row_scale(uint32_t row, int bytes, float* scale, int m, int lane) {
+    uint32_t mx = 0u;
+#pragma unroll 4
+    for (int o = lane * 16; o < bytes; o += 512) {
+        uint32_t v[4];
+        lds_v4(row + o, v);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) mx = half2_magnitude_max(mx, v[q]);
+    }
+    float up, down;
+    int8_row_scale(__reduce_max_sync(0xffffffffu, max(mx & 0xFFFFu, mx >> 16)), up, down);
+    if (lane == 0) {
+        scale[m] = up;
+        scale[16 + m] = down;
+    }
+}
+
+// One unit (stream_core.cuh: step_fp16, block_q4; the same products in the same order): i counts the warp's units of the chunk,
 // s the row's units.  Loads and arithmetic are apart so that two units' loads can be on their way together.
-template <int FMT, int NT>
+template <int NT>
 struct BatchFrag {
-    uint32_t w[2][2][4], b[4][NT][2];   // [32-byte half][row block]; [k16 step] (fp16: two steps)
+    uint32_t w[2][2][4], b[2][NT][2];   // [32-byte half][row block]; [k16 step]
 };
-template <int FMT, int NT>
-__device__ __forceinline__ void batch_load(const BatchGeo<NT>& L, uint32_t sw, int i, int s, BatchFrag<FMT, NT>& f) {
+template <int NT>
+__device__ __forceinline__ void batch_load(const BatchGeo<NT>& L, uint32_t sw, int i, int s, BatchFrag<NT>& f) {
     const uint32_t col = sw + (uint32_t)i * L.col_bytes;
 #pragma unroll
     for (int h = 0; h < 2; ++h) ldsm_x4(col + L.a0 + (L.a_off ^ (32u * h)), f.w[h][0][0], f.w[h][0][1], f.w[h][0][2], f.w[h][0][3]);
@@ -253,45 +284,48 @@ __device__ __forceinline__ void batch_load(const BatchGeo<NT>& L, uint32_t sw, i
 #pragma unroll
         for (int h = 0; h < 2; ++h) ldsm_x4(col + L.a0 + L.up + (L.a_off ^ (32u * h)), f.w[h][1][0], f.w[h][1][1], f.w[h][1][2], f.w[h][1][3]);
     }
-    if constexpr (FMT == FMT_FP16) {
-        const uint32_t off = (uint32_t)(s >> 1) * 128u + ((L.b_q ^ ((L.b_x + (uint32_t)(s >> 1)) & 7u)) << 4);
+    const uint32_t off = (uint32_t)(s >> 1) * 128u + ((L.b_q ^ ((L.b_x + (uint32_t)(s >> 1)) & 7u)) << 4);
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) ldsm_x4(L.b + nt * L.b_up + off, f.b[0][nt][0], f.b[0][nt][1], f.b[1][nt][0], f.b[1][nt][1]);
-    } else {
-        const uint32_t x = (L.b_x + (uint32_t)s) & 7u, at = (uint32_t)s * 128u + (L.b_q & 1u) * 8u;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) lds_v2(L.b + nt * L.b_up + at + (((2u * j + (L.b_q >> 1)) ^ x) << 4), f.b[j][nt][0], f.b[j][nt][1]);
-    }
+    for (int nt = 0; nt < NT; ++nt) ldsm_x4(L.b + nt * L.b_up + off, f.b[0][nt][0], f.b[0][nt][1], f.b[1][nt][0], f.b[1][nt][1]);
 }
-template <int FMT, int NT>
-__device__ __forceinline__ void batch_mac(const BatchFrag<FMT, NT>& f, bool two, float (&ac)[2][NT][4]) {
+template <int NT>
+__device__ __forceinline__ void batch_mac(const BatchFrag<NT>& f, bool two, float (&ac)[2][NT][4]) {
 #pragma unroll
     for (int rb = 0; rb < 2; ++rb) {
         if (rb == 1 && !two) continue;
-        if constexpr (FMT == FMT_FP16) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt) mma_16816(ac[rb][nt], f.w[h][rb][0], f.w[h][rb][1], f.w[h][rb][2], f.w[h][rb][3], f.b[h][nt][0], f.b[h][nt][1]);
-        } else {
-            float d[NT][4];
+            for (int nt = 0; nt < NT; ++nt) mma_16816(ac[rb][nt], f.w[h][rb][0], f.w[h][rb][1], f.w[h][rb][2], f.w[h][rb][3], f.b[h][nt][0], f.b[h][nt][1]);
+    }
+}
+// int8: one unit of 64 values.  The codes go into the integer MMAs as they are; the limbs of the activations (stream_core.cuh: int8_limbs) are
+// made here from the fp16 rows: each value belongs to one warp of the tile, and the limb planes of 16 rows would take half as much
+// shared memory again as the rows.  Four neighbouring values are the four bytes of a lane's B register, so there is nothing to exchange.
+template <int NT>
+__device__ __forceinline__ void batch_unit_int8(const BatchGeo<NT>& L, uint32_t sw, int i, int s, const float (&up)[NT], int (&ac)[3][2][NT][4]) {
+    const uint32_t col = sw + (uint32_t)i * L.col_bytes, x = (L.b_x + (uint32_t)s) & 7u, at = (uint32_t)s * 128u + (L.b_q & 1u) * 8u;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                uint32_t a0, a1, a2, a3;
-                int8x4_to_half2x2(f.w[j / 2][rb][2 * (j & 1)], a0, a2);
-                int8x4_to_half2x2(f.w[j / 2][rb][2 * (j & 1) + 1], a1, a3);
+    for (int h = 0; h < 2; ++h) {
+        uint32_t w[2][4], v[NT][2][2];
+        ldsm_x4(col + L.a0 + (L.a_off ^ (32u * h)), w[0][0], w[0][1], w[0][2], w[0][3]);
+        if (L.two) ldsm_x4(col + L.a0 + L.up + (L.a_off ^ (32u * h)), w[1][0], w[1][1], w[1][2], w[1][3]);
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    if (j == 0) mma_16816_c(d[nt], a0, a1, a2, a3, f.b[j][nt][0], f.b[j][nt][1], make_float4(0.f, 0.f, 0.f, 0.f));
-                    else mma_16816(d[nt], a0, a1, a2, a3, f.b[j][nt][0], f.b[j][nt][1]);
-                }
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) lds_v2(L.b + nt * L.b_up + at + (((2u * (2 * h + j) + (L.b_q >> 1)) ^ x) << 4), v[nt][j][0], v[nt][j][1]);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            uint32_t b[2][3];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) int8_limbs(v[nt][j][0], v[nt][j][1], up[nt], b[j]);
+#pragma unroll
+            for (int rb = 0; rb < 2; ++rb) {
+                if (rb == 1 && !L.two) continue;
+                imma_16832<true>(ac[0][rb][nt], w[rb][0], w[rb][1], w[rb][2], w[rb][3], b[0][0], b[1][0]);
+                imma_16832<false>(ac[1][rb][nt], w[rb][0], w[rb][1], w[rb][2], w[rb][3], b[0][1], b[1][1]);
+                imma_16832<false>(ac[2][rb][nt], w[rb][0], w[rb][1], w[rb][2], w[rb][3], b[0][2], b[1][2]);
             }
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-                for (int k = 0; k < 4; ++k) ac[rb][nt][k] += d[nt][k];
         }
     }
 }
@@ -345,7 +379,11 @@ template <int FMT, int NT>
 __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __grid_constant__ typename BatchMapsFor<FMT>::type km, const BatchArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int M = a.M, K = a.K, stages = a.stages, ntiles = a.ntiles, groups = a.groups, kcb = a.kcb, rowbytes = a.rowbytes, nchunks = a.nchunks;
+    // Token halves (int8, 9..16 rows): the second block of a pair takes the last eight rows, and stores those from the ninth on.
+    const bool halves = FMT == FMT_INT8 && a.halves;
+    const int bx = halves ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, gx = halves ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+    const int m_off = halves && (blockIdx.x & 1u) ? a.M - 8 : 0, m_lo = m_off ? 8 - m_off : 0;   // first row here; first one that is stored
+    const int M = halves ? 8 : a.M, K = a.K, stages = a.stages, ntiles = a.ntiles, groups = a.groups, kcb = a.kcb, rowbytes = a.rowbytes, nchunks = a.nchunks;
     const bool dual = a.epi == EPI_SWIGLU;
     const int tile_rows = a.tile_rows;
     const uint32_t base = (smem_u32(smem) + 1023u) & ~1023u;
@@ -356,6 +394,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
     if (tid < BATCH_STAGES) mbar_init(full0 + tid * 8, 1u);
     else if (tid < 2 * BATCH_STAGES) mbar_init(full0 + tid * 8, (uint32_t)BCW);
     else if (tid == 2 * BATCH_STAGES) mbar_init(xbar, 1u);
+    if (FMT == FMT_INT8 && tid < 32) reinterpret_cast<float*>(sm + OFF_SCALE)[tid] = 1.f;   // (absent rows)
     mbar_init_fence();
     // Absent rows are zeros, but not by the copy: 128 bytes past the end take it five times as long as those that are there (9 rows of a
     // 24-layer, 896-wide int8 model 613 us with boxes of 16 rows, 493 so; 2 rows of a 16-layer, 1024-wide Q4 one 440 and 316).
@@ -370,10 +409,10 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
         // ---- producer: the weights of the ring's first pass, the activations once the launch before is over, the rest ----
         pdl_launch_dependents();
         const uint64_t policy = a.evict_first ? l2_policy_evict_first() : l2_policy_evict_normal();
-        const int per_block = ((int)blockIdx.x < ntiles ? (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0) * groups;
+        const int per_block = (bx < ntiles ? (ntiles - bx + gx - 1) / gx : 0) * groups;
         const int ahead = min(stages, per_block), cols = a.cols;
         const int sw_bytes = (dual ? 2 : 1) * cols * (int)col_bytes, sc_row = cols * 16;   // sc_row: bytes of Q4 block scales per row of a stage
-        int tile = blockIdx.x, cg = 0, stage = 0;
+        int tile = bx, cg = 0, stage = 0;
         uint32_t phase = 1u;
 #pragma unroll 1
         for (int it = 0; it <= per_block; ++it) {
@@ -383,7 +422,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
                     // One copy for all rows.  A copy takes some 50 clocks to issue, whatever its size: 16 rows of
                     // 896 values are there after 1330 clocks, as pieces of 1 KB after 2900 (155 KB: 2600 and 10000).
                     mbar_arrive_expect_tx(xbar, (uint32_t)(M * xpitch + (a.norm_w ? K * 2 : 0)));
-                    tma_load_3d(base + OFF_X, &km.x, 0, 0, 0, xbar, l2_policy_evict_normal());
+                    tma_load_3d(base + OFF_X, &km.x, 0, 0, m_off, xbar, l2_policy_evict_normal());
                     if (a.norm_w) bulk_g2s(base + a.off_red, a.norm_w, (uint32_t)K * 2u, xbar, l2_policy_evict_normal());   // (the sums come later)
                 }
             }
@@ -415,39 +454,46 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
                 }
             }
             __syncwarp();
-            if (++cg == groups) { cg = 0; tile += gridDim.x; }
+            if (++cg == groups) { cg = 0; tile += gx; }
             if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
         return;
     }
 
     // ---- consumers: warp 2 j + set takes the units of parity `set` of the tile's K chunks j, j + 4, .. ----
-    constexpr int PART = 8 * NT * RED_TS;   // one warp's sums, as [token][row]
+    constexpr bool IMMA = FMT == FMT_INT8;
+    constexpr int PART = batch_part_words(FMT, NT);   // one warp's sums, as [token][row]
     const int box = warp >> 1, set = warp & 1, g = lane >> 2, t = lane & 3;
-    // the finish: pairs of neighbouring rows, one pair of one token at a time
-    const int plog = 30 - __clz(tile_rows), pair = tid & ((1 << plog) - 1), m_first = tid >> plog, m_step = (BCW * 32) >> plog;
+    // the finish: a pair of neighbouring rows of one token per thread
+    const int plog = 30 - __clz(tile_rows), pair = tid & ((1 << plog) - 1), m = tid >> plog;
+    static_assert((BCW * 32) / (WARP_ROWS / 2) >= 16, "one pass over the rows of activations");
     const int prow = 2 * pair;   // in the tile
     const bool inplace = a.epi == EPI_RESIDUAL || a.epi == EPI_SILU_GATE;
     // what a tile's finish needs besides the sums: fetched ahead (raw bits: the loads are waited for where they are used)
-    uint16_t p_sc[2] = {0, 0}, p_sc2[2] = {0, 0}, p_bias[2] = {0, 0}, p_old[2] = {0, 0};
+    uint16_t p_sc = 0, p_add[2] = {0, 0}, p_old[2] = {0, 0};
     auto fetch_rows = [&](int tile) {
         const BatchSeg sg = seg_at(dual ? 0 : segment(tile));
+        if (IMMA) {   // (one warp, a row per lane: the int8 sums leave few registers)
+            const int n = min((tile - sg.tile0) * tile_rows + lane, sg.N - 1);
+            if (warp == 1) {
+                p_sc = sg.scale[n];
+                if (dual) p_add[0] = a.scale2[n];
+                else if (sg.bias) p_add[0] = sg.bias[n];
+            }
+            return;
+        }
         const int n0 = (tile - sg.tile0) * tile_rows + prow;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int n = min(n0 + i, sg.N - 1);
-            if (FMT == FMT_INT8H) p_sc[i] = sg.scale[n];
-            if (FMT == FMT_INT8H && dual) p_sc2[i] = a.scale2[n];
-            if (sg.bias) p_bias[i] = sg.bias[n];
-        }
+        for (int i = 0; i < 2; ++i)
+            if (sg.bias) p_add[i] = sg.bias[min(n0 + i, sg.N - 1)];
     };
     auto fetch_old = [&](int tile) {
         const BatchSeg sg = seg_at(segment(tile));
         const int n0 = (tile - sg.tile0) * tile_rows + prow;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) p_old[i] = (n0 + i < sg.N && m_first < M) ? sg.out[(size_t)m_first * sg.ld + n0 + i] : (uint16_t)0;
+        for (int i = 0; i < 2; ++i) p_old[i] = (n0 + i < sg.N && m < M && m >= m_lo) ? sg.out[(size_t)(m_off + m) * sg.ld + n0 + i] : (uint16_t)0;
     };
-    int tile = blockIdx.x;
+    int tile = bx;
     if (tile < ntiles) fetch_rows(tile);
     BatchGeo<NT> lg;
     {
@@ -461,7 +507,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
         lg.a_off = (uint32_t)(((4 * set + (lane >> 4)) ^ (lane & 7)) << 4);
         const int n = FMT == FMT_FP16 ? lane & 7 : g;
         lg.b_x = (uint32_t)(n * a.xcols) & 7u;
-        lg.b_q = (uint32_t)(FMT == FMT_INT8H ? t : 4 * set + (FMT == FMT_FP16 ? lane >> 3 : t));
+        lg.b_q = (uint32_t)(IMMA ? t : 4 * set + (FMT == FMT_FP16 ? lane >> 3 : t));
         lg.b = base + OFF_X + (uint32_t)(n * xpitch);
         lg.b_up = 8u * (uint32_t)xpitch;
         const int pairs = (M + 1) / 2;
@@ -488,7 +534,16 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
             const NormRow rows[1] = {NormRow(base + OFF_X + warp * xpitch, warp * a.xcols, lane)};
             norm_rows<1>(rows, base + a.off_red + lane * 16, a.norm_eps, K, lane);
         }
+        if (IMMA) __syncwarp();   // (a warp's rows are its own until their scales are there)
+        else batch_sync();
+    }
+    float *const scale = reinterpret_cast<float*>(sm + OFF_SCALE), *const rows = reinterpret_cast<float*>(sm + OFF_ROW);
+    float up[NT];
+    if (IMMA) {
+        for (int m = warp; m < M; m += BCW) batch_row_scale(base + OFF_X + m * xpitch, K * 2, scale, m, lane);
         batch_sync();
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) up[nt] = scale[g + 8 * nt];
     }
     if (FMT == FMT_Q4) {
         const int pairs = (M + 1) / 2, blocks = K / 32;
@@ -505,14 +560,19 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
     int stage = 0;
     uint32_t phase = 0u;
 #pragma unroll 1
-    for (; tile < ntiles; tile += gridDim.x) {
+    for (; tile < ntiles; tile += gx) {
         float acc[2][NT][4];
+        int iacc[IMMA ? 3 : 1][2][NT][4];
 #pragma unroll
         for (int rb = 0; rb < 2; ++rb)
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) acc[rb][nt][i] = 0.f;
+                for (int i = 0; i < 4; ++i) {
+                    acc[rb][nt][i] = 0.f;
+#pragma unroll
+                    for (int l = 0; l < (IMMA ? 3 : 1); ++l) iacc[l][rb][nt][i] = 0;
+                }
 #pragma unroll 1
         for (int cg = 0; cg < groups; ++cg) {
             const int c = cg * NCW + box;
@@ -531,17 +591,21 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
                 const uint8_t* const sc[2] = {scb + g * sstr, scb + (g + (dual ? tile_rows : 16)) * sstr};
 #pragma unroll 1
                 for (int u = set; u < cb / 16; u += 2) batch_block_q4<NT>(lg, sw, u, s0 + u, acc, sc, sstr, (uint32_t)lane & 7u);
+            } else if constexpr (IMMA) {
+                const int s0 = c * kcb / 64;
+#pragma unroll 1
+                for (int u = set; u < cb / 64; u += 2) batch_unit_int8<NT>(lg, sw, u >> 1, s0 + u, up, iacc);
             } else {
                 const int s0 = c * kcb / 64;
                 const int n = (cb / 64 - set + 1) >> 1;   // the warp's units
-                constexpr bool PAIR = FMT == FMT_FP16 && NT == 1;   // two units' operands fit in registers
+                constexpr bool PAIR = NT == 1;   // two units' operands fit in registers
 #pragma unroll 1
                 for (int i = 0; i < n; i += PAIR ? 2 : 1) {
-                    BatchFrag<FMT, NT> f0, f1;
-                    batch_load<FMT, NT>(lg, sw, i, s0 + 2 * i + set, f0);
-                    if (PAIR && i + 1 < n) batch_load<FMT, NT>(lg, sw, i + 1, s0 + 2 * i + 2 + set, f1);
-                    batch_mac<FMT, NT>(f0, lg.two, acc);
-                    if (PAIR && i + 1 < n) batch_mac<FMT, NT>(f1, lg.two, acc);
+                    BatchFrag<NT> f0, f1;
+                    batch_load<NT>(lg, sw, i, s0 + 2 * i + set, f0);
+                    if (PAIR && i + 1 < n) batch_load<NT>(lg, sw, i + 1, s0 + 2 * i + 2 + set, f1);
+                    batch_mac<NT>(f0, lg.two, acc);
+                    if (PAIR && i + 1 < n) batch_mac<NT>(f1, lg.two, acc);
                 }
             }
             __syncwarp();
@@ -551,68 +615,90 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
         // the parts meet in shared memory as [part][token][row]
         batch_sync();   // (the finish before this one has read them)
         float* const mine = reinterpret_cast<float*>(sm + mine_off);
+        if (IMMA) {
+            // a chunk's two sets as integers (exact, so their order does not matter), then one fp32 sum per chunk, as int8_recombine has it
+            int* const pair = reinterpret_cast<int*>(sm + a.off_red) + box * 2 * PART + lane;
+            if (warp == 1) {
+                rows[lane] = __half2float(__ushort_as_half(p_sc));
+                rows[32 + lane] = __half2float(__ushort_as_half(p_add[0]));
+            }
+            if (set == 1) {
 #pragma unroll
-        for (int rb = 0; rb < 2; ++rb)
+                for (int l = 0; l < 3; ++l)
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
+                    for (int i = 0; i < 8 * NT; ++i) pair[(l * 8 * NT + i) * 32] = iacc[l % (IMMA ? 3 : 1)][i / (4 * NT)][(i >> 2) % NT][i & 3];
+            }
+            asm volatile("bar.sync %0, 64;" ::"r"(2 + box) : "memory");
+            if (set == 0) {
+                const float* const down = scale + 16 + 2 * t;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) mine[(nt * 8 + (i & 1)) * RED_TS + rb * 16 + (i >> 1) * 8] = acc[rb][nt][i];
+                for (int i = 0; i < 8 * NT; ++i) {
+                    auto limb = [&](int l) { return (float)(iacc[l % (IMMA ? 3 : 1)][i / (4 * NT)][(i >> 2) % NT][i & 3] + pair[(l * 8 * NT + i) * 32]); };
+                    acc[i / (4 * NT)][(i >> 2) % NT][i & 3] = fmaf(limb(0), 65536.f, fmaf(limb(1), 256.f, limb(2))) * down[(i >> 2) % NT * 8 + (i & 1)];
+                }
+                __syncwarp();
+            }
+        }
+        if (!IMMA || set == 0) {
+#pragma unroll
+            for (int rb = 0; rb < 2; ++rb)
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) mine[(nt * 8 + (i & 1)) * RED_TS + rb * 16 + (i >> 1) * 8] = acc[rb][nt][i];
+        }
         batch_sync();
         const BatchSeg sg = seg_at(dual ? 0 : segment(tile));
         const int n = (tile - sg.tile0) * tile_rows + prow;
         const bool two = n + 1 < sg.N, biased = sg.bias != nullptr;
         const float* const src = reinterpret_cast<const float*>(sm + src_off);
-        if (n < sg.N) {
-#pragma unroll 1
-            for (int m = m_first; m < M; m += m_step) {
-                auto sum = [&](int up) {   // a chunk's two sets first, then the chunks in order
-                    const float* const s = src + m * RED_TS + up;
-                    auto both = [&](int j) {
-                        const float2 v = *reinterpret_cast<const float2*>(s + 2 * j * PART), o = *reinterpret_cast<const float2*>(s + (2 * j + 1) * PART);
-                        return make_float2(v.x + o.x, v.y + o.y);
-                    };
-                    float2 v = both(0);
-#pragma unroll
-                    for (int j = 1; j < NCW; ++j) {
-                        const float2 o = both(j);
-                        v.x += o.x;
-                        v.y += o.y;
-                    }
-                    return v;
+        if (n < sg.N && m < M && m >= m_lo) {
+            auto sum = [&](int up) {   // a chunk's two sets first, then the chunks in order
+                const float* const s = src + m * RED_TS + up;
+                auto both = [&](int j) {
+                    if (IMMA) return *reinterpret_cast<const float2*>(s + 2 * j * PART);
+                    const float2 v = *reinterpret_cast<const float2*>(s + 2 * j * PART), o = *reinterpret_cast<const float2*>(s + (2 * j + 1) * PART);
+                    return make_float2(v.x + o.x, v.y + o.y);
                 };
-                const float2 s0 = sum(0);
-                const float2 s1 = dual ? sum(16) : make_float2(0.f, 0.f);
-                uint16_t* const dst = sg.out + (size_t)m * sg.ld + n;
-                if (inplace && m != m_first) {
-                    p_old[0] = dst[0];
-                    p_old[1] = two ? dst[1] : (uint16_t)0;
-                }
-                uint16_t hv[2];
+                float2 v = both(0);
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {   // roundings as in finish_row and finish_swiglu
-                    float v = i ? s0.y : s0.x;
-                    if (FMT == FMT_INT8H) v = __fmul_rn(v, __half2float(__ushort_as_half(p_sc[i])));
-                    const float gt = dual ? v : __half2float(__ushort_as_half(p_old[i]));
-                    if (dual) {
-                        float uv = i ? s1.y : s1.x;
-                        if (FMT == FMT_INT8H) uv *= __half2float(__ushort_as_half(p_sc2[i]));
-                        v = (gt / (1.0f + expf(-gt))) * uv;
-                    } else {
-                        if (biased) v = __fadd_rn(__half2float(__float2half_rn(v)), __half2float(__ushort_as_half(p_bias[i])));
-                        if (a.epi == EPI_RESIDUAL) v = __fadd_rn(gt, v);
-                        else if (a.epi == EPI_SILU_GATE) v = gt * (1.0f / (1.0f + expf(-gt))) * v;
-                    }
-                    hv[i] = __half_as_ushort(__float2half_rn(v));
+                for (int j = 1; j < NCW; ++j) {
+                    const float2 o = both(j);
+                    v.x += o.x;
+                    v.y += o.y;
                 }
-                if (two && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
-                    *reinterpret_cast<uint32_t*>(dst) = (uint32_t)hv[0] | (uint32_t)hv[1] << 16;
+                return v;
+            };
+            const float2 s0 = sum(0);
+            const float2 s1 = dual ? sum(16) : make_float2(0.f, 0.f);
+            uint16_t* const dst = sg.out + (size_t)(m_off + m) * sg.ld + n;
+            const float2 sc = IMMA ? *reinterpret_cast<const float2*>(rows + prow) : make_float2(0.f, 0.f);
+            const float2 add = IMMA ? *reinterpret_cast<const float2*>(rows + 32 + prow) : make_float2(__half2float(__ushort_as_half(p_add[0])), __half2float(__ushort_as_half(p_add[1])));
+            uint16_t hv[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {   // roundings as in finish_row and finish_swiglu
+                float v = i ? s0.y : s0.x;
+                if (IMMA) v = __fmul_rn(v, i ? sc.y : sc.x);
+                const float gt = dual ? v : __half2float(__ushort_as_half(p_old[i]));
+                if (dual) {
+                    float uv = i ? s1.y : s1.x;
+                    if (IMMA) uv *= i ? add.y : add.x;
+                    v = (gt / (1.0f + expf(-gt))) * uv;
                 } else {
-                    dst[0] = hv[0];
-                    if (two) dst[1] = hv[1];
+                    if (biased) v = __fadd_rn(__half2float(__float2half_rn(v)), i ? add.y : add.x);
+                    if (a.epi == EPI_RESIDUAL) v = __fadd_rn(gt, v);
+                    else if (a.epi == EPI_SILU_GATE) v = gt * (1.0f / (1.0f + expf(-gt))) * v;
                 }
+                hv[i] = __half_as_ushort(__float2half_rn(v));
+            }
+            if (two && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
+                *reinterpret_cast<uint32_t*>(dst) = (uint32_t)hv[0] | (uint32_t)hv[1] << 16;
+            } else {
+                dst[0] = hv[0];
+                if (two) dst[1] = hv[1];
             }
         }
-        const int next = tile + (int)gridDim.x;
+        const int next = tile + gx;
         if (next < ntiles) {
             fetch_rows(next);
             if (inplace) fetch_old(next);
@@ -671,7 +757,7 @@ cudaError_t launch_f(const LinArgs& a, const BatchPlan& p, cudaStream_t st, bool
         if (!weight_map(&km.tm[i], a.seg[i].W, a.seg[i].N)) return cudaErrorInvalidValue;
     }
     if (dual && !weight_map(&km.tm[3], a.W2, a.seg[0].N)) return cudaErrorInvalidValue;
-    if (!make_rows_map(&km.x, a.x, a.M, a.K * 2, a.x_pitch ? a.x_pitch : a.K * 2, p.xcols, a.M)) return cudaErrorInvalidValue;
+    if (!make_rows_map(&km.x, a.x, a.M, a.K * 2, a.x_pitch ? a.x_pitch : a.K * 2, p.xcols, p.halves ? 8 : a.M)) return cudaErrorInvalidValue;
     if (!fill_scale_maps(km, a, p.cols * 16, tile_rows)) return cudaErrorInvalidValue;
     b.scale2 = a.scale2;
     b.norm_w = a.norm_w;
@@ -679,6 +765,7 @@ cudaError_t launch_f(const LinArgs& a, const BatchPlan& p, cudaStream_t st, bool
     b.status = a.status;
     b.M = a.M;
     b.K = a.K;
+    b.halves = p.halves ? 1 : 0;
     b.cols = p.cols;
     b.wide = wide ? 1 : 0;
     b.xcols = p.xcols;
@@ -695,7 +782,10 @@ cudaError_t launch_f(const LinArgs& a, const BatchPlan& p, cudaStream_t st, bool
     b.off_ctab = p.off_ctab;
     b.off_red = p.off_red;
     b.off_ring = p.off_ring;
-    return a.M > 8 ? launch_n<FMT, 2>(km, b, p, st, pdl) : launch_n<FMT, 1>(km, b, p, st, pdl);
+    if constexpr (FMT != FMT_INT8) {
+        if (a.M > 8) return launch_n<FMT, 2>(km, b, p, st, pdl);
+    }
+    return launch_n<FMT, 1>(km, b, p, st, pdl);
 }
 
 }  // namespace
@@ -704,7 +794,7 @@ cudaError_t batch_configure() {
     cudaError_t e = cudaSuccess;
 #define SET_SMEM(F, N) \
     if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_batch_kernel<F, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    SET_SMEM(FMT_FP16, 1) SET_SMEM(FMT_FP16, 2) SET_SMEM(FMT_INT8H, 1) SET_SMEM(FMT_INT8H, 2) SET_SMEM(FMT_Q4, 1) SET_SMEM(FMT_Q4, 2)
+    SET_SMEM(FMT_FP16, 1) SET_SMEM(FMT_FP16, 2) SET_SMEM(FMT_INT8, 1) SET_SMEM(FMT_Q4, 1) SET_SMEM(FMT_Q4, 2)
 #undef SET_SMEM
     return e;
 }
@@ -733,38 +823,39 @@ BatchPlan batch_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit)
         if (sp.ok && sp.kcb == part.kcb) return p;   // (rows so long that it takes smaller chunks, and so other sums, stay here)
     }
     const bool dual = a.epi == EPI_SWIGLU;
-    const int rb = fmt_row_bytes(fmt, a.K), nt = a.M > 8 ? 2 : 1, warp_rows = dual ? 16 : WARP_ROWS;
+    p.halves = fmt == FMT_INT8 && a.M > 8;
+    const int rb = fmt_row_bytes(fmt, a.K), nt = a.M > 8 && !p.halves ? 2 : 1, warp_rows = dual ? 16 : WARP_ROWS;
     p.kcb = part.kcb;
     p.tile_rows = warp_rows;
     const int nchunks = (rb + p.kcb - 1) / p.kcb, groups = (nchunks + NCW - 1) / NCW;
     // Few tiles of long rows: half tiles on twice the SMs, whose warps have half the weights each (tiles do not enter the sums): Q4
     // 1024 x 4608, 8 rows, 8.4 -> 7.4 us.  Rows of one stage gain nothing (1024 x 1024: 3.3 against 3.5 us).
-    if (!dual && groups > 1 && count_tiles(a, WARP_ROWS) * 2 <= sm_count) p.tile_rows = 16;
+    if (!dual && groups > 1 && count_tiles(a, WARP_ROWS) * (p.halves ? 4 : 2) <= sm_count) p.tile_rows = 16;
     p.ntiles = count_tiles(a, p.tile_rows);
     if (fmt == FMT_Q4 && p.ntiles > (a.norm_w ? 4 : 2) * sm_count) return p;
     p.cols = groups == 1 ? (rb + 127) / 128 : NCW * (p.kcb / 128);   // (not more than there are: what lies past the end takes a copy long)
     p.xcols = batch_xcols(fmt, a.K);
     if (a.K % 64 != 0 || p.xcols > 256 || p.cols * 16 > 256) return p;   // one copy's reach
-    if (a.norm_w && a.K * 2 > BCW * 8 * nt * RED_TS * 4) return p;       // the norm weight lies where the sums will
+    if (a.norm_w && a.K * 2 > batch_red_bytes(fmt, nt)) return p;       // the norm weight lies where the sums will
     const int sets = dual ? 2 : 1;
     p.stage_bytes = (sets * p.tile_rows * p.cols * (128 + (fmt == FMT_Q4 ? 16 : 0)) + 1023) / 1024 * 1024;
     p.off_ring = OFF_X + 8 * nt * p.xcols * 128;
     // Two blocks per SM where that leaves each at least two stages (or all of its items): a block of the next launch can then be
     // resident, with its weights on their way, before this one's is done.
-    const int ctab = ctab_bytes_of(fmt, a.M, a.K), rest = ctab + BCW * 8 * nt * RED_TS * 4;
+    const int ctab = ctab_bytes_of(fmt, a.M, a.K), red = batch_red_bytes(fmt, nt), rest = ctab + red;
     for (int ps = 2; ps >= 1; --ps) {
         const long long budget = (long long)((smem_limit + 1024) / ps) - 1024 - 1024 - p.off_ring - rest;   // 1 KB to align the start
-        const int resident = sm_count * ps, waves = (p.ntiles + resident - 1) / resident, items = waves * groups;
+        const int resident = sm_count * ps / (p.halves ? 2 : 1), waves = (p.ntiles + resident - 1) / resident, items = waves * groups;
         const int least = items < 2 ? 1 : 2;
         int st = (int)(budget / p.stage_bytes);
         if (budget < 0 || st < least) continue;
         if (st > items) st = items;
         if (st > BATCH_STAGES) st = BATCH_STAGES;
         p.stages = st;
-        p.grid = p.ntiles < resident ? p.ntiles : resident;
+        p.grid = (p.ntiles < resident ? p.ntiles : resident) * (p.halves ? 2 : 1);
         p.off_ctab = p.off_ring + st * p.stage_bytes;
         p.off_red = p.off_ctab + ctab;
-        p.smem = (size_t)p.off_red + BCW * 8 * nt * RED_TS * 4 + 1024;
+        p.smem = (size_t)p.off_red + red + 1024;
         p.ok = true;
         break;
     }
@@ -773,7 +864,7 @@ BatchPlan batch_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit)
 
 cudaError_t launch_batch(int fmt, const LinArgs& a, const BatchPlan& p, cudaStream_t st, bool pdl) {
     if (fmt == FMT_FP16) return launch_f<FMT_FP16>(a, p, st, pdl);
-    if (fmt == FMT_INT8H) return launch_f<FMT_INT8H>(a, p, st, pdl);
+    if (fmt == FMT_INT8) return launch_f<FMT_INT8>(a, p, st, pdl);
     if (fmt == FMT_Q4) return launch_f<FMT_Q4>(a, p, st, pdl);
     return cudaErrorInvalidValue;
 }

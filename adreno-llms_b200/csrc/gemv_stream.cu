@@ -128,8 +128,11 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     // Scalars used all over the kernel are read from the parameter block once.  The block's
     // address is taken (the tensor maps in it are handed to the TMA unit), so the compiler must
     // assume that any store may change it and would otherwise re-read a field after every store.
-    const int bx = (int)blockIdx.x, gx = (int)gridDim.x;
-    const int aM = ONE ? 1 : a.M, aK = a.K, a_epi = a.epi, a_nseg = a.nseg;
+    // Token halves (int8, 9..16 rows; see stream_plan): blocks 2 i and 2 i + 1 share the tiles of block i, eight rows each.
+    const bool halves = !ONE && !EXT && FMT == FMT_INT8 && NT == 1 && a.halves;
+    const int M_all = ONE ? 1 : a.M, m_first = halves ? (int)(blockIdx.x & 1u) * 8 : 0, gM = ONE ? 1 : halves ? 8 : M_all;   // gM: rows the layout has room for
+    const int bx = halves ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, gx = halves ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+    const int aM = ONE ? 1 : halves ? min(8, M_all - m_first) : M_all, aK = a.K, a_epi = a.epi, a_nseg = a.nseg;
     int* const a_status = a.status;
     const int seg1_tile0 = a.seg[1].tile0, seg2_tile0 = a.seg[2].tile0;
     const int stages = ka.stages, kcb = a.kcb;
@@ -137,7 +140,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     const int rowbytes = ka.rowbytes, nchunks = ka.nchunks;
     const bool a_norm = VAR >= 1 && a.norm_w != nullptr;
     const int xcols = VAR == 3 ? a.xcols : 0;
-    const Geo geo = make_geo(FMT, aM, aK, kcb, stages, NT, a_norm, xcols);
+    const Geo geo = make_geo(FMT, gM, aK, kcb, stages, NT, a_norm, xcols);
     const int warp_rows = DUAL ? 16 : WARP_ROWS;                       // rows of each weight per warp
     const int tile_rows = ksplit ? warp_rows : NCW * warp_rows;        // rows of each weight per block tile
     const int groups = ksplit ? (nchunks + NCW - 1) / NCW : nchunks;   // pipeline items per tile
@@ -150,7 +153,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     const uint32_t ring = (s_base + geo.off_ring + 1023u) & ~1023u;
 
     if (tid < HDR_BYTES / 4) reinterpret_cast<uint32_t*>(smem)[tid] = 0u;
-    if (FMT == FMT_INT8 && !xcols && tid >= 32 && tid < 48) reinterpret_cast<uint32_t*>(xs + 3 * aM * geo.xstride)[tid - 32] = 0u;  // per-row max words
+    if (FMT == FMT_INT8 && !xcols && tid >= 32 && tid < 48) reinterpret_cast<uint32_t*>(xs + 3 * gM * geo.xstride)[tid - 32] = 0u;  // per-row max words
     const uint32_t xbar = s_base + geo.off_x - 8;  // batched calls: the staged activations have landed
     if (tid == 0) {
         for (int s = 0; s < stages; ++s) {
@@ -272,7 +275,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
             // copies rows, once the launch that staged them is over; the weights of the first stages do not wait for that.
             const int xrows = (FMT == FMT_INT8 ? 3 : 1) * aM, ximg = x_stride_of(FMT, aK);
             constexpr int XB = FMT == FMT_INT8 ? 1 : 2;   // bytes per value
-            auto cols = [&](int cg) { return min(xcols, x_values_of(FMT, aK) - cg * xcols) * XB; };
+            auto cols = [&](int cg) { return min(xcols, aK - cg * xcols) * XB; };
             int tile_s = tile_first, cg = 0, stage = 0, tile_w = tile_first, cg_w = 0;
             for (int it = 0; it < n_items; ++it) {
                 if (it == 0) {
@@ -292,8 +295,11 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
                     __syncwarp();
                 }
                 const uint32_t dst = ring + stage * geo.stage_bytes + geo.off_sx, n = (uint32_t)cols(cg);
-                for (int r = lane; r < xrows; r += 32)
-                    bulk_g2s(dst + r * geo.xstride, a.staged + (size_t)r * ximg + (size_t)cg * xcols * XB, n, full0 + stage * 8, l2_policy_evict_normal());
+                for (int r = lane; r < xrows; r += 32) {
+                    // (halves: rows m_first .. of every plane)
+                    const int l = halves ? r / aM : 0, to = halves ? l * gM + r - l * aM : r, from = halves ? l * M_all + m_first + r - l * aM : r;
+                    bulk_g2s(dst + to * geo.xstride, a.staged + (size_t)from * ximg + (size_t)cg * xcols * XB, n, full0 + stage * 8, l2_policy_evict_normal());
+                }
                 if (++cg == groups) { cg = 0; tile_s += tile_step; }
                 if (++stage == stages) stage = 0;
             }
@@ -315,8 +321,8 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     // ================= consumer warps =================
     const int g = lane >> 2, t = lane & 3;
     LaneGeo<NT> lg;
-    lane_geo_init<FMT, NT>(lg, DUAL, warp, lane, aM, smem_u32(xs), geo.xstride, zero_addr, smem + geo.off_ctab);
-    const float* rowscale = reinterpret_cast<const float*>(xs + (xcols ? 0 : 3 * aM * geo.xstride) + 64);
+    lane_geo_init<FMT, NT>(lg, DUAL, warp, lane, gM, smem_u32(xs), geo.xstride, zero_addr, smem + geo.off_ctab);
+    const float* rowscale = reinterpret_cast<const float*>(xs + (xcols ? 0 : 3 * gM * geo.xstride) + 64) + m_first;
 
     // rows of this warp inside its tile, and which warp writes results
     const int wrow_off = ksplit ? 0 : warp * warp_rows;
@@ -347,14 +353,14 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int n = min(row0 + 2 * f_pair + i, sg.N - 1);
-                if (int8_weights(FMT)) p_sc[i] = sg.scale[n];
-                if (int8_weights(FMT) && DUAL) p_sc2[i] = a.scale2[n];
+                if (FMT == FMT_INT8) p_sc[i] = sg.scale[n];
+                if (FMT == FMT_INT8 && DUAL) p_sc2[i] = a.scale2[n];
                 if (VAR >= 1 && !DUAL && sg.bias) p_bias[i] = sg.bias[n];
             }
             return;
         }
         if (VAR >= 1 && !DUAL && sg.bias) bias1 = sg.bias[min(row0 + lane, sg.N - 1)];
-        if (!int8_weights(FMT)) return;
+        if (FMT != FMT_INT8) return;
         if (DUAL) {   // lane L (< 16) finishes row L of the warp's 16 rows
             const int n = min(row0 + (lane & 15), sg.N - 1);
             sc1 = sg.scale[n];
@@ -411,7 +417,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int n = row0 + 2 * f_pair + i, m = f_m0 + k * f_step;
-                p_res[k][i] = (n < sg.N && m < aM) ? sg.out[(size_t)m * sg.ld_out + n] : (uint16_t)0;
+                p_res[k][i] = (n < sg.N && m < aM) ? sg.out[(size_t)(m_first + m) * sg.ld_out + n] : (uint16_t)0;
             }
     };
 
@@ -429,11 +435,15 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
         // the launch before this one (stage_image_kernel) wrote the staged form of all M rows in this
         // kernel's shared-memory layout: one bulk copy instead of M rows converted by every block
         // (rows that travel with the weights: only the int8 row scales behind them)
-        const uint32_t skip = xcols ? 3u * (uint32_t)aM * (uint32_t)x_stride_of(FMT, aK) : 0u, bytes = xcols ? 192u : a.staged_bytes;
+        const uint32_t row = (uint32_t)x_stride_of(FMT, aK), skip = xcols || halves ? 3u * (uint32_t)M_all * row : 0u, bytes = xcols || halves ? 192u : a.staged_bytes;
         const bool some = !xcols || FMT == FMT_INT8;
         if (tid == 0 && some) {
-            mbar_arrive_expect_tx(xbar, bytes);
-            bulk_g2s(smem_u32(xs), a.staged + skip, bytes, xbar, l2_policy_evict_normal());
+            const bool planes = halves && !xcols;
+            mbar_arrive_expect_tx(xbar, bytes + (planes ? 3u * (uint32_t)aM * row : 0u));
+            if (planes)
+                for (int l = 0; l < 3; ++l)
+                    bulk_g2s(smem_u32(xs) + (uint32_t)(l * gM) * row, a.staged + (size_t)(l * M_all + m_first) * row, (uint32_t)aM * row, xbar, l2_policy_evict_normal());
+            bulk_g2s(smem_u32(xs) + (planes ? 3u * (uint32_t)gM * row : 0u), a.staged + skip, bytes, xbar, l2_policy_evict_normal());
         }
         if (some && !mbar_wait_bounded(xbar, 0u)) *reinterpret_cast<volatile int*>(a_status) = 5;
     } else {
@@ -496,8 +506,8 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
         if constexpr (VAR == 3) {   // this stage's activations begin at its first column
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
-                const int n = b_row<FMT>(lane) + nt * 8;
-                if (n < aM) lg.b_base[nt] = sw + geo.off_sx + n * geo.xstride + b_lane_off<FMT>(lane) - (uint32_t)(cg * xcols * (FMT == FMT_INT8 ? 1 : 2));
+                const int n = (lane & 7) + nt * 8;
+                if (n < gM) lg.b_base[nt] = sw + geo.off_sx + n * geo.xstride + (lane >> 3) * 16 - (uint32_t)(cg * xcols * (FMT == FMT_INT8 ? 1 : 2));
             }
         }
         const int cb = (failed || !active) ? 0 : min(kcb, rowbytes - c * kcb);
@@ -506,8 +516,6 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
             chunk_fp16<NT>(lg, sw, c, kcb, cb, acc);
         } else if constexpr (FMT == FMT_INT8) {
             chunk_int8<NT>(lg, sw, c, kcb, cb, iacc);
-        } else if constexpr (FMT == FMT_INT8H) {
-            chunk_int8h<NT>(lg, sw, c, kcb, cb, acc);
         } else {
             // scale rows of this warp's two row blocks inside the stage's scale region: the
             // cp.async path keeps each warp's 32 rows together; tensor copies land whole boxes,
@@ -669,8 +677,8 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
                         old[0] = p_res[1][0];
                         old[1] = p_res[1][1];
                         if (k > 1) {
-                            old[0] = seg_out[(size_t)m * seg_ld + n];
-                            old[1] = two ? seg_out[(size_t)m * seg_ld + n + 1] : (uint16_t)0;
+                            old[0] = seg_out[(size_t)(m_first + m) * seg_ld + n];
+                            old[1] = two ? seg_out[(size_t)(m_first + m) * seg_ld + n + 1] : (uint16_t)0;
                         }
                     }
                     uint16_t hv[2];
@@ -679,13 +687,13 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
                         float v = i ? s0.y : s0.x;
                         if (DUAL) {
                             float uv = i ? s1.y : s1.x;
-                            if (int8_weights(FMT)) {
+                            if (FMT == FMT_INT8) {
                                 v *= __half2float(__ushort_as_half(p_sc[i]));
                                 uv *= __half2float(__ushort_as_half(p_sc2[i]));
                             }
                             v = (v / (1.0f + expf(-v))) * uv;
                         } else {
-                            if (int8_weights(FMT)) v = __fmul_rn(v, __half2float(__ushort_as_half(p_sc[i])));  // roundings as in finish_row
+                            if (FMT == FMT_INT8) v = __fmul_rn(v, __half2float(__ushort_as_half(p_sc[i])));  // roundings as in finish_row
                             if (VAR >= 1 && biased) v = __fadd_rn(__half2float(__float2half_rn(v)), __half2float(__ushort_as_half(p_bias[i])));
                             const float gt = __half2float(__ushort_as_half(old[i]));
                             if (epi == EPI_RESIDUAL) v = __fadd_rn(gt, v);
@@ -693,7 +701,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
                         }
                         hv[i] = __half_as_ushort(__float2half_rn(v));
                     }
-                    const size_t o = (size_t)m * seg_ld + n;
+                    const size_t o = (size_t)(m_first + m) * seg_ld + n;
                     auto put = [&](uint16_t* dst) {
                         if (two && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
                             *reinterpret_cast<uint32_t*>(dst) = (uint32_t)hv[0] | (uint32_t)hv[1] << 16;
@@ -720,7 +728,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
             float gv = hi ? g1 : g0, uv = hi ? u1 : u0;
             const int n = tile * tile_rows + wrow_off + lane;
             if (lane < 16 && n < seg_n) {
-                if (int8_weights(FMT)) {
+                if (FMT == FMT_INT8) {
                     gv *= __half2float(__ushort_as_half(sc1));
                     uv *= __half2float(__ushort_as_half(res1));
                 }
@@ -741,7 +749,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
             float v = sel == 0 ? v00 : sel == 1 ? v01 : sel == 2 ? v10 : v11;
             const int n = row0 + lane;
             if (n < seg_n) {
-                if (int8_weights(FMT)) v = __fmul_rn(v, __half2float(__ushort_as_half(sc1)));  // roundings as in finish_row
+                if (FMT == FMT_INT8) v = __fmul_rn(v, __half2float(__ushort_as_half(sc1)));  // roundings as in finish_row
                 if (VAR >= 1 && biased) v = __fadd_rn(__half2float(__float2half_rn(v)), __half2float(__ushort_as_half(bias1)));
                 if (epi == EPI_RESIDUAL) {
                     v = __fadd_rn(__half2float(__ushort_as_half(res1)), v);
@@ -932,7 +940,7 @@ int ext_blocks_per_sm(int fmt, int nt, bool dual, bool one, size_t smem) {
         if (one) return dual ? ext_occupancy<F, 1, true, true>(smem) : ext_occupancy<F, 1, false, true>(smem);       \
         return dual ? ext_occupancy<F, 1, true, false>(smem) : ext_occupancy<F, 1, false, false>(smem);              \
     }
-    OCC(FMT_FP16) OCC(FMT_INT8) OCC(FMT_INT8H) OCC(FMT_Q4)
+    OCC(FMT_FP16) OCC(FMT_INT8) OCC(FMT_Q4)
 #undef OCC
     return 0;
 }
@@ -984,7 +992,6 @@ cudaError_t stream_configure() {
 #define CFG(F, N, D) if ((e = configure_one<F, N, D>()) != cudaSuccess) return e;
     CFG(FMT_FP16, 1, false) CFG(FMT_FP16, 2, false) CFG(FMT_FP16, 1, true) CFG(FMT_FP16, 2, true)
     CFG(FMT_INT8, 1, false) CFG(FMT_INT8, 2, false) CFG(FMT_INT8, 1, true) CFG(FMT_INT8, 2, true)
-    CFG(FMT_INT8H, 1, false) CFG(FMT_INT8H, 2, false) CFG(FMT_INT8H, 1, true) CFG(FMT_INT8H, 2, true)
     CFG(FMT_Q4, 1, false) CFG(FMT_Q4, 2, false) CFG(FMT_Q4, 1, true) CFG(FMT_Q4, 2, true)
 #undef CFG
     if ((e = decode_plan_configure()) != cudaSuccess) return e;
@@ -1007,7 +1014,7 @@ bool stream_supported(int fmt, int M, int K, const LinArgs& a) {
         if (a.npeer > 0 || a.sig.world > 0 || (fmt == FMT_Q4 && !q4_scale_views(a, base, &pitch))) return false;
     }
     // int8: the limb sums are 32-bit; |code| <= 128 times a limb <= 255 over K terms must stay below 2^31
-    if (int8_weights(fmt) && K > 65536) return false;
+    if (fmt == FMT_INT8 && K > 65536) return false;
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     for (int i = 0; i < a.nseg; ++i) {
         if (!al16(a.seg[i].W)) return false;
@@ -1044,7 +1051,13 @@ StreamPlan stream_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limi
     const int K = a.K;
     const bool dual = a.epi == EPI_SWIGLU, norm = a.norm_w != nullptr;
     const int rb = fmt_row_bytes(fmt, K);
-    const int M = a.M;
+    // int8, 9..16 staged rows, an operator whose 32-row tiles take at most half the SMs: two blocks per tile, eight rows each.
+    // The integer MMAs set the pace (60 % of the SM's cycles on 896 x 4864, 28 blocks), and the weights come from L2 twice for
+    // little: that operator 19.0 -> 9.5 us.  Beyond half of the SMs the second block would only queue.  (Most such calls take the
+    // batch kernel; here come those it does not take: rows too long for it, or of an odd number of 32 values, outputs over the rows.)
+    p.halves = fmt == FMT_INT8 && a.M > 8 && a.staged && !norm && a.npeer == 0 && a.sig.world == 0 && !a.argmax_slot && a.seg[0].out &&
+               count_tiles(a, dual ? 16 : WARP_ROWS) * 2 <= sm_count;
+    const int M = p.halves ? 8 : a.M;
     const int nt = M > 8 ? 2 : 1;
     const int rb_cols = ((rb + 127) / 128) * 128;
     const int warp_rows = dual ? 16 : WARP_ROWS;
@@ -1119,6 +1132,7 @@ StreamPlan stream_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limi
             p.grid = resident;
         }
     }
+    if (p.halves) p.grid *= 2;
     p.xcols = xcols;
     p.kcb = kcb;
     p.kw = kw;
@@ -1134,6 +1148,7 @@ cudaError_t launch_stream(int fmt, const LinArgs& a, const StreamPlan& p, cudaSt
     ka.a = a;
     ka.a.kcb = p.kcb;
     ka.a.xcols = p.xcols;
+    ka.a.halves = p.halves ? 1 : 0;
     ka.a.kw = p.kw;
     ka.a.ntiles = p.ntiles;
     ka.a.streamk = p.streamk ? 1 : 0;
@@ -1144,7 +1159,7 @@ cudaError_t launch_stream(int fmt, const LinArgs& a, const StreamPlan& p, cudaSt
     for (int i = 0; i < a.nseg; ++i) wbytes += (size_t)a.seg[i].N * ka.rowbytes;
     ka.evict_first = wbytes > ((size_t)96 << 20) ? 1 : 0;  // weights that cannot stay in L2 anyway are streamed evict-first
     const bool dual = a.epi == EPI_SWIGLU;
-    const int nt = a.M > 8 ? 2 : 1;
+    const int nt = a.M > 8 && !p.halves ? 2 : 1;
     const int warp_rows = dual ? 16 : WARP_ROWS;
     const int tile_rows = p.kw == 1 ? NCW * warp_rows : warp_rows;
     int t0 = 0;
@@ -1172,7 +1187,7 @@ cudaError_t launch_stream(int fmt, const LinArgs& a, const StreamPlan& p, cudaSt
         if (dual) return nt == 2 ? launch_t<F, 2, true>(ka, p, st, pdl) : launch_t<F, 1, true>(ka, p, st, pdl); \
         return nt == 2 ? launch_t<F, 2, false>(ka, p, st, pdl) : launch_t<F, 1, false>(ka, p, st, pdl);         \
     }
-    GO(FMT_FP16) GO(FMT_INT8) GO(FMT_INT8H) GO(FMT_Q4)
+    GO(FMT_FP16) GO(FMT_INT8) GO(FMT_Q4)
 #undef GO
     return cudaErrorInvalidValue;
 }

@@ -7,8 +7,7 @@
 
 namespace nnb {
 
-enum Fmt : int { FMT_FP16 = 0, FMT_INT8 = 1, FMT_Q4 = 2,
-                 FMT_INT8H = 3 };   // inside the streaming kernels: int8 weights multiplied as fp16 (stream_format)
+enum Fmt : int { FMT_FP16 = 0, FMT_INT8 = 1, FMT_Q4 = 2 };
 
 // What work-item 0 of the reference kernels does with the reduced sum.
 enum Epi : int {
@@ -82,6 +81,7 @@ struct LinArgs {
     // stage_image_kernel in the kernel's own shared-memory layout; every block copies it in
     const uint8_t* staged;
     unsigned staged_bytes;
+    int halves;      // two blocks per tile, eight rows each (StreamPlan)
     int xcols;       // > 0: the staged rows travel with the weights, this many values of each per stage (StreamPlan)
     // host side only: Q4 scales with rows padded to a multiple of 16 bytes (seg[0..2], then the second weight of the
     // two-weight form), for the tensor copies when K / 16 is not such a multiple; all null otherwise
@@ -98,6 +98,7 @@ struct StreamPlan {  // launch geometry chosen on the host
     int kw;      // warps splitting K of one tile
     int warps;   // warps per block
     int stages;  // ring depth
+    bool halves; // 9..16 rows: two blocks per tile, eight rows each (grid counts both)
     int xcols;   // > 0: batched activations travel with the weights, this many values of every row per stage
     int ntiles;  // block tiles over all segments
     size_t smem;
@@ -112,6 +113,7 @@ struct BatchPlan {
     int grid, kcb, tile_rows, cols, xcols, stages, stage_bytes, ntiles;
     int off_ctab, off_red, off_ring;   // shared memory
     size_t smem;
+    bool halves;   // 9..16 rows: two blocks per tile, eight rows each (grid counts both)
     bool ok;
 };
 BatchPlan batch_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit);
@@ -121,11 +123,6 @@ cudaError_t batch_configure();
 // gemv_stream.cu
 int count_tiles(const LinArgs& a, int tile_rows);
 StreamPart stream_part(int fmt, const LinArgs& a, int sm_count);
-// How an operator of up to 16 rows multiplies int8 weights.  Operators whose tiles split K (the layers of a model: latency) take
-// FMT_INT8H: the codes become fp16 and meet the activations as they are, with nothing to be built from those before the first MMA.
-// Whole-row tiles (an lm_head: throughput) keep FMT_INT8: the codes go into integer MMAs as they are, against three limbs of the
-// activations; turning them into fp16 takes five instructions per four codes, and one row of 151936 x 896 so took 29.2 us instead of 25.3.
-inline int stream_format(int fmt, const LinArgs& a, int sm_count) { return fmt == FMT_INT8 && stream_part(fmt, a, sm_count).kw != 1 ? (int)FMT_INT8H : fmt; }
 constexpr int SK_MAX_BLOCKS = 1024;                         // grid limit of a balanced launch (sizes its scratch)
 constexpr size_t SK_SCRATCH_BYTES = (size_t)SK_MAX_BLOCKS * 128 * 16 * sizeof(float);
 bool stream_supported(int fmt, int M, int K, const LinArgs& a);
@@ -201,7 +198,7 @@ inline bool q4_scale_views(const LinArgs& a, const uint16_t* base[4], int* pitch
 }
 cudaError_t launch_l2_flush(void* buf, size_t bytes, cudaStream_t st);
 // the staged activations of a batched call (layout of the streaming kernel's shared memory), with the optional RMSNorm
-constexpr size_t STAGE_IMG_BYTES = (size_t)1 << 20;   // the context's room for them (16 rows of 32 000 values)
+constexpr size_t STAGE_IMG_BYTES = (size_t)1 << 20;   // the context's room for them (int8: 16 rows of 21 000 values)
 size_t stage_image_bytes(int fmt, int M, int K);
 int stage_row_bytes(int K);   // of a row of fp16 values in such an image
 cudaError_t launch_stage_image(int fmt, const uint16_t* x, int M, int K, const uint16_t* norm_w, float eps, uint8_t* img, cudaStream_t st,

@@ -192,7 +192,7 @@ cudaError_t build_run(const std::vector<RecordedOp>& rec, const std::vector<OpDe
         size_t wbytes = 0;
         for (int k = 0; k < a.nseg; ++k) wbytes += (size_t)a.seg[k].N * rowbytes;
         s.flags = (wbytes > ((size_t)96 << 20) ? PLAN_EVICT_FIRST : 0) | (r.fmt == FMT_Q4 ? PLAN_SCALE_TMA : 0);
-        if (int8_weights(r.fmt)) {
+        if (r.fmt == FMT_INT8) {
             // the row scales are static data like the weights: the producer brings them along
             bool aligned = true;
             for (int k = 0; k < a.nseg; ++k) aligned = aligned && (reinterpret_cast<uintptr_t>(a.seg[k].scale) & 15) == 0;

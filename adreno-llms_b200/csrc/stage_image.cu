@@ -2,7 +2,7 @@
 //
 // The streaming kernel keeps the whole activation batch in shared memory in a per-format staged
 // form (int8: three limb planes of a per-row 24-bit fixed-point copy plus the row scales; Q4: rows
-// permuted for ldmatrix plus the table of -72 * (sum of a block's activations); fp16, int8 as fp16: the rows).
+// permuted for ldmatrix plus the table of -72 * (sum of a block's activations); fp16: the rows).
 // With one token every block builds that form itself out of a few KB.  With M rows the same work
 // (up to 230 KB of output) repeated by every block of the launch is what bounds batched decode, so
 // a small grid, one block per activation row, writes the staged image (byte for byte the shared-
@@ -43,10 +43,9 @@ __global__ void __launch_bounds__(ST_MAX) stage_image_kernel(const uint16_t* __r
         row = xn;
     }
     const int xstride = x_stride_of(FMT, K);
-    if (FMT == FMT_FP16 || FMT == FMT_INT8H) {
+    if (FMT == FMT_FP16) {
         uint8_t* dst = img + (size_t)m * xstride;
-        for (int p = tid; p < x_values_of(FMT, K) / 8; p += nthr)
-            *reinterpret_cast<uint4*>(dst + p * 16) = p < K / 8 ? *reinterpret_cast<const uint4*>(row + p * 8) : make_uint4(0, 0, 0, 0);
+        for (int p = tid; p < K / 8; p += nthr) *reinterpret_cast<uint4*>(dst + p * 16) = *reinterpret_cast<const uint4*>(row + p * 8);
     } else if (FMT == FMT_INT8) {
         // the row's largest magnitude, then 24-bit fixed point in three 8-bit limbs (see stage_x_int8)
         const int per_row = K / 8;
@@ -154,7 +153,6 @@ cudaError_t launch_stage_image(int fmt, const uint16_t* x, int M, int K, const u
     cfg.numAttrs = 1;
     if (fmt == FMT_FP16) return cudaLaunchKernelEx(&cfg, stage_image_kernel<FMT_FP16>, x, M, K, norm_w, eps, img);
     if (fmt == FMT_INT8) return cudaLaunchKernelEx(&cfg, stage_image_kernel<FMT_INT8>, x, M, K, norm_w, eps, img);
-    if (fmt == FMT_INT8H) return cudaLaunchKernelEx(&cfg, stage_image_kernel<FMT_INT8H>, x, M, K, norm_w, eps, img);
     if (fmt == FMT_Q4) return cudaLaunchKernelEx(&cfg, stage_image_kernel<FMT_Q4>, x, M, K, norm_w, eps, img);
     return cudaErrorInvalidValue;
 }

@@ -25,7 +25,6 @@ constexpr int CTA_BOX = NCW * BOX_BYTES;    // one column box of the whole block
 constexpr int HDR_BYTES = 128;              // zeros: the B operand of absent token rows
 
 __host__ __device__ inline int fmt_row_bytes(int fmt, int K) { return fmt == FMT_FP16 ? K * 2 : fmt == FMT_Q4 ? K / 2 : K; }
-__host__ __device__ constexpr bool int8_weights(int fmt) { return fmt == FMT_INT8 || fmt == FMT_INT8H; }
 
 // Bytes of one pipeline stage: nbox column boxes of the block, then (Q4) the block scales of the
 // stage's rows (row pitch sstride for per-lane copies; tensor copies land them densely).
@@ -34,15 +33,10 @@ __host__ __device__ inline int stage_sstride(int kcb) { return kcb / 8 + 16; }
 __host__ __device__ inline int stage_bytes_of(int fmt, int kcb) {
     return stage_nbox(kcb) * CTA_BOX + (fmt == FMT_Q4 ? ((NCW * WARP_ROWS * stage_sstride(kcb) + 1023) / 1024) * 1024 : 0);
 }
-// Staged activations.  fp16, Q4, int8 as fp16 (FMT_INT8H, whose 8-byte loads want rows 32 bytes apart modulo 128 where ldmatrix wants
-// 16): fp16 rows; int8: three 8-bit limb planes of a 24-bit fixed-point
-// copy (row stride K + 16 bytes) followed by 192 bytes of per-row maximum and scale words.
-// The values of a staged row.  An int8 step is 64 values: the second half of a row's last step may lie past the row's end, where the
-// weights are zeros (the tensor copy's fill) and the activations must be numbers: zeros, in the fp16 form (in the integer form any bytes are).
-__host__ __device__ inline int x_values_of(int fmt, int K) { return fmt == FMT_INT8H ? (K + 63) / 64 * 64 : K; }
-__host__ __device__ inline int x_stride_of(int fmt, int K) {
-    return fmt == FMT_INT8 ? K + 16 : fmt == FMT_INT8H ? x_values_of(fmt, K) * 2 + 32 : K * 2 + 16;
-}
+// Staged activations.  fp16 / Q4: fp16 rows; int8: three 8-bit limb planes of a 24-bit fixed-point
+// copy (row stride K + 16 bytes) followed by 192 bytes of per-row maximum and scale words.  An int8 step is 64 values: the second
+// half of a row's last step may lie past the row's end, where the weights are zeros (the tensor copy's fill) and any limbs will do.
+__host__ __device__ inline int x_stride_of(int fmt, int K) { return fmt == FMT_INT8 ? K + 16 : K * 2 + 16; }
 __host__ __device__ inline int x_bytes_of(int fmt, int M, int K) {
     return (((fmt == FMT_INT8 ? 3 * M * x_stride_of(fmt, K) + 192 : M * x_stride_of(fmt, K)) + 127) / 128) * 128;
 }
@@ -65,6 +59,27 @@ constexpr int KPARTS = 2 * NCW;
 // the weight row's scale.  A row holding Inf or NaN is flagged and produces NaN.
 // Layout: limb planes [3][M][K + 16] (natural k order), then 16 row-maximum words (which the
 // caller has cleared) and 16 floats 2^-p.
+// The scale 2^p of a row, from the fp16 bits of its largest magnitude, and 2^-p (NaN for a row that holds Inf or NaN).
+__device__ __forceinline__ void int8_row_scale(unsigned mx, float& up, float& down) {
+    const bool bad = mx >= 0x7C00u;
+    // exponent of the largest magnitude: fp16 normal 2^(e-15), subnormals counted as 2^-14
+    const int e = (int)(mx >> 10) > 0 ? (int)(mx >> 10) - 15 : -14;
+    const int pw = (mx == 0u || bad) ? 0 : 22 - e;  // max|x| * 2^pw < 2^23
+    up = __int_as_float((127 + pw) << 23);
+    down = bad ? __int_as_float(0x7FC00000) : __int_as_float((127 - pw) << 23);
+}
+// The limbs (0: signed, 1, 2: unsigned) of four neighbouring values, a byte each in order.
+__device__ __forceinline__ void int8_limbs(uint32_t x01, uint32_t x23, float up, uint32_t (&limb)[3]) {
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&x01)), b = __half22float2(*reinterpret_cast<const __half2*>(&x23));
+    const uint32_t f0 = (uint32_t)__float2int_rn(a.x * up), f1 = (uint32_t)__float2int_rn(a.y * up);
+    const uint32_t f2 = (uint32_t)__float2int_rn(b.x * up), f3 = (uint32_t)__float2int_rn(b.y * up);
+    const uint32_t lo01 = __byte_perm(f0, f1, 0x5140), lo23 = __byte_perm(f2, f3, 0x5140);   // bytes 0, 0, 1, 1
+    limb[2] = __byte_perm(lo01, lo23, 0x5410);
+    limb[1] = __byte_perm(lo01, lo23, 0x7632);
+    limb[0] = __byte_perm(__byte_perm(f0, f1, 0x0062), __byte_perm(f2, f3, 0x0062), 0x5410);
+}
+// The larger magnitudes of two fp16 pairs, half by half (fp16 bits without the sign).
+__device__ __forceinline__ uint32_t half2_magnitude_max(uint32_t mx, uint32_t v) { return __vmaxu2(mx, v & 0x7FFF7FFFu); }
 __device__ __forceinline__ void stage_x_int8(const uint16_t* __restrict__ x, int M, int K, uint8_t* xs, int xstride, int tid,
                                              int nthreads) {
     unsigned int* rowmax = reinterpret_cast<unsigned int*>(xs + 3 * M * xstride);  // [16] max |x| bits, then [16] floats
@@ -160,12 +175,12 @@ __device__ __forceinline__ void stage_x_int8(const uint16_t* __restrict__ x, int
 
 // Stage the activations [M, K] fp16 into shared memory, permuted per format so
 // that ldmatrix over 16-byte pieces yields B fragments in the weights' packed order:
-//   fp16, int8 as fp16: identity
+//   fp16: identity
 //   Q4  : per 32 k   -> piece j, pair t = (k 8t+j, k 8t+j+4)
 template <int FMT>
 __device__ __forceinline__ void stage_x(const uint16_t* __restrict__ x, int M, int K, uint8_t* xs, int xstride, float* ctab, int tid,
                                         int nthreads) {
-    if (FMT != FMT_Q4) {
+    if (FMT == FMT_FP16) {
         const int per_row = K / 8;  // 16-byte pieces
         constexpr int BATCH = 8;    // loads first, then the stores (see stage_x_int8)
         for (int i0 = tid; i0 < M * per_row; i0 += BATCH * nthreads) {
@@ -183,10 +198,6 @@ __device__ __forceinline__ void stage_x(const uint16_t* __restrict__ x, int M, i
                     *reinterpret_cast<uint4*>(xs + m * xstride + p * 16) = v[j];
                 }
             }
-        }
-        if (FMT == FMT_INT8H) {
-            const int tail = x_values_of(FMT, K) / 8 - per_row;
-            for (int i = tid; i < M * tail; i += nthreads) *reinterpret_cast<uint4*>(xs + i / tail * xstride + (per_row + i % tail) * 16) = make_uint4(0, 0, 0, 0);
         }
     } else {
         const int per_row = K / 32;
@@ -361,8 +372,7 @@ struct LaneGeo {
     uint32_t a_row_off, a_q_lane; // fp16 / int8 ldmatrix.x4: (rows 0-7, piece q) (rows 8-15, q) (rows 0-7, q+1) (rows 8-15, q+1)
     uint32_t aq_off;              // Q4 ldmatrix.x4: the four 8-row groups (both row blocks) of one 16-byte piece
     uint32_t xr;
-    // B: matrix j = lane/8 (16-byte piece j of the 32-k step), row n = lane%8 (+8 per n tile); int8 as fp16: row n = lane/4, four
-    // values from 4 * (lane%4) on of each 16
+    // B: matrix j = lane/8 (16-byte piece j of the 32-k step), row n = lane%8 (+8 per n tile)
     uint32_t b_base[NT], b_step[NT], b_plane[NT];  // b_plane: int8 only, bytes between limb planes
     const uint8_t* ctab_lane[NT];  // Q4: this lane's accumulator-start quads (token pair t of each n tile), one per 32-weight block
     int ctab_step;
@@ -371,9 +381,6 @@ struct LaneGeo {
         return sw + (q >> 3) * CTA_BOX + off + (((q & 7) ^ xr) << 4);
     }
 };
-
-template <int FMT> __device__ __forceinline__ int b_row(int lane) { return FMT == FMT_INT8H ? lane >> 2 : lane & 7; }
-template <int FMT> __device__ __forceinline__ uint32_t b_lane_off(int lane) { return (uint32_t)(FMT == FMT_INT8H ? (lane & 3) * 8 : (lane >> 3) * 16); }
 
 // `two_weights`: the stage holds 16 rows of each of two weights per warp (gate rows in the first
 // half of a column box, up rows in the second half) instead of 32 rows of one.
@@ -391,10 +398,10 @@ __device__ __forceinline__ void lane_geo_init(LaneGeo<NT>& L, bool two_weights, 
     L.ctab_step = npair * 16;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-        const int n = b_row<FMT>(lane) + nt * 8;
+        const int n = (lane & 7) + nt * 8;
         const bool valid = n < aM;
-        L.b_base[nt] = valid ? xs_addr + n * xstride + b_lane_off<FMT>(lane) : zero_addr;
-        L.b_step[nt] = valid ? (FMT == FMT_INT8H ? 128u : 64u) : 0u;
+        L.b_base[nt] = valid ? xs_addr + n * xstride + (lane >> 3) * 16 : zero_addr;
+        L.b_step[nt] = valid ? 64u : 0u;
         L.b_plane[nt] = (FMT == FMT_INT8 && valid) ? (uint32_t)(aM * xstride) : 0u;
         L.ctab_lane[nt] = ctab + min(t + 4 * nt, npair - 1) * 16;
     }
@@ -406,9 +413,10 @@ __device__ __forceinline__ void lane_geo_init(LaneGeo<NT>& L, bool two_weights, 
 // A tile whose K is split over the four consumers (few-row operators) therefore is the sum of eight
 // K parts, part 2 * (chunk mod 4) + (unit mod 2): each consumer's two sets added first, then the four
 // consumers' sums in consumer order.  The resident kernel (decode_plan.cu) gives every part a warp of
-// its own, built from the same unit functions below (step_fp16 / step_int8h / block_q4_at), and adds
-// the parts in the same order, hence the same bits.  The integer sums of whole-row int8 tiles are exact
-// until the tile's end, so how a consumer's steps are dealt out does not matter there.
+// its own, built from the same unit functions below (step_fp16 / step_int8 / block_q4_at), and adds
+// the parts in the same order, hence the same bits.  int8 sums are exact integers until a consumer's
+// share of the tile ends, so how its steps are dealt out does not matter: kernels that give the two
+// sets warps of their own add their integers first.
 
 // fp16: one step = 64 bytes of each row = 32 k = two MMAs per row block.  `s` counts steps from the
 // start of the row (it addresses the activations), `s_in_chunk` from the start of the chunk.
@@ -491,76 +499,6 @@ __device__ __forceinline__ void int8_recombine(const int (&iacc)[3][2][NT][4], f
                 const float v = fmaf((float)iacc[0][rb][nt][i], 65536.f, fmaf((float)iacc[1][rb][nt][i], 256.f, (float)iacc[2][rb][nt][i]));
                 acc[rb][nt][i] = m < aM ? v * rowscale[m] : 0.f;
             }
-}
-
-// int8 as fp16: one step = 64 bytes of each row = 64 k = four MMAs per row block.  ldmatrix gives lane (g, t) the codes 4t .. 4t+3 of a
-// 16-byte piece of rows g and g + 8; as fp16 (exact) they are its two A registers per row of a k16 step whose k order is (4t, 4t+1)
-// for the first pairs and (4t+2, 4t+3) for the second, so the B registers are four neighbouring activations: one 8-byte load.
-// Against integer MMAs with limbs (above) there is no copy of the row to build (its maximum, the split: two barriers) and two bytes of
-// shared memory per activation instead of three: a recorded token of a 30-layer, 576-wide model 370 -> 324 us.
-//
-// The four MMAs of a unit start from zero and their sum is added in fp32: the tensor core cuts off what lies below its running sum
-// instead of rounding, so a chain over a long row would lose more than the additions do.
-template <int NT>
-struct FragInt8H {
-    uint32_t w[2][2][4], b[4][NT][2];   // [32-byte half][row block]; [k16 step]
-};
-template <int NT>
-__device__ __forceinline__ void load_int8h(const LaneGeo<NT>& L, uint32_t sw, int s, int s_in_chunk, FragInt8H<NT>& f) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int rb = 0; rb < 2; ++rb)
-            ldsm_x4(L.piece_addr(sw, (rb ? L.rb_base1 : L.rb_base0) + L.a_row_off, (uint32_t)s_in_chunk * 4 + 2 * h + L.a_q_lane), f.w[h][rb][0],
-                        f.w[h][rb][1], f.w[h][rb][2], f.w[h][rb][3]);
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) lds_v2(L.b_base[nt] + s * L.b_step[nt] + j * 32, f.b[j][nt][0], f.b[j][nt][1]);
-}
-template <int NT>
-__device__ __forceinline__ void mac_int8h(const FragInt8H<NT>& f, float (&ac)[2][NT][4]) {
-#pragma unroll
-    for (int rb = 0; rb < 2; ++rb) {
-        float d[NT][4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            uint32_t a0, a1, a2, a3;
-            int8x4_to_half2x2(f.w[j / 2][rb][2 * (j & 1)], a0, a2);
-            int8x4_to_half2x2(f.w[j / 2][rb][2 * (j & 1) + 1], a1, a3);
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-                if (j == 0) mma_16816_c(d[nt], a0, a1, a2, a3, f.b[j][nt][0], f.b[j][nt][1], make_float4(0.f, 0.f, 0.f, 0.f));
-                else mma_16816(d[nt], a0, a1, a2, a3, f.b[j][nt][0], f.b[j][nt][1]);
-            }
-        }
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) ac[rb][nt][i] += d[nt][i];
-    }
-}
-template <int NT>
-__device__ __forceinline__ void step_int8h(const LaneGeo<NT>& L, uint32_t sw, int s, int s_in_chunk, float (&ac)[2][NT][4]) {
-    FragInt8H<NT> f;
-    load_int8h<NT>(L, sw, s, s_in_chunk, f);
-    mac_int8h<NT>(f, ac);
-}
-// K chunk c.  The next unit's operands are on their way while this one's codes are converted.
-template <int NT>
-__device__ __forceinline__ void chunk_int8h(const LaneGeo<NT>& L, uint32_t sw, int c, int kcb, int cb, float (&acc)[2][2][NT][4]) {
-    const int s0 = (c * kcb) / 64, ns = (cb + 63) / 64;
-    if (ns <= 0) return;
-    FragInt8H<NT> f[2];
-    load_int8h<NT>(L, sw, s0, 0, f[0]);
-    int u = 0;
-    for (; u + 2 <= ns; u += 2) {
-        load_int8h<NT>(L, sw, s0 + u + 1, u + 1, f[1]);
-        mac_int8h<NT>(f[0], acc[0]);
-        if (u + 2 < ns) load_int8h<NT>(L, sw, s0 + u + 2, u + 2, f[0]);
-        mac_int8h<NT>(f[1], acc[1]);
-    }
-    if (u < ns) mac_int8h<NT>(f[0], acc[0]);
 }
 
 // Q4: one step = 16 bytes of each row = one 32-weight block = two MMAs per row block on the
@@ -658,7 +596,7 @@ template <int FMT>
 __device__ __forceinline__ uint16_t finish_row(float v, uint16_t scale_bits, int epi, uint16_t prev) {
     // explicit roundings (no fused multiply-add across the two steps): every kernel that finishes a row
     // (single-token, batched, resident) must give the same bits
-    if (int8_weights(FMT)) v = __fmul_rn(v, __half2float(__ushort_as_half(scale_bits)));
+    if (FMT == FMT_INT8) v = __fmul_rn(v, __half2float(__ushort_as_half(scale_bits)));
     if (epi == EPI_RESIDUAL) {
         v = __fadd_rn(__half2float(__ushort_as_half(prev)), v);
     } else if (epi == EPI_SILU_GATE) {
@@ -670,7 +608,7 @@ __device__ __forceinline__ uint16_t finish_row(float v, uint16_t scale_bits, int
 // ... and of one SwiGLU row from its gate and up sums
 template <int FMT>
 __device__ __forceinline__ uint16_t finish_swiglu(float gv, float uv, uint16_t gscale_bits, uint16_t uscale_bits) {
-    if (int8_weights(FMT)) {
+    if (FMT == FMT_INT8) {
         gv *= __half2float(__ushort_as_half(gscale_bits));
         uv *= __half2float(__ushort_as_half(uscale_bits));
     }
