@@ -893,11 +893,19 @@ bool cached_map(CUtensorMap* m, const MapKey& k) {
     const cuuint64_t strides[2] = {cols_first ? 128 : k.stride1, cols_first ? k.stride1 : 128};
     const cuuint32_t box[3] = {cols_last || cols_first ? 128u : k.box0, cols_first ? k.box0 : k.box1, cols_first ? k.box1 : k.box0};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
-    if (g_encode_tiled(m, (k.kind & 1u) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, cols_last || cols_first ? 3 : 2, const_cast<void*>(k.base), dims, strides,
-                       box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, (k.kind & 2u) ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                       (k.kind & 4u) ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return false;
+    auto encode = [&] {
+        return g_encode_tiled(m, (k.kind & 1u) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, cols_last || cols_first ? 3 : 2,
+                              const_cast<void*>(k.base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              (k.kind & 2u) ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                              (k.kind & 4u) ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    if (!encode()) {
+        // A thread whose first CUDA call this is has no device context current, which the driver's encoder asks for and the runtime's
+        // calls bring along.
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess || !encode()) return false;
+    }
     s.key = k;
     s.map = *m;
     return true;

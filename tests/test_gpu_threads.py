@@ -47,3 +47,31 @@ def test_threads_leave_no_memory_behind(nnb, ctx):
     q.release()
     for b in (xb, ob):
         ctx.free(b)
+
+
+@pytest.mark.parametrize("fmt", ["fp16", "int8", "q4"])
+@pytest.mark.parametrize("M", [1, 2, 16, 40])
+def test_a_projection_as_a_threads_first_call(nnb, ctx, fmt, M):
+    N, K = 320, 768
+    q = nnb.QuantWeight(ctx, fmt, *make_weight(fmt, N, K, 3))
+    xb, ob = ctx.upload(make_x(M, K, 4).view(np.uint16)), ctx.alloc(M * N * 2)
+    ctx.linear(M, N, K, xb, q.buf, ob)
+    want = ctx.download(ob, (M, N), np.uint16)
+    ctx.upload(np.full((M, N), 0x7E00, np.uint16), ob)
+    ctx.sync()
+    errors = []
+
+    def work():
+        try:
+            ctx.linear(M, N, K, xb, q.buf, ob)
+        except Exception as e:                       # noqa: BLE001
+            errors.append(e)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert not errors, errors
+    assert np.array_equal(ctx.download(ob, (M, N), np.uint16), want)
+    q.release()
+    for b in (xb, ob):
+        ctx.free(b)
