@@ -86,6 +86,9 @@ __host__ __device__ inline int batch_xcols(int fmt, int K) {
     return (n + 3) / 8 * 8 + 4;
 }
 
+// Rows of activations that have room in shared memory: those there are, and one of zeros that stands for all absent ones.
+__host__ __device__ inline int batch_xrows(int M, int nt) { return M < 8 * nt ? M + 1 : 8 * nt; }
+
 // Keeps a value's computation where it stands: the compiler would move it past the waits to its first use.
 __device__ __forceinline__ void pin(uint32_t& v) { asm volatile("" : "+r"(v)); }
 __device__ __forceinline__ void pin(int& v) { asm volatile("" : "+r"(v)); }
@@ -398,7 +401,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
     mbar_init_fence();
     // Absent rows are zeros, but not by the copy: 128 bytes past the end take it five times as long as those that are there (9 rows of a
     // 24-layer, 896-wide int8 model 613 us with boxes of 16 rows, 493 so; 2 rows of a 16-layer, 1024-wide Q4 one 440 and 316).
-    for (uint32_t i = (uint32_t)(M * xpitch + tid * 16); i < (uint32_t)(8 * NT * xpitch); i += BATCH_THREADS * 16) *reinterpret_cast<uint4*>(sm + OFF_X + i) = make_uint4(0, 0, 0, 0);
+    for (uint32_t i = (uint32_t)(M * xpitch + tid * 16); i < (uint32_t)(batch_xrows(M, NT) * xpitch); i += BATCH_THREADS * 16) *reinterpret_cast<uint4*>(sm + OFF_X + i) = make_uint4(0, 0, 0, 0);
     __syncthreads();
 
     auto segment = [&](int tile) { return (a.nseg > 2 && tile >= a.seg[2].tile0) ? 2 : (a.nseg > 1 && tile >= a.seg[1].tile0) ? 1 : 0; };
@@ -508,8 +511,8 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
         const int n = FMT == FMT_FP16 ? lane & 7 : g;
         lg.b_x = (uint32_t)(n * a.xcols) & 7u;
         lg.b_q = (uint32_t)(IMMA ? t : 4 * set + (FMT == FMT_FP16 ? lane >> 3 : t));
-        lg.b = base + OFF_X + (uint32_t)(n * xpitch);
-        lg.b_up = 8u * (uint32_t)xpitch;
+        lg.b = base + OFF_X + (uint32_t)(min(n, M) * xpitch);
+        lg.b_up = (uint32_t)((min(n + 8, M) - min(n, M)) * xpitch);   // (eight rows of columns are whole turns of the swizzle)
         const int pairs = (M + 1) / 2;
         lg.start_step = pairs * 16;
 #pragma unroll
@@ -839,7 +842,7 @@ BatchPlan batch_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit)
     if (a.norm_w && a.K * 2 > batch_red_bytes(fmt, nt)) return p;       // the norm weight lies where the sums will
     const int sets = dual ? 2 : 1;
     p.stage_bytes = (sets * p.tile_rows * p.cols * (128 + (fmt == FMT_Q4 ? 16 : 0)) + 1023) / 1024 * 1024;
-    p.off_ring = OFF_X + 8 * nt * p.xcols * 128;
+    p.off_ring = OFF_X + (batch_xrows(p.halves ? 8 : a.M, nt) * p.xcols * 128 + 1023) / 1024 * 1024;
     // Two blocks per SM where that leaves each at least two stages (or all of its items): a block of the next launch can then be
     // resident, with its weights on their way, before this one's is done.
     const int ctab = ctab_bytes_of(fmt, a.M, a.K), red = batch_red_bytes(fmt, nt), rest = ctab + red;
