@@ -771,7 +771,7 @@ __global__ void __launch_bounds__(PLAN_BLOCK, 1) decode_plan_kernel(const __grid
     const int nops = P.nops;
     const int ring_off = (int)(((s_base + (uint32_t)P.off_ring + 1023u) & ~1023u) - s_base);
 
-    if (tid < HDR_BYTES / 4) reinterpret_cast<uint32_t*>(smem)[tid] = 0u;  // B operand of absent token rows
+    if (tid < ZERO_BYTES / 4) reinterpret_cast<uint32_t*>(smem)[tid] = 0u;  // B operand of absent token rows
     if (tid == 0) {
         *s_issued = 0xFFFFFFFFu;
         for (int s = 0; s < PLAN_SLOTS; ++s) {

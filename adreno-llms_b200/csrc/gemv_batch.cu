@@ -32,7 +32,7 @@ namespace {
 constexpr int BCW = KPARTS;                  // consumer warps
 constexpr int BATCH_THREADS = BCW * 32 + 32; // + the producer warp
 constexpr int BATCH_STAGES = 6;              // ring stages at most
-constexpr int OFF_BARS = HDR_BYTES;          // full[], empty[], and one for the activations
+constexpr int OFF_BARS = 0;                  // full[], empty[], and one for the activations
 constexpr int OFF_SCALE = 512;               // int8: 2^p of the 16 rows, then 2^-p
 constexpr int OFF_ROW = 640;                 // int8: a tile's 32 weight-row scales, then what is added or the second weight's scales
 constexpr int OFF_X = 1024;                  // (128-byte swizzle: 1 KB boundaries)

@@ -67,8 +67,8 @@ __host__ __device__ inline Geo make_geo(int fmt, int M, int K, int kcb, int stag
     g.off_sx = stage_bytes_of(fmt, kcb);
     g.xstride = x_stride_of(fmt, xcols ? xcols : K);
     g.stage_bytes = g.off_sx + (xcols ? ((fmt == FMT_INT8 ? 3 : 1) * M * g.xstride + 1023) / 1024 * 1024 : 0);
-    g.off_bar = HDR_BYTES;  // full[stages], empty[stages], and one for the staged activations
-    g.off_x = HDR_BYTES + ((stages * 16 + 8 + 127) / 128) * 128;
+    g.off_bar = ZERO_BYTES;  // full[stages], empty[stages], and in the last word before the activations one for those
+    g.off_x = 128 + ((stages * 16 + 127) / 128) * 128;
     g.off_ctab = g.off_x + (xcols ? 256 : x_bytes_of(fmt, M, K));   // (travelling int8 rows: their scales stay)
     // fused RMSNorm: the normalised fp16 activations [M][K], from which the staging then reads
     g.off_norm = g.off_ctab + (xcols ? 0 : ctab_bytes_of(fmt, M, K));
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(THREADS) linear_stream_kernel(const __grid_con
     float* red = reinterpret_cast<float*>(smem + geo.off_red);
     const uint32_t ring = (s_base + geo.off_ring + 1023u) & ~1023u;
 
-    if (tid < HDR_BYTES / 4) reinterpret_cast<uint32_t*>(smem)[tid] = 0u;
+    if (tid < ZERO_BYTES / 4) reinterpret_cast<uint32_t*>(smem)[tid] = 0u;
     if (FMT == FMT_INT8 && !xcols && tid >= 32 && tid < 48) reinterpret_cast<uint32_t*>(xs + 3 * gM * geo.xstride)[tid - 32] = 0u;  // per-row max words
     const uint32_t xbar = s_base + geo.off_x - 8;  // batched calls: the staged activations have landed
     if (tid == 0) {

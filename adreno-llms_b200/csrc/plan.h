@@ -71,13 +71,13 @@ __host__ __device__ inline bool plan_stage_fast(int K, bool norm) { return K / 8
 
 constexpr int PLAN_SLOTS = 16;        // ring items in flight per block
 constexpr int PLAN_MAX_OPS = 1024;    // operators per run (their tile table sits in shared memory)
-// head of the kernel's shared memory: HDR_BYTES of zeros, full[] and empty[] barriers, the producer's
+// head of the kernel's shared memory: 64 bytes of zeros, full[] and empty[] barriers, the producer's
 // table of items in flight (offset and end of each), the count of items issued by a producer that stopped early
-constexpr int PLAN_HDR_BARS = 128;
+constexpr int PLAN_HDR_BARS = 64;
 constexpr int PLAN_HDR_SLOTS = PLAN_HDR_BARS + 2 * PLAN_SLOTS * 8;
 constexpr int PLAN_HDR_ISSUED = PLAN_HDR_SLOTS + 2 * PLAN_SLOTS * 4;
 constexpr int PLAN_HDR_STATE = PLAN_HDR_ISSUED + 16;  // the consumers' state between operators (64 bytes)
-constexpr int PLAN_HDR_BYTES = 768;
+constexpr int PLAN_HDR_BYTES = 640;
 static_assert(PLAN_HDR_STATE + 64 <= PLAN_HDR_BYTES, "header layout");
 
 struct PlanParams {

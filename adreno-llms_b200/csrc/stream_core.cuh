@@ -22,7 +22,7 @@ constexpr int STREAM_THREADS = (NCW + 1) * 32;  // + one producer warp
 constexpr int WARP_ROWS = 32;               // weight rows per consumer warp per tile
 constexpr int BOX_BYTES = WARP_ROWS * 128;  // one warp's 128-byte column box (4 KB)
 constexpr int CTA_BOX = NCW * BOX_BYTES;    // one column box of the whole block (16 KB)
-constexpr int HDR_BYTES = 128;              // zeros: the B operand of absent token rows
+constexpr int ZERO_BYTES = 64;              // at the head of shared memory: the B operand of absent token rows
 
 __host__ __device__ inline int fmt_row_bytes(int fmt, int K) { return fmt == FMT_FP16 ? K * 2 : fmt == FMT_Q4 ? K / 2 : K; }
 
