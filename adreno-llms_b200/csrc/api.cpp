@@ -488,17 +488,19 @@ static int run_batch(nn_context* c, int fmt, LinArgs a, int M, const char* who, 
     *done = false;
     a.M = M;
     if (M == 2 && !a.norm_w && a.epi == EPI_STORE && c->capturing) return NN_OK;
-    const uint16_t* norm_w = c->capturing ? nullptr : a.norm_w;
+    const uint16_t* norm_w = nullptr;   // the norm that the staging launch applies
     const int pitch = stage_row_bytes(a.K);
-    if (norm_w) {
-        if ((size_t)M * pitch > c->stage_img_bytes || (size_t)a.K * 2 > ((size_t)48 << 10)) return NN_OK;
+    BatchPlan p = {};
+    if (!a.norm_w || c->capturing) p = batch_plan(fmt, a, a.norm_w ? BatchNorm::here : BatchNorm::none, c->sm_count, c->smem_limit);
+    if (!p.ok && a.norm_w) {   // (also a recorded norm that finds no room in the kernel)
+        norm_w = a.norm_w;
+        if ((size_t)M * pitch > c->stage_img_bytes || (size_t)a.K * 2 > ((size_t)48 << 10) || (reinterpret_cast<uintptr_t>(norm_w) & 15) != 0) return NN_OK;
         a.norm_w = nullptr;
+        p = batch_plan(fmt, a, BatchNorm::staged, c->sm_count, c->smem_limit);
     }
-    const BatchPlan p = batch_plan(fmt, a, c->sm_count, c->smem_limit);
     if (!p.ok) return NN_OK;
     cudaError_t e;
     if (norm_w) {
-        if ((reinterpret_cast<uintptr_t>(norm_w) & 15) != 0) return NN_OK;
         e = launch_stage_image(FMT_FP16, a.x, M, a.K, norm_w, a.norm_eps, (uint8_t*)c->stage_img, c->stream, c->use_pdl);
         if (e != cudaSuccess) return NN_FAIL(NN_ERR_CUDA, "%s: norm launch failed: %s (M=%d K=%d)", who, cudaGetErrorString(e), M, a.K);
         c->launches++;

@@ -802,16 +802,23 @@ cudaError_t batch_configure() {
     return e;
 }
 
+// Where the streaming kernel is the faster one although its tiles split K too.  Q4 gate and up of more than 8 rows without a norm (12 rows of
+// 3000 x 2048: 8.9 us here, 8.4 with the staging launch), and Q4 of many tiles, where the chain per tile counts and not the launch (438 tiles,
+// 3 rows of 14000 x 2048: 9.9 us here, 7.8 there; 304 tiles, gate and up of 4864 x 896 with the norm, are better here).
+static bool stream_is_faster(int fmt, const LinArgs& a, BatchNorm norm, int sm_count) {
+    if (fmt != FMT_Q4) return false;
+    const bool dual = a.epi == EPI_SWIGLU;
+    if (dual && a.M > 8 && norm == BatchNorm::none) return true;
+    return count_tiles(a, dual ? 16 : WARP_ROWS) > (norm == BatchNorm::none ? 2 : 4) * sm_count;
+}
+
 // Which batched calls this kernel takes: those that the streaming kernel takes with K split, whose activations are whole 128-byte columns and fit
 // in shared memory beside two stages of weights, and (Q4) whose block scales can be reached by tensor copies.  The K parts are the single call's.
-// Not Q4 gate and up of more than 8 rows without a norm (12 rows of 3000 x 2048: 8.9 us here, 8.4 with the staging launch; in steps, with the
-// norm, they are better here: 9 rows of a 16-layer, 1024-wide model 414 us, 432 with the staging launch for normed operators).
-// Nor Q4 of more than one tile (with a norm, which is another launch there: two) for each block that fits on the machine, where the chain per tile
-// counts and not the launch (438 tiles, 3 rows of 14000 x 2048: 9.9 us here, 7.8 there; 282 tiles, 14 rows of 9000 x 4096, 14.1 in both; 304
-// tiles, gate and up of 4864 x 896 with the norm, are better here).
+// Not those that are faster there (above), unless it would take other K parts than the single call's: a batch's rows have the single call's
+// bits, and a recorded call those of the eager one, whichever way each goes.
 // Nor whole-row tiles (an lm_head): the finish there needs no meeting of warps in the streaming kernel (16 rows of 151936 x 896 in fp16: 48 us in
 // both; 8 rows of 65536 x 1024 in Q4 20.6 against 16.5).
-BatchPlan batch_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit) {
+BatchPlan batch_plan(int fmt, const LinArgs& a, BatchNorm norm, int sm_count, size_t smem_limit) {
     BatchPlan p = {};
     if (a.M < 2 || a.npeer > 0 || a.sig.world > 0 || a.argmax_slot || !stream_supported(fmt, a.M, a.K, a)) return p;
     for (int i = 0; i < a.nseg; ++i)
@@ -821,10 +828,7 @@ BatchPlan batch_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit)
     if (fmt == FMT_Q4 && !q4_scale_views(a, base, &pitch)) return p;
     const StreamPart part = stream_part(fmt, a, sm_count);
     if (part.kw == 1) return p;
-    if (fmt == FMT_Q4 && a.M > 8 && !a.norm_w && a.epi == EPI_SWIGLU) {
-        const StreamPlan sp = stream_plan(fmt, a, sm_count, smem_limit);
-        if (sp.ok && sp.kcb == part.kcb) return p;   // (rows so long that it takes smaller chunks, and so other sums, stay here)
-    }
+    if (stream_is_faster(fmt, a, norm, sm_count) && stream_keeps_parts(fmt, a, part, smem_limit)) return p;
     const bool dual = a.epi == EPI_SWIGLU;
     p.halves = fmt == FMT_INT8 && a.M > 8;
     const int rb = fmt_row_bytes(fmt, a.K), nt = a.M > 8 && !p.halves ? 2 : 1, warp_rows = dual ? 16 : WARP_ROWS;
@@ -835,7 +839,6 @@ BatchPlan batch_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit)
     // 1024 x 4608, 8 rows, 8.4 -> 7.4 us.  Rows of one stage gain nothing (1024 x 1024: 3.3 against 3.5 us).
     if (!dual && groups > 1 && count_tiles(a, WARP_ROWS) * (p.halves ? 4 : 2) <= sm_count) p.tile_rows = 16;
     p.ntiles = count_tiles(a, p.tile_rows);
-    if (fmt == FMT_Q4 && p.ntiles > (a.norm_w ? 4 : 2) * sm_count) return p;
     p.cols = groups == 1 ? (rb + 127) / 128 : NCW * (p.kcb / 128);   // (not more than there are: what lies past the end takes a copy long)
     p.xcols = batch_xcols(fmt, a.K);
     if (a.K % 64 != 0 || p.xcols > 256 || p.cols * 16 > 256) return p;   // one copy's reach

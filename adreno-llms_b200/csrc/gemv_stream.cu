@@ -1034,7 +1034,8 @@ bool stream_supported(int fmt, int M, int K, const LinArgs& a) {
     return true;
 }
 
-// Tiles and K parts of an operator: they set the order of its sums, and do not depend on the number of activation rows.
+// Tiles and K parts of an operator: they set the order of its sums.  They do not depend on the number of activation rows, but rows that leave
+// too little room for two stages make stream_plan take smaller chunks than these.
 StreamPart stream_part(int fmt, const LinArgs& a, int sm_count) {
     const int rb = fmt_row_bytes(fmt, a.K), rb_cols = ((rb + 127) / 128) * 128, warp_rows = a.epi == EPI_SWIGLU ? 16 : WARP_ROWS;
     StreamPart p;
@@ -1044,8 +1045,35 @@ StreamPart stream_part(int fmt, const LinArgs& a, int sm_count) {
         p.kcb = (((rb + NCW - 1) / NCW + 127) / 128) * 128;  // one chunk per consumer when the row is short
         if (p.kcb > 384) p.kcb = 256;
     }
+    if (p.kw != 1 && fmt == FMT_Q4 && a.sk_scratch && a.sk_flags) {
+        // Between one and two 128-row tiles per SM with long rows (28672 x 8192: 224 tiles of 16 chunks): whole-row
+        // tiles dealt out evenly as pipeline items (the balanced launch below) beat the K split, which pays a
+        // four-way reduction and an epilogue per 32 rows (measured 33.8 against 37.6 us); with fewer than eight
+        // items per block the balanced launch does not apply and the K split stays (24576 x 4096: 16.6 against 19.6 us)
+        const int t128 = count_tiles(a, NCW * warp_rows);
+        const long long items = (long long)t128 * ((rb + 255) / 256);
+        if (t128 > sm_count && items >= (long long)8 * 2 * sm_count) {
+            p.kw = 1;
+            p.kcb = 256;
+        }
+    }
     if (p.kcb > rb_cols) p.kcb = rb_cols;
     return p;
+}
+
+// Rows too many or too long to be resident beside two stages (int8, 16 rows of 4864 values: 234 KB of limbs) travel with the
+// weights instead of being walked in slices that stream the weights again: the values of each row per stage, 0 when they are resident.
+static int travelling_cols(int fmt, const LinArgs& a, int M, int nt, bool norm, const StreamPart& part, size_t smem_limit) {
+    if (M < 2 || fmt == FMT_Q4 || norm || a.npeer > 0 || a.sig.world > 0 || stage_image_bytes(fmt, a.M, a.K) > STAGE_IMG_BYTES ||
+        (size_t)make_geo(fmt, M, a.K, part.kcb, 2, nt, norm, 0).total <= smem_limit)
+        return 0;
+    const int xcols = (part.kw == 1 ? 1 : NCW) * part.kcb / (fmt == FMT_FP16 ? 2 : 1);
+    return (size_t)make_geo(fmt, M, a.K, part.kcb, 2, nt, norm, xcols).total <= smem_limit ? xcols : 0;
+}
+
+bool stream_keeps_parts(int fmt, const LinArgs& a, const StreamPart& part, size_t smem_limit) {
+    const int nt = a.M > 8 ? 2 : 1;
+    return (size_t)make_geo(fmt, a.M, a.K, part.kcb, 2, nt, false, travelling_cols(fmt, a, a.M, nt, false, part, smem_limit)).total <= smem_limit;
 }
 
 // Geometry heuristics:
@@ -1067,30 +1095,11 @@ StreamPlan stream_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limi
                count_tiles(a, dual ? 16 : WARP_ROWS) * 2 <= sm_count;
     const int M = p.halves ? 8 : a.M;
     const int nt = M > 8 ? 2 : 1;
-    const int rb_cols = ((rb + 127) / 128) * 128;
     const int warp_rows = dual ? 16 : WARP_ROWS;
     const StreamPart part = stream_part(fmt, a, sm_count);
-    int kw = part.kw, kcb = part.kcb;
-    if (kw != 1 && fmt == FMT_Q4 && a.sk_scratch && a.sk_flags) {
-        // Between one and two 128-row tiles per SM with long rows (28672 x 8192: 224 tiles of 16 chunks): whole-row
-        // tiles dealt out evenly as pipeline items (the balanced launch below) beat the K split, which pays a
-        // four-way reduction and an epilogue per 32 rows (measured 33.8 against 37.6 us); with fewer than eight
-        // items per block the balanced launch does not apply and the K split stays (24576 x 4096: 16.6 against 19.6 us)
-        const int t128 = count_tiles(a, NCW * warp_rows);
-        const long long items = (long long)t128 * ((rb + 255) / 256);
-        if (t128 > sm_count && items >= (long long)8 * 2 * sm_count) {
-            kw = 1;
-            kcb = rb_cols < 256 ? rb_cols : 256;
-        }
-    }
-    // Rows too many or too long to be resident beside two stages (int8, 16 rows of 4864 values: 234 KB of limbs) travel with the
-    // weights instead of being walked in slices that stream the weights again.
-    int xcols = 0;
-    if (M > 1 && fmt != FMT_Q4 && !norm && a.npeer == 0 && a.sig.world == 0 && stage_image_bytes(fmt, a.M, K) <= STAGE_IMG_BYTES &&
-        (size_t)make_geo(fmt, M, K, kcb, 2, nt, norm, 0).total > smem_limit) {
-        xcols = (kw == 1 ? 1 : NCW) * kcb / (fmt == FMT_FP16 ? 2 : 1);
-        if ((size_t)make_geo(fmt, M, K, kcb, 2, nt, norm, xcols).total > smem_limit) xcols = 0;
-    }
+    const int kw = part.kw;
+    int kcb = part.kcb;
+    const int xcols = travelling_cols(fmt, a, M, nt, norm, part, smem_limit);
     while ((size_t)make_geo(fmt, M, K, kcb, 2, nt, norm, xcols).total > smem_limit && kcb > 128) kcb -= 128;
     if ((size_t)make_geo(fmt, M, K, kcb, 2, nt, norm, xcols).total > smem_limit) { p.ok = false; return p; }
     const int ntiles = count_tiles(a, kw == 1 ? NCW * warp_rows : warp_rows);

@@ -118,13 +118,15 @@ struct BatchPlan {
     bool halves;   // 9..16 rows: two blocks per tile, eight rows each (grid counts both)
     bool ok;
 };
-BatchPlan batch_plan(int fmt, const LinArgs& a, int sm_count, size_t smem_limit);
+enum class BatchNorm { none, here, staged };   // the call's RMSNorm: in the kernel, or applied by the staging launch before it
+BatchPlan batch_plan(int fmt, const LinArgs& a, BatchNorm norm, int sm_count, size_t smem_limit);
 cudaError_t launch_batch(int fmt, const LinArgs& a, const BatchPlan& p, cudaStream_t st, bool pdl);
 cudaError_t batch_configure();
 
 // gemv_stream.cu
 int count_tiles(const LinArgs& a, int tile_rows);
 StreamPart stream_part(int fmt, const LinArgs& a, int sm_count);
+bool stream_keeps_parts(int fmt, const LinArgs& a, const StreamPart& part, size_t smem_limit);   // a batched call whose rows are staged
 constexpr int SK_MAX_BLOCKS = 1024;                         // grid limit of a balanced launch (sizes its scratch)
 constexpr size_t SK_SCRATCH_BYTES = (size_t)SK_MAX_BLOCKS * 128 * 16 * sizeof(float);
 bool stream_supported(int fmt, int M, int K, const LinArgs& a);

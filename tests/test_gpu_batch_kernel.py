@@ -55,16 +55,22 @@ def test_rows_are_the_single_calls(nnb, ctx, fmt, N, K):
 
 
 @pytest.mark.parametrize("fmt", ["fp16", "int8", "q4"])
-@pytest.mark.parametrize("N,K", [(96, 256), (70, 1024), (70, 1088), (64, 4608), (64, 4672)])   # passes of 1024 values; the longest row, and one more
+# passes of 1024 values; the longest row that is normalised in the kernel by up to 8 rows of activations, and longer ones
+@pytest.mark.parametrize("N,K", [(96, 256), (70, 1024), (70, 1088), (64, 4608), (64, 4672), (2048, 8192)])
 def test_norm_in_a_recorded_launch(nnb, ctx, fmt, N, K):
     W, s = make_weight(fmt, N, K, 411)
     qw = nnb.QuantWeight(ctx, fmt, W, s)
     x, g = make_x(16, K, 412), (1.0 + 0.1 * np.random.default_rng(413).standard_normal(K)).astype(np.float16)
     x[2] *= np.float16(30.0)
     xb, gb, ob = ctx.upload(x.view(np.uint16)), ctx.upload(g.view(np.uint16)), ctx.alloc(16 * N * 2)
+    for m in range(16):
+        ctx.rmsnorm_linear(1, N, K, xb + m * K * 2, gb, 1e-5, qw.buf, ob + m * N * 2)
+    single = ctx.download(ob, (16, N), np.uint16)
     for M in (2, 5, 8, 11, 16):
         ctx.rmsnorm_linear(M, N, K, xb, gb, 1e-5, qw.buf, ob)
         want = ctx.download(ob, (M, N), np.uint16)
+        if K <= 4672:   # (longer rows in Q4 may go to the streaming kernel in smaller chunks: other sums than the single call's)
+            assert np.array_equal(want, single[:M]), f"{fmt} {N}x{K} M={M}"
         ctx.plan_begin()
         ctx.rmsnorm_linear(M, N, K, xb, gb, 1e-5, qw.buf, ob)
         plan = ctx.plan_end()
@@ -75,5 +81,35 @@ def test_norm_in_a_recorded_launch(nnb, ctx, fmt, N, K):
         ctx.sync()
         ctx.L.nn_plan_free(plan)
     qw.release()
+    for p in (xb, gb, ob):
+        ctx.free(p)
+
+
+# Gate and up with the norm: blocks that take several tiles, and both sides of the lines between the two kernels
+@pytest.mark.parametrize("fmt,N,K", [("q4", 2300, 320), ("q4", 4864, 896), ("q4", 8192, 2752), ("int8", 4864, 896), ("int8", 2300, 320), ("fp16", 9400, 320), ("fp16", 4864, 896)])
+def test_gate_and_up_with_the_norm(nnb, ctx, fmt, N, K):
+    (W, s), (U, u) = make_weight(fmt, N, K, 421), make_weight(fmt, N, K, 422)
+    qw, qu = nnb.QuantWeight(ctx, fmt, W, s), nnb.QuantWeight(ctx, fmt, U, u)
+    x, g = make_x(16, K, 423), (1.0 + 0.1 * np.random.default_rng(424).standard_normal(K)).astype(np.float16)
+    xb, gb, ob = ctx.upload(x.view(np.uint16)), ctx.upload(g.view(np.uint16)), alloc_with_canary(ctx, 16 * N * 2)
+    for m in range(16):
+        ctx.rmsnorm_gate_up_silu(1, N, K, xb + m * K * 2, gb, 1e-5, qw.buf, qu.buf, ob + m * N * 2)
+    single = ctx.download(ob, (16, N), np.uint16)
+    for M in (2, 8, 9, 16):
+        ctx.upload(np.full((M, N), 0x7E00, np.uint16), ob)
+        ctx.rmsnorm_gate_up_silu(M, N, K, xb, gb, 1e-5, qw.buf, qu.buf, ob)
+        want = ctx.download(ob, (M, N), np.uint16)
+        assert np.array_equal(want, single[:M]), f"{fmt} {N}x{K} M={M}"
+        ctx.upload(np.full((M, N), 0x7E00, np.uint16), ob)
+        ctx.plan_begin()
+        ctx.rmsnorm_gate_up_silu(M, N, K, xb, gb, 1e-5, qw.buf, qu.buf, ob)
+        plan = ctx.plan_end()
+        ctx.plan_launch(plan)
+        assert np.array_equal(ctx.download(ob, (M, N), np.uint16), want), f"{fmt} {N}x{K} M={M} recorded"
+        ctx.sync()
+        ctx.L.nn_plan_free(plan)
+    check_canary(ctx, ob, 16 * N * 2, f"{fmt} {N}x{K}")
+    for q in (qw, qu):
+        q.release()
     for p in (xb, gb, ob):
         ctx.free(p)
