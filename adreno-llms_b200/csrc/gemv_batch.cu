@@ -845,16 +845,20 @@ BatchPlan batch_plan(int fmt, const LinArgs& a, BatchNorm norm, int sm_count, si
     if (a.norm_w && a.K * 2 > batch_red_bytes(fmt, nt)) return p;       // the norm weight lies where the sums will
     const int sets = dual ? 2 : 1;
     p.stage_bytes = (sets * p.tile_rows * p.cols * (128 + (fmt == FMT_Q4 ? 16 : 0)) + 1023) / 1024 * 1024;
-    p.off_ring = OFF_X + (batch_xrows(p.halves ? 8 : a.M, nt) * p.xcols * 128 + 1023) / 1024 * 1024;
-    // Two blocks per SM where that leaves each at least two stages (or all of its items): a block of the next launch can then be
-    // resident, with its weights on their way, before this one's is done.
+    const int xrow = p.xcols * 128;
+    p.off_ring = OFF_X + (batch_xrows(p.halves ? 8 : a.M, nt) * xrow + 1023) / 1024 * 1024;
+    // Two blocks per SM where that leaves each at least two stages (or all of its items): a block of the next launch can then be resident, with
+    // its weights on their way, before this one's is done.  With long rows one block and a deep ring are better, also for so few rows of
+    // activations that two blocks would fit (fp16 2048 x 8192, 3 rows: 14.4 us as two blocks, 10.5 as one); so are few tiles, where it asks for
+    // so much shared memory that the next launch's blocks go to SMs that are idle (Q4 1024 x 4608, 3 rows: 6.9 and 6.0 us).
+    const bool deep = groups > 4 || p.ntiles * (p.halves ? 2 : 1) * 2 <= sm_count;
     const int ctab = ctab_bytes_of(fmt, a.M, a.K), red = batch_red_bytes(fmt, nt), rest = ctab + red;
     for (int ps = 2; ps >= 1; --ps) {
-        const long long budget = (long long)((smem_limit + 1024) / ps) - 1024 - 1024 - p.off_ring - rest;   // 1 KB to align the start
+        const long long budget = (long long)((smem_limit + 1024) / ps) - 1024 - 1024 - rest;   // 1 KB to align the start
         const int resident = sm_count * ps / (p.halves ? 2 : 1), waves = (p.ntiles + resident - 1) / resident, items = waves * groups;
         const int least = items < 2 ? 1 : 2;
-        int st = (int)(budget / p.stage_bytes);
-        if (budget < 0 || st < least) continue;
+        if (budget - (ps == 2 && deep ? OFF_X + 8 * nt * xrow : p.off_ring) < (long long)least * p.stage_bytes) continue;
+        int st = (int)((budget - p.off_ring) / p.stage_bytes);
         if (st > items) st = items;
         if (st > BATCH_STAGES) st = BATCH_STAGES;
         p.stages = st;
@@ -862,6 +866,7 @@ BatchPlan batch_plan(int fmt, const LinArgs& a, BatchNorm norm, int sm_count, si
         p.off_ctab = p.off_ring + st * p.stage_bytes;
         p.off_red = p.off_ctab + ctab;
         p.smem = (size_t)p.off_red + red + 1024;
+        if (ps == 1 && p.smem < (smem_limit + 1024) / 2) p.smem = (smem_limit + 1024) / 2;
         p.ok = true;
         break;
     }
