@@ -492,7 +492,7 @@ static int run_batch(nn_context* c, int fmt, LinArgs a, int M, const char* who, 
     const int pitch = stage_row_bytes(a.K);
     BatchPlan p = {};
     if (!a.norm_w || c->capturing) p = batch_plan(fmt, a, a.norm_w ? BatchNorm::here : BatchNorm::none, c->sm_count, c->smem_limit);
-    if (!p.ok && a.norm_w) {   // (also a recorded norm that finds no room in the kernel)
+    if (!p.ok && !p.streams && a.norm_w) {   // (also a recorded norm that finds no room in the kernel)
         norm_w = a.norm_w;
         if ((size_t)M * pitch > c->stage_img_bytes || (size_t)a.K * 2 > ((size_t)48 << 10) || (reinterpret_cast<uintptr_t>(norm_w) & 15) != 0) return NN_OK;
         a.norm_w = nullptr;

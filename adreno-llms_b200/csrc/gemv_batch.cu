@@ -802,14 +802,48 @@ cudaError_t batch_configure() {
     return e;
 }
 
-// Where the streaming kernel is the faster one although its tiles split K too.  Q4 gate and up of more than 8 rows without a norm (12 rows of
-// 3000 x 2048: 8.9 us here, 8.4 with the staging launch), and Q4 of many tiles, where the chain per tile counts and not the launch (438 tiles,
-// 3 rows of 14000 x 2048: 9.9 us here, 7.8 there; 304 tiles, gate and up of 4864 x 896 with the norm, are better here).
+// Where the streaming kernel is the faster one although its tiles split K too: there the rows are staged by a launch before (small Q4 batches
+// without a norm: by each block), here they come into every block, which applies the norm and builds the Q4 starts or the int8 limbs anew.
+// The more tiles and the longer the rows, the more of that, and the less a launch counts.  All times in us, "here / there", of recorded
+// operators one after another over weights that come from memory.
 static bool stream_is_faster(int fmt, const LinArgs& a, BatchNorm norm, int sm_count) {
-    if (fmt != FMT_Q4) return false;
-    const bool dual = a.epi == EPI_SWIGLU;
-    if (dual && a.M > 8 && norm == BatchNorm::none) return true;
-    return count_tiles(a, dual ? 16 : WARP_ROWS) > (norm == BatchNorm::none ? 2 : 4) * sm_count;
+    const int tiles = count_tiles(a, a.epi == EPI_SWIGLU ? 16 : WARP_ROWS), M = a.M, K = a.K;
+    const int two_per_sm = 2 * sm_count + 8;   // (with a few blocks that take a second tile: 4864 x 896, gate and up, has 304)
+    if (norm == BatchNorm::staged && tiles * K <= 100 * 1024) return false;   // two launches both ways, and the host is what counts: q/k/v 2048 x 1024: 6.5 / 7.2
+    if (fmt == FMT_Q4) {
+        if (norm == BatchNorm::staged) return true;            // gate and up 8192 x 1536, 2 rows: 12.2 / 8.4
+        if (norm == BatchNorm::here) {
+            if (K > 1536) return true;                         // 2048 x 2048, 2 rows: 6.1 / 5.5; 1024 x 1024: 3.5 / 4.2
+            if (M > 8) return M * K > 9216 || tiles > 48;      // two rows to normalise per warp: 1536 x 576, gate and up, 16 rows: 5.6 / 5.0; 896 x 896, 9 rows: 4.6 / 4.8
+            if (tiles > sm_count) return M * K > 4608 || tiles > two_per_sm;   // gate and up 4608 x 1024, 8 rows: 6.6 / 5.7; 4864 x 896, 5 rows: 6.2 / 6.9
+            return M * K > 8192;                               // 576 x 1536, 8 rows: 5.1 / 4.9, 5 rows: 4.8 / 5.1
+        }
+        if (tiles <= 48) return false;                         // 896 x 4864, 8 rows: 7.1 / 8.4; 896 x 896: 2.9 / 3.1
+        if (K > 4096) return tiles > sm_count;                 // 2048 x 8192, 8 rows: 10.7 / 13.9; q/k/v 6000 x 8192, 4 rows: 18.0 / 16.9
+        if (K <= 1024 && M >= 6) return tiles > (M <= 8 ? two_per_sm : sm_count);   // 4864 x 896, 8 rows: 4.1 / 4.7; gate and up, 16 rows: 7.3 / 7.1
+        return true;                                           // 2048 x 2048, 5 rows: 5.6 / 4.8; 9400 x 1024, 2 rows: 4.9 / 3.9
+    }
+    if (fmt == FMT_INT8) {
+        // limbs: three bytes per value, which must leave room for the ring there
+        const bool roomy = 3ll * M * K <= (M <= 8 ? 40000 : 147456);
+        if (norm == BatchNorm::staged || (norm == BatchNorm::here && K > 1536))
+            return roomy || tiles <= 3 * sm_count;             // 3000 x 2048, gate and up, 5 rows: 7.7 / 6.5; 9000 x 4096, 8 rows: 20.6 / 27.0
+        if (norm == BatchNorm::here) {
+            if (M <= 8) return tiles > 200;                    // gate and up 4608 x 1024, 5 rows: 5.9 / 5.2; q/k/v 2048 x 1024: 4.5 / 4.7
+            if (M > 12 && K <= 960 && tiles <= two_per_sm) return false;   // gate and up 4864 x 896, 16 rows: 8.7 / 9.3
+            return tiles > (K <= 640 ? sm_count : 48);         // two blocks per tile: 4864 x 896, 9 rows: 6.7 / 5.7; q/k/v 1152 x 896: 4.4 / 4.6
+        }
+        if (!roomy) return false;                              // 28672 x 4096, 8 rows: 27.7 / 35.5, 16 rows: 47.4 / 75.4
+        if (M <= 8) return tiles > two_per_sm && K >= 512 && (K < 2048 || K % 128 != 0);   // 18900 x 1024, 8 rows: 8.7 / 7.4; gate and up 14000 x 2048, 5 rows: 14.1 / 15.0
+        if (tiles > 2 * two_per_sm) return true;               // 30000 x 320, 16 rows: 14.0 / 10.1
+        return K >= 512 && (M < 12 ? tiles > 120 : tiles * K > 450000);   // 4096 x 4096, 9 rows: 10.5 / 9.3; 9400 x 1536, 12 rows: 16.6 / 12.7; 4864 x 896: 5.7 / 6.7
+    }
+    if (norm == BatchNorm::staged)   // gate and up 4864 x 896, 2 rows: 7.7 / 6.9; 2048 x 2048, 2 rows: 7.4 / 8.7, 9 rows: 8.0 / 6.3; gate and up 9000 x 4096, 8 rows: 29.5 / 48.5
+        return K < 4096 && (tiles > sm_count ? M * K <= 16384 : K < 2048 || M > 8);
+    if (norm == BatchNorm::here)
+        return (K >= 1024 && K <= 1088 && tiles > 200 && tiles <= 2 * sm_count) ||             // gate and up 4608 x 1024, 8 rows: 6.9 / 6.1; 4864 x 896: 6.5 / 8.2
+               (M > 8 && M * K >= 16384 && K < 4096 && tiles >= 32 && tiles <= sm_count);      // 2048 x 2048, 12 rows: 8.1 / 6.4
+    return false;                                              // 576 x 576, 2 rows: 2.1 / 3.3; 28672 x 4096, 16 rows: 52 / 69
 }
 
 // Which batched calls this kernel takes: those that the streaming kernel takes with K split, whose activations are whole 128-byte columns and fit
@@ -828,7 +862,8 @@ BatchPlan batch_plan(int fmt, const LinArgs& a, BatchNorm norm, int sm_count, si
     if (fmt == FMT_Q4 && !q4_scale_views(a, base, &pitch)) return p;
     const StreamPart part = stream_part(fmt, a, sm_count);
     if (part.kw == 1) return p;
-    if (stream_is_faster(fmt, a, norm, sm_count) && stream_keeps_parts(fmt, a, part, smem_limit)) return p;
+    p.streams = stream_is_faster(fmt, a, norm, sm_count) && stream_keeps_parts(fmt, a, part, smem_limit);
+    if (p.streams) return p;
     const bool dual = a.epi == EPI_SWIGLU;
     p.halves = fmt == FMT_INT8 && a.M > 8;
     const int rb = fmt_row_bytes(fmt, a.K), nt = a.M > 8 && !p.halves ? 2 : 1, warp_rows = dual ? 16 : WARP_ROWS;

@@ -116,6 +116,7 @@ struct BatchPlan {
     int off_ctab, off_red, off_ring;   // shared memory
     size_t smem;
     bool halves;   // 9..16 rows: two blocks per tile, eight rows each (grid counts both)
+    bool streams;  // not ok because the streaming kernel is faster
     bool ok;
 };
 enum class BatchNorm { none, here, staged };   // the call's RMSNorm: in the kernel, or applied by the staging launch before it
