@@ -481,6 +481,17 @@ static void note_recorded(nn_context* c, int fmt, const LinArgs& a, const Stream
     c->rec.push_back(r);
 }
 
+// Whether an output lies over the activations.  Calls of 2..16 rows whose rows are staged by a launch of their own have read them before they write.
+static bool outputs_over_rows(const LinArgs& a, int rows) {
+    const uintptr_t x = (uintptr_t)a.x, end = x + (size_t)rows * a.K * 2;
+    bool over = false;
+    for (int i = 0; i < a.nseg; ++i) {
+        const uintptr_t o = (uintptr_t)a.seg[i].out;
+        over |= o < end && x < o + (size_t)rows * a.seg[i].ld_out * 2;
+    }
+    return over;
+}
+
 // 2..16 activation rows in one launch of the batch kernel, where it takes the shape.  Two kinds of call stay two launches, which callers
 // count (nn_launch_count, nn_plan_num_recorded and the tests of both say so): a norm outside a recording, where a call costs the host as much
 // as the device, is applied by the staging launch; a plain projection of two rows inside a recording takes that launch and the streaming kernel.
@@ -488,10 +499,13 @@ static int run_batch(nn_context* c, int fmt, LinArgs a, int M, const char* who, 
     *done = false;
     a.M = M;
     if (M == 2 && !a.norm_w && a.epi == EPI_STORE && c->capturing) return NN_OK;
+    // (its blocks fetch the rows one by one and store when they are done: rows under an output are staged first)
+    const bool over = outputs_over_rows(a, M);
+    if (over && !a.norm_w) return NN_OK;
     const uint16_t* norm_w = nullptr;   // the norm that the staging launch applies
     const int pitch = stage_row_bytes(a.K);
     BatchPlan p = {};
-    if (!a.norm_w || c->capturing) p = batch_plan(fmt, a, a.norm_w ? BatchNorm::here : BatchNorm::none, c->sm_count, c->smem_limit);
+    if (!a.norm_w || (c->capturing && !over)) p = batch_plan(fmt, a, a.norm_w ? BatchNorm::here : BatchNorm::none, c->sm_count, c->smem_limit);
     if (!p.ok && !p.streams && a.norm_w) {   // (also a recorded norm that finds no room in the kernel)
         norm_w = a.norm_w;
         if ((size_t)M * pitch > c->stage_img_bytes || (size_t)a.K * 2 > ((size_t)48 << 10) || (reinterpret_cast<uintptr_t>(norm_w) & 15) != 0) return NN_OK;
@@ -589,7 +603,7 @@ static int run_linear(nn_context* c, int fmt, LinArgs a, int M_total, const char
         LinArgs b = a;
         // Measured on whole batched steps: int8 and fp16 always gain from the staging launch; Q4 rows are cheap to
         // stage in place, so it pays only from about 12K activation values (or when there is a norm to apply)
-        const bool stage_pays = fmt != FMT_Q4 || (long long)a.M * a.K >= 12288 || a.norm_w != nullptr;
+        const bool stage_pays = fmt != FMT_Q4 || (long long)a.M * a.K >= 12288 || a.norm_w != nullptr || outputs_over_rows(a, a.M);
         if (a.M >= 2 && stage_pays && stream_supported(fmt, a.M, a.K, a) && stage_image_bytes(fmt, a.M, a.K) <= c->stage_img_bytes) {
             // batched: the activations (normalised when asked) are staged once, by a launch of their own
             b.norm_w = nullptr;

@@ -14,6 +14,8 @@
  *     The library never frees caller buffers.  Activations, scales and outputs
  *     are IEEE binary16; weights keep the exact on-disk byte layout written by
  *     scripts/convert_hf_to_bin.py and src/models/<model>/scripts/quantize_*.py.
+ *   - The activations x of a call must not overlap its outputs: they are read while results are written.
+ *     (Calls of 2..16 rows do read them first where their shape is taken by the streaming or the batch kernel.)
  *   - Every call is asynchronous on the context's single stream (the role of the
  *     reference's one in-order cl_command_queue): a result is visible to the next
  *     call on the same context without a host sync (nn_sync to wait on the host).

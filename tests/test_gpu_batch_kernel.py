@@ -140,3 +140,45 @@ def test_gate_and_up_with_the_norm(nnb, ctx, fmt, N, K):
         q.release()
     for p in (xb, gb, ob):
         ctx.free(p)
+
+
+@pytest.mark.parametrize("fmt", ["fp16", "int8", "q4"])
+@pytest.mark.parametrize("K", [576, 1024])
+def test_outputs_over_the_rows(nnb, ctx, fmt, K):
+    """A call of 2..16 rows has read its rows before it writes over them (the staging launch copies them)."""
+    (W, s), (U, u) = make_weight(fmt, K, K, 431), make_weight(fmt, K, K, 432)
+    qw, qu = nnb.QuantWeight(ctx, fmt, W, s), nnb.QuantWeight(ctx, fmt, U, u)
+    x, g = make_x(16, K, 433), (1.0 + 0.1 * np.random.default_rng(434).standard_normal(K)).astype(np.float16)
+    xb, gb, ob = ctx.upload(x.view(np.uint16)), ctx.upload(g.view(np.uint16)), ctx.alloc(16 * K * 2)
+    calls = {
+        "plain": lambda M, out: ctx.linear(M, K, K, xb, qw.buf, out),
+        "add": lambda M, out: ctx.linear_add(M, K, K, xb, qw.buf, out),
+        "swiglu": lambda M, out: ctx.fused_gate_up_silu(M, K, K, xb, qw.buf, qu.buf, out),
+        "norm": lambda M, out: ctx.rmsnorm_linear(M, K, K, xb, gb, 1e-5, qw.buf, out),
+    }
+    for form, call in calls.items():
+        for M in (2, 8, 16):
+            ctx.upload(x.view(np.uint16), xb)
+            ctx.upload(x.view(np.uint16), ob)
+            call(M, ob)
+            want = ctx.download(ob, (M, K), np.uint16)
+            for recorded in (False, True):
+                ctx.upload(x.view(np.uint16), xb)
+                before = ctx.launch_count()
+                if recorded:
+                    ctx.plan_begin()
+                    call(M, xb)
+                    plan = ctx.plan_end()
+                    assert ctx.L.nn_plan_num_recorded(plan) == 2, (form, M)
+                    ctx.plan_launch(plan)
+                else:
+                    call(M, xb)
+                    assert ctx.launch_count() - before == 2, (form, M)
+                assert np.array_equal(ctx.download(xb, (M, K), np.uint16), want), f"{fmt} {form} M={M} recorded={recorded}"
+                ctx.sync()
+                if recorded:
+                    ctx.L.nn_plan_free(plan)
+    for q in (qw, qu):
+        q.release()
+    for p in (xb, gb, ob):
+        ctx.free(p)
