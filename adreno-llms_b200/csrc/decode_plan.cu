@@ -94,12 +94,9 @@ struct CState {            // consumer-side state carried from operator to opera
     int ti;                // tiles finished so far (selects the reduction buffer)
     bool failed;
     unsigned ebase;        // epoch of operator i of this launch = ebase + i + 1
-    // what the staged activations in shared memory currently hold
-    const void* st_src;
-    unsigned st_epoch;
-    int st_fmt;
-    const void* st_norm;
+    int staged;            // which activations shared memory holds in staged form (PLAN_STAGED_SHIFT); 0: none
 };
+static_assert(sizeof(CState) <= 64, "PLAN_HDR_STATE");
 
 __device__ __noinline__ void report_failure(int* status, unsigned* state, int code) {
     *reinterpret_cast<volatile int*>(status) = code;
@@ -567,20 +564,16 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
     if (tile_first < ntiles) claim_item(off_first, slot_first);
 
     // ---------------- activations: fetch (poll the producer's words), normalise, stage ----------------
-    const void* src_id = D.x_ll ? (const void*)D.x_ll : (const void*)D.x;
     const unsigned x_epoch = D.x_ll ? S.ebase + (unsigned)D.x_epoch : 0u;
-    const bool reuse = S.st_src == src_id && S.st_epoch == x_epoch && S.st_fmt == FMT && S.st_norm == (const void*)D.norm_w;
+    const int wanted = D.flags >> PLAN_STAGED_SHIFT;
     LaneGeo<1> lg;
     lane_geo_init<FMT, 1>(lg, DUAL, quarter, lane, 1, s_base + (uint32_t)P.off_xs, xstride, s_base, smem + P.off_ctab);
     const float* rowscale = reinterpret_cast<const float*>(xs + 3 * xstride + 64);
-    if (!reuse) {
+    if (S.staged != wanted) {
         // (everyone is done with the previous staging and reduction buffers: the consumers met at this operator's start)
         S.failed = plan_stage_fast(aK, D.norm_w != nullptr) ? stage_fast<FMT>(P, D, smem, x_epoch, S.failed, tid, lane, warp)
                                                             : stage_general<FMT>(P, D, smem, x_epoch, S.failed, tid, lane, warp);
-        S.st_src = src_id;
-        S.st_epoch = x_epoch;
-        S.st_fmt = FMT;
-        S.st_norm = (const void*)D.norm_w;
+        S.staged = wanted;
     }
 
     for (int tile = tile_first; tile < ntiles;) {
@@ -931,10 +924,7 @@ __global__ void __launch_bounds__(PLAN_BLOCK, 1) decode_plan_kernel(const __grid
         S.ti = 0;
         S.failed = false;
         S.ebase = ld_relaxed_u32(P.state) * (unsigned)(nops + 1);
-        S.st_src = nullptr;
-        S.st_epoch = 0u;
-        S.st_fmt = -1;
-        S.st_norm = nullptr;
+        S.staged = 0;
         *reinterpret_cast<CState*>(smem + PLAN_HDR_STATE) = S;
     }
 

@@ -254,6 +254,12 @@ cudaError_t build_run(const std::vector<RecordedOp>& rec, const std::vector<OpDe
         }
         s.norm_w = a.norm_w;
         s.norm_eps = a.norm_eps;
+        auto same_rows = [&](const PlanOpScalars& q) {
+            return q.x == s.x && q.x_ll == s.x_ll && q.norm_w == s.norm_w && q.norm_eps == s.norm_eps && q.K == s.K && q.fmt == s.fmt;
+        };
+        int first_of = 0;
+        while (first_of < i && !same_rows(ops[first_of].s)) ++first_of;
+        s.flags |= (first_of + 1) << PLAN_STAGED_SHIFT;
         // the row as it was fetched: Q4 permutes it from there; rows too long for registers pass through it
         const bool fast = plan_stage_fast(a.K, a.norm_w != nullptr);
         if ((r.fmt == FMT_Q4 || !fast) && a.K > k_ll) k_ll = a.K;

@@ -60,6 +60,9 @@ enum : int {
     PLAN_ROW_SCALES = 4,   // int8: the tile's row scales arrive with its last item (bulk copy), when the tile's rows allow it
     PLAN_BIAS = 8,         // a bias row per segment is added to the stored result (PlanParams::bias)
 };
+// The flags' upper bits: a number from 1 on for what the operator stages (buffer and length, norm weight and eps, format).  A block whose
+// shared memory holds an operator's activations from one before does not stage them again.
+constexpr int PLAN_STAGED_SHIFT = 8;
 constexpr int PLAN_ROW_SCALE_BYTES = 1024;  // room for them at the end of an item: first weight at +0, second at +512
 // Bulk copies move multiples of 16 bytes: a tile's row scales travel with it when its valid rows are a multiple of 8.
 __host__ __device__ inline bool plan_rows_bulk_ok(int rows_valid) { return rows_valid > 0 && (rows_valid & 7) == 0; }
