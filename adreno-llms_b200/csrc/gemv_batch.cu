@@ -580,8 +580,8 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
         for (int cg = 0; cg < groups; ++cg) {
             const int c = cg * NCW + box;
             // A wait that runs out records an error and skips the arithmetic from then on; the warp still walks its items so that
-            // the block's barriers stay matched.
-            if (!failed && !mbar_wait_bounded(full0 + stage * 8, phase)) {
+            // the block's barriers stay matched, and still waits (not as long) for each copy, so that none is in flight when the block ends.
+            if (!mbar_wait_bounded(full0 + stage * 8, phase, failed ? WAIT_CYCLES / 64 : WAIT_CYCLES)) {
                 failed = true;
                 *reinterpret_cast<volatile int*>(a.status) = 1;
             }
