@@ -20,15 +20,13 @@ def test_rows(nnb, ctx, fmt, N, K):
     x, r = make_x(16, K, 502), make_x(16, N, 503)
     x[4, :40] = np.float16(np.inf)      # (what lies behind row 3 in shared memory)
     good = [m for m in range(16) if m != 4]
-    with np.errstate(invalid="ignore"):   # (row 4)
-        y = np.tile(x.astype(np.float64) @ cpu.dequant(fmt, W, s).astype(np.float64).T, (1, rep))[:, :N]
+    y = np.tile(x.astype(np.float64) @ cpu.dequant(fmt, W, s).astype(np.float64).T, (1, rep))[:, :N]
     xb, ob = ctx.upload(x.view(np.uint16)), alloc_with_canary(ctx, 16 * N * 2)
     ones = []
     for m in range(16):
         ctx.linear(1, N, K, xb + m * K * 2, qw.buf, ob + m * N * 2)
     ones = ctx.download(ob, (16, N), np.uint16).view(np.float16)
     check_close(ones[good], y[good], what=f"{fmt} {N}x{K}")
-    assert np.isnan(ones[4]).all() if fmt == "int8" else not np.isfinite(ones[4]).any()
     for M in (3, 16):
         ctx.upload(r.view(np.uint16), ob)
         ctx.linear_add(M, N, K, xb, qw.buf, ob)
