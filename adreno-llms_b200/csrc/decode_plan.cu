@@ -607,7 +607,7 @@ __device__ __noinline__ void run_op(const PlanParams& P, const PlanOpScalars& D,
                 if constexpr (WIDE) {
                     const int s0 = (c * kcb) / 64;
 #pragma unroll 1
-                    for (int u = set; u < (cb + 63) / 64; u += 2) step_int8<1>(lg, sw, s0 + u, u, iacc);
+                    for (int u = set; u < cb / 64; u += 2) step_int8<1>(lg, sw, s0 + u, u, iacc);
                 } else {
                     chunk_int8<1>(lg, sw, c, kcb, cb, iacc);
                 }

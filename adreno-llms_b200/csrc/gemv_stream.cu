@@ -1170,10 +1170,11 @@ cudaError_t launch_stream(int fmt, const LinArgs& a, const StreamPlan& p, cudaSt
     ka.a.ntiles = p.ntiles;
     ka.a.streamk = p.streamk ? 1 : 0;
     ka.stages = p.stages;
-    ka.rowbytes = fmt_row_bytes(fmt, a.K);
-    ka.nchunks = (ka.rowbytes + p.kcb - 1) / p.kcb;
+    const int rowbytes = fmt_row_bytes(fmt, a.K);
+    ka.rowbytes = step_row_bytes(fmt, a.K);
+    ka.nchunks = (rowbytes + p.kcb - 1) / p.kcb;
     size_t wbytes = 0;
-    for (int i = 0; i < a.nseg; ++i) wbytes += (size_t)a.seg[i].N * ka.rowbytes;
+    for (int i = 0; i < a.nseg; ++i) wbytes += (size_t)a.seg[i].N * rowbytes;
     ka.evict_first = wbytes > ((size_t)96 << 20) ? 1 : 0;  // weights that cannot stay in L2 anyway are streamed evict-first
     const bool dual = a.epi == EPI_SWIGLU;
     const int nt = a.M > 8 && !p.halves ? 2 : 1;
@@ -1183,9 +1184,9 @@ cudaError_t launch_stream(int fmt, const LinArgs& a, const StreamPlan& p, cudaSt
     for (int i = 0; i < a.nseg; ++i) {
         ka.a.seg[i].tile0 = t0;
         t0 += (a.seg[i].N + tile_rows - 1) / tile_rows;
-        if (!make_weight_map(&ka.tm[i], a.seg[i].W, a.seg[i].N, ka.rowbytes, tile_rows)) return cudaErrorInvalidValue;
+        if (!make_weight_map(&ka.tm[i], a.seg[i].W, a.seg[i].N, rowbytes, tile_rows)) return cudaErrorInvalidValue;
     }
-    if (dual && !make_weight_map(&ka.tm[3], a.W2, a.seg[0].N, ka.rowbytes, tile_rows)) return cudaErrorInvalidValue;
+    if (dual && !make_weight_map(&ka.tm[3], a.W2, a.seg[0].N, rowbytes, tile_rows)) return cudaErrorInvalidValue;
     // Q4 block scales by tensor copy: the scale rows (K / 16 bytes each) must keep 16-byte
     // pitch and alignment; otherwise the consumers fetch them with cp.async
     ka.scale_tma = 0;

@@ -182,7 +182,7 @@ cudaError_t build_run(const std::vector<RecordedOp>& rec, const std::vector<OpDe
         s.dual = dual ? 1 : 0;
         s.ksplit = r.p.kw > 1 ? 1 : 0;
         s.kcb = r.p.kcb;
-        s.rowbytes = rowbytes;
+        s.rowbytes = step_row_bytes(r.fmt, a.K);
         s.nchunks = (rowbytes + r.p.kcb - 1) / r.p.kcb;
         s.groups = s.ksplit ? (s.nchunks + NCW - 1) / NCW : s.nchunks;
         s.K = a.K;
