@@ -16,7 +16,7 @@
 //   * int8 has eight rows of activations per block at most, and two blocks per tile for 9..16: its exact sums are 24 registers per
 //     lane and eight rows (with 16 rows in a block, 48 registers of sums and some spills, the step below took 830 us).
 // Steps of 16 rows of a 24-layer, 896-wide model (staging launch + streaming kernel before): int8 771 -> 620 us, fp16 1063 -> 610; 8 rows
-// of a 16-layer, 1024-wide Q4 model 396 -> 364; 4 rows of a 30-layer, 576-wide int8 model 540 -> 449.
+// of a 16-layer, 1024-wide Q4 model 397 -> 360; 4 rows of a 30-layer, 576-wide int8 model 540 -> 449.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -399,8 +399,8 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) linear_batch_kernel(const __
     else if (tid == 2 * BATCH_STAGES) mbar_init(xbar, 1u);
     if (FMT == FMT_INT8 && tid < 32) reinterpret_cast<float*>(sm + OFF_SCALE)[tid] = 1.f;   // (absent rows)
     mbar_init_fence();
-    // Absent rows are zeros, but not by the copy: 128 bytes past the end take it five times as long as those that are there (9 rows of a
-    // 24-layer, 896-wide int8 model 613 us with boxes of 16 rows, 493 so; 2 rows of a 16-layer, 1024-wide Q4 one 440 and 316).
+    // Absent rows are zeros, but not by the copy: 128 bytes past the end take it five times as long as those that are there (a
+    // step of 2 rows, 16-layer, 1024-wide Q4 model: 440 us with boxes of 8 rows, 316 so).
     for (uint32_t i = (uint32_t)(M * xpitch + tid * 16); i < (uint32_t)(batch_xrows(M, NT) * xpitch); i += BATCH_THREADS * 16) *reinterpret_cast<uint4*>(sm + OFF_X + i) = make_uint4(0, 0, 0, 0);
     __syncthreads();
 
@@ -810,15 +810,22 @@ static bool stream_is_faster(int fmt, const LinArgs& a, BatchNorm norm, int sm_c
     const int tiles = count_tiles(a, a.epi == EPI_SWIGLU ? 16 : WARP_ROWS), M = a.M, K = a.K;
     const int two_per_sm = 2 * sm_count + 8;   // (with a few blocks that take a second tile: 4864 x 896, gate and up, has 304)
     if (norm == BatchNorm::staged && tiles * K <= 100 * 1024) return false;   // two launches both ways, and the host is what counts: q/k/v 2048 x 1024: 6.5 / 7.2
+    const bool two_waves = tiles > two_per_sm - sm_count / 3 && tiles <= two_per_sm;   // int8 above 8 rows: a wave is a tile per SM
     if (fmt == FMT_Q4) {
         if (norm == BatchNorm::staged) return true;            // gate and up 8192 x 1536, 2 rows: 12.2 / 8.4
         if (norm == BatchNorm::here) {
             if (K > 1536) return true;                         // 2048 x 2048, 2 rows: 6.1 / 5.5; 1024 x 1024: 3.5 / 4.2
             if (M > 8) return M * K > 9216 || tiles > 48;      // two rows to normalise per warp: 1536 x 576, gate and up, 16 rows: 5.6 / 5.0; 896 x 896, 9 rows: 4.6 / 4.8
-            if (tiles > sm_count) return M * K > 4608 || tiles > two_per_sm;   // gate and up 4608 x 1024, 8 rows: 6.6 / 5.7; 4864 x 896, 5 rows: 6.2 / 6.9
-            return M * K > 8192;                               // 576 x 1536, 8 rows: 5.1 / 4.9, 5 rows: 4.8 / 5.1
+            // gate and up 4608 x 1024, 8 rows: 6.6 / 5.7; 4864 x 896, 5 rows: 6.2 / 6.9; 9461 x 384, 6 rows: 5.7 / 5.1
+            if (tiles > sm_count) return M * K > 4608 || tiles > two_per_sm || (M >= 4 && K <= 640);
+            // 4494 x 832, 5 rows: 5.1 / 4.7; 576 x 1536, 8 rows: 5.1 / 4.9; gate and up 719 x 1536, 5 rows: 5.6 / 5.3
+            return M * K > 8192 || (M >= 4 && K > 768 && tiles > 110) || (M >= 5 && K > 1408 && tiles > 40);
         }
-        if (tiles <= 48) return false;                         // 896 x 4864, 8 rows: 7.1 / 8.4; 896 x 896: 2.9 / 3.1
+        if (M * K < 12288) {                                   // one launch there too
+            if (K <= 384) return M > 4 || tiles > 48;          // q/k/v 5625 x 384, 8 rows: 4.4 / 3.4; gate and up 970 x 320, 9 rows: 3.4 / 3.0
+            if (K <= 640 && M >= 6 && tiles > 140) return true;   // 8770 x 448, 8 rows: 4.8 / 4.0
+        }
+        if (tiles <= 48) return M > 14 && K > 2048 && K <= 2816;   // 896 x 4864, 8 rows: 7.1 / 8.4; 896 x 896: 2.9 / 3.1; 500 x 2624, 16 rows: 7.1 / 6.3
         if (K > 4096) return tiles > sm_count;                 // 2048 x 8192, 8 rows: 10.7 / 13.9; q/k/v 6000 x 8192, 4 rows: 18.0 / 16.9
         if (K <= 1024 && M >= 6) return tiles > (M <= 8 ? two_per_sm : sm_count);   // 4864 x 896, 8 rows: 4.1 / 4.7; gate and up, 16 rows: 7.3 / 7.1
         return true;                                           // 2048 x 2048, 5 rows: 5.6 / 4.8; 9400 x 1024, 2 rows: 4.9 / 3.9
@@ -829,19 +836,30 @@ static bool stream_is_faster(int fmt, const LinArgs& a, BatchNorm norm, int sm_c
         if (norm == BatchNorm::staged || (norm == BatchNorm::here && K > 1536))
             return roomy || tiles <= 3 * sm_count;             // 3000 x 2048, gate and up, 5 rows: 7.7 / 6.5; 9000 x 4096, 8 rows: 20.6 / 27.0
         if (norm == BatchNorm::here) {
-            if (M <= 8) return tiles > 200;                    // gate and up 4608 x 1024, 5 rows: 5.9 / 5.2; q/k/v 2048 x 1024: 4.5 / 4.7
-            if (M > 12 && K <= 960 && tiles <= two_per_sm) return false;   // gate and up 4864 x 896, 16 rows: 8.7 / 9.3
-            return tiles > (K <= 640 ? sm_count : 48);         // two blocks per tile: 4864 x 896, 9 rows: 6.7 / 5.7; q/k/v 1152 x 896: 4.4 / 4.6
+            // gate and up 4608 x 1024, 5 rows: 5.9 / 5.2; 3757 x 1152, 4 rows: 5.3 / 4.9; q/k/v 2203 x 1472, 8 rows: 6.0 / 5.2; 2048 x 1024: 4.5 / 4.7
+            if (M <= 8) return tiles > (K <= 928 ? 200 : K <= 1408 ? 110 : 60);
+            if (M > 12 && K <= 960 && two_waves) return false; // gate and up 4864 x 896, 16 rows: 8.7 / 9.3; 6764 x 960, 212 tiles: 7.9 / 7.2
+            // two blocks per tile: 4864 x 896, 9 rows: 6.7 / 5.7; 4318 x 512, 9 rows: 5.1 / 4.6; q/k/v 1152 x 896: 4.4 / 4.6; gate and up 532 x 1216, 14 rows: 5.4 / 4.7
+            return tiles > (K <= 384 ? sm_count : K <= 640 ? 128 : K <= 1088 ? 48 : 32);
         }
         if (!roomy) return false;                              // 28672 x 4096, 8 rows: 27.7 / 35.5, 16 rows: 47.4 / 75.4
-        if (M <= 8) return tiles > two_per_sm && K >= 512 && (K < 2048 || K % 128 != 0);   // 18900 x 1024, 8 rows: 8.7 / 7.4; gate and up 14000 x 2048, 5 rows: 14.1 / 15.0
+        if (M <= 8) {                                          // 18900 x 1024, 8 rows: 8.7 / 7.4; gate and up 14000 x 2048, 5 rows: 14.1 / 15.0; 4534 x 4288, 2 rows: 15.2 / 11.9
+            const bool parts = K >= 2048 && K % 128 != 0;      // (a copy per column)
+            return K >= 512 && (parts ? tiles > sm_count : K < 2048 && tiles > two_per_sm);
+        }
         if (tiles > 2 * two_per_sm) return true;               // 30000 x 320, 16 rows: 14.0 / 10.1
-        return K >= 512 && (M < 12 ? tiles > 120 : tiles * K > 450000);   // 4096 x 4096, 9 rows: 10.5 / 9.3; 9400 x 1536, 12 rows: 16.6 / 12.7; 4864 x 896: 5.7 / 6.7
+        // 17167 x 448, 9 rows: 9.9 / 6.6; 9543 x 384, 12 rows: 6.5 / 6.8; gate and up 7162 x 384, 9 rows: 7.1 / 6.6 (16 weight rows a tile)
+        if (K < 512) return a.epi != EPI_SWIGLU && tiles > 160 && !two_waves;
+        // 4096 x 4096, 9 rows: 10.5 / 9.3; 9400 x 1536, 12 rows: 16.6 / 12.7; 5323 x 768, 12 rows: 5.9 / 5.5; q/k/v 13939 x 576, 14 rows: 11.6 / 8.4; 4864 x 896, 16 rows: 5.7 / 6.7
+        if (M <= 12) return tiles > (M < 12 && K > 640 ? 120 : sm_count);
+        return tiles * K > 450000 || (K <= 640 && tiles > two_per_sm);
     }
     if (norm == BatchNorm::staged)   // gate and up 4864 x 896, 2 rows: 7.7 / 6.9; 2048 x 2048, 2 rows: 7.4 / 8.7, 9 rows: 8.0 / 6.3; gate and up 9000 x 4096, 8 rows: 29.5 / 48.5
         return K < 4096 && (tiles > sm_count ? M * K <= 16384 : K < 2048 || M > 8);
     if (norm == BatchNorm::here)
         return (K >= 1024 && K <= 1088 && tiles > 200 && tiles <= 2 * sm_count) ||             // gate and up 4608 x 1024, 8 rows: 6.9 / 6.1; 4864 x 896: 6.5 / 8.2
+               (M <= 8 && K >= 448 && K <= 768 && tiles > 3 * sm_count) ||                     // q/k/v 11903 x 768, 4 rows: 8.5 / 7.1
+               (a.epi == EPI_SWIGLU && M > 8 && K < 512 && tiles > sm_count) ||                // gate and up 12522 x 384, 16 rows: 8.8 / 7.7
                (M > 8 && M * K >= 16384 && K < 4096 && tiles >= 32 && tiles <= sm_count);      // 2048 x 2048, 12 rows: 8.1 / 6.4
     return false;                                              // 576 x 576, 2 rows: 2.1 / 3.3; 28672 x 4096, 16 rows: 52 / 69
 }

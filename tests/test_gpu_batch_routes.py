@@ -44,6 +44,26 @@ def test_rows_of_several_groups_and_tiles(nnb, ctx, fmt, N, K):
         ctx.free(p)
 
 
+@pytest.mark.parametrize("fmt,N,K,M,launches", [("int8", 9601, 384, 9, 1), ("int8", 10305, 384, 9, 2), ("int8", 5120, 384, 16, 1), ("int8", 5153, 384, 16, 2), ("int8", 9600, 576, 16, 1),
+                                                ("int8", 9760, 576, 16, 2), ("int8", 4800, 2112, 2, 2), ("int8", 4800, 2048, 2, 1), ("q4", 500, 2624, 16, 2), ("q4", 500, 2048, 16, 1)])
+def test_plain_rows_on_both_sides_of_a_line(nnb, ctx, fmt, N, K, M, launches):
+    W, s = make_weight(fmt, N, K, 441)
+    qw = nnb.QuantWeight(ctx, fmt, W, s)
+    xb, ob = ctx.upload(make_x(M, K, 442).view(np.uint16)), alloc_with_canary(ctx, M * N * 2)
+    for m in range(M):
+        ctx.linear(1, N, K, xb + m * K * 2, qw.buf, ob + m * N * 2)
+    want = ctx.download(ob, (M, N), np.uint16)
+    ctx.upload(np.full((M, N), 0x7E00, np.uint16), ob)
+    before = ctx.launch_count()
+    ctx.linear(M, N, K, xb, qw.buf, ob)
+    assert ctx.launch_count() - before == launches
+    assert np.array_equal(ctx.download(ob, (M, N), np.uint16), want)
+    check_canary(ctx, ob, M * N * 2, f"{fmt} {N}x{K}")
+    qw.release()
+    for p in (xb, ob):
+        ctx.free(p)
+
+
 @pytest.mark.parametrize("fmt", ["fp16", "int8", "q4"])
 @pytest.mark.parametrize("N,K", [(70, 1088), (64, 4608), (64, 4672), (2048, 8192)])   # the longest row that up to 8 rows are normalised in the kernel with, and longer ones
 def test_a_norm_gives_the_same_bits_recorded_and_row_by_row(nnb, ctx, fmt, N, K):
@@ -75,7 +95,7 @@ def test_a_norm_gives_the_same_bits_recorded_and_row_by_row(nnb, ctx, fmt, N, K)
 
 # Gate and up with the norm, on both sides of the lines between the two kernels (on a B200: 148 multiprocessors); blocks that take several tiles
 ONE_LAUNCH = {("q4", 8192, 16), ("q4", 4864, 2), ("q4", 2300, 2), ("q4", 2300, 8), ("int8", 4864, 16), ("int8", 2300, 2), ("int8", 2300, 8), ("int8", 2300, 9),
-              ("int8", 2300, 16), ("fp16", 9400, 2), ("fp16", 9400, 8), ("fp16", 9400, 9), ("fp16", 9400, 16), ("fp16", 4864, 2), ("fp16", 4864, 8), ("fp16", 4864, 9),
+              ("int8", 2300, 16), ("fp16", 9400, 2), ("fp16", 9400, 8), ("fp16", 4864, 2), ("fp16", 4864, 8), ("fp16", 4864, 9),
               ("fp16", 4864, 16)}
 
 
